@@ -105,7 +105,7 @@ typedef struct paddi_attempt_log {
     int32_t found;        /* 1 when the attempt produced the requested discords */
     int64_t n_cand;       /* "# Candidates": windows never pruned (nn >= r2) */
     int64_t n_disc;       /* "# Discords": windows with nn > r2 */
-    int64_t n_phase1;     /* candidates left after phase 1 */
+    int64_t n_phase1;     /* candidates left after phase 1 (PALMAD: and the witnesses) */
     int32_t n_recheck;    /* windows whose distance was recomputed in FP64 */
     paddi_discord top;    /* best discord of the attempt */
     float ms_stats;       /* window statistics (once per length, logged on its first attempt) */

@@ -38,8 +38,7 @@ constexpr int FG_HALF = 4;      // accumulators per thread
 constexpr int FG_MAXM = 1024;
 
 __global__ void __launch_bounds__(FG_THREADS)
-k_fragile(const float *__restrict__ x, const double *__restrict__ mu64,
-          const double *__restrict__ inv64, const int32_t *__restrict__ cand,
+k_fragile(const float *__restrict__ x, const double2 *__restrict__ ms64, const int32_t *__restrict__ cand,
           const int32_t *__restrict__ list, const int32_t *__restrict__ list_count,
           uint8_t *pruned, uint32_t *rho_max, const int32_t *__restrict__ frag,
           const int32_t *__restrict__ frag_count, int32_t m, float thr, int32_t col_lo,
@@ -70,14 +69,14 @@ k_fragile(const float *__restrict__ x, const double *__restrict__ mu64,
             cp[t] = pos;
             cw[t] = w;
             live[t] = pos >= 0 && !__ldcg(pruned + pos);
-            civ[t] = inv64[w];
+            civ[t] = ms64[w].y;
             if (live[t]) atomicOr(&s_any, 1);
         }
         __syncthreads();
         if (!s_any) continue;
         for (int e = t; e < FG_CAND * mp; e += FG_THREADS) {
             const int c = e / mp, k = e - c * mp;
-            fg_a[e] = (live[c] && k < m) ? (double)x[cw[c] + k] - mu64[cw[c]] : 0.0;
+            fg_a[e] = (live[c] && k < m) ? (double)x[cw[c] + k] - ms64[cw[c]].x : 0.0;
         }
         __syncthreads();
         const int fi = chunk * FG_THREADS + t;
@@ -93,7 +92,7 @@ k_fragile(const float *__restrict__ x, const double *__restrict__ mu64,
 #pragma unroll
             for (int c = 0; c < FG_HALF; ++c) any |= live[c0 + c] != 0;
             if (!any || !fok) continue; // any: uniform over the block
-            const double mf = mu64[f];
+            const double mf = ms64[f].x;
             const float *y = x + f;
             const double2 *a2 = reinterpret_cast<const double2 *>(fg_a + c0 * mp);
             const int mh = mp >> 1;
@@ -111,7 +110,7 @@ k_fragile(const float *__restrict__ x, const double *__restrict__ mu64,
                     acc[c] = fma(av.y, v1, fma(av.x, v0, acc[c]));
                 }
             }
-            const double ivf = inv64[f];
+            const double ivf = ms64[f].y;
 #pragma unroll
             for (int c = 0; c < FG_HALF; ++c) {
                 const int ci = c0 + c;
@@ -142,7 +141,7 @@ k_fragile(const float *__restrict__ x, const double *__restrict__ mu64,
 
 } // namespace
 
-cudaError_t paddi_launch_fragile(const float *x, const double *mu64, const double *inv64,
+cudaError_t paddi_launch_fragile(const float *x, const double2 *ms64,
                                  const int32_t *cand, const int32_t *list,
                                  const int32_t *list_count, uint8_t *pruned, uint32_t *rho_max,
                                  const int32_t *frag, const int32_t *frag_count, int32_t m,
@@ -153,7 +152,7 @@ cudaError_t paddi_launch_fragile(const float *x, const double *mu64, const doubl
     const size_t smem = sizeof(double) * (size_t)FG_CAND * (size_t)((m + 1) & ~1);
     cudaError_t e = paddi_raise_smem_limit((const void *)k_fragile, smem);
     if (e != cudaSuccess) return e;
-    k_fragile<<<num_sms * 4, FG_THREADS, smem, st>>>(x, mu64, inv64, cand, list, list_count,
+    k_fragile<<<num_sms * 4, FG_THREADS, smem, st>>>(x, ms64, cand, list, list_count,
                                                     pruned, rho_max, frag, frag_count, m, thr,
                                                     col_lo, col_hi);
     return cudaGetLastError();

@@ -141,8 +141,7 @@ __device__ __forceinline__ void guide_finish(double best, double *red, PaddiGuid
 
 // Reuse and slide.  Leaves without a trace when a rebuild is due.
 __global__ void __launch_bounds__(GD_THREADS, GD_STREAM_CTAS_PER_SM)
-k_guide_stream(const float *__restrict__ x, const double *__restrict__ mu64,
-               const double *__restrict__ inv64, const uint8_t *__restrict__ flat, int32_t N,
+k_guide_stream(const float *__restrict__ x, const double2 *__restrict__ ms64, const uint8_t *__restrict__ flat, int32_t N,
                int32_t m, const PaddiAttemptResult *__restrict__ prev, int32_t w_host,
                PaddiGuide *g, double *__restrict__ G0, double *__restrict__ G1)
 {
@@ -165,7 +164,7 @@ k_guide_stream(const float *__restrict__ x, const double *__restrict__ mu64,
     const double s = g->s;
     const double *Gin = gcur ? G1 : G0;
     double *Gout = gcur ? G0 : G1; // slide only
-    const double iw = inv64[w];
+    const double iw = ms64[w].y;
     const int fw = flat[w];
     double cw = 0.0; // A: cov = G[j] - A (mu_j - s)
     for (int k = t; k < m; k += GD_THREADS) cw += (double)x[w + k] - s;
@@ -205,8 +204,8 @@ k_guide_stream(const float *__restrict__ x, const double *__restrict__ mu64,
             v = block_sum(v, redm);
             if (t == 0) Gout[jj] = v;
             if (admissible(w, jj, m)) {
-                const double cov = v - cw * (mu64[jj] - s);
-                best = fmin(best, pair_dist(cov, iw, inv64[jj], fw, flat[jj], m));
+                const double cov = v - cw * (ms64[jj].x - s);
+                best = fmin(best, pair_dist(cov, iw, ms64[jj].y, fw, flat[jj], m));
             }
         }
     }
@@ -225,8 +224,9 @@ k_guide_stream(const float *__restrict__ x, const double *__restrict__ mu64,
             const int j = j0 + u * stride;
             const bool ok = j < bhi;
             gv[u] = ok ? Gin[j - shift] : 0.0;
-            mv[u] = ok ? mu64[j] : 0.0;
-            iv[u] = ok ? inv64[j] : 0.0;
+            const double2 s2 = ok ? ms64[j] : make_double2(0.0, 0.0);
+            mv[u] = s2.x;
+            iv[u] = s2.y;
             fv[u] = ok ? flat[j] : 0;
         }
         for (int k = 0; k < nt; ++k) {
@@ -259,8 +259,7 @@ k_guide_stream(const float *__restrict__ x, const double *__restrict__ mu64,
 // register ring over the staged series.  Leaves when the state is current
 // (k_guide_stream did this length) or there is no window.
 __global__ void __launch_bounds__(GD_THREADS)
-k_guide_build(const float *__restrict__ x, const double *__restrict__ mu64,
-              const double *__restrict__ inv64, const uint8_t *__restrict__ flat, int32_t N,
+k_guide_build(const float *__restrict__ x, const double2 *__restrict__ ms64, const uint8_t *__restrict__ flat, int32_t N,
               int32_t m, const PaddiAttemptResult *__restrict__ prev, int32_t w_host,
               PaddiGuide *g, double *__restrict__ G0, double *__restrict__ G1)
 {
@@ -273,8 +272,8 @@ k_guide_build(const float *__restrict__ x, const double *__restrict__ mu64,
     if (w < 0 || guide_mode(g, w, m) != PADDI_GUIDE_BUILT) return;
     const int ncur = g->cur ^ 1;
     double *Gout = ncur ? G1 : G0;
-    const double s = mu64[w];
-    const double iw = inv64[w];
+    const double s = ms64[w].x;
+    const double iw = ms64[w].y;
     const int fw = flat[w];
     double cw = 0.0; // A: s is w's FP64 mean, so A is only its rounding residue
     for (int k = t; k < m; k += GD_THREADS) {
@@ -321,8 +320,9 @@ k_guide_build(const float *__restrict__ x, const double *__restrict__ mu64,
             if (j < N) {
                 Gout[j] = acc[c];
                 if (admissible(w, j, m)) {
-                    const double cov = acc[c] - cw * (mu64[j] - s);
-                    best = fmin(best, pair_dist(cov, iw, inv64[j], fw, flat[j], m));
+                    const double2 sj = ms64[j];
+                    const double cov = acc[c] - cw * (sj.x - s);
+                    best = fmin(best, pair_dist(cov, iw, sj.y, fw, flat[j], m));
                 }
             }
         }
@@ -332,7 +332,7 @@ k_guide_build(const float *__restrict__ x, const double *__restrict__ mu64,
 
 } // namespace
 
-cudaError_t paddi_launch_guide(const float *x, const double *mu64, const double *inv64,
+cudaError_t paddi_launch_guide(const float *x, const double2 *ms64,
                                const uint8_t *flat, int32_t N, int32_t m,
                                const PaddiAttemptResult *prev, int32_t w_host, PaddiGuide *g,
                                double *G, size_t g_stride, int32_t num_sms, cudaStream_t st)
@@ -344,11 +344,11 @@ cudaError_t paddi_launch_guide(const float *x, const double *mu64, const double 
     if (e != cudaSuccess) return e;
     // the stream grid also covers the slide's boundary windows (one per CTA)
     const int sgrid = std::max(GD_STREAM_CTAS_PER_SM * num_sms, GD_MAX_SLIDE + 1);
-    k_guide_stream<<<sgrid, GD_THREADS, 0, st>>>(x, mu64, inv64, flat, N, m, prev, w_host, g, G,
+    k_guide_stream<<<sgrid, GD_THREADS, 0, st>>>(x, ms64, flat, N, m, prev, w_host, g, G,
                                                  G + g_stride);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    k_guide_build<<<4 * num_sms, GD_THREADS, 0, st>>>(x, mu64, inv64, flat, N, m, prev, w_host,
+    k_guide_build<<<4 * num_sms, GD_THREADS, 0, st>>>(x, ms64, flat, N, m, prev, w_host,
                                                       g, G, G + g_stride);
     return cudaGetLastError();
 }

@@ -63,6 +63,7 @@ constexpr int P1_THREADS = 32;                // one warp per task
 constexpr int P1_GPT = 4;                     // diagonal pairs per thread
 constexpr int P1_H = P1_THREADS * P1_GPT;     // partner offset (128)
 constexpr int P1_D = 2 * P1_H;                // diagonals per chunk
+static_assert(P1_H == WT_PARTNER, "witness hints name phase 1's diagonals");
 static_assert(P1_GPT == 4, "the walk's ring and row maximum are written for 4 pairs");
 constexpr int P1_MAXM = 1024;
 constexpr int P1_SUMBLK = 64;                 // start dot products: terms per partial sum
@@ -109,12 +110,15 @@ struct P1Smem {
 // diagonals at row 0, already lowered by the start and comparison margins;
 // dsub (the next 32 steps' rounding bound) is subtracted at the start of
 // every 32-row block.
-template <bool BOUND>
+// WT: flags name the lane that hit (for the witness hints), else they are 1.
+template <bool BOUND, bool WT>
 __device__ __forceinline__ void p1_walk(const P1Smem &S, float2 (&cov)[P1_GPT], int R, int rows,
                                         int lim, float dsub, int t)
 {
     const int lane = threadIdx.x & 31;
     const int c0 = P1_GPT * t;
+    // a column's flag names the lane, 32 more for a partner diagonal
+    const uint8_t fx = WT ? (uint8_t)(1 + lane) : 1, fy = WT ? (uint8_t)(33 + lane) : 1;
     float4 rxy[4];
     float2 rz[4];
 #pragma unroll
@@ -150,12 +154,15 @@ __device__ __forceinline__ void p1_walk(const P1Smem &S, float2 (&cov)[P1_GPT], 
         // the row's maximum as a tree of depth 2, off the walk's dependency chain
         const float rmax = fmax3(fmax3(v[0].x, v[0].y, v[1].x), fmax3(v[1].y, v[2].x, v[2].y),
                                  fmaxf(v[3].x, v[3].y));
-        if (__ballot_sync(0xffffffffu, rmax > 0.f) && lane == 0) S.rowflag[s] = 1;
+        // (WT: the flag names the last lane that hit, 1 + lane: its diagonals stay
+        // admissible for most lengths)
+        const unsigned hit = __ballot_sync(0xffffffffu, rmax > 0.f);
+        if (hit && lane == 0) S.rowflag[s] = WT ? (uint8_t)(32 - __clz(hit)) : 1;
     };
     // the column in ring slot sl leaves: flag it, load column q + 4 into the slot
     auto leave = [&](int sl, int q) {
-        if (cm[sl].x > 0.f) S.colflag[q] = 1;
-        if (cm[sl].y > 0.f) S.colflag[q + P1_H] = 1;
+        if (cm[sl].x > 0.f) S.colflag[q] = fx;
+        if (cm[sl].y > 0.f) S.colflag[q + P1_H] = fy;
         cm[sl] = make_float2(-INFINITY, -INFINITY);
         const int qn = csw(q + 4);
         rxy[sl] = S.colxy[qn];
@@ -193,17 +200,19 @@ __device__ __forceinline__ void p1_walk(const P1Smem &S, float2 (&cov)[P1_GPT], 
 #pragma unroll
     for (int e = 0; e < 3; ++e) {
         const int sl = (R + e) & 3;
-        if (cm[sl].x > 0.f) S.colflag[R + c0 + e] = 1;
-        if (cm[sl].y > 0.f) S.colflag[R + c0 + e + P1_H] = 1;
+        if (cm[sl].x > 0.f) S.colflag[R + c0 + e] = fx;
+        if (cm[sl].y > 0.f) S.colflag[R + c0 + e + P1_H] = fy;
     }
 }
 
+template <bool WT>
 __global__ void __launch_bounds__(P1_THREADS, 16)
 k_phase1(const float *__restrict__ x, const float4 *__restrict__ wst, const float *__restrict__ mu,
-         const double *__restrict__ mu64, uint8_t *alive, int32_t N, int32_t m, int32_t R,
-         int32_t max_chunks, float thr, int32_t row_lo, int32_t row_hi, int32_t *task_counter,
-         int32_t *walked)
+         const double2 *__restrict__ ms64, uint8_t *alive, int32_t N, int32_t m, int32_t R,
+         int32_t max_chunks, float thr, int32_t row_lo, int32_t row_hi, PaddiAttemptDev *att,
+         PaddiWitness W, int32_t enough)
 {
+    if (WT && att->n_fail - att->n_rescued <= enough) return;
     extern __shared__ __align__(16) unsigned char p1_smem[];
     const int mpad = (m + 7) & ~7;
     const int ncp = p1_ncp(R);
@@ -227,7 +236,7 @@ k_phase1(const float *__restrict__ x, const float4 *__restrict__ wst, const floa
     const float g_dot = (float)(P1_SUMBLK + (mpad + P1_SUMBLK - 1) / P1_SUMBLK + 2) * kU;
     const float g_z = (float)(mpad / 32 + 6) * kU;
     for (;;) {
-        if (t == 0) s_task = atomicAdd(task_counter, 1);
+        if (t == 0) s_task = atomicAdd(&att->task_next, 1);
         __syncwarp();
         const int task = s_task;
         __syncwarp();
@@ -237,7 +246,7 @@ k_phase1(const float *__restrict__ x, const float4 *__restrict__ wst, const floa
         const int rows = min(R, row_hi - i0);
         const int d0 = (m - 1) + chunk * P1_D;
         if (i0 + d0 >= N) continue; // no admissible pair in this task
-        if (chunk > 0) { // continue only while some row is still a candidate
+        if (WT || chunk > 0) { // only while some row is still a candidate
             int any = 0;
             for (int s = t; s < rows; s += P1_THREADS) any |= __ldcg(alive + i0 + s);
             if (!__any_sync(0xffffffffu, any)) continue;
@@ -257,7 +266,7 @@ k_phase1(const float *__restrict__ x, const float4 *__restrict__ wst, const floa
         for (int q = t; q < R + P1_D; q += P1_THREADS) S.colflag[q] = 0;
         // ---- start dot products: row window centred with its two-float mean,
         //      series shifted by the first column window's mean
-        const double m0 = mu64[i0];
+        const double m0 = ms64[i0].x;
         const float mhi = (float)m0, mlo = (float)(m0 - (double)mhi);
         float zs = 0.f;
         for (int q = t; q < mpad; q += P1_THREADS) {
@@ -348,19 +357,37 @@ k_phase1(const float *__restrict__ x, const float4 *__restrict__ wst, const floa
                 cov[k] = make_float2(cov[k].x - first, cov[k].y - first);
             __syncwarp();
             // ---- walk the R rows
-            if (t == 0) atomicAdd(walked, 1);
+            if (t == 0) atomicAdd(&att->p1_walked, 1);
             const int lim = N - cbase; // column q is a window iff q < lim
             const bool bound = (rows < R) || (R + P1_D > lim);
-            if (bound && thr < 0.f) p1_walk<true>(S, cov, R, rows, lim, dsub, t);
-            else p1_walk<false>(S, cov, R, rows, lim, dsub, t);
+            if (bound && thr < 0.f) p1_walk<true, WT>(S, cov, R, rows, lim, dsub, t);
+            else p1_walk<false, WT>(S, cov, R, rows, lim, dsub, t);
         }
         __syncwarp();
         // ---- flush pruning marks
-        for (int s = t; s < rows; s += P1_THREADS)
-            if (S.rowflag[s]) alive[i0 + s] = 0;
         const int lim = N - cbase;
-        for (int q = t; q < R + P1_D; q += P1_THREADS)
-            if (S.colflag[q] && q < lim) alive[cbase + q] = 0;
+        if (!WT) {
+            for (int s = t; s < rows; s += P1_THREADS)
+                if (S.rowflag[s]) alive[i0 + s] = 0;
+            for (int q = t; q < R + P1_D; q += P1_THREADS)
+                if (S.colflag[q] && q < lim) alive[cbase + q] = 0;
+        } else { // the pairs behind a flag: 8 per row, 4 per column
+            for (int s = t; s < rows; s += P1_THREADS) {
+                const int f = S.rowflag[s];
+                if (f && __ldcg(alive + i0 + s)) {
+                    alive[i0 + s] = 0;
+                    wt_hint(W, i0 + s, WT_ROW, cbase + s + P1_GPT * (f - 1));
+                }
+            }
+            for (int q = t; q < R + P1_D; q += P1_THREADS) {
+                const int f = S.colflag[q];
+                if (f && q < lim && __ldcg(alive + cbase + q)) {
+                    alive[cbase + q] = 0;
+                    wt_hint(W, cbase + q, WT_COL,
+                            i0 + q - (f > 32 ? P1_H : 0) - P1_GPT * ((f - 1) & 31));
+                }
+            }
+        }
         __syncwarp();
     }
 }
@@ -379,25 +406,26 @@ size_t paddi_phase1_smem(int R, int m)
 }
 
 cudaError_t paddi_launch_phase1_dev(const float *x, const float4 *wst, const float *mu,
-                                    const double *mu64, uint8_t *alive, int32_t N, int32_t m,
+                                    const double2 *ms64, uint8_t *alive, int32_t N, int32_t m,
                                     int32_t R, int32_t max_chunks, float thr, int32_t row_lo,
-                                    int32_t row_hi, int32_t *task_counter, int32_t *walked,
-                                    int32_t num_sms, cudaStream_t st)
+                                    int32_t row_hi, PaddiAttemptDev *att, int32_t num_sms,
+                                    cudaStream_t st, const PaddiWitness *W, int32_t enough)
 {
     if (R < 64 || R > 4096 || (R & 7) || m > P1_MAXM || max_chunks < 1 || row_lo < 0 ||
         row_hi > N || row_lo >= row_hi)
         return cudaErrorInvalidValue;
     const size_t smem = paddi_phase1_smem(R, m);
-    cudaError_t e = paddi_raise_smem_limit((const void *)k_phase1, smem);
+    auto kern = W ? k_phase1<true> : k_phase1<false>;
+    cudaError_t e = paddi_raise_smem_limit((const void *)kern, smem);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_phase1, P1_THREADS, smem);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, P1_THREADS, smem);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) return cudaErrorInvalidConfiguration;
     const int nseg = (row_hi - row_lo + R - 1) / R;
     int grid = num_sms * per_sm;
     if (grid > nseg * max_chunks) grid = nseg * max_chunks;
-    k_phase1<<<grid, P1_THREADS, smem, st>>>(x, wst, mu, mu64, alive, N, m, R, max_chunks, thr,
-                                             row_lo, row_hi, task_counter, walked);
+    kern<<<grid, P1_THREADS, smem, st>>>(x, wst, mu, ms64, alive, N, m, R, max_chunks, thr, row_lo,
+                                         row_hi, att, W ? *W : PaddiWitness{}, enough);
     return cudaGetLastError();
 }

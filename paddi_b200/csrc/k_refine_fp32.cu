@@ -69,7 +69,7 @@ k_refine_fp32(const float *__restrict__ x, const float4 *__restrict__ wst,
               const int32_t *__restrict__ list, const int32_t *__restrict__ list_count,
               PaddiAttemptDev *att, int32_t *work, uint32_t *rho_max, uint8_t *pruned, int32_t N,
               int32_t m, int32_t jb, int32_t je, float thr, int32_t grid_ctas, float E,
-              float gcap)
+              float gcap, PaddiWitness W)
 {
     extern __shared__ __align__(16) unsigned char rf_smem[];
     const int mpad = (m + 7) & ~7;
@@ -200,7 +200,7 @@ k_refine_fp32(const float *__restrict__ x, const float4 *__restrict__ wst,
                 }
             }
             // ---- epilogue
-            bool hit[4] = {false, false, false, false};
+            int hit[4] = {-1, -1, -1, -1}; // a window that prunes the candidate
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
                 const int ci = 4 * warp + c;
@@ -218,7 +218,7 @@ k_refine_fp32(const float *__restrict__ x, const float4 *__restrict__ wst,
                                            fmaf(fc, S.cflt[q], -S.cgm[q]));
                     if (ok) {
                         cmax = fmaxf(cmax, rho);
-                        hit[c] |= rho > thr;
+                        if (rho > thr) hit[c] = j;
                     }
                 }
                 rmax[c] = fmaxf(rmax[c], cmax + G); // the interval's middle
@@ -226,9 +226,11 @@ k_refine_fp32(const float *__restrict__ x, const float4 *__restrict__ wst,
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
                 const int ci = 4 * warp + c;
-                if (__any_sync(0xffffffffu, hit[c]) && lane == 0 && !dead[ci]) {
+                const unsigned any = __ballot_sync(0xffffffffu, hit[c] >= 0);
+                if (any && lane == __ffs(any) - 1 && !dead[ci]) {
                     dead[ci] = 1;
                     pruned[cp[ci]] = 1;
+                    if (W.wit) wt_hint(W, cw[ci], WT_ONE, hit[c]);
                 }
             }
             __syncthreads();
@@ -264,7 +266,8 @@ cudaError_t paddi_launch_refine_fp32(const float *x, const float4 *wst, const fl
                                      const int32_t *list_count, PaddiAttemptDev *att,
                                      int32_t *work, uint32_t *rho_max, uint8_t *pruned,
                                      int32_t N, int32_t m, int32_t jb, int32_t je, float thr,
-                                     float gcap, int32_t num_sms, cudaStream_t st)
+                                     float gcap, int32_t num_sms, cudaStream_t st,
+                                     const PaddiWitness *W)
 {
     if (m > RF_MAXM) return cudaErrorInvalidValue;
     if ((jb % RF_TW) != 0) return cudaErrorInvalidValue; // chunks on the 256-window grid
@@ -280,7 +283,8 @@ cudaError_t paddi_launch_refine_fp32(const float *x, const float4 *wst, const fl
     const int grid = num_sms * per_sm;
     k_refine_fp32<<<grid, RF_THREADS, smem, st>>>(x, wst, mu, cand, list, list_count, att, work,
                                                   rho_max, pruned, N, m, jb, je, thr, grid,
-                                                  paddi_bound_fp32(m).E, gcap);
+                                                  paddi_bound_fp32(m).E, gcap,
+                                                  W ? *W : PaddiWitness{});
     return cudaGetLastError();
 }
 

@@ -438,7 +438,7 @@ k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
               const uint16_t *__restrict__ bq, const float4 *__restrict__ wdq,
               PaddiAttemptDev *att, int32_t *work, uint32_t *rho_max, uint8_t *pruned, int32_t N,
               int32_t m, int32_t jb, int32_t je, float thr, int32_t grid_ctas, long long wl,
-              int32_t withhold, int32_t round, int32_t je_all)
+              int32_t withhold, int32_t round, int32_t je_all, PaddiWitness W)
 {
     using X = E16<BF>;
     constexpr int UM_M = MM;
@@ -793,16 +793,40 @@ k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
                     if (!rowok) tmax = -INFINITY;
                     rmax = fmaxf(rmax, tmax + Gt); // the interval's middle (-inf stays)
                     const unsigned bal = __ballot_sync(0xffffffffu, tmax > thr);
+                    bool hint = false;
                     if (lane < UM_TC / 4) {
                         const int ci = (UM_TC / 4) * g + lane;
                         if (!S.dead[ci]) {
                             if ((bal >> (8 * lane)) & 0xFFu) {
                                 S.dead[ci] = 1;
                                 pruned[S.cp[ci]] = 1;
+                                hint = W.wit != nullptr;
                             } else if (__ldcg(pruned + S.cp[ci])) {
                                 S.dead[ci] = 1; // pruned by another CTA's item
                             }
                         }
+                    }
+                    // a candidate pruned here leaves the window that did it as its
+                    // witness hint: a second pass over the accumulator, at most once
+                    // per candidate, finds its column
+                    const unsigned hints = __ballot_sync(0xffffffffu, hint);
+                    if (hints) {
+                        int jh = -1;
+                        const bool mine = rowok && ((hints >> (lane >> 3)) & 1u) && tmax > thr;
+                        for (int cb = 0; cb < 4; ++cb) {
+                            tmem_ld32_async(tb + 32 * cb, ra);
+                            tmem_wait_ld(ra);
+#pragma unroll
+                            for (int i = 0; i < 32; ++i) {
+                                const int j = j0 + 8 * (128 * hcol + 32 * cb + i) + bsh;
+                                const float4 wv = wrow[(32 * cb + i) >> 1];
+                                const float rho = fmaf(__uint_as_float(ra[i]), (i & 1) ? wv.y : wv.x,
+                                                       fmaf(-zsc, (i & 1) ? wv.w : wv.z, -Gt));
+                                const int dd = wc > j ? wc - j : j - wc;
+                                if (rho > thr && j < j_hi && dd >= m - 1) jh = j;
+                            }
+                        }
+                        if (mine && jh >= 0) wt_hint(W, wc, WT_ONE, jh);
                     }
                     __syncwarp();
                     if (warp == EPI_WARP0 && lane == 0) {
@@ -948,7 +972,8 @@ cudaError_t paddi_launch_refine_umma(bool bf16, const float *x, const float4 *ws
                                      uint32_t *rho_max, uint8_t *pruned, int32_t N, int32_t m,
                                      int32_t jb, int32_t je, float thr_prune, int32_t num_sms,
                                      cudaStream_t st, long long wait_cycles, int32_t withhold,
-                                     int32_t round, int32_t je_all, bool rows64)
+                                     int32_t round, int32_t je_all, bool rows64,
+                                     const PaddiWitness *W)
 {
     const int kp = kpad_of(m);
     if (kp > UM_KMAX64 || m < 3) return cudaErrorInvalidValue;
@@ -962,7 +987,7 @@ cudaError_t paddi_launch_refine_umma(bool bf16, const float *x, const float4 *ws
     void (*kern)(const float *, const float4 *, const float *, const int32_t *, const int32_t *,
                  const int32_t *, const uint16_t *, const float4 *, PaddiAttemptDev *, int32_t *,
                  uint32_t *, uint8_t *, int32_t, int32_t, int32_t, int32_t, float, int32_t,
-                 long long, int32_t, int32_t, int32_t);
+                 long long, int32_t, int32_t, int32_t, PaddiWitness);
     if (MM == 128) kern = bf16 ? k_refine_umma<true, 128> : k_refine_umma<false, 128>;
     else kern = bf16 ? k_refine_umma<true, 64> : k_refine_umma<false, 64>;
     cudaError_t e = paddi_raise_smem_limit((const void *)kern, smem);
@@ -971,6 +996,6 @@ cudaError_t paddi_launch_refine_umma(bool bf16, const float *x, const float4 *ws
     kern<<<grid, UM_THREADS, smem, st>>>(x, wst, mu, cand, list, list_count, bq, wdq, att, work,
                                          rho_max, pruned, N, m, jb, je, thr_prune, grid,
                                          wait_cycles > 0 ? wait_cycles : 4000000000ll, withhold,
-                                         round, je_all > 0 ? je_all : je);
+                                         round, je_all > 0 ? je_all : je, W ? *W : PaddiWitness{});
     return cudaGetLastError();
 }

@@ -346,8 +346,7 @@ constexpr int RC_SPAN = RC_THREADS * RC_JPT; // neighbour windows per block
 __device__ __forceinline__ int rpad(int d) { return d + (d >> 4); } // conflict-free at stride 8
 
 __global__ void __launch_bounds__(RC_THREADS)
-k_recheck(const float *__restrict__ x, const double *__restrict__ mu64,
-          const double *__restrict__ inv64, const uint8_t *__restrict__ flat, int32_t N,
+k_recheck(const float *__restrict__ x, const double2 *__restrict__ ms64, const uint8_t *__restrict__ flat, int32_t N,
           int32_t m, const int32_t *__restrict__ cand, const int32_t *__restrict__ recheck,
           PaddiAttemptDev *att, unsigned long long *nn64_ord, int32_t known_w)
 {
@@ -372,7 +371,7 @@ k_recheck(const float *__restrict__ x, const double *__restrict__ mu64,
         const int r = item % nr, sp = item / nr;
         const int w = cand[recheck[r]];
         if (w == known_w) continue; // exact value filled in by the finalize step
-        const double mw = mu64[w], iw = inv64[w];
+        const double mw = ms64[w].x, iw = ms64[w].y;
         const int fw = flat[w];
         double asum = 0.0;
         for (int k = t; k < m; k += RC_THREADS) {
@@ -420,10 +419,10 @@ k_recheck(const float *__restrict__ x, const double *__restrict__ mu64,
             for (int c = 0; c < RC_JPT; ++c) {
                 const int j = j0 + q0 + c;
                 if (j < j_hi && !overlaps(w, j, m)) {
-                    const double cov = acc[c] - (mu64[j] - sh) * asum;
+                    const double cov = acc[c] - (ms64[j].x - sh) * asum;
                     double rho;
                     if (fw | flat[j]) rho = (fw & flat[j]) ? 1.0 : 0.0;
-                    else rho = cov * iw * inv64[j];
+                    else rho = cov * iw * ms64[j].y;
                     double d = 2.0 * m * (1.0 - rho);
                     d = d < 0.0 ? 0.0 : d;
                     best = fmin(best, d);
@@ -615,14 +614,14 @@ cudaError_t paddi_launch_finalize(const int32_t *cand, PaddiAttemptDev *att,
     return cudaGetLastError();
 }
 
-cudaError_t paddi_launch_recheck(const float *x, const double *mu64, const double *inv64,
+cudaError_t paddi_launch_recheck(const float *x, const double2 *ms64,
                                  const uint8_t *flat, int32_t N, int32_t m,
                                  const int32_t *cand, const int32_t *recheck,
                                  PaddiAttemptDev *att, unsigned long long *nn64_ord,
                                  int32_t num_sms, int32_t known_w, cudaStream_t st)
 {
     if (m > RC_MAXM) return cudaErrorInvalidValue;
-    k_recheck<<<num_sms * 4, RC_THREADS, 0, st>>>(x, mu64, inv64, flat, N, m, cand, recheck, att,
+    k_recheck<<<num_sms * 4, RC_THREADS, 0, st>>>(x, ms64, flat, N, m, cand, recheck, att,
                                                  nn64_ord, known_w);
     return cudaGetLastError();
 }

@@ -61,7 +61,7 @@ __device__ T block_exclusive_scan(T v, T *warp_tot)
 
 __global__ void __launch_bounds__(ST_THREADS)
 k_window_stats(const float *__restrict__ x, int64_t n, int32_t m, int32_t N, float4 *wst,
-               float *mu, double *mu64, double *inv64, uint8_t *flat, int32_t *flat_count,
+               float *mu, double2 *ms64, uint8_t *flat, int32_t *flat_count,
                int32_t *flat_span)
 {
     // staged values: x[t0 .. t0 + ST_TILE + m] (one extra window for mu_{i+1})
@@ -121,8 +121,7 @@ k_window_stats(const float *__restrict__ x, int64_t n, int32_t m, int32_t N, flo
         if (i >= N) { // zeroed tail so tiles can over-read
             wst[i] = make_float4(0.f, 0.f, 0.f, 0.f);
             mu[i] = 0.f;
-            mu64[i] = 0.0;
-            inv64[i] = 0.0;
+            ms64[i] = make_double2(0.0, 0.0);
             flat[i] = 0;
             continue;
         }
@@ -146,8 +145,7 @@ k_window_stats(const float *__restrict__ x, int64_t n, int32_t m, int32_t N, flo
         }
         wst[i] = make_float4(df, dg, (float)iv, fl ? 0.f : (float)nrm);
         mu[i] = (float)mu_i;
-        mu64[i] = mu_i;
-        inv64[i] = iv;
+        ms64[i] = make_double2(mu_i, iv);
         flat[i] = (uint8_t)fl;
         nflat += fl;
         // lowest and highest flat window, both kept as maxima over a zeroed
@@ -161,27 +159,27 @@ k_window_stats(const float *__restrict__ x, int64_t n, int32_t m, int32_t N, flo
 }
 
 // mean / population std in the reference's FP32 layout (src/preprocessing.cuh:31-34)
-__global__ void k_export_stats(const double *__restrict__ mu64, const double *__restrict__ inv64,
+__global__ void k_export_stats(const double2 *__restrict__ ms64,
                                int32_t N, int32_t m, float *mean, float *sd)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= N) return;
-    mean[i] = (float)mu64[i];
-    const double iv = inv64[i];
+    mean[i] = (float)ms64[i].x;
+    const double iv = ms64[i].y;
     sd[i] = iv > 0.0 ? (float)(1.0 / (iv * sqrt((double)m))) : 0.f;
 }
 
 } // namespace
 
-cudaError_t paddi_launch_export_stats(const double *mu64, const double *inv64, int32_t N,
+cudaError_t paddi_launch_export_stats(const double2 *ms64, int32_t N,
                                       int32_t m, float *mean, float *sd, cudaStream_t st)
 {
-    k_export_stats<<<(N + 255) / 256, 256, 0, st>>>(mu64, inv64, N, m, mean, sd);
+    k_export_stats<<<(N + 255) / 256, 256, 0, st>>>(ms64, N, m, mean, sd);
     return cudaGetLastError();
 }
 
 cudaError_t paddi_launch_stats(const float *x, int64_t n, int32_t m, float4 *wst, float *mu,
-                               double *mu64, double *inv64, uint8_t *flat,
+                               double2 *ms64, uint8_t *flat,
                                int32_t *flat_count, cudaStream_t st, int32_t *flat_span)
 {
     if (m < 2 || m > ST_MAXM || n < 2 * (int64_t)m) return cudaErrorInvalidValue;
@@ -191,7 +189,7 @@ cudaError_t paddi_launch_stats(const float *x, int64_t n, int32_t m, float4 *wst
     const size_t smem = st_smem(m);
     cudaError_t e = paddi_raise_smem_limit((const void *)k_window_stats, smem);
     if (e != cudaSuccess) return e;
-    k_window_stats<<<grid, ST_THREADS, smem, st>>>(x, n, m, N, wst, mu, mu64, inv64, flat,
+    k_window_stats<<<grid, ST_THREADS, smem, st>>>(x, n, m, N, wst, mu, ms64, flat,
                                                    flat_count, flat_span);
     return cudaGetLastError();
 }

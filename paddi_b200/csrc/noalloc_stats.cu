@@ -41,9 +41,8 @@ constexpr size_t kSlots = (size_t)PADDI_NOALLOC_MAX_WINDOWS + PADDI_PAD_WIN; // 
 constexpr size_t up256(size_t b) { return (b + 255) & ~(size_t)255; }
 constexpr size_t kOffWst = 0;
 constexpr size_t kOffMu = kOffWst + up256(sizeof(float4) * kSlots);
-constexpr size_t kOffMu64 = kOffMu + up256(sizeof(float) * kSlots);
-constexpr size_t kOffInv64 = kOffMu64 + up256(sizeof(double) * kSlots);
-constexpr size_t kOffFlat = kOffInv64 + up256(sizeof(double) * kSlots);
+constexpr size_t kOffMs64 = kOffMu + up256(sizeof(float) * kSlots);
+constexpr size_t kOffFlat = kOffMs64 + up256(sizeof(double2) * kSlots);
 constexpr size_t kOffCount = kOffFlat + up256(kSlots);
 constexpr size_t kBytes = kOffCount + 256;
 
@@ -96,8 +95,7 @@ PADDI_API paddi_status paddi_compute_statistics_noalloc(const float *d_T, float 
         base = g_base[dev];
     }
     int32_t *count = reinterpret_cast<int32_t *>(base + kOffCount);
-    double *mu64 = reinterpret_cast<double *>(base + kOffMu64);
-    double *inv64 = reinterpret_cast<double *>(base + kOffInv64);
+    double2 *ms64 = reinterpret_cast<double2 *>(base + kOffMs64);
     // the flat-window counter is accumulated with atomics: it must start at 0
     if (cudaMemsetAsync(count, 0, sizeof(int32_t), st) != cudaSuccess) {
         cudaGetLastError();
@@ -105,10 +103,10 @@ PADDI_API paddi_status paddi_compute_statistics_noalloc(const float *d_T, float 
     }
     cudaError_t e = paddi_launch_stats(d_T, (int64_t)n, (int32_t)m,
                                        reinterpret_cast<float4 *>(base + kOffWst),
-                                       reinterpret_cast<float *>(base + kOffMu), mu64, inv64,
+                                       reinterpret_cast<float *>(base + kOffMu), ms64,
                                        base + kOffFlat, count, st);
     if (e == cudaSuccess)
-        e = paddi_launch_export_stats(mu64, inv64, (int32_t)N, (int32_t)m, d_mean, d_std, st);
+        e = paddi_launch_export_stats(ms64, (int32_t)N, (int32_t)m, d_mean, d_std, st);
     if (e != cudaSuccess) {
         cudaGetLastError();
         return PADDI_ERR_CUDA;

@@ -2,6 +2,7 @@
 // the PD3 and PALMAD drivers and the exported C ABI (include/paddi.h).
 //
 // One attempt (one length m, one threshold r) is
+//   witnesses   k_witness_check   (PALMAD: neighbours known from the length before)
 //   phase 1     k_phase1          (reference: gpu_local_candidate_select +
 //                                  gpu_local_define_candidates, src/PD3.cuh:18-29)
 //   compaction  k_compact         (get_node_candidates_num + local_candidates_union,
@@ -70,7 +71,7 @@ struct paddi_ctx {
     float *d_x = nullptr;
     float4 *d_wst = nullptr;
     float *d_mu = nullptr;
-    double *d_mu64 = nullptr, *d_inv64 = nullptr;
+    double2 *d_ms64 = nullptr; // {FP64 mean, FP64 inverse norm}
     uint8_t *d_flat = nullptr, *d_alive = nullptr, *d_pruned = nullptr;
     int32_t *d_cand = nullptr, *d_rcslot = nullptr, *d_recheck = nullptr;
     int32_t *d_list[2] = {nullptr, nullptr};
@@ -82,6 +83,11 @@ struct paddi_ctx {
     PaddiGuide *d_guide = nullptr, *h_guide = nullptr; // state + result (h: pinned)
     double *d_G = nullptr;                  // shifted dot products, two buffers (on first use)
     size_t G_cap = 0;                       // windows per buffer
+    // witnesses of the current PALMAD run (allocated on first use): the length
+    // they stand at (0: none in use) and the run's shortest length
+    PaddiWitness W = {};
+    size_t W_cap = 0; // windows
+    int wit_m = 0, wit_m0 = 0;
     int32_t *h_flatcount = nullptr;         // pinned
     // learned r predictor
     bool model_ok = false;
@@ -149,13 +155,22 @@ void dfree(T *&p)
     p = nullptr;
 }
 
+void free_witness(paddi_ctx *ctx)
+{
+    dfree(ctx->W.wit);
+    dfree(ctx->W.wc);
+    dfree(ctx->W.wrho);
+    dfree(ctx->W.scal);
+    ctx->W_cap = 0;
+    ctx->wit_m = 0;
+}
+
 void free_buffers(paddi_ctx *ctx)
 {
     dfree(ctx->d_x);
     dfree(ctx->d_wst);
     dfree(ctx->d_mu);
-    dfree(ctx->d_mu64);
-    dfree(ctx->d_inv64);
+    dfree(ctx->d_ms64);
     dfree(ctx->d_flat);
     dfree(ctx->d_alive);
     dfree(ctx->d_pruned);
@@ -173,6 +188,7 @@ void free_buffers(paddi_ctx *ctx)
     dfree(ctx->d_pn);
     dfree(ctx->d_G);
     ctx->G_cap = 0;
+    free_witness(ctx);
     ctx->cap_n = 0;
     ctx->rc_cap = 0;
 }
@@ -187,8 +203,7 @@ paddi_status ensure_capacity(paddi_ctx *ctx, size_t n)
     CK(dmalloc(ctx, &ctx->d_x, sizeof(float) * (n + 64)));
     CK(dmalloc(ctx, &ctx->d_wst, sizeof(float4) * W));
     CK(dmalloc(ctx, &ctx->d_mu, sizeof(float) * W));
-    CK(dmalloc(ctx, &ctx->d_mu64, sizeof(double) * W));
-    CK(dmalloc(ctx, &ctx->d_inv64, sizeof(double) * W));
+    CK(dmalloc(ctx, &ctx->d_ms64, sizeof(double2) * W));
     CK(dmalloc(ctx, &ctx->d_flat, W));
     CK(dmalloc(ctx, &ctx->d_alive, W));
     CK(dmalloc(ctx, &ctx->d_pruned, W));
@@ -249,7 +264,7 @@ paddi_status run_stats(paddi_ctx *ctx, const float *x, size_t n, int m, bool til
 {
     // d_flatcount = {flat windows, span of the flat windows (two ints), fragile windows}
     CK(cudaMemsetAsync(ctx->d_flatcount, 0, 4 * sizeof(int32_t), ctx->st));
-    CK(paddi_launch_stats(x, (int64_t)n, m, ctx->d_wst, ctx->d_mu, ctx->d_mu64, ctx->d_inv64,
+    CK(paddi_launch_stats(x, (int64_t)n, m, ctx->d_wst, ctx->d_mu, ctx->d_ms64,
                           ctx->d_flat, ctx->d_flatcount, ctx->st, ctx->d_flatcount + 1));
     const int kernel = refine_kernel_for(ctx, m);
     // the refine's per-length data: its tiles (tensor cores) and the windows
@@ -262,6 +277,35 @@ paddi_status run_stats(paddi_ctx *ctx, const float *x, size_t n, int m, bool til
         CK(paddi_launch_fragile_scan_fp32(x, ctx->d_wst, ctx->d_mu, (int32_t)(n - m + 1), m,
                                           guard_of(ctx, kernel), ctx->d_frag,
                                           ctx->d_flatcount + 3, ctx->num_sms, ctx->st));
+    return PADDI_OK;
+}
+
+// Starts a run's witnesses: no window has one.
+paddi_status start_witness(paddi_ctx *ctx, const float *x, size_t n, int m0)
+{
+    const size_t W = ctx->cap_n + PADDI_PAD_WIN + 64;
+    if (ctx->W_cap < W) {
+        free_witness(ctx);
+        CK(dmalloc(ctx, &ctx->W.wit, sizeof(int32_t) * W));
+        CK(dmalloc(ctx, &ctx->W.wc, sizeof(double) * W));
+        CK(dmalloc(ctx, &ctx->W.wrho, sizeof(float) * W));
+        CK(dmalloc(ctx, &ctx->W.scal, sizeof(uint32_t) * 4));
+        ctx->W_cap = W;
+    }
+    CK(paddi_launch_witness_start(x, (int64_t)n, (int32_t)(n - m0 + 1), ctx->W, ctx->num_sms,
+                                  ctx->st));
+    ctx->wit_m = ctx->wit_m0 = m0;
+    return PADDI_OK;
+}
+
+// Advances the run's witnesses to length m, whose statistics are current.
+paddi_status witness_to(paddi_ctx *ctx, const float *x, size_t n, int m)
+{
+    if (ctx->wit_m == 0 || ctx->wit_m == m) return PADDI_OK;
+    CK(paddi_launch_witness_step(x, ctx->d_ms64, (int32_t)(n - m + 1), m,
+                                 ctx->wit_m, ctx->wit_m0, ctx->W, ctx->d_list[1],
+                                 ctx->num_sms, ctx->st));
+    ctx->wit_m = m;
     return PADDI_OK;
 }
 
@@ -281,6 +325,11 @@ int p1_rows_of(const paddi_ctx *ctx)
     return (R + 7) & ~7;
 }
 
+// Windows without a proving witness: up to wit_limit of them look for a new
+// one, one warp each; phase 1 runs when more than wit_enough are left.
+int32_t wit_limit(int32_t N) { return std::max(4096, N / 16); }
+int32_t wit_enough(int32_t N) { return std::max(1024, N / 512); }
+
 // The correlation threshold of r^2 at length m: d < r^2 <=> rho > thr.
 float thr_of(float r2, int m) { return (float)(1.0 - (double)r2 / (2.0 * (double)m)); }
 
@@ -298,6 +347,7 @@ paddi_status refine_rounds(paddi_ctx *ctx, const float *x, int32_t N, int m, int
     ++*launches;
     const bool umma = kernel != PADDI_DIST_FP32;
     constexpr int kShifts[3] = {4, 2, 1};
+    const PaddiWitness *W = ctx->wit_m == m ? &ctx->W : nullptr;
     const int32_t range = col_hi - col_lo;
     const int nrounds = range >= (1 << 16) ? 4 : 1;
     // round edges on the refine's grid: 2048-window tiles (tensor cores),
@@ -326,12 +376,12 @@ paddi_status refine_rounds(paddi_ctx *ctx, const float *x, int32_t N, int m, int
                                         ctx->d_wdq, ctx->d_att, &ctx->d_att->work_rd[rd],
                                         ctx->d_rho, ctx->d_pruned, N, m, jb, je, thr,
                                         ctx->num_sms, st, ctx->wait_cycles, ctx->withhold, rd,
-                                        col_hi, ctx->opts.tile_rows == 64));
+                                        col_hi, ctx->opts.tile_rows == 64, W));
         else
             CK(paddi_launch_refine_fp32(x, ctx->d_wst, ctx->d_mu, ctx->d_cand, ctx->d_list[a],
                                         cnt, ctx->d_att, &ctx->d_att->work_rd[rd], ctx->d_rho,
                                         ctx->d_pruned, N, m, jb, je, thr, guard, ctx->num_sms,
-                                        st));
+                                        st, W));
         CK(cudaEventRecord(ctx->rev[2 * rd + 1], st));
         ++*launches;
         if (rd + 1 < nrounds) {
@@ -346,7 +396,7 @@ paddi_status refine_rounds(paddi_ctx *ctx, const float *x, int32_t N, int m, int
     // still unpruned, in FP64 (the kernel returns at once when there are none)
     const int a = (nrounds - 1) & 1;
     if (ctx->trace) CK(cudaEventRecord(ctx->tev[nrounds], st));
-    CK(paddi_launch_fragile(x, ctx->d_mu64, ctx->d_inv64, ctx->d_cand, ctx->d_list[a],
+    CK(paddi_launch_fragile(x, ctx->d_ms64, ctx->d_cand, ctx->d_list[a],
                             &ctx->d_att->list_count[nrounds - 1], ctx->d_pruned, ctx->d_rho,
                             ctx->d_frag, ctx->d_flatcount + 3, m, thr, col_lo, col_hi,
                             ctx->num_sms, st));
@@ -373,7 +423,7 @@ paddi_status select_passes(paddi_ctx *ctx, const float *x, size_t n, int m, floa
         CK(paddi_launch_finalize(ctx->d_cand, ctx->d_att, ctx->d_rho, ctx->d_pruned, m, r2, thr,
                                  guard, widen, top_k, ctx->d_flat, ctx->rc_cap, ctx->d_recheck,
                                  ctx->d_rcslot, ctx->d_nn64, ctx->d_res, known_w, known_ord, st));
-        CK(paddi_launch_recheck(x, ctx->d_mu64, ctx->d_inv64, ctx->d_flat, N, m, ctx->d_cand,
+        CK(paddi_launch_recheck(x, ctx->d_ms64, ctx->d_flat, N, m, ctx->d_cand,
                                 ctx->d_recheck, ctx->d_att, ctx->d_nn64, ctx->num_sms, known_w,
                                 st));
         CK(paddi_launch_select(ctx->d_cand, ctx->d_att, ctx->d_rho, ctx->d_pruned,
@@ -448,12 +498,20 @@ paddi_status run_attempt(paddi_ctx *ctx, const float *x, size_t n, int m, float 
     const int chunks = ctx->opts.phase1_chunks ? (int)ctx->opts.phase1_chunks : 12;
     cudaStream_t st = ctx->st;
     CK(cudaEventRecord(ctx->ev[0], st));
-    CK(cudaMemsetAsync(ctx->d_alive, 1, (size_t)N, st));
     CK(cudaMemsetAsync(ctx->d_att, 0, sizeof(PaddiAttemptDev), st));
     int launches = 0;
-    CK(paddi_launch_phase1_dev(x, ctx->d_wst, ctx->d_mu, ctx->d_mu64, ctx->d_alive, N, m, R,
-                               chunks, thr, 0, N, &ctx->d_att->task_next,
-                               &ctx->d_att->p1_walked, ctx->num_sms, st));
+    const bool wit = ctx->wit_m == m;
+    if (wit) {
+        CK(paddi_launch_witness_check(ctx->d_ms64, x, N, m, thr, ctx->wit_m0, ctx->W,
+                                      ctx->d_alive, ctx->d_list[0], ctx->d_att, wit_limit(N),
+                                      ctx->num_sms, st));
+        launches += 2;
+    } else {
+        CK(cudaMemsetAsync(ctx->d_alive, 1, (size_t)N, st));
+    }
+    CK(paddi_launch_phase1_dev(x, ctx->d_wst, ctx->d_mu, ctx->d_ms64, ctx->d_alive, N, m, R,
+                               chunks, thr, 0, N, ctx->d_att, ctx->num_sms, st,
+                               wit ? &ctx->W : nullptr, wit_enough(N)));
     ++launches;
     CK(cudaEventRecord(ctx->ev[1], st));
     CK(paddi_launch_compact(ctx->d_alive, N, ctx->d_cand, ctx->d_rho, ctx->d_pruned,
@@ -470,6 +528,8 @@ paddi_status run_attempt(paddi_ctx *ctx, const float *x, size_t n, int m, float 
         CK(cudaEventRecord(ctx->tev[nrounds + 1], st));
         CK(cudaMemcpyAsync(ctx->d_trace + 7, &ctx->d_att->p1_walked, sizeof(int32_t),
                            cudaMemcpyDeviceToDevice, st));
+        CK(cudaMemcpyAsync(ctx->d_trace + 5, &ctx->d_att->n_fail, 2 * sizeof(int32_t),
+                           cudaMemcpyDeviceToDevice, st)); // and n_rescued
         CK(cudaMemcpyAsync(ctx->h_trace64, &ctx->d_att->n_pairs, 2 * sizeof(unsigned long long),
                            cudaMemcpyDeviceToHost, st));
         CK(cudaMemcpyAsync(ctx->h_trace, ctx->d_trace, sizeof(int32_t) * 8,
@@ -484,6 +544,8 @@ paddi_status run_attempt(paddi_ctx *ctx, const float *x, size_t n, int m, float 
     if (spec_out) *spec_out = spec;
     if (ctx->trace) {
         std::string line = "paddi-trace m=" + std::to_string(m) + " r2=" + std::to_string(r2) +
+                           " unproven=" + std::to_string(ctx->h_trace[5]) + "-" +
+                           std::to_string(ctx->h_trace[6]) +
                            " p1=" + std::to_string(ctx->h_res->n_p1) +
                            " p1_tasks=" + std::to_string(ctx->h_trace[7]) + "x" + std::to_string(R) +
                            " rounds:";
@@ -581,12 +643,14 @@ paddi_status enqueue_prep(paddi_ctx *ctx, const float *x, size_t n, int m, bool 
     CK(cudaEventRecord(ctx->ev[4], ctx->st));
     paddi_status s = run_stats(ctx, x, n, m);
     if (s != PADDI_OK) return s;
+    s = witness_to(ctx, x, n, m);
+    if (s != PADDI_OK) return s;
     CK(cudaEventRecord(ctx->ev[5], ctx->st));
     CK(cudaMemcpyAsync(ctx->h_flatcount, ctx->d_flatcount, sizeof(int32_t),
                        cudaMemcpyDeviceToHost, ctx->st));
     if (guided) {
         CK(cudaEventRecord(ctx->ev[6], ctx->st));
-        CK(paddi_launch_guide(x, ctx->d_mu64, ctx->d_inv64, ctx->d_flat, N, m, ctx->d_res, w_host,
+        CK(paddi_launch_guide(x, ctx->d_ms64, ctx->d_flat, N, m, ctx->d_res, w_host,
                               ctx->d_guide, ctx->d_G, ctx->G_cap, ctx->num_sms, ctx->st));
         CK(cudaMemcpyAsync(ctx->h_guide, ctx->d_guide, sizeof(PaddiGuide),
                            cudaMemcpyDeviceToHost, ctx->st));
@@ -750,6 +814,15 @@ paddi_status palmad_impl(paddi_ctx *ctx, const float *x, size_t n, uint32_t minL
         // the dot products of an earlier call belong to another series
         CK(cudaMemsetAsync(ctx->d_guide, 0, sizeof(PaddiGuide), ctx->st));
     }
+    // one length: nothing to carry over
+    struct EndWitness {
+        paddi_ctx *c;
+        ~EndWitness() { c->wit_m = 0; }
+    } end_witness{ctx};
+    if (L > 1) {
+        paddi_status s = start_witness(ctx, x, n, (int)minL);
+        if (s != PADDI_OK) return s;
+    }
     Prep pre; // the length whose statistics (and bound) are current, if queued ahead
     for (int j = 0; j < L; ++j) {
         const int m = (int)minL + j;
@@ -824,6 +897,7 @@ paddi_status palmad_impl(paddi_ctx *ctx, const float *x, size_t n, uint32_t minL
                                 std::to_string(iter_cap) + " attempts");
             if (stale) { // a miss after the next length was queued: restore this one
                 s = run_stats(ctx, x, n, m);
+                if (s == PADDI_OK) s = witness_to(ctx, x, n, m);
                 if (s != PADDI_OK) return s;
                 stale = false;
             }
@@ -1159,7 +1233,7 @@ PADDI_API paddi_status paddi_compute_statistics(paddi_ctx *ctx, const float *d_T
     }
     s = run_stats(ctx, d_T, n, (int)m, /*tiles=*/false);
     if (s != PADDI_OK) return s;
-    CK(paddi_launch_export_stats(ctx->d_mu64, ctx->d_inv64, (int32_t)(n - m + 1), (int)m, d_mean,
+    CK(paddi_launch_export_stats(ctx->d_ms64, (int32_t)(n - m + 1), (int)m, d_mean,
                                  d_std, ctx->st));
     if (user != ctx->st) {
         CK(cudaEventRecord(ctx->ev[5], ctx->st));
@@ -1221,10 +1295,9 @@ PADDI_API paddi_status paddi_shard_phase1(paddi_ctx *ctx, const float *d_series,
     CK(cudaMemsetAsync(d_alive, 1, N, st));
     CK(cudaMemsetAsync(ctx->d_att, 0, sizeof(PaddiAttemptDev), st));
     const int chunks = ctx->opts.phase1_chunks ? (int)ctx->opts.phase1_chunks : 12;
-    CK(paddi_launch_phase1_dev(d_series, ctx->d_wst, ctx->d_mu, ctx->d_mu64, d_alive, (int32_t)N,
+    CK(paddi_launch_phase1_dev(d_series, ctx->d_wst, ctx->d_mu, ctx->d_ms64, d_alive, (int32_t)N,
                                (int)m, p1_rows_of(ctx), chunks, thr_of(r2, (int)m),
-                               (int32_t)row_lo, (int32_t)row_hi, &ctx->d_att->task_next,
-                               &ctx->d_att->p1_walked, ctx->num_sms, st));
+                               (int32_t)row_lo, (int32_t)row_hi, ctx->d_att, ctx->num_sms, st));
     CK(cudaStreamSynchronize(st));
     return PADDI_OK;
 }

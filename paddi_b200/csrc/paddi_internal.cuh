@@ -9,7 +9,7 @@
 //           n_i = |x_i - mu_i| (the window's norm), inv_i = 1 / n_i; both 0 for
 //           a flat window (window i is flat iff inv_i == 0)
 //   mu[i]   float  window mean
-//   mu64[i], inv64[i]  FP64 mean and inverse norm (recheck path)
+//   ms64[i].x, ms64[i].y  FP64 mean and inverse norm (recheck path)
 //   flat[i] uint8
 // The correlation of windows i, j is rho = cov(i,j) * inv_i * inv_j with
 // cov the centred dot product; the squared z-normalised distance is
@@ -92,6 +92,8 @@ struct PaddiAttemptDev {
                             // the last); zero when the attempt starts, so the compactions
                             // between rounds need no reset
     int32_t p1_walked;      // phase-1 tasks that walked their rows (instrumentation)
+    int32_t n_fail;         // windows whose witness proves nothing (k_witness.cu)
+    int32_t n_rescued;      // of those, windows that found a new witness
     int32_t covered_from;   // r + 1 when refine round r (one candidate tile left) took
                             // every remaining window; later rounds then have nothing to do
     unsigned long long n_pairs; // pairs evaluated by the refine (instrumentation)
@@ -128,26 +130,75 @@ struct PaddiGuide {
     int32_t done, item;        // kernel counters (zero between launches)
 };
 
+// Witnesses of a PALMAD run (k_witness.cu): per window a known neighbour
+// wit[i] (-1: none; WT_HINT: wc[i] holds a code for partners to evaluate), the
+// pair's centred dot product wc[i] at the run's current length, and a lower
+// bound wrho[i] of its correlation; scal: WT_AMAX the largest |x| (float bits),
+// WT_NHINT and WT_DONE counters of a step (zero between steps).
+// Codes: kind * WT_CODE + base, one 8-byte store so that two writers cannot
+// tear it: WT_ROW the partners base + {0..3} and base + WT_PARTNER + {0..3},
+// WT_COL base - {0..3}, WT_ONE base itself.
+struct PaddiWitness {
+    int32_t *wit;
+    double *wc;
+    float *wrho;
+    uint32_t *scal;
+};
+enum { WT_AMAX = 0, WT_NHINT = 1, WT_DONE = 2 };
+#define WT_HINT (-2)
+#define WT_CODE 8589934592.0 /* 2^33 */
+#define WT_PARTNER 128       /* phase 1's partner offset */
+enum { WT_ROW = 0, WT_COL = 1, WT_ONE = 2 };
+
+// Records a hint for window i (races between writers leave one of them).
+__device__ __forceinline__ void wt_hint(const PaddiWitness &W, int i, int kind, int base)
+{
+    W.wc[i] = (double)kind * WT_CODE + (double)base;
+    W.wit[i] = WT_HINT;
+}
+
 #define PADDI_MAX_TOPK 16
 #define PADDI_MAX_RECHECK 1024 /* initial FP64 recheck capacity (grows on demand) */
 
 // ---------------------------------------------------------------- launches
 // All launch wrappers enqueue on `st` and return cudaGetLastError().
 cudaError_t paddi_launch_stats(const float *x, int64_t n, int32_t m, float4 *wst, float *mu,
-                               double *mu64, double *inv64, uint8_t *flat,
+                               double2 *ms64, uint8_t *flat,
                                int32_t *flat_count, cudaStream_t st,
                                int32_t *flat_span = nullptr);
 // flat_span (optional): two zeroed ints that receive {INT_MAX - lowest flat
 // window, highest flat window + 1} (both stay 0 without flat windows).
 
+// Empties the witnesses of a run whose shortest length has N windows.
+cudaError_t paddi_launch_witness_start(const float *x, int64_t n, int32_t N, const PaddiWitness &W,
+                                       int32_t num_sms, cudaStream_t st);
+// Advances the witnesses from length `from` (m - 1, m or m + 1) to m, with the
+// statistics of m; m0 is the shortest length of the run; hint: scratch, N entries.
+cudaError_t paddi_launch_witness_step(const float *x, const double2 *ms64,
+                                      int32_t N, int32_t m, int32_t from, int32_t m0,
+                                      const PaddiWitness &W, int32_t *hint, int32_t num_sms,
+                                      cudaStream_t st);
+// Writes alive[0..N) from the witnesses at threshold thr and looks for new
+// witnesses of the others (listed in fail) while they are at most `limit`.
+cudaError_t paddi_launch_witness_check(const double2 *ms64, const float *x,
+                                       int32_t N, int32_t m, float thr, int32_t m0,
+                                       const PaddiWitness &W, uint8_t *alive, int32_t *fail,
+                                       PaddiAttemptDev *att, int32_t limit, int32_t num_sms,
+                                       cudaStream_t st);
+
 // Phase 1 at threshold thr = 1 - r^2 / (2m): an exact test (the kernel bounds
 // its own FP32 rounding, no guard band).
 // Only the rows [row_lo, row_hi) are walked (their columns reach anywhere).
+// W (optional): alive[] comes from the witnesses; the kernel returns at once
+// when at most `enough` candidates are left (att->n_fail - att->n_rescued),
+// walks only segments that hold a candidate, and leaves a hint for every
+// candidate it prunes.
 cudaError_t paddi_launch_phase1_dev(const float *x, const float4 *wst, const float *mu,
-                                    const double *mu64, uint8_t *alive, int32_t N, int32_t m,
+                                    const double2 *ms64, uint8_t *alive, int32_t N, int32_t m,
                                     int32_t R, int32_t max_chunks, float thr, int32_t row_lo,
-                                    int32_t row_hi, int32_t *task_counter, int32_t *walked,
-                                    int32_t num_sms, cudaStream_t st);
+                                    int32_t row_hi, PaddiAttemptDev *att, int32_t num_sms,
+                                    cudaStream_t st, const PaddiWitness *W = nullptr,
+                                    int32_t enough = 0);
 
 // prune_flats (r^2 > 0): flat windows with another flat window at least m-1
 // away are dropped (distance 0); flat_span as filled by paddi_launch_stats.
@@ -160,13 +211,15 @@ cudaError_t paddi_launch_compact(const uint8_t *alive, int32_t N, int32_t *cand,
 // Dense refine of the candidates in list[0..*list_count) (positions into
 // cand[]) against the windows [jb, je) (jb a multiple of 256).  thr is the
 // exact threshold 1 - r^2 / (2m): the kernel prunes on lower bounds of the
-// correlations; gcap is the guard band (fragile windows are skipped).
+// correlations; gcap is the guard band (fragile windows are skipped).  W
+// (optional): a pruned candidate leaves the window that pruned it as a hint.
 cudaError_t paddi_launch_refine_fp32(const float *x, const float4 *wst, const float *mu,
                                      const int32_t *cand, const int32_t *list,
                                      const int32_t *list_count, PaddiAttemptDev *att,
                                      int32_t *work, uint32_t *rho_max, uint8_t *pruned,
                                      int32_t N, int32_t m, int32_t jb, int32_t je, float thr,
-                                     float gcap, int32_t num_sms, cudaStream_t st);
+                                     float gcap, int32_t num_sms, cudaStream_t st,
+                                     const PaddiWitness *W = nullptr);
 
 // Fragile windows of length m in the FP32 refine's geometry, appended to
 // frag_list (frag_count zeroed by the caller).
@@ -177,7 +230,7 @@ cudaError_t paddi_launch_fragile_scan_fp32(const float *x, const float4 *wst, co
 // Exact FP64 correlations of the unpruned candidates of list[0..*list_count)
 // with the fragile windows in [col_lo, col_hi) (k_fragile.cu): prunes and
 // raises rho_max.
-cudaError_t paddi_launch_fragile(const float *x, const double *mu64, const double *inv64,
+cudaError_t paddi_launch_fragile(const float *x, const double2 *ms64,
                                  const int32_t *cand, const int32_t *list,
                                  const int32_t *list_count, uint8_t *pruned, uint32_t *rho_max,
                                  const int32_t *frag, const int32_t *frag_count, int32_t m,
@@ -199,7 +252,7 @@ cudaError_t paddi_launch_refine_umma(bool bf16, const float *x, const float4 *ws
                                      float thr_prune, int32_t num_sms, cudaStream_t st,
                                      long long wait_cycles = 0, int32_t withhold = 0,
                                      int32_t round = 0, int32_t je_all = 0,
-                                     bool rows64 = false);
+                                     bool rows64 = false, const PaddiWitness *W = nullptr);
 
 // Per-length tile data of the tensor-core refine: for every block of
 // paddi_tile_width() windows, the split 16-bit series slice (bq, at most
@@ -231,7 +284,7 @@ cudaError_t paddi_launch_finalize(const int32_t *cand, PaddiAttemptDev *att,
                                   PaddiAttemptResult *res, int32_t known_w,
                                   unsigned long long known_ord, cudaStream_t st);
 
-cudaError_t paddi_launch_recheck(const float *x, const double *mu64, const double *inv64,
+cudaError_t paddi_launch_recheck(const float *x, const double2 *ms64,
                                  const uint8_t *flat, int32_t N, int32_t m,
                                  const int32_t *cand, const int32_t *recheck,
                                  PaddiAttemptDev *att, unsigned long long *nn64_ord,
@@ -252,12 +305,12 @@ size_t paddi_phase1_smem(int R, int m);
 // of the attempt result `prev`, skipped when it has none), through the shifted
 // dot products (two buffers G of N doubles each, G + g_stride the second) and
 // their state in g; result in g->nn_ord.
-cudaError_t paddi_launch_guide(const float *x, const double *mu64, const double *inv64,
+cudaError_t paddi_launch_guide(const float *x, const double2 *ms64,
                                const uint8_t *flat, int32_t N, int32_t m,
                                const PaddiAttemptResult *prev, int32_t w_host, PaddiGuide *g,
                                double *G, size_t g_stride, int32_t num_sms, cudaStream_t st);
 
-cudaError_t paddi_launch_export_stats(const double *mu64, const double *inv64, int32_t N,
+cudaError_t paddi_launch_export_stats(const double2 *ms64, int32_t N,
                                       int32_t m, float *mean, float *sd, cudaStream_t st);
 
 cudaError_t paddi_launch_scatter(const int32_t *cand, const PaddiAttemptDev *att,
