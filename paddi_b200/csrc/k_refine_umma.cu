@@ -62,6 +62,8 @@ constexpr int UM_THREADS = 384;  // 12 warps
 constexpr int UM_TCMAX = 16;     // candidates per tile (M = 128); 8 for M = 64
 constexpr int UM_N = 256;        // windows at stride 8
 constexpr int UM_TW = UM_N * 8;  // windows per tile (one block of the grid)
+constexpr int UM_ROUNDS = 4;     // window ranges refined before and after compactions
+constexpr int UM_MIN_ROUNDS = 1 << 16; // windows from which on rounds pay
 constexpr int UM_WAVES = 1;      // work items per CTA and round when candidate tiles are few
 constexpr int UM_KMAX128 = 368;  // largest K' with M = 128 (shared-memory bound)
 constexpr int UM_KMAX64 = 736;   // largest K' with M = 64
@@ -411,6 +413,9 @@ struct UmShared {
     uint32_t tmem_base;
     int item, abort, tok;
     int built_tile; // candidate tile whose operand sits in A (-1: none)
+    int last, next; // round bookkeeping: this CTA finished the round's last item;
+                    // candidates of the next round (-1: give up)
+    int wsum[UM_THREADS / 32];
     volatile int item_dead;
     int tile_live; // live candidates at the start of the current tile (instrumentation)
     volatile int vb[2], vw;
@@ -427,18 +432,73 @@ struct UmPhases {
 
 __device__ __forceinline__ uint32_t par(uint32_t idx) { return idx & 1u; }
 
+__device__ __forceinline__ int32_t ld_acquire(const int32_t *p)
+{
+    int32_t v;
+    asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_release(int32_t *p, int32_t v)
+{
+    asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
+// Unpruned entries of in[0..C) (or of 0..C-1) to out, in order, by one CTA;
+// returns their number.  8 entries per thread and step: the survivors are a few
+// thousand at most, and 32k entries take about 15 us.
+__device__ int um_compact(const int32_t *in, bool identity, int C, const uint8_t *pruned,
+                          int32_t *out, int *wsum)
+{
+    constexpr int PER = 8;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int base = 0;
+    for (int b0 = 0; b0 < C; b0 += UM_THREADS * PER) {
+        const int i0 = b0 + threadIdx.x * PER;
+        int e[PER];
+        unsigned keep = 0;
+#pragma unroll
+        for (int q = 0; q < PER; ++q) e[q] = i0 + q < C ? (identity ? i0 + q : __ldcg(in + i0 + q)) : -1;
+#pragma unroll
+        for (int q = 0; q < PER; ++q)
+            if (e[q] >= 0 && !__ldcg(pruned + e[q])) keep |= 1u << q;
+        const int cnt = __popc(keep);
+        int inc = cnt;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += t;
+        }
+        __syncthreads(); // wsum of the step before is consumed
+        if (lane == 31) wsum[warp] = inc;
+        __syncthreads();
+        int off = base, all = 0;
+#pragma unroll
+        for (int w = 0; w < UM_THREADS / 32; ++w) {
+            const int v = wsum[w];
+            if (w < warp) off += v;
+            all += v;
+        }
+        int pos = off + inc - cnt;
+#pragma unroll
+        for (int q = 0; q < PER; ++q)
+            if ((keep >> q) & 1u) out[pos++] = e[q];
+        base += all;
+    }
+    __threadfence();
+    return base;
+}
+
 // MM = 128: 16 candidates, accumulator row r in TMEM lane r.
 // MM = 64:  8 candidates, accumulator row r in TMEM lane (r % 16) + 32 (r / 16)
 //           (lanes 16..31 of every subpartition stay unused).
 template <bool BF, int MM>
 __global__ void __launch_bounds__(UM_THREADS, 1)
 k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
-              const float *__restrict__ mu, const int32_t *__restrict__ cand,
-              const int32_t *__restrict__ list, const int32_t *__restrict__ list_count,
-              const uint16_t *__restrict__ bq, const float4 *__restrict__ wdq,
-              PaddiAttemptDev *att, int32_t *work, uint32_t *rho_max, uint8_t *pruned, int32_t N,
-              int32_t m, int32_t jb, int32_t je, float thr, int32_t grid_ctas, long long wl,
-              int32_t withhold, int32_t round, int32_t je_all, PaddiWitness W)
+              const float *__restrict__ mu, const int32_t *__restrict__ cand, int32_t *list0,
+              int32_t *list1, const uint16_t *__restrict__ bq, const float4 *__restrict__ wdq,
+              PaddiAttemptDev *att, uint32_t *rho_max, uint8_t *pruned, int32_t N, int32_t m,
+              int32_t col_lo, int32_t col_hi, float thr, int32_t grid_ctas, long long wl,
+              int32_t withhold, PaddiWitness W)
 {
     using X = E16<BF>;
     constexpr int UM_M = MM;
@@ -451,16 +511,8 @@ k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
     const UmLayout L = um_layout(MM, kp);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
-    const int C = *list_count;
-    // an earlier round with one candidate tile left took every remaining window
-    const int cov = att->covered_from;
-    if (C <= 0 || je <= jb || (cov > 0 && cov <= round)) return; // uniform, before any TMEM use
-    // one tile left: later rounds could not shrink it, so take the rest of the
-    // windows now and spare them their launches' fixed cost
-    if (C <= UM_TC && je_all > je) {
-        je = je_all;
-        if (blockIdx.x == 0 && threadIdx.x == 0) att->covered_from = round + 1;
-    }
+    int C = att->n_cand_p1;
+    if (C <= 0 || col_hi <= col_lo) return; // uniform, before any TMEM use
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < 2; ++s) {
@@ -472,7 +524,7 @@ k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
         mbar_init(&S.wd_empty, EPI_WARPS);
         mbar_init(&S.drain, 1);
         S.abort = 0;
-        S.built_tile = -1;
+        S.last = 0;
         S.last_full[0] = S.last_full[1] = S.last_wd = -1;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -490,13 +542,6 @@ k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
     UmPhases ph = {{0u, 0u}, {0u, 0u}, {0u, 0u}, 0u, 0u};
     bool mma_issued = false; // MMA thread: any MMA issued
 
-    const int range = je - jb;
-    const int tiles = (C + UM_TC - 1) / UM_TC;
-    // at most UM_WAVES items per CTA when the candidate tiles are few, items of
-    // at least one 2048-window block
-    const int splits = max(1, min(range / UM_TW, (UM_WAVES * grid_ctas) / tiles));
-    const int span = (((range + splits - 1) / splits) + UM_TW - 1) / UM_TW * UM_TW;
-    const int total = tiles * splits;
     const uint32_t idesc = idesc_f16(X::fmt, UM_M, UM_N);
     const uint32_t a_hi_s = smem_u32(um_smem + L.a_hi), a_lo_s = smem_u32(um_smem + L.a_lo);
     const int kblocks = kp / 16;
@@ -507,376 +552,447 @@ k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
     const int cidx = row >> 3, bsh = row & 7;
     const float4 *wd4 = reinterpret_cast<const float4 *>(um_smem + L.wd);
 
-    for (;;) {
-        if (threadIdx.x == 0) S.item = atomicAdd(work, 1);
-        __syncthreads();
-        const int item = S.item;
-        if (item >= total || S.abort) break;
-        const int tile = item % tiles, split = item / tiles;
-        const int j_lo = jb + split * span, j_hi = min(je, j_lo + span);
-        if (threadIdx.x < UM_TC) {
-            const int li = tile * UM_TC + threadIdx.x;
-            const bool v = li < C;
-            const int pos = v ? list[li] : 0;
-            const int w = v ? cand[pos] : 0;
-            S.cw[threadIdx.x] = w;
-            S.cp[threadIdx.x] = pos;
-            S.dead[threadIdx.x] = !v || __ldcg(pruned + pos);
-            S.cflat[threadIdx.x] = (v && wst[w].z == 0.f) ? 1.f : 0.f; // flat candidate
-            S.rmax[threadIdx.x] = f2ord(-INFINITY);
-        }
-        if (threadIdx.x == 0) {
-            S.item_dead = 0;
-            S.tok = -1;
-        }
-        __syncthreads();
-        {
-            int a = threadIdx.x < UM_TC ? !S.dead[threadIdx.x] : 0;
-            if (!__syncthreads_or(a) || j_lo >= j_hi) continue; // all threads agree
-        }
-        if (threadIdx.x == 32) { // read by the epilogue after the barriers below
-            int alive = 0;
-            for (int c = 0; c < UM_TC; ++c) alive += !S.dead[c];
-            S.tile_live = alive;
-        }
-        const int T = (j_hi - j_lo + UM_TW - 1) / UM_TW;
-        const int blk0 = j_lo / UM_TW; // j_lo is a multiple of UM_TW
-        // the first tile's slice streams into stage 0 while the operand is built
-        // (the build's scratch is stage 1 + the window data)
-        if (warp == LOAD_WARP && lane == 0) {
-            S.vb[0] = 1;
-            // test hook (withhold != 0): the CTA holding work item 0 never fills
-            // its first stage, so the MMA thread's wait runs out; nothing is in flight
-            const bool skip = withhold && item == 0;
-            if (!skip) {
-                const uint16_t *src = bq + (size_t)blk0 * 2 * cnt;
-                mbar_arrive_expect_tx(&S.full_b[0], (uint32_t)(4 * cnt));
-                bulk_g2s(um_smem + L.b[0][0], src, (uint32_t)(2 * cnt), &S.full_b[0]);
-                bulk_g2s(um_smem + L.b[0][1], src + cnt, (uint32_t)(2 * cnt), &S.full_b[0]);
-                S.last_full[0] = (int)ph.full[0];
-            }
-        }
-        // ---- candidate operand: 16 x (hi, lo) rows of scaled zhat, then 8 shifted
-        //      copies; kept from the CTA's previous item when that had the same
-        //      candidate tile (a candidate pruned since then only costs its rows'
-        //      work: its results no longer matter)
-        if (S.built_tile != tile) {
-            // scratch rows of 32-bit words: 4 zero words (8 elements) of front
-            // padding, then zhat[0..kp); stride ksw words with ksw % 32 == 8, so
-            // the four candidates a warp reads sit in disjoint bank ranges
-            const int ksw = zrow_words(kp);
-            uint32_t *zhw = reinterpret_cast<uint32_t *>(um_smem + L.b[1][0]);
-            uint32_t *zlw = zhw + UM_TC * ksw;
-            typename X::T *zh = reinterpret_cast<typename X::T *>(zhw);
-            typename X::T *zl = reinterpret_cast<typename X::T *>(zlw);
-            const int c = threadIdx.x >> 4, t16 = threadIdx.x & 15;
-            const int w = c < UM_TC ? S.cw[c] : 0;
-            const bool live = c < UM_TC && !S.dead[c];
-            const float muc = live ? mu[w] : 0.f;
-            const float ivc = live ? wst[w].z * 256.f : 0.f; // 2^ZSCALE
-            float zs = 0.f;
-            if (c < UM_TC)
-                for (int q = 4 + (kp >> 1) + t16; q < ksw; q += 16) { // tail words
-                    zhw[c * ksw + q] = 0u;
-                    zlw[c * ksw + q] = 0u;
+    // ---- rounds: the windows [jb, je) of growing ranges (1/16, 1/4, 1/2, all of
+    // them), the survivors compacted in between so that every tile is dense.  A
+    // round with one tile left takes every remaining window.
+    const int nrounds = col_hi - col_lo >= UM_MIN_ROUNDS ? UM_ROUNDS : 1;
+    int jb = col_lo;
+    for (int rd = 0; rd < nrounds; ++rd) {
+        int je = rd == nrounds - 1 ? col_hi
+                                   : col_lo + ((col_hi - col_lo) >> (rd ? 3 - rd : 4)) / UM_TW * UM_TW;
+        if (C <= UM_TC) je = col_hi;
+        int32_t *list = rd & 1 ? list1 : list0; // entries of this round (round 0: all candidates)
+        const int range = je - jb;
+        const int tiles = (C + UM_TC - 1) / UM_TC;
+        // at most UM_WAVES items per CTA when the candidate tiles are few, items of
+        // at least one 2048-window block
+        const int splits = max(1, min(range / UM_TW, (UM_WAVES * grid_ctas) / tiles));
+        const int span = (((range + splits - 1) / splits) + UM_TW - 1) / UM_TW * UM_TW;
+        const int total = tiles * splits;
+        if (threadIdx.x == 0) S.built_tile = -1;
+        bool counted = true; // this CTA's latest item is in done_rd
+        for (;;) {
+            if (threadIdx.x == 0) {
+                // everything this CTA wrote for its item is ordered before the count (the
+                // barrier at the item's end, then the fence)
+                if (!counted) {
+                    __threadfence();
+                    S.last = atomicAdd(&att->done_rd[rd], 1) == total - 1;
                 }
-            if (c < UM_TC && t16 < 4) { // front padding
-                zhw[c * ksw + t16] = 0u;
-                zlw[c * ksw + t16] = 0u;
+                S.item = atomicAdd(&att->work_rd[rd], 1);
             }
-            for (int k = t16; k < kp; k += 16) {
-                const float v = (live && k < m) ? (x[w + k] - muc) * ivc : 0.f;
-                const typename X::T h = X::cvt(v);
-                const typename X::T l = X::cvt(v - X::back(h));
-                if (c < UM_TC) {
-                    zh[c * 2 * ksw + 8 + k] = h;
-                    zl[c * 2 * ksw + 8 + k] = l;
-                }
-                zs += X::back(h) + X::back(l);
-            }
-#pragma unroll
-            for (int o = 8; o > 0; o >>= 1) zs += __shfl_xor_sync(0xffffffffu, zs, o);
-            if (t16 == 0 && c < UM_TC) S.zsum[c] = zs * (1.f / 256.f);
+            counted = false;
             __syncthreads();
-            // A[(c,b), k'] = z_c[k' - b] in K-major core matrices:
-            // byte offset ((k'/8)*RG + r/8)*128 + (r%8)*16 + (k'%8)*2.
-            // Elements k'-b .. k'-b+7 start at padded element p0 = 8 + 8 kc - b:
-            // five 32-bit words from word p0/2, funnel-shifted by 16 bits when p0 is odd.
-            const int chunks = kp / 8;
-            for (int e = threadIdx.x; e < UM_M * chunks; e += UM_THREADS) {
-                const int r = e & (UM_M - 1), kc = e / UM_M;
-                const int cc = r >> 3, b = r & 7;
-                const int p0 = 8 + 8 * kc - b;
-                const uint32_t shf = (uint32_t)(p0 & 1) * 16u;
-                const uint32_t *rh = zhw + cc * ksw + (p0 >> 1);
-                const uint32_t *rl = zlw + cc * ksw + (p0 >> 1);
-                uint32_t wh[5], wl[5], ph2[4], pl2[4];
-#pragma unroll
-                for (int q = 0; q < 5; ++q) {
-                    wh[q] = rh[q];
-                    wl[q] = rl[q];
-                }
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    ph2[q] = __funnelshift_r(wh[q], wh[q + 1], shf);
-                    pl2[q] = __funnelshift_r(wl[q], wl[q + 1], shf);
-                }
-                const uint32_t off = (uint32_t)((kc * RG + (r >> 3)) * 128 + (r & 7) * 16);
-                *reinterpret_cast<uint4 *>(um_smem + L.a_hi + off) =
-                    make_uint4(ph2[0], ph2[1], ph2[2], ph2[3]);
-                *reinterpret_cast<uint4 *>(um_smem + L.a_lo + off) =
-                    make_uint4(pl2[0], pl2[1], pl2[2], pl2[3]);
+            const int item = S.item;
+            if (item >= total) break;
+            const int tile = item % tiles, split = item / tiles;
+            const int j_lo = jb + split * span, j_hi = min(je, j_lo + span);
+            if (threadIdx.x < UM_TC) {
+                const int li = tile * UM_TC + threadIdx.x;
+                const bool v = li < C;
+                const int pos = !v ? 0 : rd ? __ldcg(list + li) : li;
+                const int w = v ? cand[pos] : 0;
+                S.cw[threadIdx.x] = w;
+                S.cp[threadIdx.x] = pos;
+                S.dead[threadIdx.x] = !v || __ldcg(pruned + pos);
+                S.cflat[threadIdx.x] = (v && wst[w].z == 0.f) ? 1.f : 0.f; // flat candidate
+                S.rmax[threadIdx.x] = f2ord(-INFINITY);
             }
-            fence_proxy_async_smem(); // A for the tensor core; scratch for the bulk copies
+            if (threadIdx.x == 0) {
+                S.item_dead = 0;
+                S.tok = -1;
+            }
             __syncthreads();
-            if (threadIdx.x == 0) S.built_tile = tile; // read after the next item's barrier
-        }
+            {
+                int a = threadIdx.x < UM_TC ? !S.dead[threadIdx.x] : 0;
+                if (!__syncthreads_or(a) || j_lo >= j_hi) continue; // all threads agree
+            }
+            if (threadIdx.x == 32) { // read by the epilogue after the barriers below
+                int alive = 0;
+                for (int c = 0; c < UM_TC; ++c) alive += !S.dead[c];
+                S.tile_live = alive;
+            }
+            const int T = (j_hi - j_lo + UM_TW - 1) / UM_TW;
+            const int blk0 = j_lo / UM_TW; // j_lo is a multiple of UM_TW
+            // the first tile's slice streams into stage 0 while the operand is built
+            // (the build's scratch is stage 1 + the window data)
+            if (warp == LOAD_WARP && lane == 0) {
+                S.vb[0] = 1;
+                // test hook (withhold != 0): the CTA holding work item 0 never fills
+                // its first stage, so the MMA thread's wait runs out; nothing is in flight
+                const bool skip = withhold && rd == 0 && item == 0;
+                if (!skip) {
+                    const uint16_t *src = bq + (size_t)blk0 * 2 * cnt;
+                    mbar_arrive_expect_tx(&S.full_b[0], (uint32_t)(4 * cnt));
+                    bulk_g2s(um_smem + L.b[0][0], src, (uint32_t)(2 * cnt), &S.full_b[0]);
+                    bulk_g2s(um_smem + L.b[0][1], src + cnt, (uint32_t)(2 * cnt), &S.full_b[0]);
+                    S.last_full[0] = (int)ph.full[0];
+                }
+            }
+            // ---- candidate operand: 16 x (hi, lo) rows of scaled zhat, then 8 shifted
+            //      copies; kept from the CTA's previous item when that had the same
+            //      candidate tile (a candidate pruned since then only costs its rows'
+            //      work: its results no longer matter)
+            if (S.built_tile != tile) {
+                // scratch rows of 32-bit words: 4 zero words (8 elements) of front
+                // padding, then zhat[0..kp); stride ksw words with ksw % 32 == 8, so
+                // the four candidates a warp reads sit in disjoint bank ranges
+                const int ksw = zrow_words(kp);
+                uint32_t *zhw = reinterpret_cast<uint32_t *>(um_smem + L.b[1][0]);
+                uint32_t *zlw = zhw + UM_TC * ksw;
+                typename X::T *zh = reinterpret_cast<typename X::T *>(zhw);
+                typename X::T *zl = reinterpret_cast<typename X::T *>(zlw);
+                const int c = threadIdx.x >> 4, t16 = threadIdx.x & 15;
+                const int w = c < UM_TC ? S.cw[c] : 0;
+                const bool live = c < UM_TC && !S.dead[c];
+                const float muc = live ? mu[w] : 0.f;
+                const float ivc = live ? wst[w].z * 256.f : 0.f; // 2^ZSCALE
+                float zs = 0.f;
+                if (c < UM_TC)
+                    for (int q = 4 + (kp >> 1) + t16; q < ksw; q += 16) { // tail words
+                        zhw[c * ksw + q] = 0u;
+                        zlw[c * ksw + q] = 0u;
+                    }
+                if (c < UM_TC && t16 < 4) { // front padding
+                    zhw[c * ksw + t16] = 0u;
+                    zlw[c * ksw + t16] = 0u;
+                }
+                for (int k = t16; k < kp; k += 16) {
+                    const float v = (live && k < m) ? (x[w + k] - muc) * ivc : 0.f;
+                    const typename X::T h = X::cvt(v);
+                    const typename X::T l = X::cvt(v - X::back(h));
+                    if (c < UM_TC) {
+                        zh[c * 2 * ksw + 8 + k] = h;
+                        zl[c * 2 * ksw + 8 + k] = l;
+                    }
+                    zs += X::back(h) + X::back(l);
+                }
+#pragma unroll
+                for (int o = 8; o > 0; o >>= 1) zs += __shfl_xor_sync(0xffffffffu, zs, o);
+                if (t16 == 0 && c < UM_TC) S.zsum[c] = zs * (1.f / 256.f);
+                __syncthreads();
+                // A[(c,b), k'] = z_c[k' - b] in K-major core matrices:
+                // byte offset ((k'/8)*RG + r/8)*128 + (r%8)*16 + (k'%8)*2.
+                // Elements k'-b .. k'-b+7 start at padded element p0 = 8 + 8 kc - b:
+                // five 32-bit words from word p0/2, funnel-shifted by 16 bits when p0 is odd.
+                const int chunks = kp / 8;
+                for (int e = threadIdx.x; e < UM_M * chunks; e += UM_THREADS) {
+                    const int r = e & (UM_M - 1), kc = e / UM_M;
+                    const int cc = r >> 3, b = r & 7;
+                    const int p0 = 8 + 8 * kc - b;
+                    const uint32_t shf = (uint32_t)(p0 & 1) * 16u;
+                    const uint32_t *rh = zhw + cc * ksw + (p0 >> 1);
+                    const uint32_t *rl = zlw + cc * ksw + (p0 >> 1);
+                    uint32_t wh[5], wl[5], ph2[4], pl2[4];
+#pragma unroll
+                    for (int q = 0; q < 5; ++q) {
+                        wh[q] = rh[q];
+                        wl[q] = rl[q];
+                    }
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        ph2[q] = __funnelshift_r(wh[q], wh[q + 1], shf);
+                        pl2[q] = __funnelshift_r(wl[q], wl[q + 1], shf);
+                    }
+                    const uint32_t off = (uint32_t)((kc * RG + (r >> 3)) * 128 + (r & 7) * 16);
+                    *reinterpret_cast<uint4 *>(um_smem + L.a_hi + off) =
+                        make_uint4(ph2[0], ph2[1], ph2[2], ph2[3]);
+                    *reinterpret_cast<uint4 *>(um_smem + L.a_lo + off) =
+                        make_uint4(pl2[0], pl2[1], pl2[2], pl2[3]);
+                }
+                fence_proxy_async_smem(); // A for the tensor core; scratch for the bulk copies
+                __syncthreads();
+                if (threadIdx.x == 0) S.built_tile = tile; // read after the next item's barrier
+            }
 
-        // ================================================================ roles
-        if (warp == LOAD_WARP && lane == 0) {
-            // slice of tile u into stage u&1 (after the MMAs of tile u-2 are done);
-            // an end token instead once the item is dead
-            auto load_slice = [&](int u) -> bool {
-                const int s = u & 1;
-                if (u >= 2 && !mbar_wait_bounded(&S.mma_done[s], par(ph.done[s] + ((u - 2) >> 1)), wl))
-                    return false;
-                S.last_full[s] = (int)(ph.full[s] + (u >> 1));
-                if (S.item_dead) {
-                    S.vb[s] = 0;
-                    S.tok = u;
-                    mbar_arrive(&S.full_b[s]);
+            // ================================================================ roles
+            if (warp == LOAD_WARP && lane == 0) {
+                // slice of tile u into stage u&1 (after the MMAs of tile u-2 are done);
+                // an end token instead once the item is dead
+                auto load_slice = [&](int u) -> bool {
+                    const int s = u & 1;
+                    if (u >= 2 && !mbar_wait_bounded(&S.mma_done[s], par(ph.done[s] + ((u - 2) >> 1)), wl))
+                        return false;
+                    S.last_full[s] = (int)(ph.full[s] + (u >> 1));
+                    if (S.item_dead) {
+                        S.vb[s] = 0;
+                        S.tok = u;
+                        mbar_arrive(&S.full_b[s]);
+                        return true;
+                    }
+                    S.vb[s] = 1;
+                    const uint16_t *src = bq + (size_t)(blk0 + u) * 2 * cnt;
+                    mbar_arrive_expect_tx(&S.full_b[s], (uint32_t)(4 * cnt));
+                    bulk_g2s(um_smem + L.b[s][0], src, (uint32_t)(2 * cnt), &S.full_b[s]);
+                    bulk_g2s(um_smem + L.b[s][1], src + cnt, (uint32_t)(2 * cnt), &S.full_b[s]);
                     return true;
+                };
+                bool ok = true; // slice 0 was issued before the operand build
+                for (int u = 0; ok && u < T; ++u) {
+                    if (u + 1 < T) ok = load_slice(u + 1);
+                    if (!ok) break;
+                    // window data of tile u (after the epilogue is done with tile u-1)
+                    if (u >= 1 && !mbar_wait_bounded(&S.wd_empty, par(ph.wde + (u - 1)), wl)) {
+                        ok = false;
+                        break;
+                    }
+                    S.last_wd = (int)(ph.wdf + u);
+                    if (S.tok == u + 1) { // end token: no window data for tile u either
+                        S.vw = 0;
+                        mbar_arrive(&S.wd_full);
+                        break;
+                    }
+                    S.vw = 1;
+                    mbar_arrive_expect_tx(&S.wd_full, (uint32_t)WD_BYTES);
+                    bulk_g2s(um_smem + L.wd, wdq + (size_t)(blk0 + u) * 8 * WD_ROW, (uint32_t)WD_BYTES,
+                             &S.wd_full);
                 }
-                S.vb[s] = 1;
-                const uint16_t *src = bq + (size_t)(blk0 + u) * 2 * cnt;
-                mbar_arrive_expect_tx(&S.full_b[s], (uint32_t)(4 * cnt));
-                bulk_g2s(um_smem + L.b[s][0], src, (uint32_t)(2 * cnt), &S.full_b[s]);
-                bulk_g2s(um_smem + L.b[s][1], src + cnt, (uint32_t)(2 * cnt), &S.full_b[s]);
-                return true;
-            };
-            bool ok = true; // slice 0 was issued before the operand build
-            for (int u = 0; ok && u < T; ++u) {
-                if (u + 1 < T) ok = load_slice(u + 1);
-                if (!ok) break;
-                // window data of tile u (after the epilogue is done with tile u-1)
-                if (u >= 1 && !mbar_wait_bounded(&S.wd_empty, par(ph.wde + (u - 1)), wl)) {
-                    ok = false;
-                    break;
-                }
-                S.last_wd = (int)(ph.wdf + u);
-                if (S.tok == u + 1) { // end token: no window data for tile u either
-                    S.vw = 0;
-                    mbar_arrive(&S.wd_full);
-                    break;
-                }
-                S.vw = 1;
-                mbar_arrive_expect_tx(&S.wd_full, (uint32_t)WD_BYTES);
-                bulk_g2s(um_smem + L.wd, wdq + (size_t)(blk0 + u) * 8 * WD_ROW, (uint32_t)WD_BYTES,
-                         &S.wd_full);
-            }
-            if (!ok) S.abort = 1;
-        } else if (warp == MMA_WARP && lane == 0) {
-            for (int u = 0; u < T; ++u) {
-                const int s = u & 1;
-                if (!mbar_wait_bounded(&S.full_b[s], par(ph.full[s] + (u >> 1)), wl)) {
-                    S.abort = 1;
-                    break;
-                }
-                // the accumulator's previous tile must be drained first, also before an
-                // end token: its commit completes a phase of mma_done[s] that the
-                // epilogue may still be waiting on for tile u-2
-                if (u >= 2 &&
-                    !mbar_wait_bounded(&S.acc_empty[s], par(ph.acc[s] + ((u - 2) >> 1)), wl)) {
-                    S.abort = 1;
-                    break;
-                }
-                if (!S.vb[s]) { // end token: pass it on (the commit also covers earlier MMAs)
-                    umma_commit(&S.mma_done[s]);
-                    break;
-                }
-                tc_fence_after();
-                const uint32_t d = tmem + (uint32_t)(s * UM_N);
-                const uint32_t bh = smem_u32(um_smem + L.b[s][0]), bl = smem_u32(um_smem + L.b[s][1]);
-                for (int kb = 0; kb < kblocks; ++kb) {
-                    // K-block kb = core-matrix columns 2kb, 2kb+1; LBO = next K column of cores
-                    const uint64_t ah = sdesc(a_hi_s + kb * (2 * RG * 128), RG * 128, 128);
-                    const uint64_t al = sdesc(a_lo_s + kb * (2 * RG * 128), RG * 128, 128);
-                    const uint64_t bhd = sdesc(bh + kb * 32, 16, 128);
-                    const uint64_t bld = sdesc(bl + kb * 32, 16, 128);
-                    umma_f16(d, ah, bhd, idesc, kb > 0 ? 1u : 0u);
-                    umma_f16(d, ah, bld, idesc, 1u);
-                    umma_f16(d, al, bhd, idesc, 1u);
-                }
-                umma_commit(&S.mma_done[s]);
-                mma_issued = true;
-            }
-        } else if (warp >= EPI_WARP0) {
-            float rmax = -INFINITY;
-            const int wc = S.cw[cidx];
-            const float zsc = S.zsum[cidx], fc = S.cflat[cidx];
-            const float2 nz2 = make_float2(-zsc, -zsc);
-            // Every lane waits (acquire) and the warp then agrees through a vote, so
-            // the warp is converged and takes the same branch at every tcgen05.ld.
-            for (int u = 0; u < T; ++u) {
-                const int s = u & 1;
-                if (!__all_sync(0xffffffffu, mbar_wait_bounded(&S.wd_full, par(ph.wdf + u), wl))) {
-                    S.abort = 1;
-                    break;
-                }
-                const int vw = __shfl_sync(0xffffffffu, S.vw, 0);
-                if (!__all_sync(0xffffffffu,
-                                mbar_wait_bounded(&S.mma_done[s], par(ph.done[s] + (u >> 1)), wl))) {
-                    S.abort = 1;
-                    break;
-                }
-                if (!vw) { // end token; its slice twin at tile u+1 is committed too
-                    const int s1 = (u + 1) & 1;
-                    if (!__all_sync(0xffffffffu, mbar_wait_bounded(&S.mma_done[s1], par(ph.done[s1] + ((u + 1) >> 1)), wl)))
+                if (!ok) S.abort = 1;
+            } else if (warp == MMA_WARP && lane == 0) {
+                for (int u = 0; u < T; ++u) {
+                    const int s = u & 1;
+                    if (!mbar_wait_bounded(&S.full_b[s], par(ph.full[s] + (u >> 1)), wl)) {
                         S.abort = 1;
-                    break;
+                        break;
+                    }
+                    // the accumulator's previous tile must be drained first, also before an
+                    // end token: its commit completes a phase of mma_done[s] that the
+                    // epilogue may still be waiting on for tile u-2
+                    if (u >= 2 &&
+                        !mbar_wait_bounded(&S.acc_empty[s], par(ph.acc[s] + ((u - 2) >> 1)), wl)) {
+                        S.abort = 1;
+                        break;
+                    }
+                    if (!S.vb[s]) { // end token: pass it on (the commit also covers earlier MMAs)
+                        umma_commit(&S.mma_done[s]);
+                        break;
+                    }
+                    tc_fence_after();
+                    const uint32_t d = tmem + (uint32_t)(s * UM_N);
+                    const uint32_t bh = smem_u32(um_smem + L.b[s][0]), bl = smem_u32(um_smem + L.b[s][1]);
+                    for (int kb = 0; kb < kblocks; ++kb) {
+                        // K-block kb = core-matrix columns 2kb, 2kb+1; LBO = next K column of cores
+                        const uint64_t ah = sdesc(a_hi_s + kb * (2 * RG * 128), RG * 128, 128);
+                        const uint64_t al = sdesc(a_lo_s + kb * (2 * RG * 128), RG * 128, 128);
+                        const uint64_t bhd = sdesc(bh + kb * 32, 16, 128);
+                        const uint64_t bld = sdesc(bl + kb * 32, 16, 128);
+                        umma_f16(d, ah, bhd, idesc, kb > 0 ? 1u : 0u);
+                        umma_f16(d, ah, bld, idesc, 1u);
+                        umma_f16(d, al, bhd, idesc, 1u);
+                    }
+                    umma_commit(&S.mma_done[s]);
+                    mma_issued = true;
                 }
-                tc_fence_after();
-                const int j0 = j_lo + u * UM_TW;
-                if (!__shfl_sync(0xffffffffu, S.item_dead, 0)) {
-                    const uint32_t tb = tmem + ((uint32_t)(32 * g) << 16) +
-                                        (uint32_t)(s * UM_N + 128 * hcol);
-                    const bool masked = (j0 + UM_TW > j_hi) ||
-                                        (wc > j0 - m + 1 && wc < j0 + UM_TW + m - 1) || fc != 0.f;
-                    const float4 *wrow = wd4 + bsh * WD_ROW + 64 * hcol;
-                    // the tile's rounding bound (tile prep): correlations are lowered
-                    // by it for the prune test and raised back for the kept maxima
-                    const float Gt = wd4[128].x;
-                    const float2 ng2 = make_float2(-Gt, -Gt);
-                    float tm[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-                    // 4 chunks of 32 columns; the load of chunk cb+1 overlaps the math of cb
-                    auto chunk = [&](const uint32_t (&r)[32], int cb) {
-                        if (!masked) {
+            } else if (warp >= EPI_WARP0) {
+                float rmax = -INFINITY;
+                const int wc = S.cw[cidx];
+                const float zsc = S.zsum[cidx], fc = S.cflat[cidx];
+                const float2 nz2 = make_float2(-zsc, -zsc);
+                // Every lane waits (acquire) and the warp then agrees through a vote, so
+                // the warp is converged and takes the same branch at every tcgen05.ld.
+                for (int u = 0; u < T; ++u) {
+                    const int s = u & 1;
+                    if (!__all_sync(0xffffffffu, mbar_wait_bounded(&S.wd_full, par(ph.wdf + u), wl))) {
+                        S.abort = 1;
+                        break;
+                    }
+                    const int vw = __shfl_sync(0xffffffffu, S.vw, 0);
+                    if (!__all_sync(0xffffffffu,
+                                    mbar_wait_bounded(&S.mma_done[s], par(ph.done[s] + (u >> 1)), wl))) {
+                        S.abort = 1;
+                        break;
+                    }
+                    if (!vw) { // end token; its slice twin at tile u+1 is committed too
+                        const int s1 = (u + 1) & 1;
+                        if (!__all_sync(0xffffffffu, mbar_wait_bounded(&S.mma_done[s1], par(ph.done[s1] + ((u + 1) >> 1)), wl)))
+                            S.abort = 1;
+                        break;
+                    }
+                    tc_fence_after();
+                    const int j0 = j_lo + u * UM_TW;
+                    if (!__shfl_sync(0xffffffffu, S.item_dead, 0)) {
+                        const uint32_t tb = tmem + ((uint32_t)(32 * g) << 16) +
+                                            (uint32_t)(s * UM_N + 128 * hcol);
+                        const bool masked = (j0 + UM_TW > j_hi) ||
+                                            (wc > j0 - m + 1 && wc < j0 + UM_TW + m - 1) || fc != 0.f;
+                        const float4 *wrow = wd4 + bsh * WD_ROW + 64 * hcol;
+                        // the tile's rounding bound (tile prep): correlations are lowered
+                        // by it for the prune test and raised back for the kept maxima
+                        const float Gt = wd4[128].x;
+                        const float2 ng2 = make_float2(-Gt, -Gt);
+                        float tm[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+                        // 4 chunks of 32 columns; the load of chunk cb+1 overlaps the math of cb
+                        auto chunk = [&](const uint32_t (&r)[32], int cb) {
+                            if (!masked) {
 #pragma unroll
-                            for (int i2 = 0; i2 < 16; ++i2) {
-                                const float4 wv = wrow[16 * cb + i2];
-                                const float2 dd = make_float2(__uint_as_float(r[2 * i2]),
-                                                              __uint_as_float(r[2 * i2 + 1]));
-                                const float2 rho = __ffma2_rn(
-                                    dd, make_float2(wv.x, wv.y),
-                                    __ffma2_rn(nz2, make_float2(wv.z, wv.w), ng2));
-                                tm[i2 & 3] = fmax3(tm[i2 & 3], rho.x, rho.y);
+                                for (int i2 = 0; i2 < 16; ++i2) {
+                                    const float4 wv = wrow[16 * cb + i2];
+                                    const float2 dd = make_float2(__uint_as_float(r[2 * i2]),
+                                                                  __uint_as_float(r[2 * i2 + 1]));
+                                    const float2 rho = __ffma2_rn(
+                                        dd, make_float2(wv.x, wv.y),
+                                        __ffma2_rn(nz2, make_float2(wv.z, wv.w), ng2));
+                                    tm[i2 & 3] = fmax3(tm[i2 & 3], rho.x, rho.y);
+                                }
+                            } else {
+#pragma unroll
+                                for (int i = 0; i < 32; ++i) {
+                                    const int col = 128 * hcol + 32 * cb + i;
+                                    const int j = j0 + 8 * col + bsh;
+                                    const float4 wv = wrow[(32 * cb + i) >> 1];
+                                    const float wa = (i & 1) ? wv.y : wv.x;
+                                    const float wb = (i & 1) ? wv.w : wv.z;
+                                    float rho = fmaf(__uint_as_float(r[i]), wa, fmaf(-zsc, wb, -Gt));
+                                    if (fc != 0.f && wa == 0.f) rho += 1.f; // two flat windows
+                                    const int dd = wc > j ? wc - j : j - wc;
+                                    if (j < j_hi && dd >= m - 1) tm[i & 3] = fmaxf(tm[i & 3], rho);
+                                }
                             }
-                        } else {
-#pragma unroll
-                            for (int i = 0; i < 32; ++i) {
-                                const int col = 128 * hcol + 32 * cb + i;
-                                const int j = j0 + 8 * col + bsh;
-                                const float4 wv = wrow[(32 * cb + i) >> 1];
-                                const float wa = (i & 1) ? wv.y : wv.x;
-                                const float wb = (i & 1) ? wv.w : wv.z;
-                                float rho = fmaf(__uint_as_float(r[i]), wa, fmaf(-zsc, wb, -Gt));
-                                if (fc != 0.f && wa == 0.f) rho += 1.f; // two flat windows
-                                const int dd = wc > j ? wc - j : j - wc;
-                                if (j < j_hi && dd >= m - 1) tm[i & 3] = fmaxf(tm[i & 3], rho);
+                        };
+                        uint32_t ra[32], rb[32];
+                        tmem_ld32_async(tb, ra);
+                        tmem_wait_ld(ra);
+                        tmem_ld32_async(tb + 32, rb);
+                        chunk(ra, 0);
+                        tmem_wait_ld(rb);
+                        tmem_ld32_async(tb + 64, ra);
+                        chunk(rb, 1);
+                        tmem_wait_ld(ra);
+                        tmem_ld32_async(tb + 96, rb);
+                        chunk(ra, 2);
+                        tmem_wait_ld(rb);
+                        chunk(rb, 3);
+                        float tmax = fmaxf(fmaxf(tm[0], tm[1]), fmaxf(tm[2], tm[3]));
+                        if (!rowok) tmax = -INFINITY;
+                        rmax = fmaxf(rmax, tmax + Gt); // the interval's middle (-inf stays)
+                        const unsigned bal = __ballot_sync(0xffffffffu, tmax > thr);
+                        bool hint = false;
+                        if (lane < UM_TC / 4) {
+                            const int ci = (UM_TC / 4) * g + lane;
+                            if (!S.dead[ci]) {
+                                if ((bal >> (8 * lane)) & 0xFFu) {
+                                    S.dead[ci] = 1;
+                                    pruned[S.cp[ci]] = 1;
+                                    hint = W.wit != nullptr;
+                                } else if (__ldcg(pruned + S.cp[ci])) {
+                                    S.dead[ci] = 1; // pruned by another CTA's item
+                                }
                             }
                         }
-                    };
-                    uint32_t ra[32], rb[32];
-                    tmem_ld32_async(tb, ra);
-                    tmem_wait_ld(ra);
-                    tmem_ld32_async(tb + 32, rb);
-                    chunk(ra, 0);
-                    tmem_wait_ld(rb);
-                    tmem_ld32_async(tb + 64, ra);
-                    chunk(rb, 1);
-                    tmem_wait_ld(ra);
-                    tmem_ld32_async(tb + 96, rb);
-                    chunk(ra, 2);
-                    tmem_wait_ld(rb);
-                    chunk(rb, 3);
-                    float tmax = fmaxf(fmaxf(tm[0], tm[1]), fmaxf(tm[2], tm[3]));
-                    if (!rowok) tmax = -INFINITY;
-                    rmax = fmaxf(rmax, tmax + Gt); // the interval's middle (-inf stays)
-                    const unsigned bal = __ballot_sync(0xffffffffu, tmax > thr);
-                    bool hint = false;
-                    if (lane < UM_TC / 4) {
-                        const int ci = (UM_TC / 4) * g + lane;
-                        if (!S.dead[ci]) {
-                            if ((bal >> (8 * lane)) & 0xFFu) {
-                                S.dead[ci] = 1;
-                                pruned[S.cp[ci]] = 1;
-                                hint = W.wit != nullptr;
-                            } else if (__ldcg(pruned + S.cp[ci])) {
-                                S.dead[ci] = 1; // pruned by another CTA's item
+                        // a candidate pruned here leaves the window that did it as its
+                        // witness hint: a second pass over the accumulator, at most once
+                        // per candidate, finds its column
+                        const unsigned hints = __ballot_sync(0xffffffffu, hint);
+                        if (hints) {
+                            int jh = -1;
+                            const bool mine = rowok && ((hints >> (lane >> 3)) & 1u) && tmax > thr;
+                            for (int cb = 0; cb < 4; ++cb) {
+                                tmem_ld32_async(tb + 32 * cb, ra);
+                                tmem_wait_ld(ra);
+#pragma unroll
+                                for (int i = 0; i < 32; ++i) {
+                                    const int j = j0 + 8 * (128 * hcol + 32 * cb + i) + bsh;
+                                    const float4 wv = wrow[(32 * cb + i) >> 1];
+                                    const float rho = fmaf(__uint_as_float(ra[i]), (i & 1) ? wv.y : wv.x,
+                                                           fmaf(-zsc, (i & 1) ? wv.w : wv.z, -Gt));
+                                    const int dd = wc > j ? wc - j : j - wc;
+                                    if (rho > thr && j < j_hi && dd >= m - 1) jh = j;
+                                }
                             }
+                            if (mine && jh >= 0) wt_hint(W, wc, WT_ONE, jh);
+                        }
+                        __syncwarp();
+                        if (warp == EPI_WARP0 && lane == 0) {
+                            atomicAdd(&att->n_pairs, (unsigned long long)UM_TC * UM_TW);
+                            int alive = 0;
+                            for (int c = 0; c < UM_TC; ++c) alive += !S.dead[c];
+                            atomicAdd(&att->n_live, (unsigned long long)S.tile_live * UM_TW);
+                            S.tile_live = alive;
+                            if (!alive) S.item_dead = 1;
                         }
                     }
-                    // a candidate pruned here leaves the window that did it as its
-                    // witness hint: a second pass over the accumulator, at most once
-                    // per candidate, finds its column
-                    const unsigned hints = __ballot_sync(0xffffffffu, hint);
-                    if (hints) {
-                        int jh = -1;
-                        const bool mine = rowok && ((hints >> (lane >> 3)) & 1u) && tmax > thr;
-                        for (int cb = 0; cb < 4; ++cb) {
-                            tmem_ld32_async(tb + 32 * cb, ra);
-                            tmem_wait_ld(ra);
-#pragma unroll
-                            for (int i = 0; i < 32; ++i) {
-                                const int j = j0 + 8 * (128 * hcol + 32 * cb + i) + bsh;
-                                const float4 wv = wrow[(32 * cb + i) >> 1];
-                                const float rho = fmaf(__uint_as_float(ra[i]), (i & 1) ? wv.y : wv.x,
-                                                       fmaf(-zsc, (i & 1) ? wv.w : wv.z, -Gt));
-                                const int dd = wc > j ? wc - j : j - wc;
-                                if (rho > thr && j < j_hi && dd >= m - 1) jh = j;
-                            }
-                        }
-                        if (mine && jh >= 0) wt_hint(W, wc, WT_ONE, jh);
-                    }
+                    tc_fence_before();
                     __syncwarp();
-                    if (warp == EPI_WARP0 && lane == 0) {
-                        atomicAdd(&att->n_pairs, (unsigned long long)UM_TC * UM_TW);
-                        int alive = 0;
-                        for (int c = 0; c < UM_TC; ++c) alive += !S.dead[c];
-                        atomicAdd(&att->n_live, (unsigned long long)S.tile_live * UM_TW);
-                        S.tile_live = alive;
-                        if (!alive) S.item_dead = 1;
+                    if (lane == 0) {
+                        mbar_arrive(&S.acc_empty[s]);
+                        mbar_arrive(&S.wd_empty);
                     }
                 }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) {
-                    mbar_arrive(&S.acc_empty[s]);
-                    mbar_arrive(&S.wd_empty);
-                }
-            }
-            // fold the running maxima (8 shifts per candidate)
-            float v = rmax;
+                // fold the running maxima (8 shifts per candidate)
+                float v = rmax;
 #pragma unroll
-            for (int o = 4; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-            if (rowok && (lane & 7) == 0 && v > -INFINITY) atomicMax(&S.rmax[cidx], f2ord(v));
-        }
-        __syncthreads();
-        // ---- phase bookkeeping (every thread, same numbers)
-        {
-            const int tok = S.tok;                 // slice index of the end token, or -1
-            const int nb = tok >= 0 ? tok + 1 : T; // full_b / mma_done phases
-            const int nw = tok >= 0 ? tok : T;     // wd_full phases
-            const int ne = tok >= 0 ? tok - 1 : T; // acc_empty / wd_empty arrivals (tok >= 1)
-            for (int s = 0; s < 2; ++s) {
-                const uint32_t cb = (uint32_t)((nb + 1 - s) >> 1);
-                const uint32_t ce = (uint32_t)((ne + 1 - s) >> 1);
-                ph.full[s] += cb;
-                ph.done[s] += cb;
-                ph.acc[s] += ce;
+                for (int o = 4; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+                if (rowok && (lane & 7) == 0 && v > -INFINITY) atomicMax(&S.rmax[cidx], f2ord(v));
             }
-            ph.wdf += (uint32_t)nw;
-            ph.wde += (uint32_t)ne;
+            __syncthreads();
+            // ---- phase bookkeeping (every thread, same numbers)
+            {
+                const int tok = S.tok;                 // slice index of the end token, or -1
+                const int nb = tok >= 0 ? tok + 1 : T; // full_b / mma_done phases
+                const int nw = tok >= 0 ? tok : T;     // wd_full phases
+                const int ne = tok >= 0 ? tok - 1 : T; // acc_empty / wd_empty arrivals (tok >= 1)
+                for (int s = 0; s < 2; ++s) {
+                    const uint32_t cb = (uint32_t)((nb + 1 - s) >> 1);
+                    const uint32_t ce = (uint32_t)((ne + 1 - s) >> 1);
+                    ph.full[s] += cb;
+                    ph.done[s] += cb;
+                    ph.acc[s] += ce;
+                }
+                ph.wdf += (uint32_t)nw;
+                ph.wde += (uint32_t)ne;
+            }
+            if (threadIdx.x < UM_TC && tile * UM_TC + threadIdx.x < C &&
+                S.rmax[threadIdx.x] != f2ord(-INFINITY))
+                atomicMax(rho_max + S.cp[threadIdx.x], S.rmax[threadIdx.x]);
+            __syncthreads();
+            if (S.abort) break;
         }
-        if (threadIdx.x < UM_TC && tile * UM_TC + threadIdx.x < C &&
-            S.rmax[threadIdx.x] != f2ord(-INFINITY))
-            atomicMax(rho_max + S.cp[threadIdx.x], S.rmax[threadIdx.x]);
-        __syncthreads();
         if (S.abort) break;
+        if (je >= col_hi) {
+            if (threadIdx.x == 0) att->last_rd = rd;
+            break;
+        }
+        // ---- between rounds (one launch for all of them: separate launches with a
+        // compaction kernel each cost 30 us an attempt, most of it for rounds
+        // without work; headline run 249 -> 229 ms).  The CTA that finished the round's last item compacts
+        // the survivors; the others wait for it.  A CTA waits only for items that
+        // other, running CTAs have taken (it found none left to take), so the wait
+        // ends whichever CTAs are resident; it is bounded all the same.
+        if (S.last) {
+            __threadfence();
+            const int nx = um_compact(list, rd == 0, C, pruned, rd & 1 ? list0 : list1, S.wsum);
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                S.last = 0;
+                S.next = nx;
+                att->list_count[rd + 1] = nx;
+                if (nx == 0) att->last_rd = rd + 1;
+                __threadfence();
+                st_release(&att->round_ready, rd + 1);
+            }
+        } else if (threadIdx.x == 0) {
+            const long long t0 = clock64();
+            S.next = 0;
+            while (ld_acquire(&att->round_ready) <= rd) {
+                if (ld_acquire(&att->status) == 3) S.next = -1; // another CTA gave up
+                else if (clock64() - t0 > wl) {
+                    atomicExch(&att->status, 3);
+                    S.next = -1;
+                }
+                if (S.next < 0) break;
+                __nanosleep(100);
+            }
+            if (S.next == 0) S.next = __ldcg(&att->list_count[rd + 1]);
+        }
+        __syncthreads();
+        C = S.next;
+        if (C <= 0) break;
+        jb = je;
+        __syncthreads(); // S.next is read by all before a later round writes it
     }
     if (S.abort) {
         if (threadIdx.x == 0) {
-            atomicExch(&att->status, 3);
+            atomicExch(&att->status, 3); // also ends the other CTAs' waits between rounds
             if (mma_issued) { // let the MMAs in flight finish before TMEM goes away
                 umma_commit(&S.drain);
                 mbar_wait_bounded(&S.drain, 0u, kDrainCycles);
@@ -966,36 +1082,33 @@ cudaError_t paddi_launch_tile_prep(bool bf16, const float *x, int64_t n, int32_t
 }
 
 cudaError_t paddi_launch_refine_umma(bool bf16, const float *x, const float4 *wst,
-                                     const float *mu, const int32_t *cand, const int32_t *list,
-                                     const int32_t *list_count, const uint16_t *bq,
-                                     const float4 *wdq, PaddiAttemptDev *att, int32_t *work,
-                                     uint32_t *rho_max, uint8_t *pruned, int32_t N, int32_t m,
-                                     int32_t jb, int32_t je, float thr_prune, int32_t num_sms,
-                                     cudaStream_t st, long long wait_cycles, int32_t withhold,
-                                     int32_t round, int32_t je_all, bool rows64,
+                                     const float *mu, const int32_t *cand, int32_t *list0,
+                                     int32_t *list1, const uint16_t *bq, const float4 *wdq,
+                                     PaddiAttemptDev *att, uint32_t *rho_max, uint8_t *pruned,
+                                     int32_t N, int32_t m, int32_t col_lo, int32_t col_hi,
+                                     float thr_prune, int32_t num_sms, cudaStream_t st,
+                                     long long wait_cycles, int32_t withhold, bool rows64,
                                      const PaddiWitness *W)
 {
     const int kp = kpad_of(m);
     if (kp > UM_KMAX64 || m < 3) return cudaErrorInvalidValue;
-    if ((jb % UM_TW) != 0 || (je % UM_TW != 0 && je != N)) return cudaErrorInvalidValue;
-    if (je_all > 0 && (je_all < je || (je_all % UM_TW != 0 && je_all != N)))
-        return cudaErrorInvalidValue;
+    if ((col_lo % UM_TW) != 0 || (col_hi % UM_TW != 0 && col_hi != N)) return cudaErrorInvalidValue;
     const int MM = (kp <= UM_KMAX128 && !rows64) ? 128 : 64;
     const UmLayout L = um_layout(MM, kp);
     // request at least half the SM's shared memory so one CTA owns the 512 TMEM columns
     const size_t smem = L.bytes < 120 * 1024 ? 120 * 1024 : L.bytes;
-    void (*kern)(const float *, const float4 *, const float *, const int32_t *, const int32_t *,
-                 const int32_t *, const uint16_t *, const float4 *, PaddiAttemptDev *, int32_t *,
-                 uint32_t *, uint8_t *, int32_t, int32_t, int32_t, int32_t, float, int32_t,
-                 long long, int32_t, int32_t, int32_t, PaddiWitness);
+    void (*kern)(const float *, const float4 *, const float *, const int32_t *, int32_t *,
+                 int32_t *, const uint16_t *, const float4 *, PaddiAttemptDev *, uint32_t *,
+                 uint8_t *, int32_t, int32_t, int32_t, int32_t, float, int32_t, long long, int32_t,
+                 PaddiWitness);
     if (MM == 128) kern = bf16 ? k_refine_umma<true, 128> : k_refine_umma<false, 128>;
     else kern = bf16 ? k_refine_umma<true, 64> : k_refine_umma<false, 64>;
     cudaError_t e = paddi_raise_smem_limit((const void *)kern, smem);
     if (e != cudaSuccess) return e;
     const int grid = num_sms;
-    kern<<<grid, UM_THREADS, smem, st>>>(x, wst, mu, cand, list, list_count, bq, wdq, att, work,
-                                         rho_max, pruned, N, m, jb, je, thr_prune, grid,
+    kern<<<grid, UM_THREADS, smem, st>>>(x, wst, mu, cand, list0, list1, bq, wdq, att, rho_max,
+                                         pruned, N, m, col_lo, col_hi, thr_prune, grid,
                                          wait_cycles > 0 ? wait_cycles : 4000000000ll, withhold,
-                                         round, je_all > 0 ? je_all : je, W ? *W : PaddiWitness{});
+                                         W ? *W : PaddiWitness{});
     return cudaGetLastError();
 }

@@ -57,13 +57,13 @@ struct paddi_ctx {
     int num_sms = 0;
     cudaStream_t st = nullptr;
     cudaEvent_t ev[8] = {};
-    cudaEvent_t rev[8] = {}; // around each refine round's launch
+    cudaEvent_t rev[8] = {}; // around each refine launch
+    int n_rev = 0;           // pairs of them used by the current attempt
     // PADDI_TRACE=1 in the environment: one stderr line per attempt with the
-    // live-candidate count and the time of every refine round
+    // candidates entering every refine round
     bool trace = false;
-    cudaEvent_t tev[9] = {};
-    int32_t *d_trace = nullptr, *h_trace = nullptr;
-    unsigned long long *h_trace64 = nullptr;
+    cudaEvent_t tev = nullptr;
+    PaddiAttemptDev *h_trace = nullptr;
     std::string err;
     size_t cap_n = 0; // series capacity (values)
     int32_t rc_cap = 0; // FP64 recheck capacity (windows)
@@ -231,7 +231,6 @@ struct AttemptOut {
     PaddiAttemptResult res;
     float ms_phase1 = 0, ms_refine = 0, ms_select = 0, ms_total = 0;
     float ms_refine_kernel = 0; // the refine launches alone
-    int nrounds = 0;
     int launches = 0;
     int kernel = PADDI_DIST_FP32;
     int p1_rows = 0; // rows per phase-1 task
@@ -333,75 +332,72 @@ int32_t wit_enough(int32_t N) { return std::max(1024, N / 512); }
 // The correlation threshold of r^2 at length m: d < r^2 <=> rho > thr.
 float thr_of(float r2, int m) { return (float)(1.0 - (double)r2 / (2.0 * (double)m)); }
 
-// Refine rounds of the compacted candidates against the windows [col_lo,
-// col_hi) (col_lo on the refine's grid), then the FP64 pass over the fragile
-// windows of that range.  Rounds over growing window ranges (1/16, 1/4, 1/2,
+// Refine of the compacted candidates against the windows [col_lo, col_hi)
+// (col_lo on the refine's grid), then the FP64 pass over the fragile windows of
+// that range.  It runs in rounds over growing window ranges (1/16, 1/4, 1/2,
 // all of the range; a sweep of 4 to 8 rounds picked 4); survivors are
-// re-compacted between rounds so every tile is dense with live candidates.
+// re-compacted between rounds so every tile is dense with live candidates.  The
+// tensor-core refine does all of them in one launch.
 paddi_status refine_rounds(paddi_ctx *ctx, const float *x, int32_t N, int m, int kernel,
-                           float thr, float guard, int32_t col_lo, int32_t col_hi,
-                           int *launches, int *nrounds_out)
+                           float thr, float guard, int32_t col_lo, int32_t col_hi, int *launches)
 {
     cudaStream_t st = ctx->st;
-    CK(paddi_launch_list_init(ctx->d_att, ctx->d_list[0], &ctx->d_att->list_count[0], st));
-    ++*launches;
-    const bool umma = kernel != PADDI_DIST_FP32;
-    constexpr int kShifts[3] = {4, 2, 1};
     const PaddiWitness *W = ctx->wit_m == m ? &ctx->W : nullptr;
-    const int32_t range = col_hi - col_lo;
-    const int nrounds = range >= (1 << 16) ? 4 : 1;
-    // round edges on the refine's grid: 2048-window tiles (tensor cores),
-    // 256-window chunks (FP32), so the fragile set depends only on the length
-    const int tw = umma ? paddi_tile_width() : 256;
-    int jb = col_lo;
-    for (int rd = 0; rd < nrounds; ++rd) {
-        int je = rd == nrounds - 1 ? col_hi
-                                   : col_lo + (int)((int64_t)range >> kShifts[rd]) / tw * tw;
-        if (je > col_hi) je = col_hi;
-        if (je < jb) je = jb;
-        // round rd: list d_list[rd & 1] of list_count[rd] entries, work counter
-        // work_rd[rd]; the compaction after it writes list_count[rd + 1].  All
-        // are zero from the attempt's reset, so no launch clears them.
-        const int a = rd & 1, b = a ^ 1;
-        int32_t *cnt = &ctx->d_att->list_count[rd];
-        if (ctx->trace) {
-            CK(cudaEventRecord(ctx->tev[rd], st));
-            CK(cudaMemcpyAsync(ctx->d_trace + rd, cnt, sizeof(int32_t),
-                               cudaMemcpyDeviceToDevice, st));
-        }
-        CK(cudaEventRecord(ctx->rev[2 * rd], st));
-        if (umma)
-            CK(paddi_launch_refine_umma(kernel == PADDI_DIST_SPLIT_BF16, x, ctx->d_wst, ctx->d_mu,
-                                        ctx->d_cand, ctx->d_list[a], cnt, ctx->d_bq,
-                                        ctx->d_wdq, ctx->d_att, &ctx->d_att->work_rd[rd],
-                                        ctx->d_rho, ctx->d_pruned, N, m, jb, je, thr,
-                                        ctx->num_sms, st, ctx->wait_cycles, ctx->withhold, rd,
-                                        col_hi, ctx->opts.tile_rows == 64, W));
-        else
+    int last = -1; // round whose list holds the survivors (-1: the kernel recorded it)
+    ctx->n_rev = 1;
+    if (kernel != PADDI_DIST_FP32) {
+        CK(cudaEventRecord(ctx->rev[0], st));
+        CK(paddi_launch_refine_umma(kernel == PADDI_DIST_SPLIT_BF16, x, ctx->d_wst, ctx->d_mu,
+                                    ctx->d_cand, ctx->d_list[0], ctx->d_list[1], ctx->d_bq,
+                                    ctx->d_wdq, ctx->d_att, ctx->d_rho, ctx->d_pruned, N, m,
+                                    col_lo, col_hi, thr, ctx->num_sms, st, ctx->wait_cycles,
+                                    ctx->withhold, ctx->opts.tile_rows == 64, W));
+        CK(cudaEventRecord(ctx->rev[1], st));
+        ++*launches;
+    } else {
+        CK(paddi_launch_list_init(ctx->d_att, ctx->d_list[0], &ctx->d_att->list_count[0], st));
+        ++*launches;
+        constexpr int kShifts[3] = {4, 2, 1};
+        const int32_t range = col_hi - col_lo;
+        const int nrounds = range >= (1 << 16) ? 4 : 1;
+        int jb = col_lo;
+        for (int rd = 0; rd < nrounds; ++rd) {
+            // round edges on the grid of 256-window chunks, so the fragile set
+            // depends only on the length
+            int je = rd == nrounds - 1 ? col_hi
+                                       : col_lo + (int)((int64_t)range >> kShifts[rd]) / 256 * 256;
+            if (je > col_hi) je = col_hi;
+            if (je < jb) je = jb;
+            // round rd: list d_list[rd & 1] of list_count[rd] entries, work counter
+            // work_rd[rd]; the compaction after it writes list_count[rd + 1].  All
+            // are zero from the attempt's reset, so no launch clears them.
+            const int a = rd & 1, b = a ^ 1;
+            int32_t *cnt = &ctx->d_att->list_count[rd];
+            CK(cudaEventRecord(ctx->rev[2 * rd], st));
             CK(paddi_launch_refine_fp32(x, ctx->d_wst, ctx->d_mu, ctx->d_cand, ctx->d_list[a],
                                         cnt, ctx->d_att, &ctx->d_att->work_rd[rd], ctx->d_rho,
                                         ctx->d_pruned, N, m, jb, je, thr, guard, ctx->num_sms,
                                         st, W));
-        CK(cudaEventRecord(ctx->rev[2 * rd + 1], st));
-        ++*launches;
-        if (rd + 1 < nrounds) {
-            CK(paddi_launch_list_compact(ctx->d_list[a], cnt, ctx->d_pruned, ctx->d_list[b],
-                                         cnt + 1, st));
+            CK(cudaEventRecord(ctx->rev[2 * rd + 1], st));
             ++*launches;
+            if (rd + 1 < nrounds) {
+                CK(paddi_launch_list_compact(ctx->d_list[a], cnt, ctx->d_pruned, ctx->d_list[b],
+                                             cnt + 1, st));
+                ++*launches;
+            }
+            jb = je;
         }
-        jb = je;
+        ctx->n_rev = nrounds;
+        last = nrounds - 1;
     }
     // the fragile windows (skipped by the refine: their rounding bound exceeds
     // the guard band) against the candidates of the last round's list that are
     // still unpruned, in FP64 (the kernel returns at once when there are none)
-    const int a = (nrounds - 1) & 1;
-    if (ctx->trace) CK(cudaEventRecord(ctx->tev[nrounds], st));
-    CK(paddi_launch_fragile(x, ctx->d_ms64, ctx->d_cand, ctx->d_list[a],
-                            &ctx->d_att->list_count[nrounds - 1], ctx->d_pruned, ctx->d_rho,
-                            ctx->d_frag, ctx->d_flatcount + 3, m, thr, col_lo, col_hi,
-                            ctx->num_sms, st));
+    if (ctx->trace) CK(cudaEventRecord(ctx->tev, st));
+    CK(paddi_launch_fragile(x, ctx->d_ms64, ctx->d_cand, ctx->d_list[0], ctx->d_list[1],
+                            ctx->d_att, last, ctx->d_pruned, ctx->d_rho, ctx->d_frag,
+                            ctx->d_flatcount + 3, m, thr, col_lo, col_hi, ctx->num_sms, st));
     *launches += 1;
-    *nrounds_out = nrounds;
     return PADDI_OK;
 }
 
@@ -520,21 +516,12 @@ paddi_status run_attempt(paddi_ctx *ctx, const float *x, size_t n, int m, float 
     ++launches;
     out->kernel = kernel;
     out->p1_rows = R;
-    int nrounds = 0;
-    paddi_status s = refine_rounds(ctx, x, N, m, kernel, thr, guard, 0, N, &launches, &nrounds);
+    paddi_status s = refine_rounds(ctx, x, N, m, kernel, thr, guard, 0, N, &launches);
     if (s != PADDI_OK) return s;
     CK(cudaEventRecord(ctx->ev[2], st));
-    if (ctx->trace) {
-        CK(cudaEventRecord(ctx->tev[nrounds + 1], st));
-        CK(cudaMemcpyAsync(ctx->d_trace + 7, &ctx->d_att->p1_walked, sizeof(int32_t),
-                           cudaMemcpyDeviceToDevice, st));
-        CK(cudaMemcpyAsync(ctx->d_trace + 5, &ctx->d_att->n_fail, 2 * sizeof(int32_t),
-                           cudaMemcpyDeviceToDevice, st)); // and n_rescued
-        CK(cudaMemcpyAsync(ctx->h_trace64, &ctx->d_att->n_pairs, 2 * sizeof(unsigned long long),
+    if (ctx->trace)
+        CK(cudaMemcpyAsync(ctx->h_trace, ctx->d_att, sizeof(PaddiAttemptDev),
                            cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(ctx->h_trace, ctx->d_trace, sizeof(int32_t) * 8,
-                           cudaMemcpyDeviceToHost, st));
-    }
     bool spec = false;
     s = select_passes(ctx, x, n, m, r2, guard, top_k, known_w, known_ord, next_m, next_guided,
                       &spec, &launches);
@@ -542,35 +529,28 @@ paddi_status run_attempt(paddi_ctx *ctx, const float *x, size_t n, int m, float 
     out->res = *ctx->h_res;
     out->launches = launches;
     if (spec_out) *spec_out = spec;
-    if (ctx->trace) {
-        std::string line = "paddi-trace m=" + std::to_string(m) + " r2=" + std::to_string(r2) +
-                           " unproven=" + std::to_string(ctx->h_trace[5]) + "-" +
-                           std::to_string(ctx->h_trace[6]) +
-                           " p1=" + std::to_string(ctx->h_res->n_p1) +
-                           " p1_tasks=" + std::to_string(ctx->h_trace[7]) + "x" + std::to_string(R) +
-                           " rounds:";
-        for (int rd = 0; rd < nrounds; ++rd) {
-            float ms = 0.f;
-            CK(cudaEventElapsedTime(&ms, ctx->tev[rd], ctx->tev[rd + 1]));
-            line += " " + std::to_string(ctx->h_trace[rd]) + "/" + std::to_string(ms);
-        }
-        float fms = 0.f;
-        CK(cudaEventElapsedTime(&fms, ctx->tev[nrounds], ctx->tev[nrounds + 1]));
-        std::fprintf(stderr, "%s disc=%lld pairs=%llu live=%llu fragile=%d/%f\n", line.c_str(),
-                     (long long)ctx->h_res->n_disc, ctx->h_trace64[0], ctx->h_trace64[1],
-                     ctx->h_res->n_fragile, fms);
-    }
     CK(cudaEventElapsedTime(&out->ms_phase1, ctx->ev[0], ctx->ev[1]));
     CK(cudaEventElapsedTime(&out->ms_refine, ctx->ev[1], ctx->ev[2]));
     out->ms_refine_kernel = 0.f;
-    for (int rd = 0; rd < nrounds; ++rd) {
+    for (int rd = 0; rd < ctx->n_rev; ++rd) {
         float ms = 0.f;
         CK(cudaEventElapsedTime(&ms, ctx->rev[2 * rd], ctx->rev[2 * rd + 1]));
         out->ms_refine_kernel += ms;
     }
-    out->nrounds = nrounds;
     CK(cudaEventElapsedTime(&out->ms_select, ctx->ev[2], ctx->ev[3]));
     CK(cudaEventElapsedTime(&out->ms_total, ctx->ev[0], ctx->ev[3]));
+    if (ctx->trace) {
+        const PaddiAttemptDev &t = *ctx->h_trace;
+        float fms = 0.f;
+        CK(cudaEventElapsedTime(&fms, ctx->tev, ctx->ev[2]));
+        std::fprintf(stderr,
+                     "paddi-trace m=%d r2=%f unproven=%d-%d p1=%d p1_tasks=%dx%d/%f "
+                     "rounds: %d %d %d %d/%f fragile=%d/%f recheck=%d disc=%lld pairs=%llu live=%llu\n",
+                     m, r2, t.n_fail, t.n_rescued, t.n_cand_p1, t.p1_walked, R, out->ms_phase1,
+                     t.n_cand_p1, t.list_count[1], t.list_count[2], t.list_count[3],
+                     out->ms_refine_kernel, ctx->h_res->n_fragile, fms, ctx->h_res->n_recheck,
+                     (long long)ctx->h_res->n_disc, t.n_pairs, t.n_live);
+    }
     return PADDI_OK;
 }
 
@@ -1037,10 +1017,8 @@ PADDI_API paddi_status paddi_ctx_create(paddi_ctx **out, const paddi_opts *opts)
         ctx->trace = tr && tr[0] && tr[0] != '0';
     }
     if (ctx->trace) {
-        for (auto &e : ctx->tev) ok = ok && cudaEventCreate(&e) == cudaSuccess;
-        ok = ok && cudaMalloc(&ctx->d_trace, 8 * sizeof(int32_t)) == cudaSuccess;
-        ok = ok && cudaMallocHost(&ctx->h_trace, 8 * sizeof(int32_t)) == cudaSuccess;
-        ok = ok && cudaMallocHost(&ctx->h_trace64, 2 * sizeof(unsigned long long)) == cudaSuccess;
+        ok = ok && cudaEventCreate(&ctx->tev) == cudaSuccess;
+        ok = ok && cudaMallocHost(&ctx->h_trace, sizeof(PaddiAttemptDev)) == cudaSuccess;
     }
     ok = ok && cudaMalloc(&ctx->d_att, sizeof(PaddiAttemptDev)) == cudaSuccess;
     ok = ok && cudaMalloc(&ctx->d_res, sizeof(PaddiAttemptResult)) == cudaSuccess;
@@ -1084,13 +1062,10 @@ PADDI_API paddi_status paddi_ctx_destroy(paddi_ctx *ctx)
     if (ctx->h_res) cudaFreeHost(ctx->h_res);
     for (auto &e : ctx->ev)
         if (e) cudaEventDestroy(e);
-    for (auto &e : ctx->tev)
-        if (e) cudaEventDestroy(e);
+    if (ctx->tev) cudaEventDestroy(ctx->tev);
     for (auto &e : ctx->rev)
         if (e) cudaEventDestroy(e);
-    if (ctx->d_trace) cudaFree(ctx->d_trace);
     if (ctx->h_trace) cudaFreeHost(ctx->h_trace);
-    if (ctx->h_trace64) cudaFreeHost(ctx->h_trace64);
     if (ctx->st) cudaStreamDestroy(ctx->st);
     delete ctx;
     return PADDI_OK;
@@ -1327,10 +1302,10 @@ PADDI_API paddi_status paddi_shard_refine(paddi_ctx *ctx, const float *d_series,
     CK(paddi_launch_compact(d_alive, (int32_t)N, ctx->d_cand, ctx->d_rho, ctx->d_pruned,
                             ctx->d_rcslot, ctx->d_att, ctx->d_flat, ctx->d_flatcount + 1, (int)m,
                             r2 > 0.f, st));
-    int launches = 0, nrounds = 0;
+    int launches = 0;
     paddi_status s = refine_rounds(ctx, d_series, (int32_t)N, (int)m, kernel, thr,
                                    guard_of(ctx, kernel), (int32_t)col_lo, (int32_t)col_hi,
-                                   &launches, &nrounds);
+                                   &launches);
     if (s != PADDI_OK) return s;
     CK(cudaMemcpyAsync(&ctx->h_res->n_p1, &ctx->d_att->n_cand_p1, sizeof(int32_t),
                        cudaMemcpyDeviceToHost, st));

@@ -94,8 +94,9 @@ struct PaddiAttemptDev {
     int32_t p1_walked;      // phase-1 tasks that walked their rows (instrumentation)
     int32_t n_fail;         // windows whose witness proves nothing (k_witness.cu)
     int32_t n_rescued;      // of those, windows that found a new witness
-    int32_t covered_from;   // r + 1 when refine round r (one candidate tile left) took
-                            // every remaining window; later rounds then have nothing to do
+    int32_t done_rd[4];     // finished work items of the tensor-core refine's rounds
+    int32_t round_ready;    // rounds whose survivors are compacted
+    int32_t last_rd;        // the round after which no window was left
     unsigned long long n_pairs; // pairs evaluated by the refine (instrumentation)
     unsigned long long n_live;  // of those, pairs of candidates still unpruned at the tile's start
 };
@@ -227,31 +228,32 @@ cudaError_t paddi_launch_fragile_scan_fp32(const float *x, const float4 *wst, co
                                            int32_t N, int32_t m, float gcap, int32_t *frag_list,
                                            int32_t *frag_count, int32_t num_sms, cudaStream_t st);
 
-// Exact FP64 correlations of the unpruned candidates of list[0..*list_count)
-// with the fragile windows in [col_lo, col_hi) (k_fragile.cu): prunes and
-// raises rho_max.
-cudaError_t paddi_launch_fragile(const float *x, const double2 *ms64,
-                                 const int32_t *cand, const int32_t *list,
-                                 const int32_t *list_count, uint8_t *pruned, uint32_t *rho_max,
-                                 const int32_t *frag, const int32_t *frag_count, int32_t m,
-                                 float thr, int32_t col_lo, int32_t col_hi, int32_t num_sms,
-                                 cudaStream_t st);
+// Exact FP64 correlations of the refine's unpruned candidates with the fragile
+// windows in [col_lo, col_hi) (k_fragile.cu): prunes and raises rho_max.  last:
+// the refine's last round, whose list holds the candidates (list1 if odd, else
+// list0, list_count[last] entries; round 0: all candidates); -1: att->last_rd.
+cudaError_t paddi_launch_fragile(const float *x, const double2 *ms64, const int32_t *cand,
+                                 const int32_t *list0, const int32_t *list1,
+                                 const PaddiAttemptDev *att, int32_t last, uint8_t *pruned,
+                                 uint32_t *rho_max, const int32_t *frag,
+                                 const int32_t *frag_count, int32_t m, float thr, int32_t col_lo,
+                                 int32_t col_hi, int32_t num_sms, cudaStream_t st);
 
-// Tensor-core refine over windows [jb, je) (jb a multiple of the tile width,
-// je too or je = N).  bq / wdq: the per-length tile data of
-// paddi_launch_tile_prep.  wait_cycles: limit of every barrier wait (<= 0:
-// about 2 s); a wait that runs out sets att->status = 3 and the kernel
-// returns.  withhold != 0 is a test hook: the CTA holding work item 0 never
-// fills that item's first stage, so its waits run out.
+// Tensor-core refine of all att->n_cand_p1 candidates over the windows
+// [col_lo, col_hi) (col_lo a multiple of the tile width, col_hi too or N), all
+// rounds in one launch; list0 / list1: scratch, one entry per candidate each;
+// att->list_count[r] receives the candidates of round r > 0.  bq / wdq: the
+// per-length tile data of paddi_launch_tile_prep.  wait_cycles: limit of every
+// wait (<= 0: about 2 s); a wait that runs out sets att->status = 3 and the
+// kernel returns.  withhold != 0 is a test hook: the CTA holding work item 0
+// never fills that item's first stage, so its waits run out.
 cudaError_t paddi_launch_refine_umma(bool bf16, const float *x, const float4 *wst,
-                                     const float *mu, const int32_t *cand, const int32_t *list,
-                                     const int32_t *list_count, const uint16_t *bq,
-                                     const float4 *wdq, PaddiAttemptDev *att, int32_t *work,
-                                     uint32_t *rho_max, uint8_t *pruned, int32_t N, int32_t m,
-                                     int32_t jb, int32_t je,
+                                     const float *mu, const int32_t *cand, int32_t *list0,
+                                     int32_t *list1, const uint16_t *bq, const float4 *wdq,
+                                     PaddiAttemptDev *att, uint32_t *rho_max, uint8_t *pruned,
+                                     int32_t N, int32_t m, int32_t col_lo, int32_t col_hi,
                                      float thr_prune, int32_t num_sms, cudaStream_t st,
                                      long long wait_cycles = 0, int32_t withhold = 0,
-                                     int32_t round = 0, int32_t je_all = 0,
                                      bool rows64 = false, const PaddiWitness *W = nullptr);
 
 // Per-length tile data of the tensor-core refine: for every block of
