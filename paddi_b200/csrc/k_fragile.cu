@@ -29,6 +29,7 @@
 #include "paddi_internal.cuh"
 
 using paddi::f2ord;
+using paddi::ord2f;
 
 namespace {
 
@@ -42,7 +43,7 @@ k_fragile(const float *__restrict__ x, const double2 *__restrict__ ms64, const i
           const int32_t *__restrict__ list0, const int32_t *__restrict__ list1,
           const PaddiAttemptDev *__restrict__ att, int32_t last, uint8_t *pruned, uint32_t *rho_max, const int32_t *__restrict__ frag,
           const int32_t *__restrict__ frag_count, int32_t m, float thr, int32_t col_lo,
-          int32_t col_hi)
+          int32_t col_hi, PaddiBlockMax B, float guard)
 {
     // [FG_CAND][mp] centred candidate values, mp = m rounded up to even
     extern __shared__ __align__(16) double fg_a[];
@@ -55,6 +56,7 @@ k_fragile(const float *__restrict__ x, const double2 *__restrict__ ms64, const i
     const int32_t *list = rd & 1 ? list1 : list0;
     const int C = rd ? att->list_count[rd] : att->n_cand_p1, F = *frag_count;
     if (C <= 0 || F <= 0) return;
+    const bool bkeep = B.kept(att->n_cand_p1);
     const int mp = (m + 1) & ~1;
     const int groups = (C + FG_CAND - 1) / FG_CAND;
     const int chunks = (F + FG_THREADS - 1) / FG_THREADS;
@@ -118,7 +120,13 @@ k_fragile(const float *__restrict__ x, const double2 *__restrict__ ms64, const i
             for (int c = 0; c < FG_HALF; ++c) {
                 const int ci = c0 + c;
                 const int d = cw[ci] > f ? cw[ci] - f : f - cw[ci];
-                if (live[ci] && d >= m - 1) b[ci] = acc[c] * civ[ci] * ivf;
+                if (live[ci] && d >= m - 1) {
+                    b[ci] = acc[c] * civ[ci] * ivf;
+                    // may be the nearest neighbour: the recheck has to look here
+                    if (bkeep && b[ci] >= (double)ord2f(__ldcg(rho_max + cp[ci])) - 2.0 * guard)
+                        atomicMax(B.v + (int64_t)cp[ci] * B.halves + f / PADDI_HALF,
+                                  f2ord((float)b[ci]));
+                }
             }
         }
         // maxima over the item's windows, per candidate
@@ -150,7 +158,7 @@ cudaError_t paddi_launch_fragile(const float *x, const double2 *ms64,
                                  uint8_t *pruned, uint32_t *rho_max,
                                  const int32_t *frag, const int32_t *frag_count, int32_t m,
                                  float thr, int32_t col_lo, int32_t col_hi, int32_t num_sms,
-                                 cudaStream_t st)
+                                 cudaStream_t st, const PaddiBlockMax *B, float guard)
 {
     if (m > FG_MAXM || m < 3) return cudaErrorInvalidValue;
     const size_t smem = sizeof(double) * (size_t)FG_CAND * (size_t)((m + 1) & ~1);
@@ -158,6 +166,6 @@ cudaError_t paddi_launch_fragile(const float *x, const double2 *ms64,
     if (e != cudaSuccess) return e;
     k_fragile<<<num_sms * 4, FG_THREADS, smem, st>>>(x, ms64, cand, list0, list1, att, last,
                                                     pruned, rho_max, frag, frag_count, m, thr,
-                                                    col_lo, col_hi);
+                                                    col_lo, col_hi, B ? *B : PaddiBlockMax{}, guard);
     return cudaGetLastError();
 }

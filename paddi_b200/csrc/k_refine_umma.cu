@@ -498,7 +498,7 @@ k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
               int32_t *list1, const uint16_t *__restrict__ bq, const float4 *__restrict__ wdq,
               PaddiAttemptDev *att, uint32_t *rho_max, uint8_t *pruned, int32_t N, int32_t m,
               int32_t col_lo, int32_t col_hi, float thr, int32_t grid_ctas, long long wl,
-              int32_t withhold, PaddiWitness W)
+              int32_t withhold, PaddiWitness W, PaddiBlockMax B)
 {
     using X = E16<BF>;
     constexpr int UM_M = MM;
@@ -513,6 +513,7 @@ k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
 
     int C = att->n_cand_p1;
     if (C <= 0 || col_hi <= col_lo) return; // uniform, before any TMEM use
+    const bool bkeep = B.kept(C);
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < 2; ++s) {
@@ -591,7 +592,7 @@ k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
                 const int li = tile * UM_TC + threadIdx.x;
                 const bool v = li < C;
                 const int pos = !v ? 0 : rd ? __ldcg(list + li) : li;
-                const int w = v ? cand[pos] : 0;
+                const int w = v ? cand[pos] : -1; // -1: no candidate in this row
                 S.cw[threadIdx.x] = w;
                 S.cp[threadIdx.x] = pos;
                 S.dead[threadIdx.x] = !v || __ldcg(pruned + pos);
@@ -865,6 +866,15 @@ k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
                         float tmax = fmaxf(fmaxf(tm[0], tm[1]), fmaxf(tm[2], tm[3]));
                         if (!rowok) tmax = -INFINITY;
                         rmax = fmaxf(rmax, tmax + Gt); // the interval's middle (-inf stays)
+                        if (bkeep) { // the half block's maximum over the 8 shifts
+                            float bm = tmax + Gt;
+#pragma unroll
+                            for (int o = 4; o > 0; o >>= 1)
+                                bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, o));
+                            if (rowok && bsh == 0 && wc >= 0)
+                                B.v[(int64_t)S.cp[cidx] * B.halves + j0 / PADDI_HALF + hcol] =
+                                    f2ord(bm);
+                        }
                         const unsigned bal = __ballot_sync(0xffffffffu, tmax > thr);
                         bool hint = false;
                         if (lane < UM_TC / 4) {
@@ -954,10 +964,11 @@ k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
         }
         // ---- between rounds (one launch for all of them: separate launches with a
         // compaction kernel each cost 30 us an attempt, most of it for rounds
-        // without work; headline run 249 -> 229 ms).  The CTA that finished the round's last item compacts
-        // the survivors; the others wait for it.  A CTA waits only for items that
-        // other, running CTAs have taken (it found none left to take), so the wait
-        // ends whichever CTAs are resident; it is bounded all the same.
+        // without work; headline run 249 -> 229 ms).  The CTA that finished the
+        // round's last item compacts the survivors; the others wait for it.  A CTA
+        // waits only for items that other, running CTAs have taken (it found none
+        // left to take), so the wait ends whichever CTAs are resident; it is bounded
+        // all the same.
         if (S.last) {
             __threadfence();
             const int nx = um_compact(list, rd == 0, C, pruned, rd & 1 ? list0 : list1, S.wsum);
@@ -1088,7 +1099,7 @@ cudaError_t paddi_launch_refine_umma(bool bf16, const float *x, const float4 *ws
                                      int32_t N, int32_t m, int32_t col_lo, int32_t col_hi,
                                      float thr_prune, int32_t num_sms, cudaStream_t st,
                                      long long wait_cycles, int32_t withhold, bool rows64,
-                                     const PaddiWitness *W)
+                                     const PaddiWitness *W, const PaddiBlockMax *B)
 {
     const int kp = kpad_of(m);
     if (kp > UM_KMAX64 || m < 3) return cudaErrorInvalidValue;
@@ -1100,7 +1111,7 @@ cudaError_t paddi_launch_refine_umma(bool bf16, const float *x, const float4 *ws
     void (*kern)(const float *, const float4 *, const float *, const int32_t *, int32_t *,
                  int32_t *, const uint16_t *, const float4 *, PaddiAttemptDev *, uint32_t *,
                  uint8_t *, int32_t, int32_t, int32_t, int32_t, float, int32_t, long long, int32_t,
-                 PaddiWitness);
+                 PaddiWitness, PaddiBlockMax);
     if (MM == 128) kern = bf16 ? k_refine_umma<true, 128> : k_refine_umma<false, 128>;
     else kern = bf16 ? k_refine_umma<true, 64> : k_refine_umma<false, 64>;
     cudaError_t e = paddi_raise_smem_limit((const void *)kern, smem);
@@ -1109,6 +1120,6 @@ cudaError_t paddi_launch_refine_umma(bool bf16, const float *x, const float4 *ws
     kern<<<grid, UM_THREADS, smem, st>>>(x, wst, mu, cand, list0, list1, bq, wdq, att, rho_max,
                                          pruned, N, m, col_lo, col_hi, thr_prune, grid,
                                          wait_cycles > 0 ? wait_cycles : 4000000000ll, withhold,
-                                         W ? *W : PaddiWitness{});
+                                         W ? *W : PaddiWitness{}, B ? *B : PaddiBlockMax{});
     return cudaGetLastError();
 }

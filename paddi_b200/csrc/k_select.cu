@@ -340,15 +340,23 @@ k_finalize(const int32_t *__restrict__ cand, PaddiAttemptDev *att,
 // consecutive neighbour windows and slides a register ring over the slice
 // (per step: one shared load of the slice, one broadcast of the candidate,
 // RC_JPT FP64 FMAs).
+// With the refine's block maxima only half blocks whose kept maximum is within
+// 2 guard of the candidate's are scanned: a kept correlation is within guard of
+// the exact one, so the nearest neighbour's is at least (maximum - 2 guard).  A
+// queued window then costs a few half blocks instead of the whole series (which
+// is bound by FP64 issue: 34 us at n = 2^21, m = 300).  Headline run: 71 -> 15 us
+// per recheck, 32 -> 6.7 ms of 228.
 constexpr int RC_JPT = 8;                    // neighbour windows per thread
 constexpr int RC_SPAN = RC_THREADS * RC_JPT; // neighbour windows per block
+static_assert(RC_SPAN == 2 * PADDI_HALF, "two half blocks per block");
 
 __device__ __forceinline__ int rpad(int d) { return d + (d >> 4); } // conflict-free at stride 8
 
 __global__ void __launch_bounds__(RC_THREADS)
 k_recheck(const float *__restrict__ x, const double2 *__restrict__ ms64, const uint8_t *__restrict__ flat, int32_t N,
           int32_t m, const int32_t *__restrict__ cand, const int32_t *__restrict__ recheck,
-          PaddiAttemptDev *att, unsigned long long *nn64_ord, int32_t known_w)
+          PaddiAttemptDev *att, unsigned long long *nn64_ord, int32_t known_w,
+          const uint32_t *__restrict__ rho_max, PaddiBlockMax B, float guard)
 {
     __shared__ double a[RC_MAXM];
     __shared__ double xs[RC_SPAN + RC_MAXM + (RC_SPAN + RC_MAXM) / 16 + 16];
@@ -362,6 +370,7 @@ k_recheck(const float *__restrict__ x, const double2 *__restrict__ ms64, const u
     const int ipc = (nblk + per - 1) / per;                        // items per queued window
     const long long total = (long long)nr * ipc;
     const int t = threadIdx.x;
+    const bool bkeep = B.kept(att->n_cand_p1);
     for (;;) {
         if (t == 0) s_item = atomicAdd(&att->recheck_next, 1);
         __syncthreads();
@@ -371,6 +380,18 @@ k_recheck(const float *__restrict__ x, const double2 *__restrict__ ms64, const u
         const int r = item % nr, sp = item / nr;
         const int w = cand[recheck[r]];
         if (w == known_w) continue; // exact value filled in by the finalize step
+        const int j_lo = sp * per * RC_SPAN;
+        const int j_hi = (int)min((long long)N, (long long)j_lo + (long long)per * RC_SPAN);
+        // half blocks of the item that can hold the nearest neighbour
+        const uint32_t *bm = B.v + (int64_t)recheck[r] * B.halves;
+        const float need = bkeep ? ord2f(rho_max[recheck[r]]) - 2.f * guard - 1e-6f : 0.f;
+        const int h_hi = (j_hi + PADDI_HALF - 1) / PADDI_HALF;
+        if (bkeep) {
+            bool any = false;
+            for (int h = j_lo / PADDI_HALF + t; h < h_hi; h += RC_THREADS)
+                any |= ord2f(bm[h]) >= need;
+            if (!__syncthreads_or(any)) continue;
+        }
         const double mw = ms64[w].x, iw = ms64[w].y;
         const int fw = flat[w];
         double asum = 0.0;
@@ -386,9 +407,15 @@ k_recheck(const float *__restrict__ x, const double2 *__restrict__ ms64, const u
         asum = 0.0;
         for (int q = 0; q < RC_THREADS / 32; ++q) asum += reda[q];
         double best = INFINITY;
-        const int j_lo = sp * per * RC_SPAN;
-        const int j_hi = (int)min((long long)N, (long long)j_lo + (long long)per * RC_SPAN);
         for (int j0 = j_lo; j0 < j_hi; j0 += RC_SPAN) {
+            bool mine = true; // this thread's half is to be scanned
+            if (bkeep) {
+                const int h = j0 / PADDI_HALF;
+                const bool a = ord2f(bm[h]) >= need;
+                const bool b = h + 1 < h_hi && ord2f(bm[h + 1]) >= need;
+                if (!a && !b) continue;
+                mine = RC_JPT * t < PADDI_HALF ? a : b;
+            }
             __syncthreads();
             const double sh = (double)x[j0];
             for (int p = t; p < RC_SPAN + m + RC_JPT; p += RC_THREADS) {
@@ -396,6 +423,7 @@ k_recheck(const float *__restrict__ x, const double2 *__restrict__ ms64, const u
                 xs[rpad(p)] = (g < N + m - 1 ? (double)x[g] : sh) - sh;
             }
             __syncthreads();
+            if (!mine) continue;
             const int q0 = RC_JPT * t;
             double acc[RC_JPT], ring[RC_JPT];
 #pragma unroll
@@ -618,11 +646,13 @@ cudaError_t paddi_launch_recheck(const float *x, const double2 *ms64,
                                  const uint8_t *flat, int32_t N, int32_t m,
                                  const int32_t *cand, const int32_t *recheck,
                                  PaddiAttemptDev *att, unsigned long long *nn64_ord,
-                                 int32_t num_sms, int32_t known_w, cudaStream_t st)
+                                 int32_t num_sms, int32_t known_w, cudaStream_t st,
+                                 const uint32_t *rho_max, const PaddiBlockMax *B, float guard)
 {
     if (m > RC_MAXM) return cudaErrorInvalidValue;
     k_recheck<<<num_sms * 4, RC_THREADS, 0, st>>>(x, ms64, flat, N, m, cand, recheck, att,
-                                                 nn64_ord, known_w);
+                                                 nn64_ord, known_w, rho_max,
+                                                 B ? *B : PaddiBlockMax{}, guard);
     return cudaGetLastError();
 }
 

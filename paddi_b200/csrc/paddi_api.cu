@@ -78,6 +78,8 @@ struct paddi_ctx {
     int32_t *d_pc = nullptr;  // range-discord profile output (allocated on first use)
     float *d_pn = nullptr;
     uint16_t *d_bq = nullptr; // tensor-core refine: split series slices per tile block
+    uint32_t *d_bmax = nullptr; // tensor-core refine: block maxima (bmax_cap entries)
+    int64_t bmax_cap = 0;
     float4 *d_wdq = nullptr;  // tensor-core refine: epilogue window data per tile block
     // r guidance: exact FP64 nn of the bound window, kept incrementally
     PaddiGuide *d_guide = nullptr, *h_guide = nullptr; // state + result (h: pinned)
@@ -184,6 +186,7 @@ void free_buffers(paddi_ctx *ctx)
     dfree(ctx->d_frag);
     dfree(ctx->d_bq);
     dfree(ctx->d_wdq);
+    dfree(ctx->d_bmax);
     dfree(ctx->d_pc);
     dfree(ctx->d_pn);
     dfree(ctx->d_G);
@@ -216,6 +219,10 @@ paddi_status ensure_capacity(paddi_ctx *ctx, size_t n)
     if (ctx->umma_ok) {
         const int64_t blocks = paddi_tile_blocks((int64_t)n);
         CK(dmalloc(ctx, &ctx->d_bq, sizeof(uint16_t) * (size_t)(blocks * paddi_tile_block_elems_max())));
+        // a row of block maxima for 2048 candidates of a long series, and for every
+        // candidate of a short one that an attempt commonly leaves
+        ctx->bmax_cap = std::max<int64_t>(2 * (int64_t)W, 1 << 23);
+        CK(dmalloc(ctx, &ctx->d_bmax, sizeof(uint32_t) * (size_t)ctx->bmax_cap));
         CK(dmalloc(ctx, &ctx->d_wdq, sizeof(float4) * (size_t)(blocks * paddi_tile_wd_entries())));
     }
     CK(dmalloc(ctx, &ctx->d_recheck, sizeof(int32_t) * PADDI_MAX_RECHECK));
@@ -332,6 +339,19 @@ int32_t wit_enough(int32_t N) { return std::max(1024, N / 512); }
 // The correlation threshold of r^2 at length m: d < r^2 <=> rho > thr.
 float thr_of(float r2, int m) { return (float)(1.0 - (double)r2 / (2.0 * (double)m)); }
 
+// The refine's block maxima for N windows, or none: the FP32 refine keeps none,
+// nor does a refine of a part of the windows.
+PaddiBlockMax block_max(const paddi_ctx *ctx, int kernel, int32_t N, bool whole)
+{
+    PaddiBlockMax B = {};
+    if (kernel != PADDI_DIST_FP32 && whole) {
+        B.v = ctx->d_bmax;
+        B.cap = ctx->bmax_cap;
+        B.halves = 2 * (int32_t)paddi_tile_blocks(N);
+    }
+    return B;
+}
+
 // Refine of the compacted candidates against the windows [col_lo, col_hi)
 // (col_lo on the refine's grid), then the FP64 pass over the fragile windows of
 // that range.  It runs in rounds over growing window ranges (1/16, 1/4, 1/2,
@@ -343,6 +363,7 @@ paddi_status refine_rounds(paddi_ctx *ctx, const float *x, int32_t N, int m, int
 {
     cudaStream_t st = ctx->st;
     const PaddiWitness *W = ctx->wit_m == m ? &ctx->W : nullptr;
+    const PaddiBlockMax B = block_max(ctx, kernel, N, col_lo == 0 && col_hi == N);
     int last = -1; // round whose list holds the survivors (-1: the kernel recorded it)
     ctx->n_rev = 1;
     if (kernel != PADDI_DIST_FP32) {
@@ -351,7 +372,7 @@ paddi_status refine_rounds(paddi_ctx *ctx, const float *x, int32_t N, int m, int
                                     ctx->d_cand, ctx->d_list[0], ctx->d_list[1], ctx->d_bq,
                                     ctx->d_wdq, ctx->d_att, ctx->d_rho, ctx->d_pruned, N, m,
                                     col_lo, col_hi, thr, ctx->num_sms, st, ctx->wait_cycles,
-                                    ctx->withhold, ctx->opts.tile_rows == 64, W));
+                                    ctx->withhold, ctx->opts.tile_rows == 64, W, &B));
         CK(cudaEventRecord(ctx->rev[1], st));
         ++*launches;
     } else {
@@ -396,7 +417,8 @@ paddi_status refine_rounds(paddi_ctx *ctx, const float *x, int32_t N, int m, int
     if (ctx->trace) CK(cudaEventRecord(ctx->tev, st));
     CK(paddi_launch_fragile(x, ctx->d_ms64, ctx->d_cand, ctx->d_list[0], ctx->d_list[1],
                             ctx->d_att, last, ctx->d_pruned, ctx->d_rho, ctx->d_frag,
-                            ctx->d_flatcount + 3, m, thr, col_lo, col_hi, ctx->num_sms, st));
+                            ctx->d_flatcount + 3, m, thr, col_lo, col_hi, ctx->num_sms, st, &B,
+                            guard));
     *launches += 1;
     return PADDI_OK;
 }
@@ -407,7 +429,7 @@ paddi_status refine_rounds(paddi_ctx *ctx, const float *x, int32_t N, int m, int
 // next_guided, the bound) of length next_m are queued behind the first pass,
 // before its result is synced; *spec tells whether they were.
 paddi_status select_passes(paddi_ctx *ctx, const float *x, size_t n, int m, float r2,
-                           float guard, int top_k, int32_t known_w, unsigned long long known_ord,
+                           float guard, const PaddiBlockMax &B, int top_k, int32_t known_w, unsigned long long known_ord,
                            int next_m, bool next_guided, bool *spec, int *launches)
 {
     const int32_t N = (int32_t)(n - m + 1);
@@ -421,7 +443,7 @@ paddi_status select_passes(paddi_ctx *ctx, const float *x, size_t n, int m, floa
                                  ctx->d_rcslot, ctx->d_nn64, ctx->d_res, known_w, known_ord, st));
         CK(paddi_launch_recheck(x, ctx->d_ms64, ctx->d_flat, N, m, ctx->d_cand,
                                 ctx->d_recheck, ctx->d_att, ctx->d_nn64, ctx->num_sms, known_w,
-                                st));
+                                st, ctx->d_rho, &B, guard));
         CK(paddi_launch_select(ctx->d_cand, ctx->d_att, ctx->d_rho, ctx->d_pruned,
                                ctx->d_recheck, ctx->d_rcslot, ctx->d_nn64, m, r2, thr, guard,
                                top_k, ctx->d_flat, ctx->d_res, st));
@@ -523,7 +545,7 @@ paddi_status run_attempt(paddi_ctx *ctx, const float *x, size_t n, int m, float 
         CK(cudaMemcpyAsync(ctx->h_trace, ctx->d_att, sizeof(PaddiAttemptDev),
                            cudaMemcpyDeviceToHost, st));
     bool spec = false;
-    s = select_passes(ctx, x, n, m, r2, guard, top_k, known_w, known_ord, next_m, next_guided,
+    s = select_passes(ctx, x, n, m, r2, guard, block_max(ctx, kernel, N, true), top_k, known_w, known_ord, next_m, next_guided,
                       &spec, &launches);
     if (s != PADDI_OK) return s;
     out->res = *ctx->h_res;
@@ -1358,7 +1380,7 @@ PADDI_API paddi_status paddi_shard_select(paddi_ctx *ctx, const float *d_series,
     CK(cudaEventRecord(ctx->ev[2], st));
     int launches = 0;
     bool spec = false;
-    paddi_status s = select_passes(ctx, d_series, n, (int)m, r2, guard_of(ctx, kernel),
+    paddi_status s = select_passes(ctx, d_series, n, (int)m, r2, guard_of(ctx, kernel), {},
                                    (int)top_k, -1, 0, 0, false, &spec, &launches);
     if (s != PADDI_OK) return s;
     AttemptOut a;

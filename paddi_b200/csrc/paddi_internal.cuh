@@ -131,6 +131,23 @@ struct PaddiGuide {
     int32_t done, item;        // kernel counters (zero between launches)
 };
 
+// Block maxima of the tensor-core refine: for candidate c and half block h
+// (windows [1024 h, 1024 h + 1024)) the largest kept correlation, as an ordered
+// image, at v[c * halves + h].  Kept while all candidates of the attempt fit
+// (every unpruned candidate meets every block exactly once, so no entry needs
+// clearing); the FP64 recheck then scans only half blocks that can hold a
+// candidate's nearest neighbour.
+struct PaddiBlockMax {
+    uint32_t *v;
+    int64_t cap; // entries
+    int32_t halves;
+    __device__ __forceinline__ bool kept(int C) const
+    {
+        return v != nullptr && (int64_t)C * halves <= cap;
+    }
+};
+#define PADDI_HALF 1024
+
 // Witnesses of a PALMAD run (k_witness.cu): per window a known neighbour
 // wit[i] (-1: none; WT_HINT: wc[i] holds a code for partners to evaluate), the
 // pair's centred dot product wc[i] at the run's current length, and a lower
@@ -237,7 +254,8 @@ cudaError_t paddi_launch_fragile(const float *x, const double2 *ms64, const int3
                                  const PaddiAttemptDev *att, int32_t last, uint8_t *pruned,
                                  uint32_t *rho_max, const int32_t *frag,
                                  const int32_t *frag_count, int32_t m, float thr, int32_t col_lo,
-                                 int32_t col_hi, int32_t num_sms, cudaStream_t st);
+                                 int32_t col_hi, int32_t num_sms, cudaStream_t st,
+                                 const PaddiBlockMax *B = nullptr, float guard = 0.f);
 
 // Tensor-core refine of all att->n_cand_p1 candidates over the windows
 // [col_lo, col_hi) (col_lo a multiple of the tile width, col_hi too or N), all
@@ -254,7 +272,8 @@ cudaError_t paddi_launch_refine_umma(bool bf16, const float *x, const float4 *ws
                                      int32_t N, int32_t m, int32_t col_lo, int32_t col_hi,
                                      float thr_prune, int32_t num_sms, cudaStream_t st,
                                      long long wait_cycles = 0, int32_t withhold = 0,
-                                     bool rows64 = false, const PaddiWitness *W = nullptr);
+                                     bool rows64 = false, const PaddiWitness *W = nullptr,
+                                     const PaddiBlockMax *B = nullptr);
 
 // Per-length tile data of the tensor-core refine: for every block of
 // paddi_tile_width() windows, the split 16-bit series slice (bq, at most
@@ -290,7 +309,8 @@ cudaError_t paddi_launch_recheck(const float *x, const double2 *ms64,
                                  const uint8_t *flat, int32_t N, int32_t m,
                                  const int32_t *cand, const int32_t *recheck,
                                  PaddiAttemptDev *att, unsigned long long *nn64_ord,
-                                 int32_t num_sms, int32_t known_w, cudaStream_t st);
+                                 int32_t num_sms, int32_t known_w, cudaStream_t st,
+                                 const uint32_t *rho_max, const PaddiBlockMax *B, float guard);
 
 cudaError_t paddi_launch_select(const int32_t *cand, PaddiAttemptDev *att,
                                 const uint32_t *rho_max, const uint8_t *pruned,
