@@ -39,9 +39,11 @@ constexpr int FG_HALF = 4;      // accumulators per thread
 constexpr int FG_MAXM = 1024;
 
 __global__ void __launch_bounds__(FG_THREADS)
-k_fragile(const float *__restrict__ x, const double2 *__restrict__ ms64, const int32_t *__restrict__ cand,
+k_fragile(const float *__restrict__ x, const double2 *__restrict__ ms64,
+          const int32_t *__restrict__ cand,
           const int32_t *__restrict__ list0, const int32_t *__restrict__ list1,
-          const PaddiAttemptDev *__restrict__ att, int32_t last, uint8_t *pruned, uint32_t *rho_max, const int32_t *__restrict__ frag,
+          const PaddiAttemptDev *__restrict__ att, uint8_t *pruned, uint32_t *rho_max,
+          const int32_t *__restrict__ frag,
           const int32_t *__restrict__ frag_count, int32_t m, float thr, int32_t col_lo,
           int32_t col_hi, PaddiBlockMax B, float guard)
 {
@@ -52,7 +54,7 @@ k_fragile(const float *__restrict__ x, const double2 *__restrict__ ms64, const i
     __shared__ double best_s[FG_CAND][FG_THREADS / 32];
     __shared__ int s_any;
     // the candidates of the refine's last round (round 0: all of them)
-    const int rd = last >= 0 ? last : att->last_rd;
+    const int rd = att->last_rd;
     const int32_t *list = rd & 1 ? list1 : list0;
     const int C = rd ? att->list_count[rd] : att->n_cand_p1, F = *frag_count;
     if (C <= 0 || F <= 0) return;
@@ -154,7 +156,7 @@ k_fragile(const float *__restrict__ x, const double2 *__restrict__ ms64, const i
 
 cudaError_t paddi_launch_fragile(const float *x, const double2 *ms64,
                                  const int32_t *cand, const int32_t *list0,
-                                 const int32_t *list1, const PaddiAttemptDev *att, int32_t last,
+                                 const int32_t *list1, const PaddiAttemptDev *att,
                                  uint8_t *pruned, uint32_t *rho_max,
                                  const int32_t *frag, const int32_t *frag_count, int32_t m,
                                  float thr, int32_t col_lo, int32_t col_hi, int32_t num_sms,
@@ -164,7 +166,7 @@ cudaError_t paddi_launch_fragile(const float *x, const double2 *ms64,
     const size_t smem = sizeof(double) * (size_t)FG_CAND * (size_t)((m + 1) & ~1);
     cudaError_t e = paddi_raise_smem_limit((const void *)k_fragile, smem);
     if (e != cudaSuccess) return e;
-    k_fragile<<<num_sms * 4, FG_THREADS, smem, st>>>(x, ms64, cand, list0, list1, att, last,
+    k_fragile<<<num_sms * 4, FG_THREADS, smem, st>>>(x, ms64, cand, list0, list1, att,
                                                     pruned, rho_max, frag, frag_count, m, thr,
                                                     col_lo, col_hi, B ? *B : PaddiBlockMax{}, guard);
     return cudaGetLastError();

@@ -54,6 +54,7 @@
 
 #include "paddi_internal.cuh"
 
+using paddi::compact_survivors;
 using paddi::f2ord;
 
 namespace {
@@ -62,8 +63,6 @@ constexpr int UM_THREADS = 384;  // 12 warps
 constexpr int UM_TCMAX = 16;     // candidates per tile (M = 128); 8 for M = 64
 constexpr int UM_N = 256;        // windows at stride 8
 constexpr int UM_TW = UM_N * 8;  // windows per tile (one block of the grid)
-constexpr int UM_ROUNDS = 4;     // window ranges refined before and after compactions
-constexpr int UM_MIN_ROUNDS = 1 << 16; // windows from which on rounds pay
 constexpr int UM_WAVES = 1;      // work items per CTA and round when candidate tiles are few
 constexpr int UM_KMAX128 = 368;  // largest K' with M = 128 (shared-memory bound)
 constexpr int UM_KMAX64 = 736;   // largest K' with M = 64
@@ -432,62 +431,6 @@ struct UmPhases {
 
 __device__ __forceinline__ uint32_t par(uint32_t idx) { return idx & 1u; }
 
-__device__ __forceinline__ int32_t ld_acquire(const int32_t *p)
-{
-    int32_t v;
-    asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ void st_release(int32_t *p, int32_t v)
-{
-    asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
-// Unpruned entries of in[0..C) (or of 0..C-1) to out, in order, by one CTA;
-// returns their number.  8 entries per thread and step: the survivors are a few
-// thousand at most, and 32k entries take about 15 us.
-__device__ int um_compact(const int32_t *in, bool identity, int C, const uint8_t *pruned,
-                          int32_t *out, int *wsum)
-{
-    constexpr int PER = 8;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int base = 0;
-    for (int b0 = 0; b0 < C; b0 += UM_THREADS * PER) {
-        const int i0 = b0 + threadIdx.x * PER;
-        int e[PER];
-        unsigned keep = 0;
-#pragma unroll
-        for (int q = 0; q < PER; ++q) e[q] = i0 + q < C ? (identity ? i0 + q : __ldcg(in + i0 + q)) : -1;
-#pragma unroll
-        for (int q = 0; q < PER; ++q)
-            if (e[q] >= 0 && !__ldcg(pruned + e[q])) keep |= 1u << q;
-        const int cnt = __popc(keep);
-        int inc = cnt;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int t = __shfl_up_sync(0xffffffffu, inc, o);
-            if (lane >= o) inc += t;
-        }
-        __syncthreads(); // wsum of the step before is consumed
-        if (lane == 31) wsum[warp] = inc;
-        __syncthreads();
-        int off = base, all = 0;
-#pragma unroll
-        for (int w = 0; w < UM_THREADS / 32; ++w) {
-            const int v = wsum[w];
-            if (w < warp) off += v;
-            all += v;
-        }
-        int pos = off + inc - cnt;
-#pragma unroll
-        for (int q = 0; q < PER; ++q)
-            if ((keep >> q) & 1u) out[pos++] = e[q];
-        base += all;
-    }
-    __threadfence();
-    return base;
-}
-
 // MM = 128: 16 candidates, accumulator row r in TMEM lane r.
 // MM = 64:  8 candidates, accumulator row r in TMEM lane (r % 16) + 32 (r / 16)
 //           (lanes 16..31 of every subpartition stay unused).
@@ -556,11 +499,10 @@ k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
     // ---- rounds: the windows [jb, je) of growing ranges (1/16, 1/4, 1/2, all of
     // them), the survivors compacted in between so that every tile is dense.  A
     // round with one tile left takes every remaining window.
-    const int nrounds = col_hi - col_lo >= UM_MIN_ROUNDS ? UM_ROUNDS : 1;
+    const int nrounds = paddi::refine_rounds(col_hi - col_lo);
     int jb = col_lo;
     for (int rd = 0; rd < nrounds; ++rd) {
-        int je = rd == nrounds - 1 ? col_hi
-                                   : col_lo + ((col_hi - col_lo) >> (rd ? 3 - rd : 4)) / UM_TW * UM_TW;
+        int je = paddi::refine_round_end(rd, nrounds, col_lo, col_hi, UM_TW);
         if (C <= UM_TC) je = col_hi;
         int32_t *list = rd & 1 ? list1 : list0; // entries of this round (round 0: all candidates)
         const int range = je - jb;
@@ -971,29 +913,16 @@ k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
         // all the same.
         if (S.last) {
             __threadfence();
-            const int nx = um_compact(list, rd == 0, C, pruned, rd & 1 ? list0 : list1, S.wsum);
+            const int nx = compact_survivors<UM_THREADS>(list, rd == 0, C, pruned,
+                                                          rd & 1 ? list0 : list1, S.wsum);
             __syncthreads();
             if (threadIdx.x == 0) {
                 S.last = 0;
                 S.next = nx;
-                att->list_count[rd + 1] = nx;
-                if (nx == 0) att->last_rd = rd + 1;
-                __threadfence();
-                st_release(&att->round_ready, rd + 1);
+                paddi::publish_round(att, rd, nx);
             }
         } else if (threadIdx.x == 0) {
-            const long long t0 = clock64();
-            S.next = 0;
-            while (ld_acquire(&att->round_ready) <= rd) {
-                if (ld_acquire(&att->status) == 3) S.next = -1; // another CTA gave up
-                else if (clock64() - t0 > wl) {
-                    atomicExch(&att->status, 3);
-                    S.next = -1;
-                }
-                if (S.next < 0) break;
-                __nanosleep(100);
-            }
-            if (S.next == 0) S.next = __ldcg(&att->list_count[rd + 1]);
+            S.next = paddi::wait_round(att, rd, wl);
         }
         __syncthreads();
         C = S.next;

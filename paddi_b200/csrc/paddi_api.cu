@@ -57,8 +57,7 @@ struct paddi_ctx {
     int num_sms = 0;
     cudaStream_t st = nullptr;
     cudaEvent_t ev[8] = {};
-    cudaEvent_t rev[8] = {}; // around each refine launch
-    int n_rev = 0;           // pairs of them used by the current attempt
+    cudaEvent_t rev[2] = {}; // around the refine launch
     // PADDI_TRACE=1 in the environment: one stderr line per attempt with the
     // candidates entering every refine round
     bool trace = false;
@@ -219,9 +218,10 @@ paddi_status ensure_capacity(paddi_ctx *ctx, size_t n)
     if (ctx->umma_ok) {
         const int64_t blocks = paddi_tile_blocks((int64_t)n);
         CK(dmalloc(ctx, &ctx->d_bq, sizeof(uint16_t) * (size_t)(blocks * paddi_tile_block_elems_max())));
-        // a row of block maxima for 2048 candidates of a long series, and for every
-        // candidate of a short one that an attempt commonly leaves
-        ctx->bmax_cap = std::max<int64_t>(2 * (int64_t)W, 1 << 23);
+        // a row of block maxima for 2048 candidates of a long series, and for all
+        // that an attempt commonly leaves of a short one
+        ctx->bmax_cap = std::min<int64_t>((int64_t)n * 2 * blocks,
+                                          std::max<int64_t>(2 * (int64_t)W, 1 << 21));
         CK(dmalloc(ctx, &ctx->d_bmax, sizeof(uint32_t) * (size_t)ctx->bmax_cap));
         CK(dmalloc(ctx, &ctx->d_wdq, sizeof(float4) * (size_t)(blocks * paddi_tile_wd_entries())));
     }
@@ -356,67 +356,33 @@ PaddiBlockMax block_max(const paddi_ctx *ctx, int kernel, int32_t N, bool whole)
 // (col_lo on the refine's grid), then the FP64 pass over the fragile windows of
 // that range.  It runs in rounds over growing window ranges (1/16, 1/4, 1/2,
 // all of the range; a sweep of 4 to 8 rounds picked 4); survivors are
-// re-compacted between rounds so every tile is dense with live candidates.  The
-// tensor-core refine does all of them in one launch.
+// re-compacted between rounds so every tile is dense with live candidates.
 paddi_status refine_rounds(paddi_ctx *ctx, const float *x, int32_t N, int m, int kernel,
                            float thr, float guard, int32_t col_lo, int32_t col_hi, int *launches)
 {
     cudaStream_t st = ctx->st;
     const PaddiWitness *W = ctx->wit_m == m ? &ctx->W : nullptr;
     const PaddiBlockMax B = block_max(ctx, kernel, N, col_lo == 0 && col_hi == N);
-    int last = -1; // round whose list holds the survivors (-1: the kernel recorded it)
-    ctx->n_rev = 1;
-    if (kernel != PADDI_DIST_FP32) {
-        CK(cudaEventRecord(ctx->rev[0], st));
+    CK(cudaEventRecord(ctx->rev[0], st));
+    if (kernel != PADDI_DIST_FP32)
         CK(paddi_launch_refine_umma(kernel == PADDI_DIST_SPLIT_BF16, x, ctx->d_wst, ctx->d_mu,
                                     ctx->d_cand, ctx->d_list[0], ctx->d_list[1], ctx->d_bq,
                                     ctx->d_wdq, ctx->d_att, ctx->d_rho, ctx->d_pruned, N, m,
                                     col_lo, col_hi, thr, ctx->num_sms, st, ctx->wait_cycles,
                                     ctx->withhold, ctx->opts.tile_rows == 64, W, &B));
-        CK(cudaEventRecord(ctx->rev[1], st));
-        ++*launches;
-    } else {
-        CK(paddi_launch_list_init(ctx->d_att, ctx->d_list[0], &ctx->d_att->list_count[0], st));
-        ++*launches;
-        constexpr int kShifts[3] = {4, 2, 1};
-        const int32_t range = col_hi - col_lo;
-        const int nrounds = range >= (1 << 16) ? 4 : 1;
-        int jb = col_lo;
-        for (int rd = 0; rd < nrounds; ++rd) {
-            // round edges on the grid of 256-window chunks, so the fragile set
-            // depends only on the length
-            int je = rd == nrounds - 1 ? col_hi
-                                       : col_lo + (int)((int64_t)range >> kShifts[rd]) / 256 * 256;
-            if (je > col_hi) je = col_hi;
-            if (je < jb) je = jb;
-            // round rd: list d_list[rd & 1] of list_count[rd] entries, work counter
-            // work_rd[rd]; the compaction after it writes list_count[rd + 1].  All
-            // are zero from the attempt's reset, so no launch clears them.
-            const int a = rd & 1, b = a ^ 1;
-            int32_t *cnt = &ctx->d_att->list_count[rd];
-            CK(cudaEventRecord(ctx->rev[2 * rd], st));
-            CK(paddi_launch_refine_fp32(x, ctx->d_wst, ctx->d_mu, ctx->d_cand, ctx->d_list[a],
-                                        cnt, ctx->d_att, &ctx->d_att->work_rd[rd], ctx->d_rho,
-                                        ctx->d_pruned, N, m, jb, je, thr, guard, ctx->num_sms,
-                                        st, W));
-            CK(cudaEventRecord(ctx->rev[2 * rd + 1], st));
-            ++*launches;
-            if (rd + 1 < nrounds) {
-                CK(paddi_launch_list_compact(ctx->d_list[a], cnt, ctx->d_pruned, ctx->d_list[b],
-                                             cnt + 1, st));
-                ++*launches;
-            }
-            jb = je;
-        }
-        ctx->n_rev = nrounds;
-        last = nrounds - 1;
-    }
+    else
+        CK(paddi_launch_refine_fp32(x, ctx->d_wst, ctx->d_mu, ctx->d_cand, ctx->d_list[0],
+                                    ctx->d_list[1], ctx->d_att, ctx->d_rho, ctx->d_pruned, N, m,
+                                    col_lo, col_hi, thr, guard, ctx->num_sms, st,
+                                    ctx->wait_cycles, W));
+    CK(cudaEventRecord(ctx->rev[1], st));
+    ++*launches;
     // the fragile windows (skipped by the refine: their rounding bound exceeds
     // the guard band) against the candidates of the last round's list that are
     // still unpruned, in FP64 (the kernel returns at once when there are none)
     if (ctx->trace) CK(cudaEventRecord(ctx->tev, st));
     CK(paddi_launch_fragile(x, ctx->d_ms64, ctx->d_cand, ctx->d_list[0], ctx->d_list[1],
-                            ctx->d_att, last, ctx->d_pruned, ctx->d_rho, ctx->d_frag,
+                            ctx->d_att, ctx->d_pruned, ctx->d_rho, ctx->d_frag,
                             ctx->d_flatcount + 3, m, thr, col_lo, col_hi, ctx->num_sms, st, &B,
                             guard));
     *launches += 1;
@@ -553,12 +519,7 @@ paddi_status run_attempt(paddi_ctx *ctx, const float *x, size_t n, int m, float 
     if (spec_out) *spec_out = spec;
     CK(cudaEventElapsedTime(&out->ms_phase1, ctx->ev[0], ctx->ev[1]));
     CK(cudaEventElapsedTime(&out->ms_refine, ctx->ev[1], ctx->ev[2]));
-    out->ms_refine_kernel = 0.f;
-    for (int rd = 0; rd < ctx->n_rev; ++rd) {
-        float ms = 0.f;
-        CK(cudaEventElapsedTime(&ms, ctx->rev[2 * rd], ctx->rev[2 * rd + 1]));
-        out->ms_refine_kernel += ms;
-    }
+    CK(cudaEventElapsedTime(&out->ms_refine_kernel, ctx->rev[0], ctx->rev[1]));
     CK(cudaEventElapsedTime(&out->ms_select, ctx->ev[2], ctx->ev[3]));
     CK(cudaEventElapsedTime(&out->ms_total, ctx->ev[0], ctx->ev[3]));
     if (ctx->trace) {

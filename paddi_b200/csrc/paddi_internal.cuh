@@ -101,6 +101,102 @@ struct PaddiAttemptDev {
     unsigned long long n_live;  // of those, pairs of candidates still unpruned at the tile's start
 };
 
+namespace paddi {
+
+// ---- rounds of a refine launch: the windows in growing ranges (1/16, 1/4,
+// 1/2, all of them), the survivors compacted in between.
+__host__ __device__ __forceinline__ int refine_rounds(int range) { return range >= (1 << 16) ? 4 : 1; }
+// last window + 1 of round rd, on a grid of `tw` windows
+__host__ __device__ __forceinline__ int refine_round_end(int rd, int rounds, int lo, int hi, int tw)
+{
+    return rd == rounds - 1 ? hi : lo + ((hi - lo) >> (rd ? 3 - rd : 4)) / tw * tw;
+}
+
+__device__ __forceinline__ int32_t ld_acquire(const int32_t *p)
+{
+    int32_t v;
+    asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_release(int32_t *p, int32_t v)
+{
+    asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
+// Unpruned entries of in[0..C) (or of 0..C-1) to out, in order, by one CTA;
+// returns their number.  8 entries per thread and step: the survivors are a few
+// thousand at most, and 32k entries take about 15 us.
+template <int NT>
+__device__ int compact_survivors(const int32_t *in, bool identity, int C, const uint8_t *pruned,
+                          int32_t *out, int *wsum)
+{
+    constexpr int PER = 8;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int base = 0;
+    for (int b0 = 0; b0 < C; b0 += NT * PER) {
+        const int i0 = b0 + threadIdx.x * PER;
+        int e[PER];
+        unsigned keep = 0;
+#pragma unroll
+        for (int q = 0; q < PER; ++q)
+            e[q] = i0 + q >= C ? -1 : identity ? i0 + q : __ldcg(in + i0 + q);
+#pragma unroll
+        for (int q = 0; q < PER; ++q)
+            if (e[q] >= 0 && !__ldcg(pruned + e[q])) keep |= 1u << q;
+        const int cnt = __popc(keep);
+        int inc = cnt;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += t;
+        }
+        __syncthreads(); // wsum of the step before is consumed
+        if (lane == 31) wsum[warp] = inc;
+        __syncthreads();
+        int off = base, all = 0;
+#pragma unroll
+        for (int w = 0; w < NT / 32; ++w) {
+            const int v = wsum[w];
+            if (w < warp) off += v;
+            all += v;
+        }
+        int pos = off + inc - cnt;
+#pragma unroll
+        for (int q = 0; q < PER; ++q)
+            if ((keep >> q) & 1u) out[pos++] = e[q];
+        base += all;
+    }
+    __threadfence();
+    return base;
+}
+
+// The CTA that compacted round rd's survivors (one thread, after a barrier).
+__device__ __forceinline__ void publish_round(PaddiAttemptDev *att, int rd, int count)
+{
+    att->list_count[rd + 1] = count;
+    if (count == 0) att->last_rd = rd + 1;
+    __threadfence();
+    st_release(&att->round_ready, rd + 1);
+}
+
+// The others (one thread): survivors of round rd, or -1 when a CTA gave up or
+// the wait ran out after `limit` clock cycles (status 3 is then recorded).
+__device__ __forceinline__ int wait_round(PaddiAttemptDev *att, int rd, long long limit)
+{
+    const long long t0 = clock64();
+    while (ld_acquire(&att->round_ready) <= rd) {
+        if (ld_acquire(&att->status) == 3) return -1;
+        if (clock64() - t0 > limit) {
+            atomicExch(&att->status, 3);
+            return -1;
+        }
+        __nanosleep(100);
+    }
+    return __ldcg(&att->list_count[rd + 1]);
+}
+
+} // namespace paddi
+
 // Result of one attempt, copied to the host at the end of the attempt.
 struct PaddiAttemptResult {
     int64_t n_cand;  // windows with nn >= r2 (never pruned)
@@ -226,18 +322,18 @@ cudaError_t paddi_launch_compact(const uint8_t *alive, int32_t N, int32_t *cand,
                                  const int32_t *flat_span, int32_t m, bool prune_flats,
                                  cudaStream_t st);
 
-// Dense refine of the candidates in list[0..*list_count) (positions into
-// cand[]) against the windows [jb, je) (jb a multiple of 256).  thr is the
-// exact threshold 1 - r^2 / (2m): the kernel prunes on lower bounds of the
-// correlations; gcap is the guard band (fragile windows are skipped).  W
-// (optional): a pruned candidate leaves the window that pruned it as a hint.
+// FP32 refine of all att->n_cand_p1 candidates over the windows [col_lo, col_hi)
+// (col_lo a multiple of 256), all rounds in one launch; list0 / list1 and
+// att->list_count as in paddi_launch_refine_umma.  thr is the exact threshold
+// 1 - r^2 / (2m): the kernel prunes on lower bounds of the correlations; gcap
+// is the guard band.  W (optional): a pruned candidate leaves the window that
+// pruned it as a hint.
 cudaError_t paddi_launch_refine_fp32(const float *x, const float4 *wst, const float *mu,
-                                     const int32_t *cand, const int32_t *list,
-                                     const int32_t *list_count, PaddiAttemptDev *att,
-                                     int32_t *work, uint32_t *rho_max, uint8_t *pruned,
-                                     int32_t N, int32_t m, int32_t jb, int32_t je, float thr,
-                                     float gcap, int32_t num_sms, cudaStream_t st,
-                                     const PaddiWitness *W = nullptr);
+                                     const int32_t *cand, int32_t *list0, int32_t *list1,
+                                     PaddiAttemptDev *att, uint32_t *rho_max, uint8_t *pruned,
+                                     int32_t N, int32_t m, int32_t col_lo, int32_t col_hi,
+                                     float thr, float gcap, int32_t num_sms, cudaStream_t st,
+                                     long long wait_cycles = 0, const PaddiWitness *W = nullptr);
 
 // Fragile windows of length m in the FP32 refine's geometry, appended to
 // frag_list (frag_count zeroed by the caller).
@@ -246,13 +342,12 @@ cudaError_t paddi_launch_fragile_scan_fp32(const float *x, const float4 *wst, co
                                            int32_t *frag_count, int32_t num_sms, cudaStream_t st);
 
 // Exact FP64 correlations of the refine's unpruned candidates with the fragile
-// windows in [col_lo, col_hi) (k_fragile.cu): prunes and raises rho_max.  last:
-// the refine's last round, whose list holds the candidates (list1 if odd, else
-// list0, list_count[last] entries; round 0: all candidates); -1: att->last_rd.
+// windows in [col_lo, col_hi) (k_fragile.cu): prunes and raises rho_max.  The
+// candidates are those of the refine's last round att->last_rd (list1 if odd,
+// else list0, list_count[last_rd] entries; round 0: all candidates).
 cudaError_t paddi_launch_fragile(const float *x, const double2 *ms64, const int32_t *cand,
                                  const int32_t *list0, const int32_t *list1,
-                                 const PaddiAttemptDev *att, int32_t last, uint8_t *pruned,
-                                 uint32_t *rho_max, const int32_t *frag,
+                                 const PaddiAttemptDev *att, uint8_t *pruned, uint32_t *rho_max, const int32_t *frag,
                                  const int32_t *frag_count, int32_t m, float thr, int32_t col_lo,
                                  int32_t col_hi, int32_t num_sms, cudaStream_t st,
                                  const PaddiBlockMax *B = nullptr, float guard = 0.f);
@@ -289,13 +384,6 @@ cudaError_t paddi_launch_tile_prep(bool bf16, const float *x, int64_t n, int32_t
                                    const float4 *wst, const float *mu, uint16_t *bq, float4 *wdq,
                                    float gcap, int32_t *frag_list, int32_t *frag_count,
                                    cudaStream_t st);
-
-cudaError_t paddi_launch_list_init(const PaddiAttemptDev *att, int32_t *list, int32_t *count,
-                                   cudaStream_t st);
-
-cudaError_t paddi_launch_list_compact(const int32_t *in, const int32_t *in_count,
-                                      const uint8_t *pruned, int32_t *out, int32_t *out_count,
-                                      cudaStream_t st);
 
 cudaError_t paddi_launch_finalize(const int32_t *cand, PaddiAttemptDev *att,
                                   const uint32_t *rho_max, const uint8_t *pruned, int32_t m,

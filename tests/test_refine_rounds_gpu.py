@@ -1,0 +1,38 @@
+"""The refines' rounds in one launch.
+
+Rounds start at 65536 windows; a candidate tile holds 16 (tensor cores, 8 for
+64-row tiles) or 8 (FP32) candidates.  Thresholds are taken from the FP64 nn
+profile so that a chosen number of candidates survives: none, one, a tile's
+worth and one more, many.  Counts must equal the profile's exactly.
+"""
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+from paddi_b200 import datagen
+
+pytestmark = pytest.mark.gpu
+
+M = 40
+
+
+@pytest.fixture(scope="module", params=[65536 - 1, 65536, 65536 + 2048 + 7])
+def case(request):
+    n = request.param + M - 1
+    x, _ = datagen.pd3_series(n=n, seed=11, n_anom=4, anom_len=100)
+    return x, np.sort(O.nn_profile_fast(x, M).astype(np.float32))
+
+
+@pytest.mark.parametrize("dist,rows", [("fp32", 0), ("fp16", 0), ("fp16", 64), ("bf16", 0)])
+def test_survivor_counts_across_rounds(case, dist, rows):
+    import paddi_b200 as P
+    x, nn = case
+    k = {"fp32": P.DIST_FP32, "fp16": P.DIST_SPLIT_FP16, "bf16": P.DIST_SPLIT_BF16}[dist]
+    with P.Context(device=0, distance_kernel=k, tile_rows=rows) as ctx:
+        for keep in (0, 1, 8, 9, 16, 17, 300, 5000):
+            v = float(nn[-1]) * 1.01 if keep == 0 else 0.5 * (float(nn[-keep]) + float(nn[-keep - 1]))
+            r = float(np.sqrt(np.float32(v)))
+            r2 = float(np.float32(r) * np.float32(r))
+            _, (a,) = ctx.pd3(x, M, r=r)
+            assert a["n_cand"] == int((nn >= r2).sum()), keep
+            assert a["n_disc"] == int((nn > r2).sum()), keep
