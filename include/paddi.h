@@ -77,7 +77,9 @@ typedef struct paddi_opts {
     int32_t distance_kernel;  /* paddi_distance_kernel */
     int32_t r_policy;         /* paddi_r_policy */
     uint32_t segment_len;     /* phase-1 rows per segment (reference SEGMENT_N); 0 = 256,
-                                 else 64..4096 (others: PADDI_ERR_UNSUPPORTED) */
+                                 else 64..4096 (others: PADDI_ERR_UNSUPPORTED); a segment
+                                 is split where a series is too short to fill the GPU, and
+                                 above 512 rows */
     uint32_t phase1_chunks;   /* 256-diagonal chunks a segment scans before the refine; 0 = 12 */
     uint32_t iter_cap;        /* attempts allowed per length; 0 = 200 */
     float guard;              /* guard band in correlation units: the largest per-window

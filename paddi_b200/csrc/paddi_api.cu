@@ -322,13 +322,23 @@ paddi_status witness_to(paddi_ctx *ctx, const float *x, size_t n, int m)
 paddi_status enqueue_prep(paddi_ctx *ctx, const float *x, size_t n, int m, bool guided,
                           int32_t w_host);
 
-// Phase-1 rows per task (the reference's SEGMENT_N); validated at the ABI
-// (segment_len_ok), rounded up to a multiple of 8 rows.
-int p1_rows_of(const paddi_ctx *ctx)
+// Phase-1 rows per task for `rows` rows: at most the segment length (the
+// reference's SEGMENT_N; validated at the ABI, rounded up to a multiple of 8),
+// and few enough to give every resident warp of the GPU a task.  Both attempts
+// of a PD3 search, phase 1 only, us (the segment length alone decided before):
+//   n = 131072, m = 128: 64 rows 118, 128 135, 256 186, 4096 1582
+//   n = 131072, m = 600: 64 rows 237, 128 224, 256 241 (start dot products: m per
+//                        diagonal and task)
+//   n = 600000, m = 500: 64 rows 587, 128 461, 256 473
+//   n = 1500007, m = 300: 128 rows 737, 192 715, 256 726, 1024 1580
+int p1_rows_of(const paddi_ctx *ctx, int64_t rows, int m)
 {
     int R = (int)ctx->opts.segment_len;
     if (R <= 0) R = 256;
-    return (R + 7) & ~7;
+    R = (R + 7) & ~7;
+    const int64_t tasks = 15ll * ctx->num_sms; // resident one-warp tasks
+    const int fit = rows <= 64 * tasks && m <= 256 ? 64 : rows <= 512 * tasks ? 128 : 512;
+    return std::min(R, fit);
 }
 
 // Windows without a proving witness: up to wit_limit of them look for a new
@@ -478,7 +488,7 @@ paddi_status run_attempt(paddi_ctx *ctx, const float *x, size_t n, int m, float 
     const int kernel = refine_kernel_for(ctx, m);
     const float guard = guard_of(ctx, kernel);
     const float thr = thr_of(r2, m);
-    const int R = p1_rows_of(ctx);
+    const int R = p1_rows_of(ctx, N, m);
     const int chunks = ctx->opts.phase1_chunks ? (int)ctx->opts.phase1_chunks : 12;
     cudaStream_t st = ctx->st;
     CK(cudaEventRecord(ctx->ev[0], st));
@@ -1254,7 +1264,7 @@ PADDI_API paddi_status paddi_shard_phase1(paddi_ctx *ctx, const float *d_series,
     CK(cudaMemsetAsync(ctx->d_att, 0, sizeof(PaddiAttemptDev), st));
     const int chunks = ctx->opts.phase1_chunks ? (int)ctx->opts.phase1_chunks : 12;
     CK(paddi_launch_phase1_dev(d_series, ctx->d_wst, ctx->d_mu, ctx->d_ms64, d_alive, (int32_t)N,
-                               (int)m, p1_rows_of(ctx), chunks, thr_of(r2, (int)m),
+                               (int)m, p1_rows_of(ctx, (int64_t)(row_hi - row_lo), (int)m), chunks, thr_of(r2, (int)m),
                                (int32_t)row_lo, (int32_t)row_hi, ctx->d_att, ctx->num_sms, st));
     CK(cudaStreamSynchronize(st));
     return PADDI_OK;

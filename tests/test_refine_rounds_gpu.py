@@ -1,4 +1,4 @@
-"""The refines' rounds in one launch.
+"""The refines' rounds in one launch, and phase 1's split segments.
 
 Rounds start at 65536 windows; a candidate tile holds 16 (tensor cores, 8 for
 64-row tiles) or 8 (FP32) candidates.  Thresholds are taken from the FP64 nn
@@ -36,3 +36,17 @@ def test_survivor_counts_across_rounds(case, dist, rows):
             _, (a,) = ctx.pd3(x, M, r=r)
             assert a["n_cand"] == int((nn >= r2).sum()), keep
             assert a["n_disc"] == int((nn > r2).sum()), keep
+
+
+@pytest.mark.parametrize("n,m", [(300, 20), (64 * 15 * 148 // 8, 30), (64 * 15 * 148 + 40, 40)])
+@pytest.mark.parametrize("seg", [64, 72, 256, 520, 4096])
+def test_phase1_tasks_do_not_change_results(n, m, seg):
+    """Every split of the rows gives the same candidates (the last n has more rows
+    than one 64-row task per resident warp covers)."""
+    import paddi_b200 as P
+    x, _ = datagen.pd3_series(n=n, seed=5, n_anom=2, anom_len=max(10, min(100, n // 40)))
+    with P.Context(device=0) as ctx:
+        ref, rl = ctx.pd3(x, m, segment_len=256)
+        got, gl = ctx.pd3(x, m, segment_len=seg)
+    assert [(d.ind, d.dist) for d in got] == [(d.ind, d.dist) for d in ref]
+    assert [(a["n_cand"], a["n_disc"]) for a in gl] == [(a["n_cand"], a["n_disc"]) for a in rl]
