@@ -42,7 +42,7 @@ __global__ void __launch_bounds__(FG_THREADS)
 k_fragile(const float *__restrict__ x, const double2 *__restrict__ ms64,
           const int32_t *__restrict__ cand,
           const int32_t *__restrict__ list0, const int32_t *__restrict__ list1,
-          const PaddiAttemptDev *__restrict__ att, uint8_t *pruned, uint32_t *rho_max,
+          PaddiAttemptDev *att, uint8_t *pruned, uint32_t *rho_max,
           const int32_t *__restrict__ frag,
           const int32_t *__restrict__ frag_count, int32_t m, float thr, int32_t col_lo,
           int32_t col_hi, PaddiBlockMax B, float guard)
@@ -53,10 +53,12 @@ k_fragile(const float *__restrict__ x, const double2 *__restrict__ ms64,
     __shared__ double civ[FG_CAND];
     __shared__ double best_s[FG_CAND][FG_THREADS / 32];
     __shared__ int s_any;
+    paddi::chain_begin();
+    paddi::stamp_begin(att->t + PADDI_T_FRAGILE);
     // the candidates of the refine's last round (round 0: all of them)
     const int rd = att->last_rd;
     const int32_t *list = rd & 1 ? list1 : list0;
-    const int C = rd ? att->list_count[rd] : att->n_cand_p1, F = *frag_count;
+    const int C = rd ? att->list_count[rd] : att->n_cand_p1, F = __ldcg(frag_count);
     if (C <= 0 || F <= 0) return;
     const bool bkeep = B.kept(att->n_cand_p1);
     const int mp = (m + 1) & ~1;
@@ -156,7 +158,7 @@ k_fragile(const float *__restrict__ x, const double2 *__restrict__ ms64,
 
 cudaError_t paddi_launch_fragile(const float *x, const double2 *ms64,
                                  const int32_t *cand, const int32_t *list0,
-                                 const int32_t *list1, const PaddiAttemptDev *att,
+                                 const int32_t *list1, PaddiAttemptDev *att,
                                  uint8_t *pruned, uint32_t *rho_max,
                                  const int32_t *frag, const int32_t *frag_count, int32_t m,
                                  float thr, int32_t col_lo, int32_t col_hi, int32_t num_sms,
@@ -166,8 +168,7 @@ cudaError_t paddi_launch_fragile(const float *x, const double2 *ms64,
     const size_t smem = sizeof(double) * (size_t)FG_CAND * (size_t)((m + 1) & ~1);
     cudaError_t e = paddi_raise_smem_limit((const void *)k_fragile, smem);
     if (e != cudaSuccess) return e;
-    k_fragile<<<num_sms * 4, FG_THREADS, smem, st>>>(x, ms64, cand, list0, list1, att,
+    return paddi_launch(true, k_fragile, num_sms * 4, FG_THREADS, smem, st, x, ms64, cand, list0, list1, att,
                                                     pruned, rho_max, frag, frag_count, m, thr,
                                                     col_lo, col_hi, B ? *B : PaddiBlockMax{}, guard);
-    return cudaGetLastError();
 }

@@ -113,7 +113,9 @@ __device__ __forceinline__ int guide_mode(const PaddiGuide *g, int w, int m)
 
 // Grid minimum into g->nn_ord; the last CTA to arrive publishes the state.
 __device__ __forceinline__ void guide_finish(double best, double *red, PaddiGuide *g, int w, int m,
-                                             double s, int cur, int age, int mode)
+                                             double s, int cur, int age, int mode,
+                                             volatile PaddiGuide *host, const int32_t *flat_count,
+                                             unsigned long long *t)
 {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) best = fmin(best, __shfl_xor_sync(0xffffffffu, best, o));
@@ -135,6 +137,12 @@ __device__ __forceinline__ void guide_finish(double best, double *red, PaddiGuid
             g->mode = mode;
             g->done = 0;
             g->item = 0;
+            __threadfence();
+            host->nn_ord = __ldcg(&g->nn_ord);
+            host->w_used = w;
+            host->mode = mode;
+            host->n_flat = *flat_count;
+            t[PADDI_T_GUIDE_E] = paddi::time_ns();
         }
     }
 }
@@ -143,8 +151,12 @@ __device__ __forceinline__ void guide_finish(double best, double *red, PaddiGuid
 __global__ void __launch_bounds__(GD_THREADS, GD_STREAM_CTAS_PER_SM)
 k_guide_stream(const float *__restrict__ x, const double2 *__restrict__ ms64, const uint8_t *__restrict__ flat, int32_t N,
                int32_t m, const PaddiAttemptResult *__restrict__ prev, int32_t w_host,
-               PaddiGuide *g, double *__restrict__ G0, double *__restrict__ G1)
+               PaddiGuide *g, double *__restrict__ G0, double *__restrict__ G1,
+               volatile PaddiGuide *host, const int32_t *__restrict__ flat_count,
+               unsigned long long *t_prep)
 {
+    paddi::chain_begin();
+    paddi::stamp_begin(t_prep + PADDI_T_GUIDE_B);
     __shared__ double redm[GD_THREADS / 32];
     __shared__ double cf[2 * GD_MAX_SLIDE + 2]; // slide coefficients, signed
     __shared__ int coff[2 * GD_MAX_SLIDE + 2];  // their partner offsets (from j)
@@ -154,6 +166,10 @@ k_guide_stream(const float *__restrict__ x, const double2 *__restrict__ ms64, co
         if (blockIdx.x == 0 && t == 0) {
             g->w_used = -1;
             g->mode = PADDI_GUIDE_SKIPPED;
+            host->w_used = -1;
+            host->mode = PADDI_GUIDE_SKIPPED;
+            host->n_flat = *flat_count;
+            t_prep[PADDI_T_GUIDE_E] = paddi::time_ns();
         }
         return;
     }
@@ -251,7 +267,8 @@ k_guide_stream(const float *__restrict__ x, const double2 *__restrict__ ms64, co
         }
     }
     const bool slid = mode == PADDI_GUIDE_SLID;
-    guide_finish(best, redm, g, w, m, s, slid ? gcur ^ 1 : gcur, gage + (slid ? 1 : 0), mode);
+    guide_finish(best, redm, g, w, m, s, slid ? gcur ^ 1 : gcur, gage + (slid ? 1 : 0), mode, host,
+                 flat_count, t_prep);
 }
 
 // Rebuild: direct dot products of w with blocks of GD_SPAN windows, handed
@@ -261,8 +278,11 @@ k_guide_stream(const float *__restrict__ x, const double2 *__restrict__ ms64, co
 __global__ void __launch_bounds__(GD_THREADS)
 k_guide_build(const float *__restrict__ x, const double2 *__restrict__ ms64, const uint8_t *__restrict__ flat, int32_t N,
               int32_t m, const PaddiAttemptResult *__restrict__ prev, int32_t w_host,
-              PaddiGuide *g, double *__restrict__ G0, double *__restrict__ G1)
+              PaddiGuide *g, double *__restrict__ G0, double *__restrict__ G1,
+              volatile PaddiGuide *host, const int32_t *__restrict__ flat_count,
+              unsigned long long *t_prep)
 {
+    paddi::chain_begin();
     __shared__ double a[GD_MAXM];
     __shared__ double xs[GD_SPAN + GD_MAXM + (GD_SPAN + GD_MAXM) / 16 + 16];
     __shared__ double redm[GD_THREADS / 32];
@@ -327,28 +347,23 @@ k_guide_build(const float *__restrict__ x, const double2 *__restrict__ ms64, con
             }
         }
     }
-    guide_finish(best, redm, g, w, m, s, ncur, 0, PADDI_GUIDE_BUILT);
+    guide_finish(best, redm, g, w, m, s, ncur, 0, PADDI_GUIDE_BUILT, host, flat_count, t_prep);
 }
 
 } // namespace
 
-cudaError_t paddi_launch_guide(const float *x, const double2 *ms64,
-                               const uint8_t *flat, int32_t N, int32_t m,
-                               const PaddiAttemptResult *prev, int32_t w_host, PaddiGuide *g,
-                               double *G, size_t g_stride, int32_t num_sms, cudaStream_t st)
+cudaError_t paddi_launch_guide(const float *x, const double2 *ms64, const uint8_t *flat, int32_t N,
+                               int32_t m, const PaddiAttemptResult *prev, int32_t w_host,
+                               PaddiGuide *g, double *G, size_t g_stride, int32_t num_sms,
+                               cudaStream_t st, PaddiGuide *host, const int32_t *flat_count,
+                               unsigned long long *t)
 {
     if (m < 3 || m > GD_MAXM || N < 1 || g_stride < (size_t)N) return cudaErrorInvalidValue;
-    // the result's ordered image starts at +inf (all ones: above every finite
-    // image); the rest of the record is written by the kernels
-    cudaError_t e = cudaMemsetAsync(&g->nn_ord, 0xff, sizeof(g->nn_ord), st);
-    if (e != cudaSuccess) return e;
     // the stream grid also covers the slide's boundary windows (one per CTA)
     const int sgrid = std::max(GD_STREAM_CTAS_PER_SM * num_sms, GD_MAX_SLIDE + 1);
-    k_guide_stream<<<sgrid, GD_THREADS, 0, st>>>(x, ms64, flat, N, m, prev, w_host, g, G,
-                                                 G + g_stride);
-    e = cudaGetLastError();
+    cudaError_t e = paddi_launch(true, k_guide_stream, sgrid, GD_THREADS, 0, st, x, ms64, flat, N, m,
+                                 prev, w_host, g, G, G + g_stride, host, flat_count, t);
     if (e != cudaSuccess) return e;
-    k_guide_build<<<4 * num_sms, GD_THREADS, 0, st>>>(x, ms64, flat, N, m, prev, w_host,
-                                                      g, G, G + g_stride);
-    return cudaGetLastError();
+    return paddi_launch(true, k_guide_build, 4 * num_sms, GD_THREADS, 0, st, x, ms64, flat, N, m,
+                        prev, w_host, g, G, G + g_stride, host, flat_count, t);
 }

@@ -212,6 +212,8 @@ k_phase1(const float *__restrict__ x, const float4 *__restrict__ wst, const floa
          int32_t max_chunks, float thr, int32_t row_lo, int32_t row_hi, PaddiAttemptDev *att,
          PaddiWitness W, int32_t enough)
 {
+    paddi::chain_begin();
+    if (!WT) paddi::stamp_begin(att->t + PADDI_T_BEGIN);
     if (WT && att->n_fail - att->n_rescued <= enough) return;
     extern __shared__ __align__(16) unsigned char p1_smem[];
     const int mpad = (m + 7) & ~7;
@@ -425,7 +427,6 @@ cudaError_t paddi_launch_phase1_dev(const float *x, const float4 *wst, const flo
     const int nseg = (row_hi - row_lo + R - 1) / R;
     int grid = num_sms * per_sm;
     if (grid > nseg * max_chunks) grid = nseg * max_chunks;
-    kern<<<grid, P1_THREADS, smem, st>>>(x, wst, mu, ms64, alive, N, m, R, max_chunks, thr, row_lo,
+    return paddi_launch(true, kern, grid, P1_THREADS, smem, st, x, wst, mu, ms64, alive, N, m, R, max_chunks, thr, row_lo,
                                          row_hi, att, W ? *W : PaddiWitness{}, enough);
-    return cudaGetLastError();
 }

@@ -94,8 +94,13 @@ k_refine_fp32(const float *__restrict__ x, const float4 *__restrict__ wst,
     __shared__ float cf[RF_TC], zsum[RF_TC];
     __shared__ uint8_t dead[RF_TC];
 
+    paddi::chain_begin();
+    paddi::stamp_begin(att->t + PADDI_T_REFINE_B);
     int C = att->n_cand_p1;
-    if (C <= 0 || col_hi <= col_lo) return;
+    if (C <= 0 || col_hi <= col_lo) {
+        paddi::stamp_begin(att->t + PADDI_T_REFINE_E);
+        return;
+    }
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int cg = warp % RF_CG, sub = warp / RF_CG;
     if (threadIdx.x == 0) s_last = 0;
@@ -324,6 +329,7 @@ k_refine_fp32(const float *__restrict__ x, const float4 *__restrict__ wst,
         jb = je;
         __syncthreads(); // s_next is read by all before a later round writes it
     }
+    if (threadIdx.x == 0) paddi::stamp_end(att->t + PADDI_T_REFINE_E);
 }
 
 } // namespace
@@ -347,11 +353,9 @@ cudaError_t paddi_launch_refine_fp32(const float *x, const float4 *wst, const fl
     if (e != cudaSuccess) return e;
     if (per_sm < 1) return cudaErrorInvalidConfiguration;
     const int grid = num_sms * per_sm;
-    k_refine_fp32<<<grid, RF_THREADS, smem, st>>>(
-        x, wst, mu, cand, list0, list1, att, rho_max, pruned, N, m, col_lo, col_hi, thr,
+    return paddi_launch(true, k_refine_fp32, grid, RF_THREADS, smem, st, x, wst, mu, cand, list0, list1, att, rho_max, pruned, N, m, col_lo, col_hi, thr,
         paddi_bound_fp32(m).E, gcap, wait_cycles > 0 ? wait_cycles : 4000000000ll,
         W ? *W : PaddiWitness{});
-    return cudaGetLastError();
 }
 
 PaddiBound paddi_bound_fp32(int m)
@@ -372,8 +376,10 @@ PaddiBound paddi_bound_fp32(int m)
 // windows shifted by their first value): the same test as the refine applies.
 __global__ void k_fragile_scan_fp32(const float *__restrict__ x, const float4 *__restrict__ wst,
                                     const float *__restrict__ mu, int32_t N, int32_t m, float E,
-                                    float gcap, int32_t *frag_list, int32_t *frag_count)
+                                    float gcap, int32_t *frag_list, int32_t *frag_count,
+                                    unsigned long long *t_end)
 {
+    paddi::chain_begin();
     const int lane = threadIdx.x & 31;
     for (int j0 = blockIdx.x * blockDim.x; j0 < N; j0 += gridDim.x * blockDim.x) {
         const int j = j0 + threadIdx.x;
@@ -390,13 +396,15 @@ __global__ void k_fragile_scan_fp32(const float *__restrict__ x, const float4 *_
             if (frag) frag_list[base + __popc(bal & ((1u << lane) - 1u))] = j;
         }
     }
+    __syncthreads();
+    if (threadIdx.x == 0) paddi::stamp_end(t_end);
 }
 
 cudaError_t paddi_launch_fragile_scan_fp32(const float *x, const float4 *wst, const float *mu,
                                            int32_t N, int32_t m, float gcap, int32_t *frag_list,
-                                           int32_t *frag_count, int32_t num_sms, cudaStream_t st)
+                                           int32_t *frag_count, int32_t num_sms, cudaStream_t st,
+                                           unsigned long long *t_end)
 {
-    k_fragile_scan_fp32<<<num_sms * 4, 256, 0, st>>>(x, wst, mu, N, m, paddi_bound_fp32(m).E, gcap,
-                                                    frag_list, frag_count);
-    return cudaGetLastError();
+    return paddi_launch(true, k_fragile_scan_fp32, num_sms * 4, 256, 0, st, x, wst, mu, N, m,
+                        paddi_bound_fp32(m).E, gcap, frag_list, frag_count, t_end);
 }

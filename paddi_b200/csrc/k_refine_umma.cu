@@ -263,9 +263,10 @@ __global__ void __launch_bounds__(TP_THREADS)
 k_tile_prep(const float *__restrict__ x, int64_t nser, int32_t cnt, int32_t m,
             const float4 *__restrict__ wst, const float *__restrict__ mu, uint16_t *__restrict__ bq,
             float4 *__restrict__ wdq, float E, float Fu, float gcap, int32_t *frag_list,
-            int32_t *frag_count)
+            int32_t *frag_count, unsigned long long *t_end)
 {
     using X = E16<BF>;
+    paddi::chain_begin();
     __shared__ float red[4][TP_THREADS / 32];
     const int b = blockIdx.x;
     const int64_t j0 = (int64_t)b * UM_TW;
@@ -372,6 +373,7 @@ k_tile_prep(const float *__restrict__ x, int64_t nser, int32_t cnt, int32_t m,
         float G = 0.f;
         for (int k = 0; k < TP_THREADS / 32; ++k) G = fmaxf(G, red[0][k]);
         wf[(0 * WD_ROW + 128) * 4] = G; // padding entry of shift row 0
+        paddi::stamp_end(t_end);
     }
 }
 
@@ -454,8 +456,13 @@ k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
     const UmLayout L = um_layout(MM, kp);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
+    paddi::chain_begin();
+    paddi::stamp_begin(att->t + PADDI_T_REFINE_B);
     int C = att->n_cand_p1;
-    if (C <= 0 || col_hi <= col_lo) return; // uniform, before any TMEM use
+    if (C <= 0 || col_hi <= col_lo) { // uniform, before any TMEM use
+        paddi::stamp_begin(att->t + PADDI_T_REFINE_E);
+        return;
+    }
     const bool bkeep = B.kept(C);
 
     if (threadIdx.x == 0) {
@@ -951,6 +958,7 @@ k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    if (threadIdx.x == 0) paddi::stamp_end(att->t + PADDI_T_REFINE_E);
     if (warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u)
                      : "memory");
@@ -1005,20 +1013,16 @@ PaddiBound paddi_bound_tc(int m, bool bf16)
 cudaError_t paddi_launch_tile_prep(bool bf16, const float *x, int64_t n, int32_t m,
                                    const float4 *wst, const float *mu, uint16_t *bq, float4 *wdq,
                                    float gcap, int32_t *frag_list, int32_t *frag_count,
-                                   cudaStream_t st)
+                                   cudaStream_t st, unsigned long long *t_end)
 {
     const int kp = kpad_of(m);
     if (kp > UM_KMAX64 || m < 3) return cudaErrorInvalidValue;
     const int64_t N = n - m + 1;
     const unsigned grid = (unsigned)paddi_tile_blocks(N);
     const PaddiBound B = paddi_bound_tc(m, bf16);
-    if (bf16)
-        k_tile_prep<true><<<grid, TP_THREADS, 0, st>>>(x, n, slice_cnt(kp), m, wst, mu, bq, wdq,
-                                                       B.E, B.F, gcap, frag_list, frag_count);
-    else
-        k_tile_prep<false><<<grid, TP_THREADS, 0, st>>>(x, n, slice_cnt(kp), m, wst, mu, bq, wdq,
-                                                        B.E, B.F, gcap, frag_list, frag_count);
-    return cudaGetLastError();
+    return paddi_launch(true, bf16 ? k_tile_prep<true> : k_tile_prep<false>, grid, TP_THREADS, 0, st,
+                        x, n, slice_cnt(kp), m, wst, mu, bq, wdq, B.E, B.F, gcap, frag_list,
+                        frag_count, t_end);
 }
 
 cudaError_t paddi_launch_refine_umma(bool bf16, const float *x, const float4 *wst,
@@ -1046,9 +1050,8 @@ cudaError_t paddi_launch_refine_umma(bool bf16, const float *x, const float4 *ws
     cudaError_t e = paddi_raise_smem_limit((const void *)kern, smem);
     if (e != cudaSuccess) return e;
     const int grid = num_sms;
-    kern<<<grid, UM_THREADS, smem, st>>>(x, wst, mu, cand, list0, list1, bq, wdq, att, rho_max,
+    return paddi_launch(true, kern, grid, UM_THREADS, smem, st, x, wst, mu, cand, list0, list1, bq, wdq, att, rho_max,
                                          pruned, N, m, col_lo, col_hi, thr_prune, grid,
                                          wait_cycles > 0 ? wait_cycles : 4000000000ll, withhold,
                                          W ? *W : PaddiWitness{}, B ? *B : PaddiBlockMax{});
-    return cudaGetLastError();
 }

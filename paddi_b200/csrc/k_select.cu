@@ -41,13 +41,15 @@ constexpr int RC_MAXM = 1024;
 constexpr int CP_WIN = 16;                 // windows per thread
 constexpr int CP_CTHREADS = 256;
 __global__ void __launch_bounds__(CP_CTHREADS)
-k_compact(const uint8_t *__restrict__ alive, int32_t N, int32_t *cand, uint32_t *rho_max,
+k_compact(uint8_t *__restrict__ alive, int32_t reset, int32_t N, int32_t *cand, uint32_t *rho_max,
           uint8_t *pruned, int32_t *rc_slot, PaddiAttemptDev *att,
           const uint8_t *__restrict__ flat, const int32_t *__restrict__ flat_span, int32_t m,
           int32_t prune_flats)
 {
     __shared__ int wcnt[CP_CTHREADS / 32];
     __shared__ int base;
+    paddi::chain_begin();
+    paddi::stamp_begin(att->t + PADDI_T_COMPACT);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int i0 = (blockIdx.x * CP_CTHREADS + threadIdx.x) * CP_WIN;
     uint8_t f[CP_WIN];
@@ -56,9 +58,15 @@ k_compact(const uint8_t *__restrict__ alive, int32_t N, int32_t *cand, uint32_t 
         const uint32_t u[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
         for (int b = 0; b < CP_WIN; ++b) f[b] = (u[b >> 2] >> (8 * (b & 3))) & 0xffu;
+        if (reset)
+            *reinterpret_cast<uint4 *>(alive + i0) =
+                make_uint4(0x01010101u, 0x01010101u, 0x01010101u, 0x01010101u);
     } else {
 #pragma unroll
-        for (int b = 0; b < CP_WIN; ++b) f[b] = i0 + b < N ? alive[i0 + b] : 0;
+        for (int b = 0; b < CP_WIN; ++b) {
+            f[b] = i0 + b < N ? alive[i0 + b] : 0;
+            if (reset && i0 + b < N) alive[i0 + b] = 1;
+        }
     }
     uint32_t mask = 0;
     int lo = 0, hi = -1;
@@ -208,6 +216,8 @@ k_finalize(const int32_t *__restrict__ cand, PaddiAttemptDev *att,
     __shared__ VI redv[32];
     __shared__ int picks[PADDI_MAX_TOPK];
     __shared__ int s_nr;
+    paddi::chain_begin();
+    paddi::stamp_begin(att->t + PADDI_T_SELECT);
     const int C = att->n_cand_p1;
     if (threadIdx.x == 0) s_nr = 0;
     __syncthreads();
@@ -319,6 +329,7 @@ k_recheck(const float *__restrict__ x, const double2 *__restrict__ ms64, const u
     __shared__ double reda[RC_THREADS / 32];
     __shared__ double redm[RC_THREADS / 32];
     __shared__ int s_item;
+    paddi::chain_begin();
     const int nr = att->n_recheck;
     const int nblk = (N + RC_SPAN - 1) / RC_SPAN;
     const long long want = 4ll * gridDim.x;
@@ -433,8 +444,11 @@ k_select(const int32_t *__restrict__ cand, PaddiAttemptDev *att,
          const uint32_t *__restrict__ rho_max, const uint8_t *__restrict__ pruned,
          const int32_t *__restrict__ recheck, const int32_t *__restrict__ rc_slot,
          const unsigned long long *__restrict__ nn64_ord, int32_t m, float r2, float thr,
-         float guard, int32_t top_k, const uint8_t *__restrict__ flat, PaddiAttemptResult *res)
+         float guard, int32_t top_k, const uint8_t *__restrict__ flat,
+         const int32_t *__restrict__ flat_count, const unsigned long long *__restrict__ t_prep,
+         PaddiAttemptDev *next, PaddiAttemptResult *res, PaddiAttemptResult *host)
 {
+    paddi::chain_begin();
     __shared__ long long redl[32];
     __shared__ VI redv[32];
     __shared__ int picks_w[PADDI_MAX_TOPK];
@@ -506,7 +520,19 @@ k_select(const int32_t *__restrict__ cand, PaddiAttemptDev *att,
         res->n_live = att->n_live;
         res->p1_walked = att->p1_walked;
         res->status = att->status ? att->status : (s_need ? 2 : 0);
+        res->n_fragile = flat_count[3];
+        res->n_flat = flat_count[0];
+        res->n_unproven = att->n_fail;
+        for (int k = 0; k < PADDI_T_PREP; ++k) res->t_prep[k] = t_prep[k];
+        for (int k = 0; k < PADDI_T_END; ++k) res->t[k] = att->t[k];
+        res->t[PADDI_T_END] = paddi::time_ns();
     }
+    __syncthreads();
+    // the result to the host, and a clean state for the next attempt
+    for (int k = threadIdx.x; k < (int)(sizeof(PaddiAttemptResult) / 4); k += FZ_THREADS)
+        reinterpret_cast<volatile int32_t *>(host)[k] = reinterpret_cast<int32_t *>(res)[k];
+    for (int k = threadIdx.x; k < (int)(sizeof(PaddiAttemptDev) / 4); k += FZ_THREADS)
+        reinterpret_cast<int32_t *>(next)[k] = 0;
 }
 
 // Candidate flags and distances in the reference's per-window layout
@@ -555,7 +581,7 @@ cudaError_t paddi_launch_scatter(const int32_t *cand, const PaddiAttemptDev *att
     return cudaGetLastError();
 }
 
-cudaError_t paddi_launch_compact(const uint8_t *alive, int32_t N, int32_t *cand,
+cudaError_t paddi_launch_compact(uint8_t *alive, bool reset, int32_t N, int32_t *cand,
                                  uint32_t *rho_max, uint8_t *pruned, int32_t *rc_slot,
                                  PaddiAttemptDev *att, const uint8_t *flat,
                                  const int32_t *flat_span, int32_t m, bool prune_flats,
@@ -563,9 +589,8 @@ cudaError_t paddi_launch_compact(const uint8_t *alive, int32_t N, int32_t *cand,
 {
     const int per_cta = CP_CTHREADS * CP_WIN;
     const unsigned grid = (unsigned)((N + per_cta - 1) / per_cta);
-    k_compact<<<grid, CP_CTHREADS, 0, st>>>(alive, N, cand, rho_max, pruned, rc_slot, att, flat,
+    return paddi_launch(true, k_compact, grid, CP_CTHREADS, 0, st, alive, reset ? 1 : 0, N, cand, rho_max, pruned, rc_slot, att, flat,
                                            flat_span, m, prune_flats ? 1 : 0);
-    return cudaGetLastError();
 }
 
 cudaError_t paddi_launch_finalize(const int32_t *cand, PaddiAttemptDev *att,
@@ -577,10 +602,9 @@ cudaError_t paddi_launch_finalize(const int32_t *cand, PaddiAttemptDev *att,
                                   unsigned long long known_ord, cudaStream_t st)
 {
     if (top_k < 1 || top_k > PADDI_MAX_TOPK) return cudaErrorInvalidValue;
-    k_finalize<<<1, FZ_THREADS, 0, st>>>(cand, att, rho_max, pruned, m, r2, thr, guard, widen,
+    return paddi_launch(true, k_finalize, 1, FZ_THREADS, 0, st, cand, att, rho_max, pruned, m, r2, thr, guard, widen,
                                          top_k, flat, rc_cap, recheck, rc_slot, nn64_ord, res,
                                          known_w, known_ord);
-    return cudaGetLastError();
 }
 
 cudaError_t paddi_launch_recheck(const float *x, const double2 *ms64,
@@ -591,10 +615,9 @@ cudaError_t paddi_launch_recheck(const float *x, const double2 *ms64,
                                  const uint32_t *rho_max, const PaddiBlockMax *B, float guard)
 {
     if (m > RC_MAXM) return cudaErrorInvalidValue;
-    k_recheck<<<num_sms * 4, RC_THREADS, 0, st>>>(x, ms64, flat, N, m, cand, recheck, att,
+    return paddi_launch(true, k_recheck, num_sms * 4, RC_THREADS, 0, st, x, ms64, flat, N, m, cand, recheck, att,
                                                  nn64_ord, known_w, rho_max,
                                                  B ? *B : PaddiBlockMax{}, guard);
-    return cudaGetLastError();
 }
 
 cudaError_t paddi_launch_select(const int32_t *cand, PaddiAttemptDev *att,
@@ -602,9 +625,10 @@ cudaError_t paddi_launch_select(const int32_t *cand, PaddiAttemptDev *att,
                                 const int32_t *recheck, const int32_t *rc_slot,
                                 const unsigned long long *nn64_ord, int32_t m, float r2,
                                 float thr, float guard, int32_t top_k, const uint8_t *flat,
-                                PaddiAttemptResult *res, cudaStream_t st)
+                                const int32_t *flat_count, const unsigned long long *t_prep,
+                                PaddiAttemptDev *next, PaddiAttemptResult *res,
+                                PaddiAttemptResult *host, cudaStream_t st)
 {
-    k_select<<<1, FZ_THREADS, 0, st>>>(cand, att, rho_max, pruned, recheck, rc_slot, nn64_ord,
-                                       m, r2, thr, guard, top_k, flat, res);
-    return cudaGetLastError();
+    return paddi_launch(true, k_select, 1, FZ_THREADS, 0, st, cand, att, rho_max, pruned, recheck, rc_slot, nn64_ord,
+                                       m, r2, thr, guard, top_k, flat, flat_count, t_prep, next, res, host);
 }

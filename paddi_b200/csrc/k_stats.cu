@@ -62,8 +62,15 @@ __device__ T block_exclusive_scan(T v, T *warp_tot)
 __global__ void __launch_bounds__(ST_THREADS)
 k_window_stats(const float *__restrict__ x, int64_t n, int32_t m, int32_t N, float4 *wst,
                float *mu, double2 *ms64, uint8_t *flat, int32_t *flat_count,
-               int32_t *flat_span)
+               int32_t *flat_span, PaddiStatsExtra extra)
 {
+    paddi::chain_begin();
+    paddi::stamp_begin(extra.t);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        if (extra.next)
+            for (int k = 0; k < 4; ++k) extra.next[k] = 0;
+        if (extra.guide) extra.guide->nn_ord = ~0ull;
+    }
     // staged values: x[t0 .. t0 + ST_TILE + m] (one extra window for mu_{i+1})
     extern __shared__ __align__(16) unsigned char st_mem[];
     const int LS = ST_TILE + m + 2;
@@ -147,6 +154,7 @@ k_window_stats(const float *__restrict__ x, int64_t n, int32_t m, int32_t N, flo
         mu[i] = (float)mu_i;
         ms64[i] = make_double2(mu_i, iv);
         flat[i] = (uint8_t)fl;
+        if (extra.alive) extra.alive[i] = 1;
         nflat += fl;
         // lowest and highest flat window, both kept as maxima over a zeroed
         // pair: {INT_MAX - lowest, highest + 1} (flat windows are rare)
@@ -180,7 +188,8 @@ cudaError_t paddi_launch_export_stats(const double2 *ms64, int32_t N,
 
 cudaError_t paddi_launch_stats(const float *x, int64_t n, int32_t m, float4 *wst, float *mu,
                                double2 *ms64, uint8_t *flat,
-                               int32_t *flat_count, cudaStream_t st, int32_t *flat_span)
+                               int32_t *flat_count, cudaStream_t st, int32_t *flat_span,
+                               bool chained, const PaddiStatsExtra &extra)
 {
     if (m < 2 || m > ST_MAXM || n < 2 * (int64_t)m) return cudaErrorInvalidValue;
     const int32_t N = (int32_t)(n - m + 1);
@@ -189,7 +198,6 @@ cudaError_t paddi_launch_stats(const float *x, int64_t n, int32_t m, float4 *wst
     const size_t smem = st_smem(m);
     cudaError_t e = paddi_raise_smem_limit((const void *)k_window_stats, smem);
     if (e != cudaSuccess) return e;
-    k_window_stats<<<grid, ST_THREADS, smem, st>>>(x, n, m, N, wst, mu, ms64, flat,
-                                                   flat_count, flat_span);
-    return cudaGetLastError();
+    return paddi_launch(chained, k_window_stats, grid, ST_THREADS, smem, st, x, n, m, N, wst, mu, ms64, flat,
+                                                   flat_count, flat_span, extra);
 }

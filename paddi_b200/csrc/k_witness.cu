@@ -99,6 +99,7 @@ k_witness_step(const float *__restrict__ x, const double2 *__restrict__ ms64, in
                float *__restrict__ wrho, int32_t *__restrict__ hint, uint32_t *scal,
                double dscale)
 {
+    paddi::chain_begin();
     const int i0 = blockIdx.x * (WT_THREADS * WT_SWIN) + threadIdx.x;
     const double t1 = dscale * (double)__uint_as_float(scal[WT_AMAX]);
     // the window's new value: the last one of length m, or (back to the length
@@ -181,8 +182,9 @@ __global__ void __launch_bounds__(WT_THREADS)
 k_witness_hints(const float *__restrict__ x, const double2 *__restrict__ ms64, int32_t N,
                 int32_t m, int32_t *__restrict__ wit, double *__restrict__ wc,
                 float *__restrict__ wrho, const int32_t *__restrict__ hint, uint32_t *scal,
-                double dscale)
+                double dscale, unsigned long long *t_end)
 {
+    paddi::chain_begin();
     const int nh = (int)scal[WT_NHINT];
     const int lane = threadIdx.x & 31;
     const int nser = N + m - 1;
@@ -266,6 +268,7 @@ k_witness_hints(const float *__restrict__ x, const double2 *__restrict__ ms64, i
             scal[WT_NHINT] = 0;
             scal[WT_DONE] = 0;
         }
+        paddi::stamp_end(t_end);
     }
 }
 
@@ -287,8 +290,10 @@ k_absmax(const float *__restrict__ x, int64_t n, uint32_t *amax)
 // within a CTA kept).  5 B per window.
 __global__ void __launch_bounds__(WT_THREADS)
 k_witness_check(const float *__restrict__ wrho, int32_t N, float thr, uint8_t *__restrict__ alive,
-                int32_t *__restrict__ fail, int32_t *n_fail)
+                int32_t *__restrict__ fail, PaddiAttemptDev *att)
 {
+    paddi::chain_begin();
+    paddi::stamp_begin(att->t + PADDI_T_BEGIN);
     __shared__ int wcnt[WT_THREADS / 32];
     __shared__ int base;
     const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
@@ -330,7 +335,7 @@ k_witness_check(const float *__restrict__ wrho, int32_t N, float thr, uint8_t *_
             wcnt[q] = s;
             s += t;
         }
-        base = s ? atomicAdd(n_fail, s) : 0;
+        base = s ? atomicAdd(&att->n_fail, s) : 0;
     }
     __syncthreads();
     int pos = base + wcnt[wp] + inc - cnt;
@@ -358,7 +363,8 @@ k_witness_rescue(const float *__restrict__ x, const double2 *__restrict__ ms64, 
                  const uint32_t *__restrict__ scal, double dscale)
 {
     extern __shared__ float wt_a[]; // per warp: the centred window
-    const int nf = *n_fail;
+    paddi::chain_begin();
+    const int nf = __ldcg(n_fail);
     if (nf > limit) return;
     const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
     float *a = wt_a + (size_t)wp * m;
@@ -489,17 +495,16 @@ cudaError_t paddi_launch_witness_start(const float *x, int64_t n, int32_t N, con
 cudaError_t paddi_launch_witness_step(const float *x, const double2 *ms64,
                                       int32_t N, int32_t m, int32_t from, int32_t m0,
                                       const PaddiWitness &W, int32_t *hint, int32_t num_sms,
-                                      cudaStream_t st)
+                                      cudaStream_t st, unsigned long long *t_end)
 {
     if (m < 3 || m > WT_MAXM || N < 1 || from < m - 1 || from > m + 1) return cudaErrorInvalidValue;
     const int per = WT_THREADS * WT_SWIN;
-    k_witness_step<<<(unsigned)(N / per + 1), WT_THREADS, 0, st>>>(
-        x, ms64, N, m, from, W.wit, W.wc, W.wrho, hint, W.scal, wt_dscale(m0));
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = paddi_launch(true, k_witness_step, (unsigned)(N / per + 1), WT_THREADS, 0, st, x,
+                                 ms64, N, m, from, W.wit, W.wc, W.wrho, hint, W.scal,
+                                 wt_dscale(m0));
     if (e != cudaSuccess) return e;
-    k_witness_hints<<<num_sms * 4, WT_THREADS, 0, st>>>(x, ms64, N, m, W.wit, W.wc, W.wrho, hint,
-                                                       W.scal, wt_dscale(m0));
-    return cudaGetLastError();
+    return paddi_launch(true, k_witness_hints, num_sms * 4, WT_THREADS, 0, st, x, ms64, N, m, W.wit,
+                        W.wc, W.wrho, hint, W.scal, wt_dscale(m0), t_end);
 }
 
 cudaError_t paddi_launch_witness_check(const double2 *ms64, const float *x,
@@ -509,13 +514,11 @@ cudaError_t paddi_launch_witness_check(const double2 *ms64, const float *x,
                                        cudaStream_t st)
 {
     const int per = WT_THREADS * WT_CWIN;
-    k_witness_check<<<(unsigned)((N + per - 1) / per), WT_THREADS, 0, st>>>(W.wrho, N, thr, alive,
-                                                                          fail, &att->n_fail);
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = paddi_launch(true, k_witness_check, (unsigned)((N + per - 1) / per), WT_THREADS,
+                                 0, st, W.wrho, N, thr, alive, fail, att);
     if (e != cudaSuccess) return e;
     const size_t smem = sizeof(float) * (size_t)WT_RWARPS * (size_t)m;
-    k_witness_rescue<<<num_sms * 8, 32 * WT_RWARPS, smem, st>>>(
-        x, ms64, N, m, thr, fail, &att->n_fail, limit, W.wit, W.wc, W.wrho, alive,
-        &att->n_rescued, W.scal, wt_dscale(m0));
-    return cudaGetLastError();
+    return paddi_launch(true, k_witness_rescue, num_sms * 8, 32 * WT_RWARPS, smem, st, x, ms64, N, m,
+                        thr, fail, &att->n_fail, limit, W.wit, W.wc, W.wrho, alive,
+                        &att->n_rescued, W.scal, wt_dscale(m0));
 }

@@ -56,12 +56,10 @@ struct paddi_ctx {
     int device = 0;
     int num_sms = 0;
     cudaStream_t st = nullptr;
-    cudaEvent_t ev[8] = {};
-    cudaEvent_t rev[2] = {}; // around the refine launch
+    cudaEvent_t ev[4] = {}; // ordering against a caller's stream (0, 1), autotuner (2, 3)
     // PADDI_TRACE=1 in the environment: one stderr line per attempt with the
     // candidates entering every refine round
     bool trace = false;
-    cudaEvent_t tev = nullptr;
     PaddiAttemptDev *h_trace = nullptr;
     std::string err;
     size_t cap_n = 0; // series capacity (values)
@@ -89,7 +87,6 @@ struct paddi_ctx {
     PaddiWitness W = {};
     size_t W_cap = 0; // windows
     int wit_m = 0, wit_m0 = 0;
-    int32_t *h_flatcount = nullptr;         // pinned
     // learned r predictor
     bool model_ok = false;
     float model_margin = 1.f;
@@ -99,9 +96,16 @@ struct paddi_ctx {
     float *h_feat = nullptr;                // pinned: features [12] then prediction
     uint32_t *d_rho = nullptr;
     unsigned long long *d_nn64 = nullptr;
-    PaddiAttemptDev *d_att = nullptr;
+    // state of the current attempt: one of two, the selection of each attempt
+    // clears the other (dirty: an attempt broke off before that)
+    PaddiAttemptDev *d_att = nullptr, *d_att2[2] = {nullptr, nullptr};
+    bool att_dirty = false;
+    unsigned long long *d_tprep = nullptr; // time stamps of the current length's preparation
     PaddiAttemptResult *d_res = nullptr;
-    int32_t *d_flatcount = nullptr; // {flat windows, flat span (2), fragile windows}
+    // {flat windows, flat span (2), fragile windows} of the current length: one of
+    // two, the statistics of each length clear the other
+    int32_t *d_flatcount = nullptr, *d_flat2[2] = {nullptr, nullptr};
+    int prep_launches = 0;          // kernels of the current length's preparation
     int32_t *d_frag = nullptr;      // fragile windows of the current length
     PaddiAttemptResult *h_res = nullptr;
     bool umma_ok = false;
@@ -234,8 +238,14 @@ paddi_status ensure_capacity(paddi_ctx *ctx, size_t n)
     return PADDI_OK;
 }
 
+float ms_between(unsigned long long a, unsigned long long b)
+{
+    return a && b > a ? (float)((double)(b - a) * 1e-6) : 0.f;
+}
+
 struct AttemptOut {
     PaddiAttemptResult res;
+    float ms_stats = 0, ms_guide = 0; // the preparation of the length
     float ms_phase1 = 0, ms_refine = 0, ms_select = 0, ms_total = 0;
     float ms_refine_kernel = 0; // the refine launches alone
     int launches = 0;
@@ -266,23 +276,32 @@ float guard_of(const paddi_ctx *ctx, int kernel)
 
 // Statistics of length m for the series in `x` (n values); with `tiles`, also
 // the tensor-core refine's tile data when that kernel serves this length.
-paddi_status run_stats(paddi_ctx *ctx, const float *x, size_t n, int m, bool tiles = true)
+// chained: the stream's previous operation is a kernel of this context.
+paddi_status run_stats(paddi_ctx *ctx, const float *x, size_t n, int m, bool tiles = true,
+                       bool chained = false)
 {
-    // d_flatcount = {flat windows, span of the flat windows (two ints), fragile windows}
-    CK(cudaMemsetAsync(ctx->d_flatcount, 0, 4 * sizeof(int32_t), ctx->st));
-    CK(paddi_launch_stats(x, (int64_t)n, m, ctx->d_wst, ctx->d_mu, ctx->d_ms64,
-                          ctx->d_flat, ctx->d_flatcount, ctx->st, ctx->d_flatcount + 1));
+    const int cur = ctx->d_flatcount == ctx->d_flat2[0] ? 1 : 0;
+    ctx->d_flatcount = ctx->d_flat2[cur];
+    PaddiStatsExtra ex;
+    ex.alive = ctx->d_alive;
+    ex.next = ctx->d_flat2[cur ^ 1];
+    ex.guide = ctx->d_guide;
+    ex.t = ctx->d_tprep + PADDI_T_STATS_B;
+    unsigned long long *t_end = ctx->d_tprep + PADDI_T_STATS_E;
+    CK(paddi_launch_stats(x, (int64_t)n, m, ctx->d_wst, ctx->d_mu, ctx->d_ms64, ctx->d_flat,
+                          ctx->d_flatcount, ctx->st, ctx->d_flatcount + 1, chained, ex));
+    ctx->prep_launches = tiles ? 2 : 1;
     const int kernel = refine_kernel_for(ctx, m);
     // the refine's per-length data: its tiles (tensor cores) and the windows
     // whose rounding bound exceeds the guard band (both refine kernels)
     if (tiles && kernel != PADDI_DIST_FP32)
         CK(paddi_launch_tile_prep(kernel == PADDI_DIST_SPLIT_BF16, x, (int64_t)n, m, ctx->d_wst,
                                   ctx->d_mu, ctx->d_bq, ctx->d_wdq, guard_of(ctx, kernel),
-                                  ctx->d_frag, ctx->d_flatcount + 3, ctx->st));
+                                  ctx->d_frag, ctx->d_flatcount + 3, ctx->st, t_end));
     else if (tiles)
         CK(paddi_launch_fragile_scan_fp32(x, ctx->d_wst, ctx->d_mu, (int32_t)(n - m + 1), m,
                                           guard_of(ctx, kernel), ctx->d_frag,
-                                          ctx->d_flatcount + 3, ctx->num_sms, ctx->st));
+                                          ctx->d_flatcount + 3, ctx->num_sms, ctx->st, t_end));
     return PADDI_OK;
 }
 
@@ -310,7 +329,8 @@ paddi_status witness_to(paddi_ctx *ctx, const float *x, size_t n, int m)
     if (ctx->wit_m == 0 || ctx->wit_m == m) return PADDI_OK;
     CK(paddi_launch_witness_step(x, ctx->d_ms64, (int32_t)(n - m + 1), m,
                                  ctx->wit_m, ctx->wit_m0, ctx->W, ctx->d_list[1],
-                                 ctx->num_sms, ctx->st));
+                                 ctx->num_sms, ctx->st, ctx->d_tprep + PADDI_T_STATS_E));
+    ctx->prep_launches += 2;
     ctx->wit_m = m;
     return PADDI_OK;
 }
@@ -320,7 +340,7 @@ paddi_status witness_to(paddi_ctx *ctx, const float *x, size_t n, int m)
 // length is already known (its ordered image known_ord, from the guide
 // kernel); the recheck skips it.
 paddi_status enqueue_prep(paddi_ctx *ctx, const float *x, size_t n, int m, bool guided,
-                          int32_t w_host);
+                          int32_t w_host, bool chained);
 
 // Phase-1 rows per task for `rows` rows: at most the segment length (the
 // reference's SEGMENT_N; validated at the ABI, rounded up to a multiple of 8),
@@ -373,7 +393,6 @@ paddi_status refine_rounds(paddi_ctx *ctx, const float *x, int32_t N, int m, int
     cudaStream_t st = ctx->st;
     const PaddiWitness *W = ctx->wit_m == m ? &ctx->W : nullptr;
     const PaddiBlockMax B = block_max(ctx, kernel, N, col_lo == 0 && col_hi == N);
-    CK(cudaEventRecord(ctx->rev[0], st));
     if (kernel != PADDI_DIST_FP32)
         CK(paddi_launch_refine_umma(kernel == PADDI_DIST_SPLIT_BF16, x, ctx->d_wst, ctx->d_mu,
                                     ctx->d_cand, ctx->d_list[0], ctx->d_list[1], ctx->d_bq,
@@ -385,12 +404,10 @@ paddi_status refine_rounds(paddi_ctx *ctx, const float *x, int32_t N, int m, int
                                     ctx->d_list[1], ctx->d_att, ctx->d_rho, ctx->d_pruned, N, m,
                                     col_lo, col_hi, thr, guard, ctx->num_sms, st,
                                     ctx->wait_cycles, W));
-    CK(cudaEventRecord(ctx->rev[1], st));
     ++*launches;
     // the fragile windows (skipped by the refine: their rounding bound exceeds
     // the guard band) against the candidates of the last round's list that are
     // still unpruned, in FP64 (the kernel returns at once when there are none)
-    if (ctx->trace) CK(cudaEventRecord(ctx->tev, st));
     CK(paddi_launch_fragile(x, ctx->d_ms64, ctx->d_cand, ctx->d_list[0], ctx->d_list[1],
                             ctx->d_att, ctx->d_pruned, ctx->d_rho, ctx->d_frag,
                             ctx->d_flatcount + 3, m, thr, col_lo, col_hi, ctx->num_sms, st, &B,
@@ -422,19 +439,20 @@ paddi_status select_passes(paddi_ctx *ctx, const float *x, size_t n, int m, floa
                                 st, ctx->d_rho, &B, guard));
         CK(paddi_launch_select(ctx->d_cand, ctx->d_att, ctx->d_rho, ctx->d_pruned,
                                ctx->d_recheck, ctx->d_rcslot, ctx->d_nn64, m, r2, thr, guard,
-                               top_k, ctx->d_flat, ctx->d_res, st));
+                               top_k, ctx->d_flat, ctx->d_flatcount, ctx->d_tprep,
+                               ctx->d_att2[ctx->d_att == ctx->d_att2[0]], ctx->d_res, ctx->h_res,
+                               st));
         *launches += 3;
-        CK(cudaEventRecord(ctx->ev[3], st));
-        CK(cudaMemcpyAsync(&ctx->d_res->n_fragile, ctx->d_flatcount + 3, sizeof(int32_t),
-                           cudaMemcpyDeviceToDevice, st));
-        CK(cudaMemcpyAsync(ctx->h_res, ctx->d_res, sizeof(PaddiAttemptResult),
-                           cudaMemcpyDeviceToHost, st));
+        if (ctx->trace)
+            CK(cudaMemcpyAsync(ctx->h_trace, ctx->d_att, sizeof(PaddiAttemptDev),
+                               cudaMemcpyDeviceToHost, st));
         if (pass == 0 && next_m > 0) {
-            paddi_status s = enqueue_prep(ctx, x, n, next_m, next_guided, -1);
+            paddi_status s = enqueue_prep(ctx, x, n, next_m, next_guided, -1, !ctx->trace);
             if (s != PADDI_OK) return s;
             *spec = true;
         }
         CK(cudaStreamSynchronize(st));
+        ctx->att_dirty = false;
         ctx->last_passes = pass + 1;
         if (ctx->h_res->status == 3) // a refine wait ran out: no redo can help
             return fail(ctx, PADDI_ERR_CUDA, "tensor-core refine: a barrier wait timed out (m=" +
@@ -491,8 +509,11 @@ paddi_status run_attempt(paddi_ctx *ctx, const float *x, size_t n, int m, float 
     const int R = p1_rows_of(ctx, N, m);
     const int chunks = ctx->opts.phase1_chunks ? (int)ctx->opts.phase1_chunks : 12;
     cudaStream_t st = ctx->st;
-    CK(cudaEventRecord(ctx->ev[0], st));
-    CK(cudaMemsetAsync(ctx->d_att, 0, sizeof(PaddiAttemptDev), st));
+    // the attempt's state and the alive flags are clean: the previous attempt's
+    // selection, the statistics and the compaction leave them so
+    ctx->d_att = ctx->d_att2[ctx->d_att == ctx->d_att2[0]];
+    if (ctx->att_dirty) CK(cudaMemsetAsync(ctx->d_att, 0, sizeof(PaddiAttemptDev), st));
+    ctx->att_dirty = true;
     int launches = 0;
     const bool wit = ctx->wit_m == m;
     if (wit) {
@@ -500,15 +521,12 @@ paddi_status run_attempt(paddi_ctx *ctx, const float *x, size_t n, int m, float 
                                       ctx->d_alive, ctx->d_list[0], ctx->d_att, wit_limit(N),
                                       ctx->num_sms, st));
         launches += 2;
-    } else {
-        CK(cudaMemsetAsync(ctx->d_alive, 1, (size_t)N, st));
     }
     CK(paddi_launch_phase1_dev(x, ctx->d_wst, ctx->d_mu, ctx->d_ms64, ctx->d_alive, N, m, R,
                                chunks, thr, 0, N, ctx->d_att, ctx->num_sms, st,
                                wit ? &ctx->W : nullptr, wit_enough(N)));
     ++launches;
-    CK(cudaEventRecord(ctx->ev[1], st));
-    CK(paddi_launch_compact(ctx->d_alive, N, ctx->d_cand, ctx->d_rho, ctx->d_pruned,
+    CK(paddi_launch_compact(ctx->d_alive, !wit, N, ctx->d_cand, ctx->d_rho, ctx->d_pruned,
                             ctx->d_rcslot, ctx->d_att, ctx->d_flat, ctx->d_flatcount + 1, m,
                             r2 > 0.f, st));
     ++launches;
@@ -516,10 +534,6 @@ paddi_status run_attempt(paddi_ctx *ctx, const float *x, size_t n, int m, float 
     out->p1_rows = R;
     paddi_status s = refine_rounds(ctx, x, N, m, kernel, thr, guard, 0, N, &launches);
     if (s != PADDI_OK) return s;
-    CK(cudaEventRecord(ctx->ev[2], st));
-    if (ctx->trace)
-        CK(cudaMemcpyAsync(ctx->h_trace, ctx->d_att, sizeof(PaddiAttemptDev),
-                           cudaMemcpyDeviceToHost, st));
     bool spec = false;
     s = select_passes(ctx, x, n, m, r2, guard, block_max(ctx, kernel, N, true), top_k, known_w, known_ord, next_m, next_guided,
                       &spec, &launches);
@@ -527,15 +541,17 @@ paddi_status run_attempt(paddi_ctx *ctx, const float *x, size_t n, int m, float 
     out->res = *ctx->h_res;
     out->launches = launches;
     if (spec_out) *spec_out = spec;
-    CK(cudaEventElapsedTime(&out->ms_phase1, ctx->ev[0], ctx->ev[1]));
-    CK(cudaEventElapsedTime(&out->ms_refine, ctx->ev[1], ctx->ev[2]));
-    CK(cudaEventElapsedTime(&out->ms_refine_kernel, ctx->rev[0], ctx->rev[1]));
-    CK(cudaEventElapsedTime(&out->ms_select, ctx->ev[2], ctx->ev[3]));
-    CK(cudaEventElapsedTime(&out->ms_total, ctx->ev[0], ctx->ev[3]));
+    const unsigned long long *T = out->res.t, *P = out->res.t_prep;
+    out->ms_stats = ms_between(P[PADDI_T_STATS_B], P[PADDI_T_STATS_E]);
+    out->ms_guide = ms_between(P[PADDI_T_GUIDE_B], P[PADDI_T_GUIDE_E]);
+    out->ms_phase1 = ms_between(T[PADDI_T_BEGIN], T[PADDI_T_COMPACT]);
+    out->ms_refine = ms_between(T[PADDI_T_COMPACT], T[PADDI_T_SELECT]);
+    out->ms_refine_kernel = ms_between(T[PADDI_T_REFINE_B], T[PADDI_T_REFINE_E]);
+    out->ms_select = ms_between(T[PADDI_T_SELECT], T[PADDI_T_END]);
+    out->ms_total = ms_between(T[PADDI_T_BEGIN], T[PADDI_T_END]);
     if (ctx->trace) {
         const PaddiAttemptDev &t = *ctx->h_trace;
-        float fms = 0.f;
-        CK(cudaEventElapsedTime(&fms, ctx->tev, ctx->ev[2]));
+        const float fms = ms_between(T[PADDI_T_FRAGILE], T[PADDI_T_SELECT]);
         std::fprintf(stderr,
                      "paddi-trace m=%d r2=%f unproven=%d-%d p1=%d p1_tasks=%dx%d/%f "
                      "rounds: %d %d %d %d/%f fragile=%d/%f recheck=%d disc=%lld pairs=%llu live=%llu\n",
@@ -576,7 +592,7 @@ void fill_log(paddi_attempt_log *L, int m, float r, float r2, int top_k, const A
     L->p1_pairs = (int64_t)a.res.p1_walked * (int64_t)a.p1_rows * 256;
     L->ms_refine_kernel = a.ms_refine_kernel;
     L->n_fragile = a.res.n_fragile;
-    L->n_launches = a.launches + (ms_stats > 0.f ? 1 : 0);
+    L->n_launches = a.launches;
     L->refine_kernel = a.kernel;
     L->r_source = 0;
     L->ms_guide = 0.f;
@@ -593,12 +609,11 @@ bool valid_lengths(size_t n, uint32_t minL, uint32_t maxL)
            n < (size_t)INT32_MAX - PADDI_PAD_WIN - 64;
 }
 
-// What is known about one length before its first attempt: the timing of
-// its statistics, its flat-window count and, for the guided r policies, the
-// exact FP64 nn of the bound window (the previous length's top-1 window).
+// What is known about one length before its first attempt: its flat-window
+// count and, for the guided r policies, the exact FP64 nn of the bound window
+// (the previous length's top-1 window).
 struct Prep {
     int m = 0;                        // length prepared (0: none)
-    float ms_stats = 0.f, ms_guide = 0.f;
     int32_t flatcount = 0;
     int32_t known_w = -1;             // bound window with a finite exact nn (-1: none)
     unsigned long long known_ord = 0; // its ordered image
@@ -610,52 +625,39 @@ struct Prep {
 // on the device, so this can be queued before the host has read it).  No
 // sync: read_prep collects the values after the next one.
 paddi_status enqueue_prep(paddi_ctx *ctx, const float *x, size_t n, int m, bool guided,
-                          int32_t w_host)
+                          int32_t w_host, bool chained)
 {
-    const int32_t N = (int32_t)(n - m + 1);
-    CK(cudaEventRecord(ctx->ev[4], ctx->st));
-    paddi_status s = run_stats(ctx, x, n, m);
+    paddi_status s = run_stats(ctx, x, n, m, true, chained);
     if (s != PADDI_OK) return s;
     s = witness_to(ctx, x, n, m);
     if (s != PADDI_OK) return s;
-    CK(cudaEventRecord(ctx->ev[5], ctx->st));
-    CK(cudaMemcpyAsync(ctx->h_flatcount, ctx->d_flatcount, sizeof(int32_t),
-                       cudaMemcpyDeviceToHost, ctx->st));
     if (guided) {
-        CK(cudaEventRecord(ctx->ev[6], ctx->st));
-        CK(paddi_launch_guide(x, ctx->d_ms64, ctx->d_flat, N, m, ctx->d_res, w_host,
-                              ctx->d_guide, ctx->d_G, ctx->G_cap, ctx->num_sms, ctx->st));
-        CK(cudaMemcpyAsync(ctx->h_guide, ctx->d_guide, sizeof(PaddiGuide),
-                           cudaMemcpyDeviceToHost, ctx->st));
-        CK(cudaEventRecord(ctx->ev[7], ctx->st));
+        CK(paddi_launch_guide(x, ctx->d_ms64, ctx->d_flat, (int32_t)(n - m + 1), m, ctx->d_res,
+                              w_host, ctx->d_guide, ctx->d_G, ctx->G_cap, ctx->num_sms, ctx->st,
+                              ctx->h_guide, ctx->d_flatcount, ctx->d_tprep));
+        ctx->prep_launches += 2;
     }
     return PADDI_OK;
 }
 
-// After a sync that covers enqueue_prep(m, guided).
-paddi_status read_prep(paddi_ctx *ctx, int m, bool guided, Prep *p)
+// After a sync that covers enqueue_prep(m, guided = true).
+void read_prep(paddi_ctx *ctx, int m, Prep *p)
 {
     *p = Prep();
     p->m = m;
-    CK(cudaEventElapsedTime(&p->ms_stats, ctx->ev[4], ctx->ev[5]));
-    p->flatcount = *ctx->h_flatcount;
-    if (guided) {
-        CK(cudaEventElapsedTime(&p->ms_guide, ctx->ev[6], ctx->ev[7]));
-        const unsigned long long u = ctx->h_guide->nn_ord;
-        const unsigned long long bits =
-            (u & 0x8000000000000000ull) ? (u & 0x7fffffffffffffffull) : ~u;
-        double d;
-        std::memcpy(&d, &bits, sizeof(d));
-        if (ctx->h_guide->w_used >= 0 && std::isfinite(d)) {
-            p->known_w = ctx->h_guide->w_used;
-            p->known_ord = u;
-            p->lb = d;
-        }
-        if (ctx->trace)
-            std::fprintf(stderr, "paddi-guide m=%d w=%d mode=%d ms=%f\n", m,
-                         ctx->h_guide->w_used, ctx->h_guide->mode, p->ms_guide);
+    p->flatcount = ctx->h_guide->n_flat;
+    const unsigned long long u = ctx->h_guide->nn_ord;
+    const unsigned long long bits = (u & 0x8000000000000000ull) ? (u & 0x7fffffffffffffffull) : ~u;
+    double d;
+    std::memcpy(&d, &bits, sizeof(d));
+    if (ctx->h_guide->w_used >= 0 && std::isfinite(d)) {
+        p->known_w = ctx->h_guide->w_used;
+        p->known_ord = u;
+        p->lb = d;
     }
-    return PADDI_OK;
+    if (ctx->trace)
+        std::fprintf(stderr, "paddi-guide m=%d w=%d mode=%d\n", m, ctx->h_guide->w_used,
+                     ctx->h_guide->mode);
 }
 
 // MERLIN's first r for length minL + j (src/main.cu:38, 171, 202-214): a pure
@@ -806,19 +808,18 @@ paddi_status palmad_impl(paddi_ctx *ctx, const float *x, size_t n, uint32_t minL
         //      evaluated exactly at this length: its nn is a lower bound on
         //      this length's top-1 distance)
         const bool g_here = guided && j >= 1 && out[j - 1].ind >= 0;
-        bool need_read = false;
         if (pre.m != m) {
             const int32_t w = g_here ? (out[j - 1].ind < N ? out[j - 1].ind : N - 1) : -1;
-            s = enqueue_prep(ctx, x, n, m, g_here, w);
+            s = enqueue_prep(ctx, x, n, m, g_here, w, false);
             if (s != PADDI_OK) return s;
-            if (g_here || ahead) { // (queueing ahead re-records the prep events)
+            if (g_here) {
                 CK(cudaStreamSynchronize(ctx->st));
-                s = read_prep(ctx, m, g_here, &pre);
-                if (s != PADDI_OK) return s;
+                read_prep(ctx, m, &pre);
             } else {
-                need_read = true; // read after the first attempt's sync
+                pre = Prep(); // nothing is known before the first attempt
             }
         }
+        const int prep_launches = ctx->prep_launches;
         Prep cur = pre; // the next length's values may replace pre during the attempts
         pre.m = 0;
         float S = 0.f;
@@ -826,7 +827,7 @@ paddi_status palmad_impl(paddi_ctx *ctx, const float *x, size_t n, uint32_t minL
         // ---- guidance: the bound and / or the model's prediction
         float lbf = 0.f, lbm = 0.f; // lbm: largest r^2 below the bound
         int source = 0;
-        if (!need_read && cur.known_w >= 0 && cur.lb > 0.0) {
+        if (cur.known_w >= 0 && cur.lb > 0.0) {
             lbf = (float)std::fmin(cur.lb, (double)FLT_MAX);
             const float rb = r_below(lbf);
             lbm = rb * rb;
@@ -881,24 +882,20 @@ paddi_status palmad_impl(paddi_ctx *ctx, const float *x, size_t n, uint32_t minL
                             &spec);
             if (s != PADDI_OK) return s;
             stale = spec;
-            if (need_read) {
-                s = read_prep(ctx, m, false, &cur);
-                if (s != PADDI_OK) return s;
-                need_read = false;
-            }
+            cur.flatcount = a.res.n_flat;
             if (a.res.n_sel > 0) {
                 out[j].ind = a.res.sel_ind[0];
                 out[j].dist = a.res.sel_dist[0];
             }
             if (log && nl < log_cap) {
-                fill_log(&log[nl], m, r, r2, 1, a, first ? cur.ms_stats : 0.f);
+                fill_log(&log[nl], m, r, r2, 1, a, first ? a.ms_stats : 0.f);
                 log[nl].r_source = source;
                 log[nl].lb = lbf;
                 log[nl].flat_frac = (float)cur.flatcount / (float)N;
                 if (first) {
-                    log[nl].ms_guide = cur.ms_guide;
-                    log[nl].ms_total += cur.ms_guide;
-                    log[nl].n_launches += (lbf > 0.f ? 1 : 0) + (source == 1 ? 1 : 0);
+                    if (g_here) log[nl].ms_guide = a.ms_guide;
+                    log[nl].ms_total += log[nl].ms_guide;
+                    log[nl].n_launches += prep_launches + (source == 1 ? 1 : 0);
                 }
             }
             ++nl;
@@ -922,8 +919,7 @@ paddi_status palmad_impl(paddi_ctx *ctx, const float *x, size_t n, uint32_t minL
             }
         }
         if (spec) { // the last attempt queued the next length
-            s = read_prep(ctx, m + 1, guided, &pre);
-            if (s != PADDI_OK) return s;
+            read_prep(ctx, m + 1, &pre);
         }
         prev_attempts = it;
         if (prof_fn) {
@@ -1004,23 +1000,28 @@ PADDI_API paddi_status paddi_ctx_create(paddi_ctx **out, const paddi_opts *opts)
     }
     bool ok = cudaStreamCreateWithFlags(&ctx->st, cudaStreamNonBlocking) == cudaSuccess;
     for (auto &e : ctx->ev) ok = ok && cudaEventCreate(&e) == cudaSuccess;
-    for (auto &e : ctx->rev) ok = ok && cudaEventCreate(&e) == cudaSuccess;
     {
         const char *tr = std::getenv("PADDI_TRACE");
         ctx->trace = tr && tr[0] && tr[0] != '0';
     }
     if (ctx->trace) {
-        ok = ok && cudaEventCreate(&ctx->tev) == cudaSuccess;
         ok = ok && cudaMallocHost(&ctx->h_trace, sizeof(PaddiAttemptDev)) == cudaSuccess;
     }
-    ok = ok && cudaMalloc(&ctx->d_att, sizeof(PaddiAttemptDev)) == cudaSuccess;
+    for (int k = 0; k < 2; ++k) {
+        ok = ok && cudaMalloc(&ctx->d_att2[k], sizeof(PaddiAttemptDev)) == cudaSuccess;
+        ok = ok && cudaMemset(ctx->d_att2[k], 0, sizeof(PaddiAttemptDev)) == cudaSuccess;
+        ok = ok && cudaMalloc(&ctx->d_flat2[k], 4 * sizeof(int32_t)) == cudaSuccess;
+        ok = ok && cudaMemset(ctx->d_flat2[k], 0, 4 * sizeof(int32_t)) == cudaSuccess;
+    }
+    ctx->d_att = ctx->d_att2[0];
+    ctx->d_flatcount = ctx->d_flat2[0];
     ok = ok && cudaMalloc(&ctx->d_res, sizeof(PaddiAttemptResult)) == cudaSuccess;
-    ok = ok && cudaMalloc(&ctx->d_flatcount, 4 * sizeof(int32_t)) == cudaSuccess;
+    ok = ok && cudaMalloc(&ctx->d_tprep, PADDI_T_PREP * sizeof(unsigned long long)) == cudaSuccess;
+    ok = ok && cudaMemset(ctx->d_tprep, 0, PADDI_T_PREP * sizeof(unsigned long long)) == cudaSuccess;
     ok = ok && cudaMallocHost(&ctx->h_res, sizeof(PaddiAttemptResult)) == cudaSuccess;
     ok = ok && cudaMalloc(&ctx->d_guide, sizeof(PaddiGuide)) == cudaSuccess;
     ok = ok && cudaMemset(ctx->d_guide, 0, sizeof(PaddiGuide)) == cudaSuccess;
     ok = ok && cudaMallocHost(&ctx->h_guide, sizeof(PaddiGuide)) == cudaSuccess;
-    ok = ok && cudaMallocHost(&ctx->h_flatcount, sizeof(int32_t)) == cudaSuccess;
     ok = ok && cudaMalloc(&ctx->d_model, sizeof(float) * MLP_NPARAM) == cudaSuccess;
     ok = ok && cudaMalloc(&ctx->d_model_bf16, 2 * MLP_NPARAM) == cudaSuccess;
     ok = ok && cudaMalloc(&ctx->d_feat, sizeof(float) * 16) == cudaSuccess;
@@ -1041,22 +1042,21 @@ PADDI_API paddi_status paddi_ctx_destroy(paddi_ctx *ctx)
     cudaSetDevice(ctx->device);
     if (ctx->st) cudaStreamSynchronize(ctx->st);
     free_buffers(ctx);
-    dfree(ctx->d_att);
+    for (int k = 0; k < 2; ++k) {
+        dfree(ctx->d_att2[k]);
+        dfree(ctx->d_flat2[k]);
+    }
     dfree(ctx->d_res);
-    dfree(ctx->d_flatcount);
+    dfree(ctx->d_tprep);
     dfree(ctx->d_guide);
     dfree(ctx->d_model);
     if (ctx->d_model_bf16) cudaFree(ctx->d_model_bf16);
     dfree(ctx->d_feat);
     dfree(ctx->d_pred);
     if (ctx->h_feat) cudaFreeHost(ctx->h_feat);
-    if (ctx->h_flatcount) cudaFreeHost(ctx->h_flatcount);
     if (ctx->h_guide) cudaFreeHost(ctx->h_guide);
     if (ctx->h_res) cudaFreeHost(ctx->h_res);
     for (auto &e : ctx->ev)
-        if (e) cudaEventDestroy(e);
-    if (ctx->tev) cudaEventDestroy(ctx->tev);
-    for (auto &e : ctx->rev)
         if (e) cudaEventDestroy(e);
     if (ctx->h_trace) cudaFreeHost(ctx->h_trace);
     if (ctx->st) cudaStreamDestroy(ctx->st);
@@ -1144,9 +1144,7 @@ PADDI_API paddi_status paddi_pd3(paddi_ctx *ctx, const float *series, size_t n, 
     const uint32_t saved_seg = ctx->opts.segment_len;
     if (segment_len) ctx->opts.segment_len = segment_len;
     CK(cudaMemcpyAsync(ctx->d_x, series, sizeof(float) * n, cudaMemcpyHostToDevice, ctx->st));
-    CK(cudaEventRecord(ctx->ev[4], ctx->st));
     s = run_stats(ctx, ctx->d_x, n, (int)m);
-    CK(cudaEventRecord(ctx->ev[5], ctx->st));
     if (s != PADDI_OK) {
         ctx->opts.segment_len = saved_seg;
         return s;
@@ -1167,9 +1165,10 @@ PADDI_API paddi_status paddi_pd3(paddi_ctx *ctx, const float *series, size_t n, 
             ctx->opts.segment_len = saved_seg;
             return s;
         }
-        float ms_stats = 0.f;
-        if (it == 0) CK(cudaEventElapsedTime(&ms_stats, ctx->ev[4], ctx->ev[5]));
-        if (log && nl < log_cap) fill_log(&log[nl], (int)m, rr, r2, (int)top_k, a, ms_stats);
+        if (log && nl < log_cap) {
+            fill_log(&log[nl], (int)m, rr, r2, (int)top_k, a, it == 0 ? a.ms_stats : 0.f);
+            if (it == 0) log[nl].n_launches += ctx->prep_launches;
+        }
         ++nl;
         const bool found = a.res.n_sel >= (int)top_k;
         if (!halving || found || r2 == 0.f) break; // r2 == 0 admits every nn > 0
@@ -1196,16 +1195,16 @@ PADDI_API paddi_status paddi_compute_statistics(paddi_ctx *ctx, const float *d_T
     if (s != PADDI_OK) return s;
     cudaStream_t user = stream ? (cudaStream_t)stream : ctx->st;
     if (user != ctx->st) { // order the context stream after the caller's
-        CK(cudaEventRecord(ctx->ev[4], user));
-        CK(cudaStreamWaitEvent(ctx->st, ctx->ev[4], 0));
+        CK(cudaEventRecord(ctx->ev[0], user));
+        CK(cudaStreamWaitEvent(ctx->st, ctx->ev[0], 0));
     }
     s = run_stats(ctx, d_T, n, (int)m, /*tiles=*/false);
     if (s != PADDI_OK) return s;
     CK(paddi_launch_export_stats(ctx->d_ms64, (int32_t)(n - m + 1), (int)m, d_mean,
                                  d_std, ctx->st));
     if (user != ctx->st) {
-        CK(cudaEventRecord(ctx->ev[5], ctx->st));
-        CK(cudaStreamWaitEvent(user, ctx->ev[5], 0));
+        CK(cudaEventRecord(ctx->ev[1], ctx->st));
+        CK(cudaStreamWaitEvent(user, ctx->ev[1], 0));
     }
     return PADDI_OK;
 }
@@ -1222,8 +1221,8 @@ PADDI_API paddi_status paddi_do_pd3(paddi_ctx *ctx, const float *d_T, size_t n, 
     if (s != PADDI_OK) return s;
     cudaStream_t user = stream ? (cudaStream_t)stream : ctx->st;
     if (user != ctx->st) {
-        CK(cudaEventRecord(ctx->ev[4], user));
-        CK(cudaStreamWaitEvent(ctx->st, ctx->ev[4], 0));
+        CK(cudaEventRecord(ctx->ev[0], user));
+        CK(cudaStreamWaitEvent(ctx->st, ctx->ev[0], 0));
     }
     s = run_stats(ctx, d_T, n, (int)m);
     if (s != PADDI_OK) return s;
@@ -1234,8 +1233,8 @@ PADDI_API paddi_status paddi_do_pd3(paddi_ctx *ctx, const float *d_T, size_t n, 
                             ctx->d_nn64, ctx->d_flat, (int32_t)(n - m + 1), (int)m, r2, d_is_cand,
                             d_nnDist, ctx->st));
     if (user != ctx->st) {
-        CK(cudaEventRecord(ctx->ev[5], ctx->st));
-        CK(cudaStreamWaitEvent(user, ctx->ev[5], 0));
+        CK(cudaEventRecord(ctx->ev[1], ctx->st));
+        CK(cudaStreamWaitEvent(user, ctx->ev[1], 0));
     } else {
         CK(cudaStreamSynchronize(ctx->st));
     }
@@ -1292,7 +1291,7 @@ PADDI_API paddi_status paddi_shard_refine(paddi_ctx *ctx, const float *d_series,
     const int kernel = refine_kernel_for(ctx, (int)m);
     const float thr = thr_of(r2, (int)m);
     CK(cudaMemsetAsync(ctx->d_att, 0, sizeof(PaddiAttemptDev), st));
-    CK(paddi_launch_compact(d_alive, (int32_t)N, ctx->d_cand, ctx->d_rho, ctx->d_pruned,
+    CK(paddi_launch_compact(const_cast<uint8_t *>(d_alive), false, (int32_t)N, ctx->d_cand, ctx->d_rho, ctx->d_pruned,
                             ctx->d_rcslot, ctx->d_att, ctx->d_flat, ctx->d_flatcount + 1, (int)m,
                             r2 > 0.f, st));
     int launches = 0;
@@ -1347,8 +1346,6 @@ PADDI_API paddi_status paddi_shard_select(paddi_ctx *ctx, const float *d_series,
     ctx->h_res->n_p1 = (int32_t)count;
     CK(cudaMemcpyAsync(&ctx->d_att->n_cand_p1, &ctx->h_res->n_p1, sizeof(int32_t),
                        cudaMemcpyHostToDevice, st));
-    CK(cudaEventRecord(ctx->ev[0], st));
-    CK(cudaEventRecord(ctx->ev[2], st));
     int launches = 0;
     bool spec = false;
     paddi_status s = select_passes(ctx, d_series, n, (int)m, r2, guard_of(ctx, kernel), {},
@@ -1358,7 +1355,7 @@ PADDI_API paddi_status paddi_shard_select(paddi_ctx *ctx, const float *d_series,
     a.res = *ctx->h_res;
     a.launches = launches;
     a.kernel = kernel;
-    CK(cudaEventElapsedTime(&a.ms_select, ctx->ev[2], ctx->ev[3]));
+    a.ms_select = ms_between(a.res.t[PADDI_T_SELECT], a.res.t[PADDI_T_END]);
     a.ms_total = a.ms_select;
     *n_out = (uint32_t)a.res.n_sel;
     for (int q = 0; q < a.res.n_sel; ++q) {
@@ -1688,16 +1685,16 @@ PADDI_API paddi_status paddi_autotune(paddi_ctx *ctx, const float *series, size_
                 for (size_t p = 0; p < probes.size(); ++p) {
                     const uint32_t a = probes[p].first, b = probes[p].second;
                     out.assign(b - a + 1, paddi_discord{-1, -FLT_MAX});
-                    CK(cudaEventRecord(ctx->ev[6], ctx->st));
+                    CK(cudaEventRecord(ctx->ev[2], ctx->st));
                     s = palmad_impl(ctx, ctx->d_x, n, a, b, out.data(), nullptr, 0, nullptr);
                     if (s != PADDI_OK) {
                         ctx->opts = saved;
                         return s;
                     }
-                    CK(cudaEventRecord(ctx->ev[7], ctx->st));
-                    CK(cudaEventSynchronize(ctx->ev[7]));
+                    CK(cudaEventRecord(ctx->ev[3], ctx->st));
+                    CK(cudaEventSynchronize(ctx->ev[3]));
                     float t = 0.f;
-                    CK(cudaEventElapsedTime(&t, ctx->ev[6], ctx->ev[7]));
+                    CK(cudaEventElapsedTime(&t, ctx->ev[2], ctx->ev[3]));
                     t_total += t;
                     if (pass == 1) {
                         if (ref.size() <= p) ref.push_back(out);

@@ -25,6 +25,36 @@
 
 namespace paddi {
 
+// ---- launches in a chain.  A kernel of an attempt starts while the one
+// before it drains (programmatic stream serialization): its first act is to
+// wait until that kernel is complete and its writes are visible, its second to
+// let the next kernel come in as soon as all of its own blocks run.  Saves the
+// launch latency between dependent kernels, about 2 us each; an attempt has a
+// dozen of 2 to 60 us.
+__device__ __forceinline__ void chain_begin()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// Time stamps instead of events between the kernels: a stamp costs one store,
+// an event a break in the stream.
+__device__ __forceinline__ unsigned long long time_ns()
+{
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+__device__ __forceinline__ void stamp_begin(unsigned long long *t)
+{
+    if (t && blockIdx.x == 0 && threadIdx.x == 0) *t = time_ns();
+}
+// by one thread of every block, when the block is done
+__device__ __forceinline__ void stamp_end(unsigned long long *t)
+{
+    if (t) atomicMax(t, time_ns());
+}
+
 // Monotone map float -> uint32 so that unsigned max == float max.
 __device__ __forceinline__ uint32_t f2ord(float f)
 {
@@ -79,6 +109,30 @@ struct PaddiBound {
 PaddiBound paddi_bound_tc(int m, bool bf16);
 PaddiBound paddi_bound_fp32(int m);
 
+// Launches `kern`; chained: as the successor of the stream's previous kernel (see
+// paddi::chain_begin, which the kernel must call first).
+template <typename... P, typename... A>
+cudaError_t paddi_launch(bool chained, void (*kern)(P...), unsigned grid, unsigned block,
+                         size_t smem, cudaStream_t st, A... args)
+{
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(block);
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    c.attrs = &at;
+    c.numAttrs = chained ? 1 : 0;
+    return cudaLaunchKernelEx(&c, kern, P(args)...);
+}
+
+// Time stamps (ns, globaltimer) of a length's preparation and of an attempt.
+enum { PADDI_T_STATS_B, PADDI_T_STATS_E, PADDI_T_GUIDE_B, PADDI_T_GUIDE_E, PADDI_T_PREP };
+enum { PADDI_T_BEGIN, PADDI_T_COMPACT, PADDI_T_REFINE_B, PADDI_T_REFINE_E, PADDI_T_FRAGILE,
+       PADDI_T_SELECT, PADDI_T_END, PADDI_T_ATTEMPT };
+
 // Per-attempt device-side state shared by the kernels of one (m, r) attempt.
 struct PaddiAttemptDev {
     int32_t n_cand_p1;      // candidates after phase 1 (compacted list length)
@@ -99,7 +153,9 @@ struct PaddiAttemptDev {
     int32_t last_rd;        // the round after which no window was left
     unsigned long long n_pairs; // pairs evaluated by the refine (instrumentation)
     unsigned long long n_live;  // of those, pairs of candidates still unpruned at the tile's start
+    unsigned long long t[PADDI_T_ATTEMPT]; // time stamps
 };
+static_assert(sizeof(PaddiAttemptDev) % 4 == 0, "cleared in words");
 
 namespace paddi {
 
@@ -197,7 +253,8 @@ __device__ __forceinline__ int wait_round(PaddiAttemptDev *att, int rd, long lon
 
 } // namespace paddi
 
-// Result of one attempt, copied to the host at the end of the attempt.
+// Result of one attempt; the selection writes it to device and to pinned host
+// memory.
 struct PaddiAttemptResult {
     int64_t n_cand;  // windows with nn >= r2 (never pruned)
     int64_t n_disc;  // windows with nn > r2
@@ -211,7 +268,11 @@ struct PaddiAttemptResult {
     unsigned long long n_live;  // of those, pairs of candidates live at the tile's start
     int32_t p1_walked;          // phase-1 tasks that walked their rows
     int32_t n_fragile;          // windows the refine left to the FP64 fragile pass
+    int32_t n_flat;             // flat windows of the length
+    int32_t n_unproven;         // windows without a proving witness
+    unsigned long long t_prep[PADDI_T_PREP], t[PADDI_T_ATTEMPT]; // time stamps
 };
+static_assert(sizeof(PaddiAttemptResult) % 4 == 0, "copied in words");
 
 // Incremental FP64 nn of the r policy's bound window (k_guide.cu): the state
 // of the shifted dot products G (two buffers), the launch's result, and
@@ -225,6 +286,8 @@ struct PaddiGuide {
     int32_t cur, age;          // state: buffer holding G, slides since the last build
     int32_t w_used, mode;      // result: window of the launch (-1: skipped), PADDI_GUIDE_*
     int32_t done, item;        // kernel counters (zero between launches)
+    int32_t n_flat;            // host copy only: flat windows of the length
+    int32_t pad;
 };
 
 // Block maxima of the tensor-core refine: for candidate c and half block h
@@ -276,10 +339,20 @@ __device__ __forceinline__ void wt_hint(const PaddiWitness &W, int i, int kind, 
 
 // ---------------------------------------------------------------- launches
 // All launch wrappers enqueue on `st` and return cudaGetLastError().
+// What the statistics kernel also prepares for the kernels after it (all
+// optional): alive[0..N) = 1; `next`, the counters of the next length, zeroed
+// (4 ints); the guide's result reset; the time stamp of its start.
+struct PaddiStatsExtra {
+    uint8_t *alive = nullptr;
+    int32_t *next = nullptr;
+    PaddiGuide *guide = nullptr;
+    unsigned long long *t = nullptr;
+};
 cudaError_t paddi_launch_stats(const float *x, int64_t n, int32_t m, float4 *wst, float *mu,
                                double2 *ms64, uint8_t *flat,
                                int32_t *flat_count, cudaStream_t st,
-                               int32_t *flat_span = nullptr);
+                               int32_t *flat_span = nullptr, bool chained = false,
+                               const PaddiStatsExtra &extra = PaddiStatsExtra());
 // flat_span (optional): two zeroed ints that receive {INT_MAX - lowest flat
 // window, highest flat window + 1} (both stay 0 without flat windows).
 
@@ -291,7 +364,7 @@ cudaError_t paddi_launch_witness_start(const float *x, int64_t n, int32_t N, con
 cudaError_t paddi_launch_witness_step(const float *x, const double2 *ms64,
                                       int32_t N, int32_t m, int32_t from, int32_t m0,
                                       const PaddiWitness &W, int32_t *hint, int32_t num_sms,
-                                      cudaStream_t st);
+                                      cudaStream_t st, unsigned long long *t_end = nullptr);
 // Writes alive[0..N) from the witnesses at threshold thr and looks for new
 // witnesses of the others (listed in fail) while they are at most `limit`.
 cudaError_t paddi_launch_witness_check(const double2 *ms64, const float *x,
@@ -314,9 +387,10 @@ cudaError_t paddi_launch_phase1_dev(const float *x, const float4 *wst, const flo
                                     cudaStream_t st, const PaddiWitness *W = nullptr,
                                     int32_t enough = 0);
 
+// reset: alive[] is all ones again when the kernel is done.
 // prune_flats (r^2 > 0): flat windows with another flat window at least m-1
 // away are dropped (distance 0); flat_span as filled by paddi_launch_stats.
-cudaError_t paddi_launch_compact(const uint8_t *alive, int32_t N, int32_t *cand,
+cudaError_t paddi_launch_compact(uint8_t *alive, bool reset, int32_t N, int32_t *cand,
                                  uint32_t *rho_max, uint8_t *pruned, int32_t *rc_slot,
                                  PaddiAttemptDev *att, const uint8_t *flat,
                                  const int32_t *flat_span, int32_t m, bool prune_flats,
@@ -339,7 +413,8 @@ cudaError_t paddi_launch_refine_fp32(const float *x, const float4 *wst, const fl
 // frag_list (frag_count zeroed by the caller).
 cudaError_t paddi_launch_fragile_scan_fp32(const float *x, const float4 *wst, const float *mu,
                                            int32_t N, int32_t m, float gcap, int32_t *frag_list,
-                                           int32_t *frag_count, int32_t num_sms, cudaStream_t st);
+                                           int32_t *frag_count, int32_t num_sms, cudaStream_t st,
+                                           unsigned long long *t_end = nullptr);
 
 // Exact FP64 correlations of the refine's unpruned candidates with the fragile
 // windows in [col_lo, col_hi) (k_fragile.cu): prunes and raises rho_max.  The
@@ -347,7 +422,7 @@ cudaError_t paddi_launch_fragile_scan_fp32(const float *x, const float4 *wst, co
 // else list0, list_count[last_rd] entries; round 0: all candidates).
 cudaError_t paddi_launch_fragile(const float *x, const double2 *ms64, const int32_t *cand,
                                  const int32_t *list0, const int32_t *list1,
-                                 const PaddiAttemptDev *att, uint8_t *pruned, uint32_t *rho_max, const int32_t *frag,
+                                 PaddiAttemptDev *att, uint8_t *pruned, uint32_t *rho_max, const int32_t *frag,
                                  const int32_t *frag_count, int32_t m, float thr, int32_t col_lo,
                                  int32_t col_hi, int32_t num_sms, cudaStream_t st,
                                  const PaddiBlockMax *B = nullptr, float guard = 0.f);
@@ -383,7 +458,7 @@ int64_t paddi_tile_wd_entries();
 cudaError_t paddi_launch_tile_prep(bool bf16, const float *x, int64_t n, int32_t m,
                                    const float4 *wst, const float *mu, uint16_t *bq, float4 *wdq,
                                    float gcap, int32_t *frag_list, int32_t *frag_count,
-                                   cudaStream_t st);
+                                   cudaStream_t st, unsigned long long *t_end = nullptr);
 
 cudaError_t paddi_launch_finalize(const int32_t *cand, PaddiAttemptDev *att,
                                   const uint32_t *rho_max, const uint8_t *pruned, int32_t m,
@@ -400,12 +475,16 @@ cudaError_t paddi_launch_recheck(const float *x, const double2 *ms64,
                                  int32_t num_sms, int32_t known_w, cudaStream_t st,
                                  const uint32_t *rho_max, const PaddiBlockMax *B, float guard);
 
+// flat_count: {flat windows, span (2), fragile windows}; next: the state of the
+// next attempt, cleared here; host: pinned copy of *res.
 cudaError_t paddi_launch_select(const int32_t *cand, PaddiAttemptDev *att,
                                 const uint32_t *rho_max, const uint8_t *pruned,
                                 const int32_t *recheck, const int32_t *rc_slot,
                                 const unsigned long long *nn64_ord, int32_t m, float r2,
                                 float thr, float guard, int32_t top_k, const uint8_t *flat,
-                                PaddiAttemptResult *res, cudaStream_t st);
+                                const int32_t *flat_count, const unsigned long long *t_prep,
+                                PaddiAttemptDev *next, PaddiAttemptResult *res,
+                                PaddiAttemptResult *host, cudaStream_t st);
 
 // with_w: room for the flat-window column data (false only when the length is
 // known to have no flat window).
@@ -414,11 +493,14 @@ size_t paddi_phase1_smem(int R, int m);
 // Exact FP64 nn at length m of window w_host (w_host < 0: the top-1 window
 // of the attempt result `prev`, skipped when it has none), through the shifted
 // dot products (two buffers G of N doubles each, G + g_stride the second) and
-// their state in g; result in g->nn_ord.
+// their state in g; result in g->nn_ord (all ones on entry: paddi_launch_stats
+// resets it), copied to pinned memory at `host` with the flat-window count.
 cudaError_t paddi_launch_guide(const float *x, const double2 *ms64,
                                const uint8_t *flat, int32_t N, int32_t m,
                                const PaddiAttemptResult *prev, int32_t w_host, PaddiGuide *g,
-                               double *G, size_t g_stride, int32_t num_sms, cudaStream_t st);
+                               double *G, size_t g_stride, int32_t num_sms, cudaStream_t st,
+                               PaddiGuide *host, const int32_t *flat_count,
+                               unsigned long long *t);
 
 cudaError_t paddi_launch_export_stats(const double2 *ms64, int32_t N,
                                       int32_t m, float *mean, float *sd, cudaStream_t st);
