@@ -17,13 +17,17 @@
 // candidate (the margin covers the FP32 rounding of thr); every value enters
 // the candidate's kept maximum.
 //
-// Work items: (a group of 8 entries of the candidate list, 256 consecutive
+// Work items: (a group of 8 entries of the candidate list, 64 consecutive
 // entries of the fragile list).  The group's centred candidate values sit in
-// shared memory (read as broadcasts, two terms per load); each thread owns
-// one fragile window, reads its values once per 4-candidate half of the group
-// straight from the series (consecutive addresses per thread, so 7 of 8
-// loads hit L1) and keeps 4 FP64 accumulators.  Halves whose candidates are
-// all pruned, and items with no live candidate, are skipped.
+// shared memory (read as broadcasts, two terms per load); a fragile window is
+// shared by four threads, two halves of the group times two halves of the
+// length, each with 4 FP64 accumulators and reading the window's values straight
+// from the series (consecutive addresses per thread, so 7 of 8 loads hit L1).
+// What bounds it is the serial chain of one thread, not FP64 issue: a headline
+// attempt has about 3000 fragile windows and a dozen candidates, 100 items for
+// 592 resident CTAs; with one thread per window and both halves in turn it took
+// 25 us, now 5.  Halves whose candidates are all pruned, and items
+// with no live candidate, are skipped.
 #include <float.h>
 
 #include "paddi_internal.cuh"
@@ -33,7 +37,8 @@ using paddi::ord2f;
 
 namespace {
 
-constexpr int FG_THREADS = 256; // fragile windows per item (one per thread)
+constexpr int FG_THREADS = 256;
+constexpr int FG_WIN = 64;      // fragile windows per item
 constexpr int FG_CAND = 8;      // candidate-list entries per item
 constexpr int FG_HALF = 4;      // accumulators per thread
 constexpr int FG_MAXM = 1024;
@@ -51,7 +56,7 @@ k_fragile(const float *__restrict__ x, const double2 *__restrict__ ms64,
     extern __shared__ __align__(16) double fg_a[];
     __shared__ int cw[FG_CAND], cp[FG_CAND], live[FG_CAND];
     __shared__ double civ[FG_CAND];
-    __shared__ double best_s[FG_CAND][FG_THREADS / 32];
+    __shared__ double best_s[FG_CAND][4];
     __shared__ int s_any;
     paddi::chain_begin();
     paddi::stamp_begin(att->t + PADDI_T_FRAGILE);
@@ -63,7 +68,7 @@ k_fragile(const float *__restrict__ x, const double2 *__restrict__ ms64,
     const bool bkeep = B.kept(att->n_cand_p1);
     const int mp = (m + 1) & ~1;
     const int groups = (C + FG_CAND - 1) / FG_CAND;
-    const int chunks = (F + FG_THREADS - 1) / FG_THREADS;
+    const int chunks = (F + FG_WIN - 1) / FG_WIN;
     const long long total = (long long)groups * chunks;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     for (long long item = blockIdx.x; item < total; item += gridDim.x) {
@@ -88,64 +93,67 @@ k_fragile(const float *__restrict__ x, const double2 *__restrict__ ms64,
             fg_a[e] = (live[c] && k < m) ? (double)x[cw[c] + k] - ms64[cw[c]].x : 0.0;
         }
         __syncthreads();
-        const int fi = chunk * FG_THREADS + t;
+        // warp: half of the group (h), 16 windows; lane: window, half of the length (s)
+        const int h = warp & 1, wsub = warp >> 1, s = lane >> 4;
+        const int fi = chunk * FG_WIN + 16 * wsub + (lane & 15);
         const int f = fi < F ? frag[fi] : -1;
         const bool fok = f >= col_lo && f < col_hi;
-        double b[FG_CAND];
+        const int c0 = h * FG_HALF;
+        double b[FG_HALF];
 #pragma unroll
-        for (int c = 0; c < FG_CAND; ++c) b[c] = -INFINITY;
+        for (int c = 0; c < FG_HALF; ++c) b[c] = -INFINITY;
+        bool any = false; // uniform over the warp
 #pragma unroll
-        for (int h = 0; h < FG_CAND / FG_HALF; ++h) {
-            const int c0 = h * FG_HALF;
-            bool any = false;
-#pragma unroll
-            for (int c = 0; c < FG_HALF; ++c) any |= live[c0 + c] != 0;
-            if (!any || !fok) continue; // any: uniform over the block
-            const double mf = ms64[f].x;
-            const float *y = x + f;
-            const double2 *a2 = reinterpret_cast<const double2 *>(fg_a + c0 * mp);
-            const int mh = mp >> 1;
+        for (int c = 0; c < FG_HALF; ++c) any |= live[c0 + c] != 0;
+        if (any) {
             double acc[FG_HALF];
 #pragma unroll
             for (int c = 0; c < FG_HALF; ++c) acc[c] = 0.0;
+            const double2 sf = fok ? ms64[f] : make_double2(0.0, 0.0);
+            const double2 *a2 = reinterpret_cast<const double2 *>(fg_a + c0 * mp);
+            const int mh = mp >> 1, q0 = s ? (mh + 1) >> 1 : 0, q1 = s ? mh : (mh + 1) >> 1;
+            if (fok) {
+                const float *y = x + f;
 #pragma unroll 4
-            for (int q = 0; q < mh; ++q) {
-                // terms 2q, 2q+1 (the even padding term has zero candidate values)
-                const double v0 = (double)__ldg(y + 2 * q) - mf;
-                const double v1 = 2 * q + 1 < m ? (double)__ldg(y + 2 * q + 1) - mf : 0.0;
+                for (int q = q0; q < q1; ++q) {
+                    // terms 2q, 2q+1 (the even padding term has zero candidate values)
+                    const double v0 = (double)__ldg(y + 2 * q) - sf.x;
+                    const double v1 = 2 * q + 1 < m ? (double)__ldg(y + 2 * q + 1) - sf.x : 0.0;
 #pragma unroll
-                for (int c = 0; c < FG_HALF; ++c) {
-                    const double2 av = a2[c * mh + q];
-                    acc[c] = fma(av.y, v1, fma(av.x, v0, acc[c]));
+                    for (int c = 0; c < FG_HALF; ++c) {
+                        const double2 av = a2[c * mh + q];
+                        acc[c] = fma(av.y, v1, fma(av.x, v0, acc[c]));
+                    }
                 }
             }
-            const double ivf = ms64[f].y;
 #pragma unroll
             for (int c = 0; c < FG_HALF; ++c) {
+                acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], 16);
                 const int ci = c0 + c;
                 const int d = cw[ci] > f ? cw[ci] - f : f - cw[ci];
-                if (live[ci] && d >= m - 1) {
-                    b[ci] = acc[c] * civ[ci] * ivf;
+                if (fok && live[ci] && d >= m - 1) {
+                    b[c] = acc[c] * civ[ci] * sf.y;
                     // may be the nearest neighbour: the recheck has to look here
-                    if (bkeep && b[ci] >= (double)ord2f(__ldcg(rho_max + cp[ci])) - 2.0 * guard)
+                    if (s == 0 && bkeep &&
+                        b[c] >= (double)ord2f(__ldcg(rho_max + cp[ci])) - 2.0 * guard)
                         atomicMax(B.v + (int64_t)cp[ci] * B.halves + f / PADDI_HALF,
-                                  f2ord((float)b[ci]));
+                                  f2ord((float)b[c]));
                 }
             }
         }
         // maxima over the item's windows, per candidate
 #pragma unroll
-        for (int c = 0; c < FG_CAND; ++c) {
+        for (int c = 0; c < FG_HALF; ++c) {
             double v = b[c];
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-            if (lane == 0) best_s[c][warp] = v;
+            for (int o = 8; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+            if (lane == 0) best_s[c0 + c][wsub] = v;
         }
         __syncthreads();
         if (t < FG_CAND && live[t]) {
             double v = -INFINITY;
 #pragma unroll
-            for (int q = 0; q < FG_THREADS / 32; ++q) v = fmax(v, best_s[t][q]);
+            for (int q = 0; q < 4; ++q) v = fmax(v, best_s[t][q]);
             if (v > -INFINITY) {
                 atomicMax(rho_max + cp[t], f2ord((float)v));
                 if (v > (double)thr + 1e-7) pruned[cp[t]] = 1;
