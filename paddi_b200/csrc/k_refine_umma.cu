@@ -63,6 +63,7 @@ constexpr int UM_THREADS = 384;  // 12 warps
 constexpr int UM_TCMAX = 16;     // candidates per tile (M = 128); 8 for M = 64
 constexpr int UM_N = 256;        // windows at stride 8
 constexpr int UM_TW = UM_N * 8;  // windows per tile (one block of the grid)
+constexpr int UM_FEW = 4;        // tiles that take all remaining windows after the first round
 constexpr int UM_WAVES = 1;      // work items per CTA and round when candidate tiles are few
 constexpr int UM_KMAX128 = 368;  // largest K' with M = 128 (shared-memory bound)
 constexpr int UM_KMAX64 = 736;   // largest K' with M = 64
@@ -510,7 +511,9 @@ k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
     int jb = col_lo;
     for (int rd = 0; rd < nrounds; ++rd) {
         int je = paddi::refine_round_end(rd, nrounds, col_lo, col_hi, UM_TW);
-        if (C <= UM_TC) je = col_hi;
+        // one tile left, or a few after the first round: a further round (about 15 us:
+        // operand builds, the wait, a last wave) costs more than it could save
+        if (C <= (rd == 0 ? 1 : UM_FEW) * UM_TC) je = col_hi;
         int32_t *list = rd & 1 ? list1 : list0; // entries of this round (round 0: all candidates)
         const int range = je - jb;
         const int tiles = (C + UM_TC - 1) / UM_TC;
@@ -607,6 +610,7 @@ k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
                     zhw[c * ksw + t16] = 0u;
                     zlw[c * ksw + t16] = 0u;
                 }
+#pragma unroll 4
                 for (int k = t16; k < kp; k += 16) {
                     const float v = (live && k < m) ? (x[w + k] - muc) * ivc : 0.f;
                     const typename X::T h = X::cvt(v);
