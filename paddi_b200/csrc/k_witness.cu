@@ -53,7 +53,7 @@ constexpr int WT_SOON = 64;     // lengths within which a partner counts as soon
 constexpr int WT_RWARPS = 4;    // warps per CTA of the rescue
 constexpr int WT_MAXM = 1024;
 constexpr int WT_BATCH = 8;     // partners ranked together
-constexpr float WT_EASY = 0.02f; // a correlation this far above thr ends the search
+constexpr float WT_EASY = 0.1f; // a correlation this far above thr ends the search
 constexpr double kU64 = 1.1102230246251565e-16;
 
 // lower bound of a pair's correlation from its centred dot product
@@ -196,23 +196,26 @@ k_witness_hints(const float *__restrict__ x, const double2 *__restrict__ ms64, i
         wrho[i] = B.j >= 0 ? wt_bound(B.c, ii, ms64[B.j].y, t1) : -INFINITY;
     };
     if (nh >= WT_MANY) {
+        // ranked in FP32, the best partner then evaluated in FP64
         for (int e = blockIdx.x * WT_THREADS + threadIdx.x; e < nh; e += gridDim.x * WT_THREADS) {
             const int i = hint[e];
             const WtGroups G = wt_decode(wc[i]);
             const double2 si = ms64[i];
             WtBest B = {-INFINITY, 0.0, -1};
+            const float mf = (float)si.x;
             for (int q = 0; q < G.n; ++q) {
                 const int g = q ? G.g1 : G.g0;
-                const double sh = at(g);
-                double acc[4] = {0.0, 0.0, 0.0, 0.0}, y[4], as = 0.0;
+                const float sh = (float)at(g);
+                float acc[4] = {0.f, 0.f, 0.f, 0.f}, y[4], as = 0.f;
+                auto atf = [&](int k) { return x[min(max(k, 0), nser - 1)] - sh; };
 #pragma unroll
-                for (int c = 0; c < 3; ++c) y[c] = at(g + c) - sh;
+                for (int c = 0; c < 3; ++c) y[c] = atf(g + c);
                 for (int k = 0; k < m; ++k) {
-                    const double a = (double)x[i + k] - si.x;
-                    y[3] = at(g + k + 3) - sh;
+                    const float a = x[i + k] - mf;
+                    y[3] = atf(g + k + 3);
                     as += a;
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) acc[c] = fma(a, y[c], acc[c]);
+                    for (int c = 0; c < 4; ++c) acc[c] = fmaf(a, y[c], acc[c]);
                     y[0] = y[1];
                     y[1] = y[2];
                     y[2] = y[3];
@@ -221,8 +224,20 @@ k_witness_hints(const float *__restrict__ x, const double2 *__restrict__ ms64, i
                 for (int c = 0; c < 4; ++c)
                     if ((G.mask >> c) & 1u && g + c >= 0 && g + c < N) {
                         const double2 sj = ms64[g + c];
-                        wt_settle(B, i, g + c, acc[c] - (sj.x - sh) * as, sj, si.y, N, m);
+                        wt_settle(B, i, g + c,
+                                  (double)acc[c] - (sj.x - (double)sh) * (double)as, sj, si.y, N, m);
                     }
+            }
+            if (B.j >= 0) {
+                const double mj = ms64[B.j].x;
+                double c0 = 0.0, c1 = 0.0;
+                int k = 0;
+                for (; k + 2 <= m; k += 2) {
+                    c0 = fma((double)x[i + k] - si.x, (double)x[B.j + k] - mj, c0);
+                    c1 = fma((double)x[i + k + 1] - si.x, (double)x[B.j + k + 1] - mj, c1);
+                }
+                if (k < m) c0 = fma((double)x[i + k] - si.x, (double)x[B.j + k] - mj, c0);
+                B.c = c0 + c1;
             }
             store(i, B, si.y);
         }
