@@ -79,17 +79,38 @@ class _Log(C.Structure):
                 ("n_fragile", C.c_int32)]
 
     def as_dict(self):
-        return {"m": self.m, "r": self.r, "r2": self.r2, "found": self.found,
-                "n_cand": self.n_cand, "n_disc": self.n_disc, "n_phase1": self.n_phase1,
-                "n_recheck": self.n_recheck, "top_ind": self.top.ind, "top_dist": self.top.dist,
-                "ms_stats": self.ms_stats, "ms_phase1": self.ms_phase1,
-                "ms_refine": self.ms_refine, "ms_select": self.ms_select,
-                "ms_total": self.ms_total, "refine_pairs": self.refine_pairs,
-                "n_launches": self.n_launches, "refine_kernel": self.refine_kernel,
-                "r_source": self.r_source, "ms_guide": self.ms_guide, "lb": self.lb,
-                "flat_frac": self.flat_frac, "p1_pairs": self.p1_pairs,
-                "refine_live_pairs": self.refine_live_pairs,
-                "ms_refine_kernel": self.ms_refine_kernel, "n_fragile": self.n_fragile}
+        return _row_dict(tuple(getattr(self, f) for f in _LOG_FIELDS[:_TOP])
+                         + ((self.top.ind, self.top.dist),)
+                         + tuple(getattr(self, f) for f in _LOG_FIELDS[_TOP + 1:]))
+
+
+_LOG_FIELDS = [f[0] for f in _Log._fields_]
+_LOG_DTYPE = np.dtype(_Log)
+_TOP = _LOG_FIELDS.index("top")
+_ROW_KEYS = _LOG_FIELDS[:_TOP] + ["top_ind", "top_dist"] + _LOG_FIELDS[_TOP + 1:]
+
+
+def _row_dict(row):
+    return dict(zip(_ROW_KEYS, row[:_TOP] + row[_TOP] + row[_TOP + 1:]))
+
+
+class _LogRows:
+    """Room for `cap` attempt rows.  The memory is not touched before the library
+    writes to it (the default of 100000 rows is 17 MB)."""
+
+    def __init__(self, cap: int):
+        self.buf = np.empty(max(cap, 1), _LOG_DTYPE)
+        self.cap = cap
+        self.n = C.c_uint32(0)
+
+    @property
+    def ptr(self):
+        return C.cast(self.buf.ctypes.data, C.POINTER(_Log))
+
+    def dicts(self):
+        """The rows written, as dicts."""
+        n = min(self.n.value, self.cap)
+        return [_row_dict(r) for r in self.buf[:n].tolist()]
 
 
 @dataclass(frozen=True)
@@ -302,12 +323,11 @@ class Context:
         x = np.ascontiguousarray(series, dtype=np.float32)
         L = maxL - minL + 1
         out = (_Discord * max(L, 1))()  # the library rejects an empty range itself
-        log = (_Log * log_cap)()
-        nl = C.c_uint32(0)
-        self._check(lib().paddi_palmad(self._h, x.ctypes.data, len(x), minL, maxL, out, log,
-                                       log_cap, C.byref(nl)))
+        log = _LogRows(log_cap)
+        self._check(lib().paddi_palmad(self._h, x.ctypes.data, len(x), minL, maxL, out, log.ptr,
+                                       log_cap, C.byref(log.n)))
         return ([Discord(out[i].ind, out[i].dist) for i in range(L)],
-                [log[i].as_dict() for i in range(min(nl.value, log_cap))])
+                log.dicts())
 
     def palmad_profiled(self, series, minL: int, maxL: int, on_profile=None,
                         log_cap: int = 100000):
@@ -319,8 +339,7 @@ class Context:
         x = np.ascontiguousarray(series, dtype=np.float32)
         L = maxL - minL + 1
         out = (_Discord * max(L, 1))()
-        log = (_Log * log_cap)()
-        nl = C.c_uint32(0)
+        log = _LogRows(log_cap)
         kept = []
 
         def cb(_user, m, ptr, N):
@@ -332,9 +351,9 @@ class Context:
 
         fn = PROFILE_FN(cb)
         self._check(lib().paddi_palmad_profiled(self._h, x.ctypes.data, len(x), minL, maxL, out,
-                                                log, log_cap, C.byref(nl), fn, None))
+                                                log.ptr, log_cap, C.byref(log.n), fn, None))
         return ([Discord(out[i].ind, out[i].dist) for i in range(L)],
-                [log[i].as_dict() for i in range(min(nl.value, log_cap))],
+                log.dicts(),
                 None if on_profile is not None else kept)
 
     def autotune(self, series, minL: int, maxL: int):
@@ -370,12 +389,11 @@ class Context:
         """PALMAD on a series already in device memory (pointer to n floats)."""
         L = maxL - minL + 1
         out = (_Discord * max(L, 1))()
-        log = (_Log * log_cap)()
-        nl = C.c_uint32(0)
+        log = _LogRows(log_cap)
         self._check(lib().paddi_palmad_device(self._h, C.c_void_p(d_series_ptr), n, minL, maxL,
-                                              out, log, log_cap, C.byref(nl)))
+                                              out, log.ptr, log_cap, C.byref(log.n)))
         return ([Discord(out[i].ind, out[i].dist) for i in range(L)],
-                [log[i].as_dict() for i in range(min(nl.value, log_cap))])
+                log.dicts())
 
     def pd3(self, series, m: int, top_k: int = 1, r: float = 0.0, segment_len: int = 0,
             log_cap: int = 1000):
@@ -383,12 +401,11 @@ class Context:
         x = np.ascontiguousarray(series, dtype=np.float32)
         out = (_Discord * max(top_k, 1))()
         n_out = C.c_uint32(0)
-        log = (_Log * log_cap)()
-        nl = C.c_uint32(0)
+        log = _LogRows(log_cap)
         self._check(lib().paddi_pd3(self._h, x.ctypes.data, len(x), m, segment_len, top_k,
-                                    float(r), out, C.byref(n_out), log, log_cap, C.byref(nl)))
+                                    float(r), out, C.byref(n_out), log.ptr, log_cap, C.byref(log.n)))
         return ([Discord(out[i].ind, out[i].dist) for i in range(n_out.value)],
-                [log[i].as_dict() for i in range(min(nl.value, log_cap))])
+                log.dicts())
 
     def compute_statistics(self, d_T: int, d_mean: int, d_std: int, n: int, m: int,
                            stream: int = 0):

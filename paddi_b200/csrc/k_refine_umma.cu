@@ -972,12 +972,13 @@ k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
 
 bool paddi_umma_supported(int device)
 {
-    cudaDeviceProp p;
-    if (cudaGetDeviceProperties(&p, device) != cudaSuccess) {
+    int major = 0, minor = 0;
+    if (cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device) != cudaSuccess ||
+        cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, device) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
-    return p.major == 10 && p.minor == 0; // sm_100 (B200)
+    return major == 10 && minor == 0; // sm_100 (B200)
 }
 
 int paddi_umma_max_m() { return UM_KMAX64 - 7; } // kpad_of(m) <= UM_KMAX64

@@ -115,6 +115,12 @@ struct paddi_ctx {
     long long wait_cycles = 0;
     int32_t withhold = 0;
     int32_t last_passes = 0; // selection passes of the last attempt
+    // the small buffers above live in one device and one pinned block
+    void *d_small = nullptr, *h_small = nullptr;
+    // worker contexts of paddi_palmad_batched, kept for the next call: as many as
+    // the last call used, destroyed with the context, after a failed call, or when
+    // an allocation of this context needs their memory
+    std::vector<paddi_ctx *> workers;
 };
 
 namespace {
@@ -143,6 +149,14 @@ paddi_status fail(paddi_ctx *c, paddi_status s, const std::string &msg)
                         std::string(#call) + ": " + cudaGetErrorString(e_));                \
     } while (0)
 
+void drop_workers(paddi_ctx *ctx, size_t keep = 0)
+{
+    while (ctx->workers.size() > keep) {
+        paddi_ctx_destroy(ctx->workers.back());
+        ctx->workers.pop_back();
+    }
+}
+
 // Every device allocation of a context goes through here, so a test can make
 // one fail (PADDI_DEBUG_FAIL_ALLOC) and check that PADDI_ERR_OUT_OF_MEMORY
 // reaches the caller.
@@ -150,7 +164,13 @@ template <typename T>
 cudaError_t dmalloc(paddi_ctx *ctx, T **p, size_t bytes)
 {
     if (ctx->fail_alloc > 0 && --ctx->fail_alloc == 0) return cudaErrorMemoryAllocation;
-    return cudaMalloc((void **)p, bytes);
+    cudaError_t e = cudaMalloc((void **)p, bytes);
+    if (e == cudaErrorMemoryAllocation && !ctx->workers.empty()) {
+        cudaGetLastError();
+        drop_workers(ctx);
+        e = cudaMalloc((void **)p, bytes);
+    }
+    return e;
 }
 
 template <typename T>
@@ -983,14 +1003,17 @@ PADDI_API paddi_status paddi_ctx_create(paddi_ctx **out, const paddi_opts *opts)
         return PADDI_ERR_NO_DEVICE;
     }
     ctx->device = ctx->opts.device;
-    cudaDeviceProp prop;
+    int major = 0;
     if (cudaSetDevice(ctx->device) != cudaSuccess ||
-        cudaGetDeviceProperties(&prop, ctx->device) != cudaSuccess || prop.major < 10) {
+        cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, ctx->device) !=
+            cudaSuccess ||
+        cudaDeviceGetAttribute(&ctx->num_sms, cudaDevAttrMultiProcessorCount, ctx->device) !=
+            cudaSuccess ||
+        major < 10) {
         cudaGetLastError();
         delete ctx;
         return PADDI_ERR_NO_DEVICE;
     }
-    ctx->num_sms = prop.multiProcessorCount;
     ctx->umma_ok = paddi_umma_supported(ctx->device);
     if ((ctx->opts.distance_kernel == PADDI_DIST_SPLIT_BF16 ||
          ctx->opts.distance_kernel == PADDI_DIST_SPLIT_FP16) &&
@@ -1004,29 +1027,46 @@ PADDI_API paddi_status paddi_ctx_create(paddi_ctx **out, const paddi_opts *opts)
         const char *tr = std::getenv("PADDI_TRACE");
         ctx->trace = tr && tr[0] && tr[0] != '0';
     }
-    if (ctx->trace) {
-        ok = ok && cudaMallocHost(&ctx->h_trace, sizeof(PaddiAttemptDev)) == cudaSuccess;
+    // small buffers, in one allocation each (256-byte steps), zeroed
+    size_t dn = 0, hn = 0;
+    auto place = [](size_t &off, size_t bytes) {
+        const size_t at = off;
+        off += (bytes + 255) & ~(size_t)255;
+        return at;
+    };
+    const size_t o_att[2] = {place(dn, sizeof(PaddiAttemptDev)), place(dn, sizeof(PaddiAttemptDev))};
+    const size_t o_flat[2] = {place(dn, 4 * sizeof(int32_t)), place(dn, 4 * sizeof(int32_t))};
+    const size_t o_res = place(dn, sizeof(PaddiAttemptResult));
+    const size_t o_tp = place(dn, PADDI_T_PREP * sizeof(unsigned long long));
+    const size_t o_guide = place(dn, sizeof(PaddiGuide));
+    const size_t o_model = place(dn, sizeof(float) * MLP_NPARAM);
+    const size_t o_bf16 = place(dn, 2 * MLP_NPARAM);
+    const size_t o_feat = place(dn, sizeof(float) * 16), o_pred = place(dn, sizeof(float) * 4);
+    const size_t p_res = place(hn, sizeof(PaddiAttemptResult)), p_guide = place(hn, sizeof(PaddiGuide));
+    const size_t p_feat = place(hn, sizeof(float) * 16), p_trace = place(hn, sizeof(PaddiAttemptDev));
+    ok = ok && cudaMalloc(&ctx->d_small, dn) == cudaSuccess;
+    ok = ok && cudaMemset(ctx->d_small, 0, dn) == cudaSuccess;
+    ok = ok && cudaMallocHost(&ctx->h_small, hn) == cudaSuccess;
+    if (ok) {
+        char *d = (char *)ctx->d_small, *h = (char *)ctx->h_small;
+        for (int k = 0; k < 2; ++k) {
+            ctx->d_att2[k] = (PaddiAttemptDev *)(d + o_att[k]);
+            ctx->d_flat2[k] = (int32_t *)(d + o_flat[k]);
+        }
+        ctx->d_att = ctx->d_att2[0];
+        ctx->d_flatcount = ctx->d_flat2[0];
+        ctx->d_res = (PaddiAttemptResult *)(d + o_res);
+        ctx->d_tprep = (unsigned long long *)(d + o_tp);
+        ctx->d_guide = (PaddiGuide *)(d + o_guide);
+        ctx->d_model = (float *)(d + o_model);
+        ctx->d_model_bf16 = d + o_bf16;
+        ctx->d_feat = (float *)(d + o_feat);
+        ctx->d_pred = (float *)(d + o_pred);
+        ctx->h_res = (PaddiAttemptResult *)(h + p_res);
+        ctx->h_guide = (PaddiGuide *)(h + p_guide);
+        ctx->h_feat = (float *)(h + p_feat);
+        ctx->h_trace = (PaddiAttemptDev *)(h + p_trace);
     }
-    for (int k = 0; k < 2; ++k) {
-        ok = ok && cudaMalloc(&ctx->d_att2[k], sizeof(PaddiAttemptDev)) == cudaSuccess;
-        ok = ok && cudaMemset(ctx->d_att2[k], 0, sizeof(PaddiAttemptDev)) == cudaSuccess;
-        ok = ok && cudaMalloc(&ctx->d_flat2[k], 4 * sizeof(int32_t)) == cudaSuccess;
-        ok = ok && cudaMemset(ctx->d_flat2[k], 0, 4 * sizeof(int32_t)) == cudaSuccess;
-    }
-    ctx->d_att = ctx->d_att2[0];
-    ctx->d_flatcount = ctx->d_flat2[0];
-    ok = ok && cudaMalloc(&ctx->d_res, sizeof(PaddiAttemptResult)) == cudaSuccess;
-    ok = ok && cudaMalloc(&ctx->d_tprep, PADDI_T_PREP * sizeof(unsigned long long)) == cudaSuccess;
-    ok = ok && cudaMemset(ctx->d_tprep, 0, PADDI_T_PREP * sizeof(unsigned long long)) == cudaSuccess;
-    ok = ok && cudaMallocHost(&ctx->h_res, sizeof(PaddiAttemptResult)) == cudaSuccess;
-    ok = ok && cudaMalloc(&ctx->d_guide, sizeof(PaddiGuide)) == cudaSuccess;
-    ok = ok && cudaMemset(ctx->d_guide, 0, sizeof(PaddiGuide)) == cudaSuccess;
-    ok = ok && cudaMallocHost(&ctx->h_guide, sizeof(PaddiGuide)) == cudaSuccess;
-    ok = ok && cudaMalloc(&ctx->d_model, sizeof(float) * MLP_NPARAM) == cudaSuccess;
-    ok = ok && cudaMalloc(&ctx->d_model_bf16, 2 * MLP_NPARAM) == cudaSuccess;
-    ok = ok && cudaMalloc(&ctx->d_feat, sizeof(float) * 16) == cudaSuccess;
-    ok = ok && cudaMalloc(&ctx->d_pred, sizeof(float) * 4) == cudaSuccess;
-    ok = ok && cudaMallocHost(&ctx->h_feat, sizeof(float) * 16) == cudaSuccess;
     if (!ok) {
         cudaGetLastError();
         paddi_ctx_destroy(ctx);
@@ -1041,24 +1081,12 @@ PADDI_API paddi_status paddi_ctx_destroy(paddi_ctx *ctx)
     if (!ctx) return PADDI_ERR_INVALID_ARG;
     cudaSetDevice(ctx->device);
     if (ctx->st) cudaStreamSynchronize(ctx->st);
+    drop_workers(ctx);
     free_buffers(ctx);
-    for (int k = 0; k < 2; ++k) {
-        dfree(ctx->d_att2[k]);
-        dfree(ctx->d_flat2[k]);
-    }
-    dfree(ctx->d_res);
-    dfree(ctx->d_tprep);
-    dfree(ctx->d_guide);
-    dfree(ctx->d_model);
-    if (ctx->d_model_bf16) cudaFree(ctx->d_model_bf16);
-    dfree(ctx->d_feat);
-    dfree(ctx->d_pred);
-    if (ctx->h_feat) cudaFreeHost(ctx->h_feat);
-    if (ctx->h_guide) cudaFreeHost(ctx->h_guide);
-    if (ctx->h_res) cudaFreeHost(ctx->h_res);
+    if (ctx->d_small) cudaFree(ctx->d_small);
+    if (ctx->h_small) cudaFreeHost(ctx->h_small);
     for (auto &e : ctx->ev)
         if (e) cudaEventDestroy(e);
-    if (ctx->h_trace) cudaFreeHost(ctx->h_trace);
     if (ctx->st) cudaStreamDestroy(ctx->st);
     delete ctx;
     return PADDI_OK;
@@ -1591,25 +1619,34 @@ PADDI_API paddi_status paddi_palmad_batched(paddi_ctx *ctx, const float *const *
     const uint32_t L = maxL - minL + 1;
     int W = streams ? (int)streams : 4;
     if ((uint32_t)W > count) W = (int)count;
-    // worker contexts share the options (and the model) of ctx
-    std::vector<paddi_ctx *> workers(W, nullptr);
+    // worker contexts share the options and the model of ctx
+    drop_workers(ctx, (size_t)W);
     paddi_status first_err = PADDI_OK;
-    for (int w = 0; w < W; ++w) {
-        paddi_status s = paddi_ctx_create(&workers[w], &ctx->opts);
-        if (s == PADDI_OK && ctx->model_ok) {
-            std::vector<float> p(MLP_NPARAM);
-            if (cudaMemcpy(p.data(), ctx->d_model, sizeof(float) * MLP_NPARAM,
-                           cudaMemcpyDeviceToHost) != cudaSuccess)
-                s = PADDI_ERR_CUDA;
-            else
-                s = paddi_model_set(workers[w], p.data(), MLP_NPARAM, ctx->model_margin);
-        }
-        if (s != PADDI_OK) {
-            for (auto *c : workers)
-                if (c) paddi_ctx_destroy(c);
-            return fail(ctx, s, "batched: cannot create worker contexts");
+    CK(cudaSetDevice(ctx->device));
+    while (ctx->workers.size() < (size_t)W) {
+        paddi_ctx *c = nullptr;
+        const paddi_status s = paddi_ctx_create(&c, &ctx->opts);
+        if (s != PADDI_OK) return fail(ctx, s, "batched: cannot create worker contexts");
+        ctx->workers.push_back(c);
+    }
+    for (paddi_ctx *c : ctx->workers) {
+        c->opts = ctx->opts;
+        c->model_ok = ctx->model_ok;
+        c->model_margin = ctx->model_margin;
+        if (ctx->model_ok) {
+            CK(cudaMemcpy(c->d_model, ctx->d_model, sizeof(float) * MLP_NPARAM,
+                          cudaMemcpyDeviceToDevice));
+            CK(cudaMemcpy(c->d_model_bf16, ctx->d_model_bf16, 2 * MLP_NPARAM,
+                          cudaMemcpyDeviceToDevice));
         }
     }
+    CK(cudaDeviceSynchronize()); // the copies precede the workers' (non-blocking) streams
+    // longest series first: a worker's buffers are sized by its first one, and the
+    // short ones even out the end
+    std::vector<uint32_t> order(count);
+    for (uint32_t k = 0; k < count; ++k) order[k] = k;
+    std::stable_sort(order.begin(), order.end(),
+                     [&](uint32_t a, uint32_t b) { return lens[a] > lens[b]; });
     std::atomic<uint32_t> next{0};
     std::vector<int32_t> st(count, (int32_t)PADDI_OK);
     std::vector<std::string> errs(count);
@@ -1617,10 +1654,11 @@ PADDI_API paddi_status paddi_palmad_batched(paddi_ctx *ctx, const float *const *
     std::vector<std::thread> pool;
     for (int w = 0; w < W; ++w) {
         pool.emplace_back([&, w]() {
-            paddi_ctx *c = workers[w];
+            paddi_ctx *c = ctx->workers[w];
             cudaSetDevice(c->device);
             std::vector<paddi_attempt_log> lg(4096);
-            for (uint32_t k = next++; k < count; k = next++) {
+            for (uint32_t q = next++; q < count; q = next++) {
+                const uint32_t k = order[q];
                 uint32_t nl = 0;
                 st[k] = (int32_t)paddi_palmad(c, series[k], lens[k], minL, maxL,
                                               out + (size_t)k * L, lg.data(),
@@ -1631,7 +1669,6 @@ PADDI_API paddi_status paddi_palmad_batched(paddi_ctx *ctx, const float *const *
         });
     }
     for (auto &t : pool) t.join();
-    for (auto *c : workers) paddi_ctx_destroy(c);
     std::string msg;
     for (uint32_t k = 0; k < count; ++k) {
         if (status) status[k] = st[k];
@@ -1641,7 +1678,10 @@ PADDI_API paddi_status paddi_palmad_batched(paddi_ctx *ctx, const float *const *
             msg = "batched: series " + std::to_string(k) + ": " + errs[k];
         }
     }
-    if (first_err != PADDI_OK) return fail(ctx, first_err, msg);
+    if (first_err != PADDI_OK) {
+        drop_workers(ctx);
+        return fail(ctx, first_err, msg);
+    }
     return PADDI_OK;
 }
 
