@@ -28,7 +28,7 @@
 // values: rho = (D 2^-(8+e) - sum(zhat') (mu_j - shift)) inv_j.
 //
 // Layout of the work.  Tiles sit on a fixed grid of 2048-window blocks.  Once
-// per length, k_tile_prep converts every block's slice into its hi / lo
+// per length, k_prep converts every block's slice into its hi / lo
 // halves and its per-window epilogue data (inv_j 2^-(8+e), (mu_j - shift)
 // inv_j) in global memory (L2-resident).  The refine is then a pipeline of
 // roles inside one persistent CTA per SM, coupled only by mbarriers:
@@ -52,6 +52,7 @@
 
 #include <cmath>
 
+#include "k_stats.cuh"
 #include "paddi_internal.cuh"
 
 using paddi::compact_survivors;
@@ -257,38 +258,51 @@ template <> struct E16<true> {
 // subtracts it from every correlation of the tile (a lower bound that is safe
 // to prune on) and adds it back to the maxima it keeps (the middle of the
 // interval, within gcap of every true value).
-constexpr int TP_THREADS = 256;
+// The statistics of the length come out of the same kernel: a block's windows
+// are a statistics tile, so the staged series and the windows' means and norms
+// are used where they are, in shared memory and registers.  As two kernels (the
+// second one re-reading 20 B a window) they took 34 us a length at n = 1500007,
+// m = 300, as one 25; headline run 168 -> 153 ms.
+static_assert(ST_TILE == UM_TW, "a statistics tile is a block of the refine's grid");
 
 template <bool BF>
-__global__ void __launch_bounds__(TP_THREADS)
-k_tile_prep(const float *__restrict__ x, int64_t nser, int32_t cnt, int32_t m,
-            const float4 *__restrict__ wst, const float *__restrict__ mu, uint16_t *__restrict__ bq,
-            float4 *__restrict__ wdq, float E, float Fu, float gcap, int32_t *frag_list,
-            int32_t *frag_count, unsigned long long *t_end)
+__global__ void __launch_bounds__(ST_THREADS)
+k_prep(const float *__restrict__ x, int64_t nser, int32_t cnt, int32_t m, int32_t N, StOut O,
+       uint16_t *__restrict__ bq, float4 *__restrict__ wdq, float E, float Fu, float gcap,
+       int32_t *frag_list, int32_t *frag_count, unsigned long long *t_end)
 {
     using X = E16<BF>;
-    paddi::chain_begin();
-    __shared__ float red[4][TP_THREADS / 32];
+    extern __shared__ __align__(16) unsigned char st_mem[];
+    __shared__ StShared S;
+    __shared__ float red[4][ST_THREADS / 32];
+    st_begin(O.extra);
     const int b = blockIdx.x;
     const int64_t j0 = (int64_t)b * UM_TW;
-    const int64_t N = nser - m + 1;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    float sw = 0.f, swm = 0.f; // sums of 1/|x_j - mu_j|^2 and mu_j/|x_j - mu_j|^2
-    for (int q = threadIdx.x; q < UM_TW; q += TP_THREADS) {
-        const int64_t j = j0 + q;
-        if (j < N) {
-            const float iv = wst[j].z;
-            const float wgt = fminf(iv * iv, 1e30f);
-            sw += wgt;
-            swm = fmaf(wgt, mu[j], swm);
-        }
+    const StTile T = st_prefix(st_mem, S, x, nser, m, j0);
+    float iv[ST_WPT], mv[ST_WPT]; // zero past N
+    st_write(T, O, j0, m, N, iv, mv);
+    if (j0 >= N) { // the zeroed tail holds no tile
+        if (threadIdx.x == 0) paddi::stamp_end(t_end);
+        return;
     }
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    // the slice reaches a few values past what is staged
+    const int staged = ST_TILE + m + 1;
+    auto val = [&](int p) { return p < staged ? T.xs[p] : x[j0 + p]; };
+    float sw = 0.f, swm = 0.f; // sums of 1/|x_j - mu_j|^2 and mu_j/|x_j - mu_j|^2
+#pragma unroll
+    for (int k = 0; k < ST_WPT; ++k)
+        if (j0 + threadIdx.x + ST_THREADS * k < N) {
+            const float wgt = fminf(iv[k] * iv[k], 1e30f);
+            sw += wgt;
+            swm = fmaf(wgt, mv[k], swm);
+        }
     float lo_v = INFINITY, hi_v = -INFINITY;
-    for (int p = threadIdx.x; p < cnt; p += TP_THREADS) {
-        const int64_t g = j0 + p;
-        if (g < nser) {
-            lo_v = fminf(lo_v, x[g]);
-            hi_v = fmaxf(hi_v, x[g]);
+    for (int p = threadIdx.x; p < cnt; p += ST_THREADS) {
+        if (j0 + p < nser) {
+            const float v = val(p);
+            lo_v = fminf(lo_v, v);
+            hi_v = fmaxf(hi_v, v);
         }
     }
 #pragma unroll
@@ -310,7 +324,7 @@ k_tile_prep(const float *__restrict__ x, int64_t nser, int32_t cnt, int32_t m,
     sw = 0.f;
     swm = 0.f;
 #pragma unroll
-    for (int k = 0; k < TP_THREADS / 32; ++k) {
+    for (int k = 0; k < ST_THREADS / 32; ++k) {
         lo_v = fminf(lo_v, red[0][k]);
         hi_v = fmaxf(hi_v, red[1][k]);
         sw += red[2][k];
@@ -334,10 +348,10 @@ k_tile_prep(const float *__restrict__ x, int64_t nser, int32_t cnt, int32_t m,
     const float dsc = ldexpf(1.f, -(ZSCALE + e));
     uint32_t *hi = reinterpret_cast<uint32_t *>(bq + (size_t)b * 2 * cnt);
     uint32_t *lo = reinterpret_cast<uint32_t *>(bq + (size_t)b * 2 * cnt + cnt);
-    for (int p2 = threadIdx.x; p2 < cnt / 2; p2 += TP_THREADS) {
+    for (int p2 = threadIdx.x; p2 < cnt / 2; p2 += ST_THREADS) {
         const int64_t g = j0 + 2 * p2;
-        const float u0 = (g < nser ? x[g] - sh : 0.f) * sc;
-        const float u1 = (g + 1 < nser ? x[g + 1] - sh : 0.f) * sc;
+        const float u0 = (g < nser ? val(2 * p2) - sh : 0.f) * sc;
+        const float u1 = (g + 1 < nser ? val(2 * p2 + 1) - sh : 0.f) * sc;
         const typename X::T h0 = X::cvt(u0), h1 = X::cvt(u1);
         const typename X::T l0 = X::cvt(u0 - X::back(h0)), l1 = X::cvt(u1 - X::back(h1));
         hi[p2] = (uint32_t)reinterpret_cast<const uint16_t &>(h0) |
@@ -348,15 +362,16 @@ k_tile_prep(const float *__restrict__ x, int64_t nser, int32_t cnt, int32_t m,
     float *wf = reinterpret_cast<float *>(wdq + (size_t)b * 8 * WD_ROW);
     const float F = Fu * mx, fm = (float)m;
     float gmax = 0.f;
-    for (int q = threadIdx.x; q < UM_TW; q += TP_THREADS) {
-        const int64_t j = j0 + q; // the padded tail beyond N is zero
-        const float iv = wst[j].z, mv = mu[j];
-        const float g = paddi::window_bound(iv, mv, sh, fm, E, F);
+#pragma unroll
+    for (int kq = 0; kq < ST_WPT; ++kq) {
+        const int q = threadIdx.x + ST_THREADS * kq;
+        const int64_t j = j0 + q;
+        const float g = paddi::window_bound(iv[kq], mv[kq], sh, fm, E, F);
         const bool frag = j < N && g > gcap;
         if (!frag) gmax = fmaxf(gmax, g);
         const int s = q & 7, i = q >> 3, k = i >> 1, slot = i & 1;
-        wf[(s * WD_ROW + k) * 4 + slot] = frag ? __int_as_float(0x7fffffff) : iv * dsc;
-        wf[(s * WD_ROW + k) * 4 + 2 + slot] = (mv - sh) * iv;
+        wf[(s * WD_ROW + k) * 4 + slot] = frag ? __int_as_float(0x7fffffff) : iv[kq] * dsc;
+        wf[(s * WD_ROW + k) * 4 + 2 + slot] = (mv[kq] - sh) * iv[kq];
         // fragile windows in index order within each warp (runs stay contiguous)
         const unsigned bal = __ballot_sync(0xffffffffu, frag);
         if (bal) {
@@ -372,7 +387,7 @@ k_tile_prep(const float *__restrict__ x, int64_t nser, int32_t cnt, int32_t m,
     __syncthreads();
     if (threadIdx.x == 0) {
         float G = 0.f;
-        for (int k = 0; k < TP_THREADS / 32; ++k) G = fmaxf(G, red[0][k]);
+        for (int k = 0; k < ST_THREADS / 32; ++k) G = fmaxf(G, red[0][k]);
         wf[(0 * WD_ROW + 128) * 4] = G; // padding entry of shift row 0
         paddi::stamp_end(t_end);
     }
@@ -1015,19 +1030,24 @@ PaddiBound paddi_bound_tc(int m, bool bf16)
     return B;
 }
 
-cudaError_t paddi_launch_tile_prep(bool bf16, const float *x, int64_t n, int32_t m,
-                                   const float4 *wst, const float *mu, uint16_t *bq, float4 *wdq,
-                                   float gcap, int32_t *frag_list, int32_t *frag_count,
-                                   cudaStream_t st, unsigned long long *t_end)
+cudaError_t paddi_launch_prep(bool bf16, const float *x, int64_t n, int32_t m, float4 *wst,
+                              float *mu, double2 *ms64, uint8_t *flat, int32_t *flat_count,
+                              uint16_t *bq, float4 *wdq, float gcap, int32_t *frag_list,
+                              cudaStream_t st, bool chained, const PaddiStatsExtra &extra,
+                              unsigned long long *t_end)
 {
     const int kp = kpad_of(m);
-    if (kp > UM_KMAX64 || m < 3) return cudaErrorInvalidValue;
-    const int64_t N = n - m + 1;
-    const unsigned grid = (unsigned)paddi_tile_blocks(N);
+    if (kp > UM_KMAX64 || m < 3 || n < 2 * (int64_t)m) return cudaErrorInvalidValue;
+    const int32_t N = (int32_t)(n - m + 1);
+    const unsigned grid = (unsigned)(((int64_t)N + PADDI_PAD_WIN + ST_TILE - 1) / ST_TILE);
     const PaddiBound B = paddi_bound_tc(m, bf16);
-    return paddi_launch(true, bf16 ? k_tile_prep<true> : k_tile_prep<false>, grid, TP_THREADS, 0, st,
-                        x, n, slice_cnt(kp), m, wst, mu, bq, wdq, B.E, B.F, gcap, frag_list,
-                        frag_count, t_end);
+    const size_t smem = st_smem(m);
+    auto kern = bf16 ? k_prep<true> : k_prep<false>;
+    cudaError_t e = paddi_raise_smem_limit((const void *)kern, smem);
+    if (e != cudaSuccess) return e;
+    const StOut O = {wst, mu, ms64, flat, flat_count, flat_count + 1, extra};
+    return paddi_launch(chained, kern, grid, ST_THREADS, smem, st, x, n, slice_cnt(kp), m, N, O, bq,
+                        wdq, B.E, B.F, gcap, frag_list, flat_count + 3, t_end);
 }
 
 cudaError_t paddi_launch_refine_umma(bool bf16, const float *x, const float4 *wst,

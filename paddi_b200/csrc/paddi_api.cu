@@ -294,11 +294,11 @@ float guard_of(const paddi_ctx *ctx, int kernel)
     return kernel == PADDI_DIST_SPLIT_BF16 ? 1e-3f : 2e-4f;
 }
 
-// Statistics of length m for the series in `x` (n values); with `tiles`, also
-// the tensor-core refine's tile data when that kernel serves this length.
-// chained: the stream's previous operation is a kernel of this context.
-paddi_status run_stats(paddi_ctx *ctx, const float *x, size_t n, int m, bool tiles = true,
-                       bool chained = false)
+// Statistics of length m for the series in `x` (n values) and the refine's
+// per-length data: its tiles (tensor cores) and the windows whose rounding
+// bound exceeds the guard band (both refine kernels).  chained: the stream's
+// previous operation is a kernel of this context.
+paddi_status run_stats(paddi_ctx *ctx, const float *x, size_t n, int m, bool chained = false)
 {
     const int cur = ctx->d_flatcount == ctx->d_flat2[0] ? 1 : 0;
     ctx->d_flatcount = ctx->d_flat2[cur];
@@ -308,20 +308,21 @@ paddi_status run_stats(paddi_ctx *ctx, const float *x, size_t n, int m, bool til
     ex.guide = ctx->d_guide;
     ex.t = ctx->d_tprep + PADDI_T_STATS_B;
     unsigned long long *t_end = ctx->d_tprep + PADDI_T_STATS_E;
-    CK(paddi_launch_stats(x, (int64_t)n, m, ctx->d_wst, ctx->d_mu, ctx->d_ms64, ctx->d_flat,
-                          ctx->d_flatcount, ctx->st, ctx->d_flatcount + 1, chained, ex));
-    ctx->prep_launches = tiles ? 2 : 1;
     const int kernel = refine_kernel_for(ctx, m);
-    // the refine's per-length data: its tiles (tensor cores) and the windows
-    // whose rounding bound exceeds the guard band (both refine kernels)
-    if (tiles && kernel != PADDI_DIST_FP32)
-        CK(paddi_launch_tile_prep(kernel == PADDI_DIST_SPLIT_BF16, x, (int64_t)n, m, ctx->d_wst,
-                                  ctx->d_mu, ctx->d_bq, ctx->d_wdq, guard_of(ctx, kernel),
-                                  ctx->d_frag, ctx->d_flatcount + 3, ctx->st, t_end));
-    else if (tiles)
-        CK(paddi_launch_fragile_scan_fp32(x, ctx->d_wst, ctx->d_mu, (int32_t)(n - m + 1), m,
-                                          guard_of(ctx, kernel), ctx->d_frag,
-                                          ctx->d_flatcount + 3, ctx->num_sms, ctx->st, t_end));
+    const float guard = guard_of(ctx, kernel);
+    if (kernel != PADDI_DIST_FP32) {
+        CK(paddi_launch_prep(kernel == PADDI_DIST_SPLIT_BF16, x, (int64_t)n, m, ctx->d_wst,
+                             ctx->d_mu, ctx->d_ms64, ctx->d_flat, ctx->d_flatcount, ctx->d_bq,
+                             ctx->d_wdq, guard, ctx->d_frag, ctx->st, chained, ex, t_end));
+        ctx->prep_launches = 1;
+    } else {
+        CK(paddi_launch_stats(x, (int64_t)n, m, ctx->d_wst, ctx->d_mu, ctx->d_ms64, ctx->d_flat,
+                              ctx->d_flatcount, ctx->st, ctx->d_flatcount + 1, chained, ex));
+        CK(paddi_launch_fragile_scan_fp32(x, ctx->d_wst, ctx->d_mu, (int32_t)(n - m + 1), m, guard,
+                                          ctx->d_frag, ctx->d_flatcount + 3, ctx->num_sms, ctx->st,
+                                          t_end));
+        ctx->prep_launches = 2;
+    }
     return PADDI_OK;
 }
 
@@ -647,7 +648,7 @@ struct Prep {
 paddi_status enqueue_prep(paddi_ctx *ctx, const float *x, size_t n, int m, bool guided,
                           int32_t w_host, bool chained)
 {
-    paddi_status s = run_stats(ctx, x, n, m, true, chained);
+    paddi_status s = run_stats(ctx, x, n, m, chained);
     if (s != PADDI_OK) return s;
     s = witness_to(ctx, x, n, m);
     if (s != PADDI_OK) return s;
@@ -1226,10 +1227,7 @@ PADDI_API paddi_status paddi_compute_statistics(paddi_ctx *ctx, const float *d_T
         CK(cudaEventRecord(ctx->ev[0], user));
         CK(cudaStreamWaitEvent(ctx->st, ctx->ev[0], 0));
     }
-    s = run_stats(ctx, d_T, n, (int)m, /*tiles=*/false);
-    if (s != PADDI_OK) return s;
-    CK(paddi_launch_export_stats(ctx->d_ms64, (int32_t)(n - m + 1), (int)m, d_mean,
-                                 d_std, ctx->st));
+    CK(paddi_launch_mean_std(d_T, (int64_t)n, (int32_t)m, d_mean, d_std, ctx->st));
     if (user != ctx->st) {
         CK(cudaEventRecord(ctx->ev[1], ctx->st));
         CK(cudaStreamWaitEvent(user, ctx->ev[1], 0));

@@ -431,7 +431,7 @@ cudaError_t paddi_launch_fragile(const float *x, const double2 *ms64, const int3
 // [col_lo, col_hi) (col_lo a multiple of the tile width, col_hi too or N), all
 // rounds in one launch; list0 / list1: scratch, one entry per candidate each;
 // att->list_count[r] receives the candidates of round r > 0.  bq / wdq: the
-// per-length tile data of paddi_launch_tile_prep.  wait_cycles: limit of every
+// per-length tile data of paddi_launch_prep.  wait_cycles: limit of every
 // wait (<= 0: about 2 s); a wait that runs out sets att->status = 3 and the
 // kernel returns.  withhold != 0 is a test hook: the CTA holding work item 0
 // never fills that item's first stage, so its waits run out.
@@ -453,12 +453,14 @@ int32_t paddi_tile_width();
 int64_t paddi_tile_blocks(int64_t N);
 int64_t paddi_tile_block_elems_max();
 int64_t paddi_tile_wd_entries();
-// Fragile windows (bound above gcap) are appended to frag_list (frag_count
-// zeroed by the caller).
-cudaError_t paddi_launch_tile_prep(bool bf16, const float *x, int64_t n, int32_t m,
-                                   const float4 *wst, const float *mu, uint16_t *bq, float4 *wdq,
-                                   float gcap, int32_t *frag_list, int32_t *frag_count,
-                                   cudaStream_t st, unsigned long long *t_end = nullptr);
+// Statistics of length m (as paddi_launch_stats) and the tensor-core refine's
+// tile data in one kernel.  flat_count: {flat windows, span (2), fragile
+// windows}, zeroed; the fragile windows (bound above gcap) go to frag_list.
+cudaError_t paddi_launch_prep(bool bf16, const float *x, int64_t n, int32_t m, float4 *wst,
+                              float *mu, double2 *ms64, uint8_t *flat, int32_t *flat_count,
+                              uint16_t *bq, float4 *wdq, float gcap, int32_t *frag_list,
+                              cudaStream_t st, bool chained, const PaddiStatsExtra &extra,
+                              unsigned long long *t_end);
 
 cudaError_t paddi_launch_finalize(const int32_t *cand, PaddiAttemptDev *att,
                                   const uint32_t *rho_max, const uint8_t *pruned, int32_t m,
@@ -502,6 +504,9 @@ cudaError_t paddi_launch_guide(const float *x, const double2 *ms64,
                                PaddiGuide *host, const int32_t *flat_count,
                                unsigned long long *t);
 
+// Mean and population standard deviation of every window of length m.
+cudaError_t paddi_launch_mean_std(const float *x, int64_t n, int32_t m, float *mean, float *sd,
+                                  cudaStream_t st);
 cudaError_t paddi_launch_export_stats(const double2 *ms64, int32_t N,
                                       int32_t m, float *mean, float *sd, cudaStream_t st);
 
