@@ -1499,18 +1499,20 @@ PADDI_API paddi_status paddi_model_grad(paddi_ctx *ctx, const float *X, const fl
     CK(dmalloc(ctx, &dY.p, sizeof(float) * n));
     CK(dmalloc(ctx, &dP.p, sizeof(float) * MLP_NPARAM));
     CK(dmalloc(ctx, &dG.p, sizeof(float) * MLP_NPARAM));
-    CK(dmalloc(ctx, &dL.p, sizeof(float)));
+    CK(dmalloc(ctx, &dL.p, sizeof(double)));
     cudaStream_t st = ctx->st;
     CK(cudaMemcpyAsync(dX.p, X, sizeof(float) * MLP_NFEAT * n, cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(dY.p, Y, sizeof(float) * n, cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(dP.p, params, sizeof(float) * MLP_NPARAM, cudaMemcpyHostToDevice, st));
     CK(cudaMemsetAsync(dG.p, 0, sizeof(float) * MLP_NPARAM, st));
-    CK(cudaMemsetAsync(dL.p, 0, sizeof(float), st));
-    CK(paddi_launch_mlp_grad((float *)dX.p, (float *)dY.p, (int)n, tau, (float *)dP.p,
-                             (float *)dG.p, (float *)dL.p, ctx->num_sms, st));
+    CK(cudaMemsetAsync(dL.p, 0, sizeof(double), st));
+    CK(paddi_launch_mlp_grad((float *)dX.p, (float *)dY.p, nullptr, (int)n, tau, (float *)dP.p,
+                             (float *)dG.p, (double *)dL.p, ctx->num_sms, st));
     CK(cudaMemcpyAsync(grad, dG.p, sizeof(float) * MLP_NPARAM, cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(loss, dL.p, sizeof(float), cudaMemcpyDeviceToHost, st));
+    double lsum = 0.0;
+    CK(cudaMemcpyAsync(&lsum, dL.p, sizeof(double), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
+    *loss = (float)lsum;
     return PADDI_OK;
 }
 
@@ -1549,54 +1551,53 @@ PADDI_API paddi_status paddi_model_train(paddi_ctx *ctx, const float *X, const f
         return fail(ctx, PADDI_ERR_INVALID_ARG, "model_train: bad argument");
     CK(cudaSetDevice(ctx->device));
     cudaStream_t st = ctx->st;
-    DevBuf dX, dY, dP, dG, dM, dV, dL;
-    CK(dmalloc(ctx, &dX.p, sizeof(float) * MLP_NFEAT * n));
-    CK(dmalloc(ctx, &dY.p, sizeof(float) * n));
-    CK(dmalloc(ctx, &dP.p, sizeof(float) * MLP_NPARAM));
-    CK(dmalloc(ctx, &dG.p, sizeof(float) * MLP_NPARAM));
-    CK(dmalloc(ctx, &dM.p, sizeof(float) * MLP_NPARAM));
-    CK(dmalloc(ctx, &dV.p, sizeof(float) * MLP_NPARAM));
-    CK(dmalloc(ctx, &dL.p, sizeof(float) * (epochs ? epochs : 1)));
-    CK(cudaMemcpyAsync(dP.p, params, sizeof(float) * MLP_NPARAM, cudaMemcpyHostToDevice, st));
-    CK(cudaMemsetAsync(dG.p, 0, sizeof(float) * MLP_NPARAM, st));
-    CK(cudaMemsetAsync(dM.p, 0, sizeof(float) * MLP_NPARAM, st));
-    CK(cudaMemsetAsync(dV.p, 0, sizeof(float) * MLP_NPARAM, st));
-    CK(cudaMemsetAsync(dL.p, 0, sizeof(float) * (epochs ? epochs : 1), st));
-    std::vector<float> xs((size_t)MLP_NFEAT * n), ys(n);
+    // one allocation: the samples, an epoch's order, parameters, gradient, Adam
+    // moments, losses
+    DevBuf buf;
+    size_t bytes = 0;
+    auto place = [&](size_t b) {
+        const size_t at = bytes;
+        bytes += (b + 255) & ~(size_t)255;
+        return at;
+    };
+    const size_t np = sizeof(float) * MLP_NPARAM, nl = sizeof(double) * (epochs ? epochs : 1);
+    const size_t oX = place(sizeof(float) * MLP_NFEAT * n), oY = place(sizeof(float) * n);
+    const size_t oI = place(sizeof(uint32_t) * n), oP = place(np), oG = place(np), oM = place(np);
+    const size_t oV = place(np), oL = place(nl);
+    CK(dmalloc(ctx, &buf.p, bytes));
+    auto at = [&](size_t o) { return reinterpret_cast<float *>(static_cast<char *>(buf.p) + o); };
+    uint32_t *dI = reinterpret_cast<uint32_t *>(at(oI));
+    CK(cudaMemsetAsync(at(oG), 0, bytes - oG, st));
+    CK(cudaMemcpyAsync(at(oP), params, np, cudaMemcpyHostToDevice, st));
+    CK(cudaMemcpyAsync(at(oX), X, sizeof(float) * MLP_NFEAT * n, cudaMemcpyHostToDevice, st));
+    CK(cudaMemcpyAsync(at(oY), Y, sizeof(float) * n, cudaMemcpyHostToDevice, st));
     std::vector<uint32_t> perm(n);
     for (uint32_t i = 0; i < n; ++i) perm[i] = i;
     uint64_t rng = seed * 6364136223846793005ull + 1442695040888963407ull;
     int step = 0;
     for (uint32_t e = 0; e < epochs; ++e) {
+        // the next order is drawn while the epoch before runs (the copy from
+        // pageable memory is done with the host's array when it returns)
         for (uint32_t i = n - 1; i > 0; --i) { // Fisher-Yates with an LCG
             rng = rng * 6364136223846793005ull + 1442695040888963407ull;
-            const uint32_t k = (uint32_t)((rng >> 33) % (i + 1));
+            const uint32_t k = (uint32_t)(rng >> 33) % (i + 1);
             std::swap(perm[i], perm[k]);
         }
-        CK(cudaStreamSynchronize(st)); // the host buffers are reused each epoch
-        for (uint32_t i = 0; i < n; ++i) {
-            std::memcpy(&xs[(size_t)i * MLP_NFEAT], &X[(size_t)perm[i] * MLP_NFEAT],
-                        sizeof(float) * MLP_NFEAT);
-            ys[i] = Y[perm[i]];
-        }
-        CK(cudaMemcpyAsync(dX.p, xs.data(), sizeof(float) * xs.size(), cudaMemcpyHostToDevice, st));
-        CK(cudaMemcpyAsync(dY.p, ys.data(), sizeof(float) * n, cudaMemcpyHostToDevice, st));
+        CK(cudaMemcpyAsync(dI, perm.data(), sizeof(uint32_t) * n, cudaMemcpyHostToDevice, st));
         for (uint32_t b0 = 0; b0 < n; b0 += batch) {
             const uint32_t bn = std::min(batch, n - b0);
-            CK(paddi_launch_mlp_grad((float *)dX.p + (size_t)b0 * MLP_NFEAT, (float *)dY.p + b0,
-                                     (int)bn, tau, (float *)dP.p, (float *)dG.p,
-                                     (float *)dL.p + e, ctx->num_sms, st));
-            CK(paddi_launch_mlp_adam((float *)dP.p, (float *)dG.p, (float *)dM.p, (float *)dV.p,
-                                     lr, ++step, st));
+            CK(paddi_launch_mlp_grad(at(oX), at(oY), dI + b0, (int)bn, tau, at(oP), at(oG),
+                                     reinterpret_cast<double *>(at(oL)) + e, ctx->num_sms, st));
+            CK(paddi_launch_mlp_adam(at(oP), at(oG), at(oM), at(oV), lr, ++step, st));
         }
     }
-    CK(cudaMemcpyAsync(params, dP.p, sizeof(float) * MLP_NPARAM, cudaMemcpyDeviceToHost, st));
-    std::vector<float> lsum(epochs ? epochs : 1);
-    CK(cudaMemcpyAsync(lsum.data(), dL.p, sizeof(float) * lsum.size(), cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(params, at(oP), np, cudaMemcpyDeviceToHost, st));
+    std::vector<double> lsum(epochs ? epochs : 1);
+    CK(cudaMemcpyAsync(lsum.data(), at(oL), nl, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     if (loss) {
         const uint32_t nb = (n + batch - 1) / batch;
-        for (uint32_t e = 0; e < epochs; ++e) loss[e] = lsum[e] / (float)nb;
+        for (uint32_t e = 0; e < epochs; ++e) loss[e] = (float)(lsum[e] / (double)nb);
     }
     return PADDI_OK;
 }

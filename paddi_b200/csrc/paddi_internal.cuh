@@ -522,8 +522,9 @@ cudaError_t paddi_launch_scatter(const int32_t *cand, const PaddiAttemptDev *att
 #define MLP_NPARAM (MLP_HIDDEN * MLP_NFEAT + MLP_HIDDEN + MLP_HIDDEN * MLP_HIDDEN + MLP_HIDDEN + MLP_HIDDEN + 1)
 cudaError_t paddi_launch_mlp_forward(const float *X, int n, const void *P, bool bf16, float *Y,
                                      cudaStream_t st);
-cudaError_t paddi_launch_mlp_grad(const float *X, const float *Y, int n, float tau,
-                                  const float *P, float *G, float *loss, int num_sms,
+// perm (optional): rows of X and Y to take, in order.
+cudaError_t paddi_launch_mlp_grad(const float *X, const float *Y, const uint32_t *perm, int n,
+                                  float tau, const float *P, float *G, double *loss, int num_sms,
                                   cudaStream_t st);
 cudaError_t paddi_launch_mlp_adam(float *P, float *G, float *M, float *V, float lr, int step,
                                   cudaStream_t st);
