@@ -52,30 +52,49 @@ __device__ __forceinline__ float ld<__nv_bfloat16>(const __nv_bfloat16 *p, int i
     return __bfloat162float(p[i]);
 }
 
-// Forward pass of one sample by one warp; returns y_hat on every lane.
+// Parameters of one model.
 template <typename W>
-__device__ float mlp_forward(const W *P, const float *x, int lane)
+struct MlpView {
+    const W *w1, *b1, *w2, *b2, *w3, *b3;
+    int w2s; // row stride of W2
+};
+
+template <typename W>
+__device__ __forceinline__ MlpView<W> packed_view(const W *P)
 {
-    float h1[2];
+    return MlpView<W>{P + OW1, P + OB1, P + OW2, P + OB2, P + OW3, P + OB3, H};
+}
+
+// Forward pass of one sample by one warp; returns y_hat on every lane and the
+// pre-activations / activations of the lane's two units per layer.
+template <typename W>
+__device__ float mlp_forward(const MlpView<W> &P, const float *x, int lane, float (&z1)[2],
+                             float (&h1)[2], float (&z2)[2], float (&h2)[2])
+{
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
         const int u = lane + 32 * q;
-        float a = ld(P + OB1, u);
+        float a = ld(P.b1, u);
 #pragma unroll
-        for (int k = 0; k < F; ++k) a = fmaf(ld(P + OW1, u * F + k), x[k], a);
+        for (int k = 0; k < F; ++k) a = fmaf(ld(P.w1, u * F + k), x[k], a);
+        z1[q] = a;
         h1[q] = gelu(a);
     }
-    float a0 = ld(P + OB2, lane), a1 = ld(P + OB2, lane + 32);
+    float a0 = ld(P.b2, lane), a1 = ld(P.b2, lane + 32);
 #pragma unroll 4
     for (int v = 0; v < H; ++v) {
         const float hv = __shfl_sync(0xffffffffu, v < 32 ? h1[0] : h1[1], v & 31);
-        a0 = fmaf(ld(P + OW2, lane * H + v), hv, a0);
-        a1 = fmaf(ld(P + OW2, (lane + 32) * H + v), hv, a1);
+        a0 = fmaf(ld(P.w2, lane * P.w2s + v), hv, a0);
+        a1 = fmaf(ld(P.w2, (lane + 32) * P.w2s + v), hv, a1);
     }
-    float y = ld(P + OW3, lane) * gelu(a0) + ld(P + OW3, lane + 32) * gelu(a1);
+    z2[0] = a0;
+    z2[1] = a1;
+    h2[0] = gelu(a0);
+    h2[1] = gelu(a1);
+    float y = ld(P.w3, lane) * h2[0] + ld(P.w3, lane + 32) * h2[1];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
-    return y + ld(P + OB3, 0);
+    return y + ld(P.b3, 0);
 }
 
 template <typename W>
@@ -85,11 +104,13 @@ __global__ void k_mlp_forward(const float *__restrict__ X, int n, const W *__res
     const int lane = threadIdx.x & 31;
     const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nw = (gridDim.x * blockDim.x) >> 5;
+    const MlpView<W> P = packed_view(Pg);
     for (int s = wid; s < n; s += nw) {
         float x[F];
 #pragma unroll
         for (int k = 0; k < F; ++k) x[k] = X[(size_t)s * F + k];
-        const float y = mlp_forward(Pg, x, lane);
+        float z1[2], h1[2], z2[2], h2[2];
+        const float y = mlp_forward(P, x, lane, z1, h1, z2, h2);
         if (lane == 0) Y[s] = y;
     }
 }
