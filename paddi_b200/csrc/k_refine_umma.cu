@@ -40,6 +40,19 @@
 //   * epilogue (8 warps, two per TMEM lane quarter, 128 columns each):
 //     double-buffered tcgen05.ld, rho with packed f32x2 FMAs, running maxima,
 //     prune flags.
+// Screening.  The three products of a tile are needed to 2e-4, but most tiles
+// hold nothing that matters: no correlation above what their live candidates are
+// known to reach.  hi * hi alone, a third of the MMAs, is within gc (about 5e-3 on
+// the headline series) of the exact value; when its maximum plus that bound stays
+// below the best value known of every live candidate (this item's tiles, other
+// CTAs' through rho_max, the candidate's witness), the other two products and the
+// full epilogue are skipped.  A candidate whose lower bound is above thr is pruned
+// at once.  Nothing kept is computed with less than all three products.  The MMA
+// thread issues tile u+1's hi * hi before it takes the verdict on tile u; 8 to 30 %
+// of the tiles need everything.  What bounds a screened tile is the epilogue (2000
+// cycles with all window data, 1000 with the screen's weights) and the hops
+// between the roles, about 3700 cycles together; headline run 154 -> 144 ms.
+//
 // The candidate operand is built by all 384 threads at the start of a work
 // item.  When every candidate of the item is pruned the loader stops and
 // sends an end token through the pipeline, so all roles consume the same
@@ -57,6 +70,7 @@
 
 using paddi::compact_survivors;
 using paddi::f2ord;
+using paddi::ord2f;
 
 namespace {
 
@@ -65,12 +79,27 @@ constexpr int UM_TCMAX = 16;     // candidates per tile (M = 128); 8 for M = 64
 constexpr int UM_N = 256;        // windows at stride 8
 constexpr int UM_TW = UM_N * 8;  // windows per tile (one block of the grid)
 constexpr int UM_FEW = 4;        // tiles that take all remaining windows after the first round
+// A tile is screened by its hi * hi product first (split-FP16, where the work item
+// has several tiles and K' is long enough; the comment at the kernel has the
+// figures): refine launches at n = 300007 with tens of thousands of candidates, all
+// products at once / screened, us: m = 64 (K' 80) 2067 / 2152, m = 100 (112) 2270 /
+// 2238, m = 200 (208) 3935 / 3035, m = 500 (512) 18700 / 10000, m = 700 (720) 27450 /
+// 14140; PALMAD 64..512 at 2^18 151 ms / 139.  With one to three tiles an item's first
+// tile, which nothing is known about yet, is most of it: MERLIN at n = 2^18 1.27 ms,
+// 1.49 screened.  BF16 leaves out 2^-8 of the slice: its screen rejects little.
+constexpr int UM_SCREEN_T = 4;
+constexpr int UM_SCREEN_K = 112;
 constexpr int UM_WAVES = 1;      // work items per CTA and round when candidate tiles are few
 constexpr int UM_KMAX128 = 368;  // largest K' with M = 128 (shared-memory bound)
 constexpr int UM_KMAX64 = 736;   // largest K' with M = 64
+constexpr int UM_STAGES = 4;      // at most
 constexpr int ZSCALE = 8;        // zhat scaled by 2^8 before splitting
 constexpr int WD_ROW = 129;      // float4 entries per shift row of the window data (128 + pad)
-constexpr int WD_BYTES = 8 * WD_ROW * 16;
+constexpr int WQ_ROW = 132;      // words per shift row of the screen's weights (128 + pad)
+constexpr int WQ_OFF = 8 * WD_ROW;   // they follow the window data (float4 entries)
+constexpr int WD_ENTRIES = WQ_OFF + 8 * WQ_ROW / 4;
+constexpr int WD_BYTES = WD_ENTRIES * 16;
+constexpr uint32_t UM_SMEM_MAX = 227 * 1024 - 896; // dynamic; the rest is UmShared
 // limit of the abort path's drain waits (~2 s at 1.9 GHz): copies and MMAs the
 // kernel issued complete on their own, so these waits end long before it
 constexpr long long kDrainCycles = 4000000000ll;
@@ -114,8 +143,9 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity)
 
 // Bounded wait for the completion of the phase with the given parity;
 // false when `limit` clock cycles passed first.
-__device__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity, long long limit)
+__device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity, long long limit)
 {
+    if (mbar_try_wait(bar, parity)) return true; // mostly: no clock is read then
     const long long t0 = clock64();
     while (!mbar_try_wait(bar, parity))
         if (clock64() - t0 > limit) return false;
@@ -228,12 +258,14 @@ template <bool BF> struct E16;
 template <> struct E16<false> {
     using T = __half;
     static constexpr uint32_t fmt = 0;
+    static constexpr float uh = 4.8828125e-4f; // 2^-11: relative rounding of a half
     __device__ static __half cvt(float v) { return __float2half_rn(v); }
     __device__ static float back(__half v) { return __half2float(v); }
 };
 template <> struct E16<true> {
     using T = __nv_bfloat16;
     static constexpr uint32_t fmt = 1;
+    static constexpr float uh = 3.90625e-3f; // 2^-8
     __device__ static __nv_bfloat16 cvt(float v) { return __float2bfloat16_rn(v); }
     __device__ static float back(__nv_bfloat16 v) { return __bfloat162float(v); }
 };
@@ -359,18 +391,26 @@ k_prep(const float *__restrict__ x, int64_t nser, int32_t cnt, int32_t m, int32_
         lo[p2] = (uint32_t)reinterpret_cast<const uint16_t &>(l0) |
                  ((uint32_t)reinterpret_cast<const uint16_t &>(l1) << 16);
     }
-    float *wf = reinterpret_cast<float *>(wdq + (size_t)b * 8 * WD_ROW);
+    // built in shared memory (the prefixes are done with), written out in one sweep
+    float *wf = reinterpret_cast<float *>(st_mem);
+    __nv_bfloat16 *wq = reinterpret_cast<__nv_bfloat16 *>(wf + 4 * WQ_OFF);
     const float F = Fu * mx, fm = (float)m;
-    float gmax = 0.f;
+    float gmax = 0.f, amax = 1.f;
 #pragma unroll
     for (int kq = 0; kq < ST_WPT; ++kq) {
         const int q = threadIdx.x + ST_THREADS * kq;
         const int64_t j = j0 + q;
         const float g = paddi::window_bound(iv[kq], mv[kq], sh, fm, E, F);
         const bool frag = j < N && g > gcap;
-        if (!frag) gmax = fmaxf(gmax, g);
+        if (!frag) {
+            gmax = fmaxf(gmax, g);
+            const float bb = (mv[kq] - sh) * iv[kq];
+            amax = fmaxf(amax, sqrtf(fmaf(fm * bb, bb, 1.f)) * 1.0001f);
+        }
         const int s = q & 7, i = q >> 3, k = i >> 1, slot = i & 1;
-        wf[(s * WD_ROW + k) * 4 + slot] = frag ? __int_as_float(0x7fffffff) : iv[kq] * dsc;
+        const float a = frag ? __int_as_float(0x7fffffff) : iv[kq] * dsc;
+        wf[(s * WD_ROW + k) * 4 + slot] = a;
+        wq[(s * WQ_ROW + k) * 2 + slot] = __float2bfloat16_rn(a);
         wf[(s * WD_ROW + k) * 4 + 2 + slot] = (mv[kq] - sh) * iv[kq];
         // fragile windows in index order within each warp (runs stay contiguous)
         const unsigned bal = __ballot_sync(0xffffffffu, frag);
@@ -382,22 +422,40 @@ k_prep(const float *__restrict__ x, int64_t nser, int32_t cnt, int32_t m, int32_
         }
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) gmax = fmaxf(gmax, __shfl_xor_sync(0xffffffffu, gmax, o));
-    if (lane == 0) red[0][w] = gmax;
+    for (int o = 16; o > 0; o >>= 1) {
+        gmax = fmaxf(gmax, __shfl_xor_sync(0xffffffffu, gmax, o));
+        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    }
+    if (lane == 0) {
+        red[0][w] = gmax;
+        red[1][w] = amax;
+    }
     __syncthreads();
     if (threadIdx.x == 0) {
-        float G = 0.f;
-        for (int k = 0; k < ST_THREADS / 32; ++k) G = fmaxf(G, red[0][k]);
+        float G = 0.f, A = 1.f;
+        for (int k = 0; k < ST_THREADS / 32; ++k) {
+            G = fmaxf(G, red[0][k]);
+            A = fmaxf(A, red[1][k]);
+        }
         wf[(0 * WD_ROW + 128) * 4] = G; // padding entry of shift row 0
-        paddi::stamp_end(t_end);
+        wf[(0 * WD_ROW + 128) * 4 + 1] = A;
     }
+    __syncthreads();
+    const float4 *src = reinterpret_cast<const float4 *>(st_mem);
+    for (int k = threadIdx.x; k < WD_ENTRIES; k += ST_THREADS) wdq[(size_t)b * WD_ENTRIES + k] = src[k];
+    if (threadIdx.x == 0) paddi::stamp_end(t_end);
 }
 
 // ------------------------------------------------------------------ shared memory
 struct UmLayout {
-    uint32_t a_hi, a_lo, b[2][2], wd, bytes;
+    uint32_t a_hi, a_lo, b[UM_STAGES][2], wd[UM_STAGES], bytes;
+    int nb, nw; // stages of slices and of window data
 };
 
+// As many stages as fit, up to 4, of a slice and its window data each (K' = 208: 4,
+// 320: 2), so that a tile's data are requested that many tiles ahead: refine
+// launches of an ECG series of 2^23 points 8.2 -> 7.0 ms, m = 64 at n = 300007 2.18 ->
+// 2.09 ms.  The largest K' have room for two slices and one set of window data.
 __host__ __device__ inline UmLayout um_layout(int MM, int kp)
 {
     UmLayout L;
@@ -405,28 +463,42 @@ __host__ __device__ inline UmLayout um_layout(int MM, int kp)
     const uint32_t b_bytes = (uint32_t)slice_cnt(kp) * 2; // multiple of 32
     L.a_hi = 0;
     L.a_lo = a_bytes;
+    const int fit = (int)((UM_SMEM_MAX - 2 * a_bytes) / (2 * b_bytes + WD_BYTES));
+    L.nb = fit >= UM_STAGES ? UM_STAGES : fit >= 2 ? fit : 2;
+    L.nw = fit >= 2 ? L.nb : 1;
+    // slice 0, the window data, the other slices: without slice 0, or without the
+    // last one, enough contiguous room is left for the operand build's scratch
     uint32_t o = 2 * a_bytes;
-    for (int s = 0; s < 2; ++s)
-        for (int h = 0; h < 2; ++h) {
-            L.b[s][h] = o;
-            o += b_bytes;
-        }
-    L.wd = o; // window data of the current tile, directly after the stages
-    o += WD_BYTES;
+    for (int s = 0; s < UM_STAGES; ++s) {
+        if (s < L.nb)
+            for (int h = 0; h < 2; ++h) {
+                L.b[s][h] = o;
+                o += b_bytes;
+            }
+        if (s == 0)
+            for (int q = 0; q < UM_STAGES; ++q) {
+                L.wd[q] = o;
+                if (q < L.nw) o += WD_BYTES;
+            }
+    }
     L.bytes = o;
     return L;
 }
 
 struct UmShared {
-    uint64_t full_b[2];    // loader -> MMA: stage holds the tile's slice (or an end token)
+    // rings over the stages (full, empty) and over the two accumulators
+    uint64_t full_b[UM_STAGES];   // loader -> MMA: the stage holds the tile's slice (or an end token)
+    uint64_t wd_full[UM_STAGES];  // loader -> epilogue: and its window data (or an end token)
+    uint64_t sl_empty[UM_STAGES]; // epilogue -> loader: done with the slice
+    uint64_t wd_empty[UM_STAGES]; // epilogue -> loader: done with the window data
     uint64_t mma_done[2];  // tcgen05.commit: the tile's MMAs are complete
     uint64_t acc_empty[2]; // epilogue -> MMA: accumulator drained
-    uint64_t wd_full;      // loader -> epilogue: window data of the tile (or an end token)
-    uint64_t wd_empty;     // epilogue -> loader: window data consumed
+    uint64_t dec[2];       // epilogue -> MMA: hi * hi product screened, need[] decided
+    uint64_t rest_done[2]; // tcgen05.commit: the products with lo halves are complete
     uint64_t drain;        // final MMA drain on abort
-    // absolute phase index of the last arrival the loader issued on full_b[s] /
-    // wd_full (-1: none yet); the abort path waits only for those
-    int last_full[2], last_wd;
+    // phase of the last arrival the loader issued on full_b[s] / wd_full[s] (-1: none
+    // yet); the abort path waits only for those
+    int last_full[UM_STAGES], last_wd[UM_STAGES];
     uint32_t tmem_base;
     int item, abort, tok;
     int built_tile; // candidate tile whose operand sits in A (-1: none)
@@ -434,20 +506,31 @@ struct UmShared {
                     // candidates of the next round (-1: give up)
     int wsum[UM_THREADS / 32];
     volatile int item_dead;
-    int tile_live; // live candidates at the start of the current tile (instrumentation)
-    volatile int vb[2], vw;
+    volatile int vb[UM_STAGES], vw[UM_STAGES];
     int cw[UM_TCMAX], cp[UM_TCMAX];
     float cflat[UM_TCMAX], zsum[UM_TCMAX];
+    // screening: sum of the hi halves, norm of what they leave out, a correlation
+    // the candidate is known to reach; need[s]: tag of the last tile in accumulator
+    // s that needs its other products
+    float zsumh[UM_TCMAX], zrest[UM_TCMAX], known[UM_TCMAX];
+    volatile uint32_t need[2];
     uint32_t rmax[UM_TCMAX];
     volatile uint8_t dead[UM_TCMAX];
 };
 
-// Completed phases of each barrier before the current work item.
-struct UmPhases {
-    uint32_t full[2], done[2], acc[2], wdf, wde;
-};
+static_assert(sizeof(UmShared) <= 896, "beside the largest operand and window data");
 
-__device__ __forceinline__ uint32_t par(uint32_t idx) { return idx & 1u; }
+// The n-th use of a ring of `stages` barriers: its barrier and phase parity.  Every
+// tile (and every end token) of a CTA takes one use of every ring, so one count
+// over the CTA's work items serves them all.
+struct Ring {
+    int s;
+    uint32_t par;
+    __device__ __forceinline__ Ring(uint32_t n, int stages)
+        : s((int)(n % (uint32_t)stages)), par((n / (uint32_t)stages) & 1u)
+    {
+    }
+};
 
 // MM = 128: 16 candidates, accumulator row r in TMEM lane r.
 // MM = 64:  8 candidates, accumulator row r in TMEM lane (r % 16) + 32 (r / 16)
@@ -459,13 +542,13 @@ k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
               int32_t *list1, const uint16_t *__restrict__ bq, const float4 *__restrict__ wdq,
               PaddiAttemptDev *att, uint32_t *rho_max, uint8_t *pruned, int32_t N, int32_t m,
               int32_t col_lo, int32_t col_hi, float thr, int32_t grid_ctas, long long wl,
-              int32_t withhold, PaddiWitness W, PaddiBlockMax B)
+              int32_t withhold, PaddiWitness W, PaddiBlockMax B, int32_t may_screen, float guard)
 {
     using X = E16<BF>;
     constexpr int UM_M = MM;
     constexpr int UM_TC = MM / 8;
     constexpr int RG = MM / 8;          // 8-row core-matrix groups of A
-    extern __shared__ __align__(1024) unsigned char um_smem[];
+    extern __shared__ __align__(128) unsigned char um_smem[];
     __shared__ UmShared S;
     const int kp = kpad_of(m);
     const int cnt = slice_cnt(kp);
@@ -482,17 +565,23 @@ k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
     const bool bkeep = B.kept(C);
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < 2; ++s) {
+        for (int s = 0; s < UM_STAGES; ++s) {
             mbar_init(&S.full_b[s], 1);
+            mbar_init(&S.wd_full[s], 1);
+            mbar_init(&S.sl_empty[s], EPI_WARPS);
+            mbar_init(&S.wd_empty[s], EPI_WARPS);
+            S.last_full[s] = S.last_wd[s] = -1;
+        }
+        for (int s = 0; s < 2; ++s) {
             mbar_init(&S.mma_done[s], 1);
             mbar_init(&S.acc_empty[s], EPI_WARPS);
+            mbar_init(&S.dec[s], EPI_WARPS);
+            mbar_init(&S.rest_done[s], 1);
+            S.need[s] = 0;
         }
-        mbar_init(&S.wd_full, 1);
-        mbar_init(&S.wd_empty, EPI_WARPS);
         mbar_init(&S.drain, 1);
         S.abort = 0;
         S.last = 0;
-        S.last_full[0] = S.last_full[1] = S.last_wd = -1;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
@@ -506,8 +595,9 @@ k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = S.tmem_base;
-    UmPhases ph = {{0u, 0u}, {0u, 0u}, {0u, 0u}, 0u, 0u};
+    uint32_t G = 0; // tiles and end tokens of this CTA before the current work item
     bool mma_issued = false; // MMA thread: any MMA issued
+    uint32_t n_rest0 = 0u, n_rest1 = 0u; // epilogue: completed phases of rest_done
 
     const uint32_t idesc = idesc_f16(X::fmt, UM_M, UM_N);
     const uint32_t a_hi_s = smem_u32(um_smem + L.a_hi), a_lo_s = smem_u32(um_smem + L.a_lo);
@@ -517,7 +607,6 @@ k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
     const bool rowok = MM == 128 || lane < 16;
     const int row = MM == 128 ? 32 * g + lane : 16 * g + (lane & 15);
     const int cidx = row >> 3, bsh = row & 7;
-    const float4 *wd4 = reinterpret_cast<const float4 *>(um_smem + L.wd);
 
     // ---- rounds: the windows [jb, je) of growing ranges (1/16, 1/4, 1/2, all of
     // them), the survivors compacted in between so that every tile is dense.  A
@@ -565,6 +654,10 @@ k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
                 S.dead[threadIdx.x] = !v || __ldcg(pruned + pos);
                 S.cflat[threadIdx.x] = (v && wst[w].z == 0.f) ? 1.f : 0.f; // flat candidate
                 S.rmax[threadIdx.x] = f2ord(-INFINITY);
+                // a correlation this candidate reaches, from its witness (the kept value
+                // of that window is within the guard band of it)
+                S.known[threadIdx.x] =
+                    (v && W.wit) ? fmaxf(W.wrho[w] - guard - 1e-5f, -INFINITY) : -INFINITY;
             }
             if (threadIdx.x == 0) {
                 S.item_dead = 0;
@@ -575,27 +668,31 @@ k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
                 int a = threadIdx.x < UM_TC ? !S.dead[threadIdx.x] : 0;
                 if (!__syncthreads_or(a) || j_lo >= j_hi) continue; // all threads agree
             }
-            if (threadIdx.x == 32) { // read by the epilogue after the barriers below
-                int alive = 0;
-                for (int c = 0; c < UM_TC; ++c) alive += !S.dead[c];
-                S.tile_live = alive;
-            }
             const int T = (j_hi - j_lo + UM_TW - 1) / UM_TW;
+            const bool screen = may_screen && T >= UM_SCREEN_T;
             const int blk0 = j_lo / UM_TW; // j_lo is a multiple of UM_TW
-            // the first tile's slice streams into stage 0 while the operand is built
-            // (the build's scratch is stage 1 + the window data)
+            // the slice of tile u (its stage is free) or an end token
+            auto put_slice = [&](int u, bool token) {
+                const Ring r(G + (uint32_t)u, L.nb);
+                S.last_full[r.s] = (int)r.par;
+                S.vb[r.s] = !token;
+                if (token) {
+                    mbar_arrive(&S.full_b[r.s]);
+                    return;
+                }
+                const uint16_t *src = bq + (size_t)(blk0 + u) * 2 * cnt;
+                mbar_arrive_expect_tx(&S.full_b[r.s], (uint32_t)(4 * cnt));
+                bulk_g2s(um_smem + L.b[r.s][0], src, (uint32_t)(2 * cnt), &S.full_b[r.s]);
+                bulk_g2s(um_smem + L.b[r.s][1], src + cnt, (uint32_t)(2 * cnt), &S.full_b[r.s]);
+            };
+            // the first tile's slice streams in while the operand is built (the build's
+            // scratch lies clear of its stage)
+            const int stage0 = Ring(G, L.nb).s;
             if (warp == LOAD_WARP && lane == 0) {
-                S.vb[0] = 1;
                 // test hook (withhold != 0): the CTA holding work item 0 never fills
                 // its first stage, so the MMA thread's wait runs out; nothing is in flight
-                const bool skip = withhold && rd == 0 && item == 0;
-                if (!skip) {
-                    const uint16_t *src = bq + (size_t)blk0 * 2 * cnt;
-                    mbar_arrive_expect_tx(&S.full_b[0], (uint32_t)(4 * cnt));
-                    bulk_g2s(um_smem + L.b[0][0], src, (uint32_t)(2 * cnt), &S.full_b[0]);
-                    bulk_g2s(um_smem + L.b[0][1], src + cnt, (uint32_t)(2 * cnt), &S.full_b[0]);
-                    S.last_full[0] = (int)ph.full[0];
-                }
+                S.vb[stage0] = 1;
+                if (!(withhold && rd == 0 && item == 0)) put_slice(0, false);
             }
             // ---- candidate operand: 16 x (hi, lo) rows of scaled zhat, then 8 shifted
             //      copies; kept from the CTA's previous item when that had the same
@@ -606,7 +703,7 @@ k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
                 // padding, then zhat[0..kp); stride ksw words with ksw % 32 == 8, so
                 // the four candidates a warp reads sit in disjoint bank ranges
                 const int ksw = zrow_words(kp);
-                uint32_t *zhw = reinterpret_cast<uint32_t *>(um_smem + L.b[1][0]);
+                uint32_t *zhw = reinterpret_cast<uint32_t *>(um_smem + (L.nw >= 2 || stage0 == 0 ? L.wd[0] : L.b[0][0]));
                 uint32_t *zlw = zhw + UM_TC * ksw;
                 typename X::T *zh = reinterpret_cast<typename X::T *>(zhw);
                 typename X::T *zl = reinterpret_cast<typename X::T *>(zlw);
@@ -615,7 +712,7 @@ k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
                 const bool live = c < UM_TC && !S.dead[c];
                 const float muc = live ? mu[w] : 0.f;
                 const float ivc = live ? wst[w].z * 256.f : 0.f; // 2^ZSCALE
-                float zs = 0.f;
+                float zs = 0.f, zsh = 0.f, zr = 0.f;
                 if (c < UM_TC)
                     for (int q = 4 + (kp >> 1) + t16; q < ksw; q += 16) { // tail words
                         zhw[c * ksw + q] = 0u;
@@ -634,11 +731,22 @@ k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
                         zh[c * 2 * ksw + 8 + k] = h;
                         zl[c * 2 * ksw + 8 + k] = l;
                     }
-                    zs += X::back(h) + X::back(l);
+                    const float hb = X::back(h), rs = v - hb;
+                    zs += hb + X::back(l);
+                    zsh += hb;
+                    zr = fmaf(rs, rs, zr);
                 }
 #pragma unroll
-                for (int o = 8; o > 0; o >>= 1) zs += __shfl_xor_sync(0xffffffffu, zs, o);
-                if (t16 == 0 && c < UM_TC) S.zsum[c] = zs * (1.f / 256.f);
+                for (int o = 8; o > 0; o >>= 1) {
+                    zs += __shfl_xor_sync(0xffffffffu, zs, o);
+                    zsh += __shfl_xor_sync(0xffffffffu, zsh, o);
+                    zr += __shfl_xor_sync(0xffffffffu, zr, o);
+                }
+                if (t16 == 0 && c < UM_TC) {
+                    S.zsum[c] = zs * (1.f / 256.f);
+                    S.zsumh[c] = zsh * (1.f / 256.f);
+                    S.zrest[c] = sqrtf(zr) * (1.01f / 256.f);
+                }
                 __syncthreads();
                 // A[(c,b), k'] = z_c[k' - b] in K-major core matrices:
                 // byte offset ((k'/8)*RG + r/8)*128 + (r%8)*16 + (k'%8)*2.
@@ -676,225 +784,378 @@ k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
 
             // ================================================================ roles
             if (warp == LOAD_WARP && lane == 0) {
-                // slice of tile u into stage u&1 (after the MMAs of tile u-2 are done);
-                // an end token instead once the item is dead
-                auto load_slice = [&](int u) -> bool {
-                    const int s = u & 1;
-                    if (u >= 2 && !mbar_wait_bounded(&S.mma_done[s], par(ph.done[s] + ((u - 2) >> 1)), wl))
-                        return false;
-                    S.last_full[s] = (int)(ph.full[s] + (u >> 1));
-                    if (S.item_dead) {
-                        S.vb[s] = 0;
-                        S.tok = u;
-                        mbar_arrive(&S.full_b[s]);
-                        return true;
-                    }
-                    S.vb[s] = 1;
-                    const uint16_t *src = bq + (size_t)(blk0 + u) * 2 * cnt;
-                    mbar_arrive_expect_tx(&S.full_b[s], (uint32_t)(4 * cnt));
-                    bulk_g2s(um_smem + L.b[s][0], src, (uint32_t)(2 * cnt), &S.full_b[s]);
-                    bulk_g2s(um_smem + L.b[s][1], src + cnt, (uint32_t)(2 * cnt), &S.full_b[s]);
-                    return true;
+                // the use `before` uses ago of a stage must be consumed (uses of earlier
+                // items are)
+                auto freed = [&](uint64_t *empty, int u, int stages) -> bool {
+                    if (G + (uint32_t)u < (uint32_t)stages) return true;
+                    const Ring r(G + (uint32_t)u - (uint32_t)stages, stages);
+                    return mbar_wait_bounded(empty + r.s, r.par, wl);
                 };
-                bool ok = true; // slice 0 was issued before the operand build
-                for (int u = 0; ok && u < T; ++u) {
-                    if (u + 1 < T) ok = load_slice(u + 1);
+                auto put_wd = [&](int u, bool token) {
+                    const Ring r(G + (uint32_t)u, L.nw);
+                    S.last_wd[r.s] = (int)r.par;
+                    S.vw[r.s] = !token;
+                    if (token) {
+                        mbar_arrive(&S.wd_full[r.s]);
+                        return;
+                    }
+                    mbar_arrive_expect_tx(&S.wd_full[r.s], (uint32_t)WD_BYTES);
+                    bulk_g2s(um_smem + L.wd[r.s], wdq + (size_t)(blk0 + u) * WD_ENTRIES,
+                             (uint32_t)WD_BYTES, &S.wd_full[r.s]);
+                };
+                // once the item is dead, an end token takes the place of a tile
+                bool ok = freed(S.wd_empty, 0, L.nw);
+                if (ok) put_wd(0, false); // slice 0 was issued before the operand build
+                for (int u = 1; ok && u < T && S.tok < 0; ++u) {
+                    ok = freed(S.sl_empty, u, L.nb);
                     if (!ok) break;
-                    // window data of tile u (after the epilogue is done with tile u-1)
-                    if (u >= 1 && !mbar_wait_bounded(&S.wd_empty, par(ph.wde + (u - 1)), wl)) {
-                        ok = false;
-                        break;
-                    }
-                    S.last_wd = (int)(ph.wdf + u);
-                    if (S.tok == u + 1) { // end token: no window data for tile u either
-                        S.vw = 0;
-                        mbar_arrive(&S.wd_full);
-                        break;
-                    }
-                    S.vw = 1;
-                    mbar_arrive_expect_tx(&S.wd_full, (uint32_t)WD_BYTES);
-                    bulk_g2s(um_smem + L.wd, wdq + (size_t)(blk0 + u) * 8 * WD_ROW, (uint32_t)WD_BYTES,
-                             &S.wd_full);
+                    const bool token = S.item_dead;
+                    if (token) S.tok = u;
+                    put_slice(u, token);
+                    ok = freed(S.wd_empty, u, L.nw);
+                    if (ok) put_wd(u, token);
                 }
                 if (!ok) S.abort = 1;
             } else if (warp == MMA_WARP && lane == 0) {
-                for (int u = 0; u < T; ++u) {
-                    const int s = u & 1;
-                    if (!mbar_wait_bounded(&S.full_b[s], par(ph.full[s] + (u >> 1)), wl)) {
-                        S.abort = 1;
+                // products of tile u: hi * hi, and (rest) hi * lo + lo * hi
+                auto issue = [&](int u, bool hihi, bool rest) {
+                    const uint32_t n = G + (uint32_t)u;
+                    const int st = Ring(n, L.nb).s;
+                    tc_fence_after();
+                    const uint32_t d = tmem + (n & 1u) * UM_N;
+                    const uint32_t bh = smem_u32(um_smem + L.b[st][0]);
+                    const uint32_t bl = smem_u32(um_smem + L.b[st][1]);
+                    // K-block kb = core-matrix columns 2kb, 2kb+1; LBO = next K column of cores.
+                    // The descriptors' address fields (16-byte units) just step along K
+                    uint64_t ah = sdesc(a_hi_s, RG * 128, 128), al = sdesc(a_lo_s, RG * 128, 128);
+                    uint64_t bhd = sdesc(bh, 16, 128), bld = sdesc(bl, 16, 128);
+                    constexpr uint64_t da = 2 * RG * 128 / 16, db = 32 / 16;
+                    if (!rest) {
+#pragma unroll 4
+                        for (int kb = 0; kb < kblocks; ++kb, ah += da, bhd += db)
+                            umma_f16(d, ah, bhd, idesc, kb > 0 ? 1u : 0u);
+                    } else {
+                        for (int kb = 0; kb < kblocks; ++kb, ah += da, al += da, bhd += db, bld += db) {
+                            if (hihi) umma_f16(d, ah, bhd, idesc, kb > 0 ? 1u : 0u);
+                            umma_f16(d, ah, bld, idesc, 1u);
+                            umma_f16(d, al, bhd, idesc, 1u);
+                        }
+                    }
+                    mma_issued = true;
+                };
+                // the screen's verdict on tile u (its own products may still be wanted)
+                auto settle = [&](int u) -> bool {
+                    const Ring a(G + (uint32_t)u, 2);
+                    if (!mbar_wait_bounded(&S.dec[a.s], a.par, wl)) return false;
+                    if (S.need[a.s] == G + (uint32_t)u + 1u) {
+                        issue(u, false, true);
+                        umma_commit(&S.rest_done[a.s]);
+                    }
+                    return true;
+                };
+                bool ok = true;
+                int u = 0;
+                for (; ok && u < T; ++u) {
+                    const uint32_t n = G + (uint32_t)u;
+                    const Ring r(n, L.nb), a(n, 2);
+                    if (!mbar_wait_bounded(&S.full_b[r.s], r.par, wl)) {
+                        ok = false;
                         break;
                     }
                     // the accumulator's previous tile must be drained first, also before an
-                    // end token: its commit completes a phase of mma_done[s] that the
-                    // epilogue may still be waiting on for tile u-2
-                    if (u >= 2 &&
-                        !mbar_wait_bounded(&S.acc_empty[s], par(ph.acc[s] + ((u - 2) >> 1)), wl)) {
-                        S.abort = 1;
+                    // end token: its commit completes a phase of mma_done that the epilogue
+                    // may still be waiting on for that tile
+                    if (n >= 2u && !mbar_wait_bounded(&S.acc_empty[a.s], Ring(n - 2u, 2).par, wl)) {
+                        ok = false;
                         break;
                     }
-                    if (!S.vb[s]) { // end token: pass it on (the commit also covers earlier MMAs)
-                        umma_commit(&S.mma_done[s]);
+                    if (!S.vb[r.s]) { // end token: pass it on (the commit also covers earlier MMAs)
+                        if (screen && u > 0) ok = settle(u - 1);
+                        umma_commit(&S.mma_done[a.s]);
                         break;
                     }
-                    tc_fence_after();
-                    const uint32_t d = tmem + (uint32_t)(s * UM_N);
-                    const uint32_t bh = smem_u32(um_smem + L.b[s][0]), bl = smem_u32(um_smem + L.b[s][1]);
-                    for (int kb = 0; kb < kblocks; ++kb) {
-                        // K-block kb = core-matrix columns 2kb, 2kb+1; LBO = next K column of cores
-                        const uint64_t ah = sdesc(a_hi_s + kb * (2 * RG * 128), RG * 128, 128);
-                        const uint64_t al = sdesc(a_lo_s + kb * (2 * RG * 128), RG * 128, 128);
-                        const uint64_t bhd = sdesc(bh + kb * 32, 16, 128);
-                        const uint64_t bld = sdesc(bl + kb * 32, 16, 128);
-                        umma_f16(d, ah, bhd, idesc, kb > 0 ? 1u : 0u);
-                        umma_f16(d, ah, bld, idesc, 1u);
-                        umma_f16(d, al, bhd, idesc, 1u);
-                    }
-                    umma_commit(&S.mma_done[s]);
-                    mma_issued = true;
+                    issue(u, true, !screen);
+                    umma_commit(&S.mma_done[a.s]);
+                    // the tile before was screened while this one's product started
+                    if (screen && u > 0) ok = settle(u - 1);
                 }
+                if (ok && screen && u == T) ok = settle(T - 1);
+                if (!ok) S.abort = 1;
             } else if (warp >= EPI_WARP0) {
                 float rmax = -INFINITY;
                 const int wc = S.cw[cidx];
                 const float zsc = S.zsum[cidx], fc = S.cflat[cidx];
-                const float2 nz2 = make_float2(-zsc, -zsc);
+                const float zsh = S.zsumh[cidx], zrest = S.zrest[cidx];
+                float known = S.known[cidx];
+                const float rsm = rsqrtf((float)m) * 1.001f;
+                // tiles of the item and their live candidates (instrumentation)
+                int n_tiles = 0, n_alive = 0;
+                int alive = __popc(__ballot_sync(0xffffffffu, lane < UM_TC && !S.dead[lane & (UM_TC - 1)]));
+                const uint8_t *gone_p = pruned + S.cp[(UM_TC / 4) * g + (lane & (UM_TC / 4 - 1))];
+                const uint32_t *known_p = rho_max + S.cp[cidx];
+                int gone_next = 0;
+                uint32_t kg_next = 0u;
                 // Every lane waits (acquire) and the warp then agrees through a vote, so
-                // the warp is converged and takes the same branch at every tcgen05.ld.
+                // the warp is converged and takes the same branch at every tcgen05.ld.  (One
+                // lane polling for the warp was slower: 40 instead of 37 ms per headline run.)
                 for (int u = 0; u < T; ++u) {
-                    const int s = u & 1;
-                    if (!__all_sync(0xffffffffu, mbar_wait_bounded(&S.wd_full, par(ph.wdf + u), wl))) {
+                    const uint32_t n = G + (uint32_t)u;
+                    const Ring a(n, 2), rw(n, L.nw);
+                    const int s = a.s;
+                    // what other CTAs have found meanwhile, asked for a tile ahead
+                    const int gone = gone_next;
+                    uint32_t kg = kg_next;
+                    if (lane < UM_TC / 4) gone_next = __ldcg(gone_p);
+                    if (screen && bsh == 0) kg_next = __ldcg(known_p);
+                    if (!__all_sync(0xffffffffu, mbar_wait_bounded(&S.wd_full[rw.s], rw.par, wl) &&
+                                                     mbar_wait_bounded(&S.mma_done[s], a.par, wl))) {
                         S.abort = 1;
                         break;
                     }
-                    const int vw = __shfl_sync(0xffffffffu, S.vw, 0);
-                    if (!__all_sync(0xffffffffu,
-                                    mbar_wait_bounded(&S.mma_done[s], par(ph.done[s] + (u >> 1)), wl))) {
-                        S.abort = 1;
+                    // an end token (its slice twin is committed too) takes its use of every ring
+                    const bool token = !__shfl_sync(0xffffffffu, S.vw[rw.s], 0);
+                    if (token) {
+                        if (lane == 0) {
+                            mbar_arrive(&S.dec[s]);
+                            mbar_arrive(&S.acc_empty[s]);
+                            mbar_arrive(&S.wd_empty[rw.s]);
+                            mbar_arrive(&S.sl_empty[Ring(n, L.nb).s]);
+                        }
                         break;
                     }
-                    if (!vw) { // end token; its slice twin at tile u+1 is committed too
-                        const int s1 = (u + 1) & 1;
-                        if (!__all_sync(0xffffffffu, mbar_wait_bounded(&S.mma_done[s1], par(ph.done[s1] + ((u + 1) >> 1)), wl)))
-                            S.abort = 1;
-                        break;
-                    }
+                    const float4 *wd4 = reinterpret_cast<const float4 *>(um_smem + L.wd[rw.s]);
                     tc_fence_after();
                     const int j0 = j_lo + u * UM_TW;
-                    if (!__shfl_sync(0xffffffffu, S.item_dead, 0)) {
+                    const uint32_t tag = n + 1u; // the tile's tag in need[s]
+                    const bool live = !__shfl_sync(0xffffffffu, S.item_dead, 0);
+                    bool full = true;
+                    if (live || screen) {
                         const uint32_t tb = tmem + ((uint32_t)(32 * g) << 16) +
                                             (uint32_t)(s * UM_N + 128 * hcol);
                         const bool masked = (j0 + UM_TW > j_hi) ||
                                             (wc > j0 - m + 1 && wc < j0 + UM_TW + m - 1) || fc != 0.f;
                         const float4 *wrow = wd4 + bsh * WD_ROW + 64 * hcol;
-                        // the tile's rounding bound (tile prep): correlations are lowered
-                        // by it for the prune test and raised back for the kept maxima
-                        const float Gt = wd4[128].x;
-                        const float2 ng2 = make_float2(-Gt, -Gt);
-                        float tm[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-                        // 4 chunks of 32 columns; the load of chunk cb+1 overlaps the math of cb
-                        auto chunk = [&](const uint32_t (&r)[32], int cb) {
-                            if (!masked) {
+                        // the tile's rounding bound and largest amplification (k_prep)
+                        const float Gt = wd4[128].x, At = wd4[128].y;
+                        uint32_t ra[32], rb[32];
+                        // maximum over the row's 128 columns of D a - z b - sub.  4 chunks of 32
+                        // columns; the load of chunk cb+1 overlaps the math of cb
+                        auto row_max = [&](float z, float sub) -> float {
+                            const float2 nz2 = make_float2(-z, -z), ns2 = make_float2(-sub, -sub);
+                            float tm[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+                            auto chunk = [&](const uint32_t (&r)[32], int cb) {
+                                if (!masked) {
 #pragma unroll
-                                for (int i2 = 0; i2 < 16; ++i2) {
-                                    const float4 wv = wrow[16 * cb + i2];
-                                    const float2 dd = make_float2(__uint_as_float(r[2 * i2]),
-                                                                  __uint_as_float(r[2 * i2 + 1]));
-                                    const float2 rho = __ffma2_rn(
-                                        dd, make_float2(wv.x, wv.y),
-                                        __ffma2_rn(nz2, make_float2(wv.z, wv.w), ng2));
-                                    tm[i2 & 3] = fmax3(tm[i2 & 3], rho.x, rho.y);
+                                    for (int i2 = 0; i2 < 16; ++i2) {
+                                        const float4 wv = wrow[16 * cb + i2];
+                                        const float2 dd = make_float2(__uint_as_float(r[2 * i2]),
+                                                                      __uint_as_float(r[2 * i2 + 1]));
+                                        const float2 rho = __ffma2_rn(
+                                            dd, make_float2(wv.x, wv.y),
+                                            __ffma2_rn(nz2, make_float2(wv.z, wv.w), ns2));
+                                        tm[i2 & 3] = fmax3(tm[i2 & 3], rho.x, rho.y);
+                                    }
+                                } else {
+#pragma unroll
+                                    for (int i = 0; i < 32; ++i) {
+                                        const int col = 128 * hcol + 32 * cb + i;
+                                        const int j = j0 + 8 * col + bsh;
+                                        const float4 wv = wrow[(32 * cb + i) >> 1];
+                                        const float wa = (i & 1) ? wv.y : wv.x;
+                                        const float wb = (i & 1) ? wv.w : wv.z;
+                                        float rho = fmaf(__uint_as_float(r[i]), wa, fmaf(-z, wb, -sub));
+                                        if (fc != 0.f && wa == 0.f) rho += 1.f; // two flat windows
+                                        const int dd = wc > j ? wc - j : j - wc;
+                                        if (j < j_hi && dd >= m - 1) tm[i & 3] = fmaxf(tm[i & 3], rho);
+                                    }
                                 }
-                            } else {
+                            };
+                            tmem_ld32_async(tb, ra);
+                            tmem_wait_ld(ra);
+                            tmem_ld32_async(tb + 32, rb);
+                            chunk(ra, 0);
+                            tmem_wait_ld(rb);
+                            tmem_ld32_async(tb + 64, ra);
+                            chunk(rb, 1);
+                            tmem_wait_ld(ra);
+                            tmem_ld32_async(tb + 96, rb);
+                            chunk(ra, 2);
+                            tmem_wait_ld(rb);
+                            chunk(rb, 3);
+                            return rowok ? fmaxf(fmaxf(tm[0], tm[1]), fmaxf(tm[2], tm[3])) : -INFINITY;
+                        };
+                        // maximum of D a alone, the weights in BF16: 8 columns per load
+                        auto screen_max = [&]() -> float {
+                            const uint4 *q4 = reinterpret_cast<const uint4 *>(wd4 + WQ_OFF) +
+                                              (bsh * WQ_ROW + 64 * hcol) / 4;
+                            float tm[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+                            auto chunk = [&](const uint32_t (&r)[32], int cb) {
 #pragma unroll
-                                for (int i = 0; i < 32; ++i) {
-                                    const int col = 128 * hcol + 32 * cb + i;
-                                    const int j = j0 + 8 * col + bsh;
-                                    const float4 wv = wrow[(32 * cb + i) >> 1];
-                                    const float wa = (i & 1) ? wv.y : wv.x;
-                                    const float wb = (i & 1) ? wv.w : wv.z;
-                                    float rho = fmaf(__uint_as_float(r[i]), wa, fmaf(-zsc, wb, -Gt));
-                                    if (fc != 0.f && wa == 0.f) rho += 1.f; // two flat windows
-                                    const int dd = wc > j ? wc - j : j - wc;
-                                    if (j < j_hi && dd >= m - 1) tm[i & 3] = fmaxf(tm[i & 3], rho);
+                                for (int i8 = 0; i8 < 4; ++i8) {
+                                    const uint4 w4 = q4[4 * cb + i8];
+                                    const uint32_t ww[4] = {w4.x, w4.y, w4.z, w4.w};
+#pragma unroll
+                                    for (int e = 0; e < 4; ++e) {
+                                        const float2 dd =
+                                            make_float2(__uint_as_float(r[8 * i8 + 2 * e]),
+                                                        __uint_as_float(r[8 * i8 + 2 * e + 1]));
+                                        const float2 aa =
+                                            make_float2(__uint_as_float(ww[e] << 16),
+                                                        __uint_as_float(ww[e] & 0xffff0000u));
+                                        const float2 v = __fmul2_rn(dd, aa);
+                                        tm[e] = fmax3(tm[e], v.x, v.y);
+                                    }
+                                }
+                            };
+                            tmem_ld32_async(tb, ra);
+                            tmem_wait_ld(ra);
+                            tmem_ld32_async(tb + 32, rb);
+                            chunk(ra, 0);
+                            tmem_wait_ld(rb);
+                            tmem_ld32_async(tb + 64, ra);
+                            chunk(rb, 1);
+                            tmem_wait_ld(ra);
+                            tmem_ld32_async(tb + 96, rb);
+                            chunk(ra, 2);
+                            tmem_wait_ld(rb);
+                            chunk(rb, 3);
+                            return rowok ? fmaxf(fmaxf(tm[0], tm[1]), fmaxf(tm[2], tm[3])) : -INFINITY;
+                        };
+                        // prunes the candidates whose lower bound `low` exceeds thr, and those
+                        // pruned elsewhere.  A candidate pruned here leaves the window that did
+                        // it as its witness hint: a second pass over the accumulator, at most
+                        // once per candidate, finds its column
+                        auto prune = [&](float low, float z, float sub) {
+                            const unsigned bal = __ballot_sync(0xffffffffu, low > thr);
+                            bool hint = false;
+                            if (lane < UM_TC / 4) {
+                                const int ci = (UM_TC / 4) * g + lane;
+                                if (!S.dead[ci]) {
+                                    if ((bal >> (8 * lane)) & 0xFFu) {
+                                        S.dead[ci] = 1;
+                                        pruned[S.cp[ci]] = 1;
+                                        hint = W.wit != nullptr;
+                                    } else if (gone) {
+                                        S.dead[ci] = 1; // pruned by another CTA's item
+                                    }
                                 }
                             }
+                            const unsigned hints = __ballot_sync(0xffffffffu, hint);
+                            if (hints) {
+                                int jh = -1;
+                                const bool mine = rowok && ((hints >> (lane >> 3)) & 1u) && low > thr;
+                                for (int cb = 0; cb < 4; ++cb) {
+                                    tmem_ld32_async(tb + 32 * cb, ra);
+                                    tmem_wait_ld(ra);
+#pragma unroll
+                                    for (int i = 0; i < 32; ++i) {
+                                        const int j = j0 + 8 * (128 * hcol + 32 * cb + i) + bsh;
+                                        const float4 wv = wrow[(32 * cb + i) >> 1];
+                                        const float rho =
+                                            fmaf(__uint_as_float(ra[i]), (i & 1) ? wv.y : wv.x,
+                                                 fmaf(-z, (i & 1) ? wv.w : wv.z, -sub));
+                                        const int dd = wc > j ? wc - j : j - wc;
+                                        if (rho > thr && j < j_hi && dd >= m - 1) jh = j;
+                                    }
+                                }
+                                if (mine && jh >= 0) wt_hint(W, wc, WT_ONE, jh);
+                            }
+                            __syncwarp();
                         };
-                        uint32_t ra[32], rb[32];
-                        tmem_ld32_async(tb, ra);
-                        tmem_wait_ld(ra);
-                        tmem_ld32_async(tb + 32, rb);
-                        chunk(ra, 0);
-                        tmem_wait_ld(rb);
-                        tmem_ld32_async(tb + 64, ra);
-                        chunk(rb, 1);
-                        tmem_wait_ld(ra);
-                        tmem_ld32_async(tb + 96, rb);
-                        chunk(ra, 2);
-                        tmem_wait_ld(rb);
-                        chunk(rb, 3);
-                        float tmax = fmaxf(fmaxf(tm[0], tm[1]), fmaxf(tm[2], tm[3]));
-                        if (!rowok) tmax = -INFINITY;
-                        rmax = fmaxf(rmax, tmax + Gt); // the interval's middle (-inf stays)
-                        if (bkeep) { // the half block's maximum over the 8 shifts
-                            float bm = tmax + Gt;
+                        // the half block's maximum (or a bound of it) over the 8 shifts
+                        auto keep_block = [&](float bm) {
+                            if (!bkeep) return;
 #pragma unroll
                             for (int o = 4; o > 0; o >>= 1)
                                 bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, o));
                             if (rowok && bsh == 0 && wc >= 0)
                                 B.v[(int64_t)S.cp[cidx] * B.halves + j0 / PADDI_HALF + hcol] =
                                     f2ord(bm);
+                        };
+                        float hup = -INFINITY;
+                        if (screen && live) {
+                            kg = __shfl_sync(0xffffffffu, kg, lane & 24);
+                            known = fmaxf(known, ord2f(kg));
+                            // hi * hi alone is within gc of the exact correlation: the hi halves
+                            // leave out zrest of the candidate's unit norm and 2^-11 (BF16: 2^-8)
+                            // of the slice, amplified by at most At; Gt covers the arithmetic
+                            // and the screen drops the candidate's residual sum (|b| <= At /
+                            // sqrt(m)) and rounds the weights to 2^-8
+                            float gc = zrest + (X::uh * 1.01f + fabsf(zsh) * rsm) * At + Gt + 1e-6f;
+                            float hh;
+                            // (one choice per warp: both read tensor memory, all lanes together)
+                            if (!__any_sync(0xffffffffu, masked)) {
+                                hh = screen_max();
+                                gc = fmaf(0.004f, fabsf(hh), gc);
+                            } else {
+                                hh = row_max(zsh, 0.f);
+                            }
+                            if (hh == -INFINITY || fc != 0.f) gc = 0.f; // a flat row is exact
+                            prune(hh - gc, zsh, gc);
+                            // a value kept after all products is at most hup
+                            hup = fc != 0.f ? hh : hh + gc + Gt;
+                            const bool want = rowok && hup > known && !S.dead[cidx];
+                            if (__any_sync(0xffffffffu, want) && lane == 0) S.need[s] = tag;
                         }
-                        const unsigned bal = __ballot_sync(0xffffffffu, tmax > thr);
-                        bool hint = false;
-                        if (lane < UM_TC / 4) {
-                            const int ci = (UM_TC / 4) * g + lane;
-                            if (!S.dead[ci]) {
-                                if ((bal >> (8 * lane)) & 0xFFu) {
-                                    S.dead[ci] = 1;
-                                    pruned[S.cp[ci]] = 1;
-                                    hint = W.wit != nullptr;
-                                } else if (__ldcg(pruned + S.cp[ci])) {
-                                    S.dead[ci] = 1; // pruned by another CTA's item
+                        if (screen) { // every warp, also one that saw the item dead already
+                            tc_fence_before(); // the accumulator has been read
+                            __syncwarp();
+                            if (lane == 0) mbar_arrive(&S.dec[s]);
+                            if (!__all_sync(0xffffffffu, mbar_wait_bounded(&S.dec[s], a.par, wl))) {
+                                S.abort = 1;
+                                break;
+                            }
+                            full = __shfl_sync(0xffffffffu, S.need[s], 0) == tag;
+                            if (full) {
+                                if (!__all_sync(0xffffffffu,
+                                                mbar_wait_bounded(&S.rest_done[s],
+                                                                  (s ? n_rest1 : n_rest0) & 1u, wl))) {
+                                    S.abort = 1;
+                                    break;
                                 }
+                                n_rest0 += s ^ 1;
+                                n_rest1 += s;
+                                tc_fence_after();
+                            } else if (live) {
+                                keep_block(hup);
                             }
                         }
-                        // a candidate pruned here leaves the window that did it as its
-                        // witness hint: a second pass over the accumulator, at most once
-                        // per candidate, finds its column
-                        const unsigned hints = __ballot_sync(0xffffffffu, hint);
-                        if (hints) {
-                            int jh = -1;
-                            const bool mine = rowok && ((hints >> (lane >> 3)) & 1u) && tmax > thr;
-                            for (int cb = 0; cb < 4; ++cb) {
-                                tmem_ld32_async(tb + 32 * cb, ra);
-                                tmem_wait_ld(ra);
+                        if (full && live) {
+                            // correlations lowered by the tile's bound for the prune test, raised
+                            // back for the kept maximum (the interval's middle; -inf stays)
+                            const float tmax = row_max(zsc, Gt);
+                            rmax = fmaxf(rmax, tmax + Gt);
+                            keep_block(tmax + Gt);
+                            prune(tmax, zsc, Gt);
+                            if (screen) { // for the other CTAs' screens, and this item's next tiles
+                                float v = rmax;
 #pragma unroll
-                                for (int i = 0; i < 32; ++i) {
-                                    const int j = j0 + 8 * (128 * hcol + 32 * cb + i) + bsh;
-                                    const float4 wv = wrow[(32 * cb + i) >> 1];
-                                    const float rho = fmaf(__uint_as_float(ra[i]), (i & 1) ? wv.y : wv.x,
-                                                           fmaf(-zsc, (i & 1) ? wv.w : wv.z, -Gt));
-                                    const int dd = wc > j ? wc - j : j - wc;
-                                    if (rho > thr && j < j_hi && dd >= m - 1) jh = j;
-                                }
+                                for (int o = 4; o > 0; o >>= 1)
+                                    v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+                                known = fmaxf(known, v);
+                                if (rowok && bsh == 0 && v > -INFINITY && wc >= 0)
+                                    atomicMax(rho_max + S.cp[cidx], f2ord(v));
                             }
-                            if (mine && jh >= 0) wt_hint(W, wc, WT_ONE, jh);
                         }
-                        __syncwarp();
-                        if (warp == EPI_WARP0 && lane == 0) {
-                            atomicAdd(&att->n_pairs, (unsigned long long)UM_TC * UM_TW);
-                            int alive = 0;
-                            for (int c = 0; c < UM_TC; ++c) alive += !S.dead[c];
-                            atomicAdd(&att->n_live, (unsigned long long)S.tile_live * UM_TW);
-                            S.tile_live = alive;
+                        if (live && warp == EPI_WARP0) {
+                            ++n_tiles;
+                            n_alive += alive;
+                            alive = __popc(__ballot_sync(0xffffffffu, lane < UM_TC && !S.dead[lane & (UM_TC - 1)]));
                             if (!alive) S.item_dead = 1;
                         }
                     }
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) {
+                        if (!screen) mbar_arrive(&S.dec[s]); // no screen: only its use of the ring
                         mbar_arrive(&S.acc_empty[s]);
-                        mbar_arrive(&S.wd_empty);
+                        mbar_arrive(&S.wd_empty[rw.s]);
+                        mbar_arrive(&S.sl_empty[Ring(n, L.nb).s]);
                     }
+                }
+                if (warp == EPI_WARP0 && lane == 0) {
+                    atomicAdd(&att->n_pairs, (unsigned long long)n_tiles * (UM_TC * UM_TW));
+                    atomicAdd(&att->n_live, (unsigned long long)n_alive * UM_TW);
                 }
                 // fold the running maxima (8 shifts per candidate)
                 float v = rmax;
@@ -903,22 +1164,7 @@ k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
                 if (rowok && (lane & 7) == 0 && v > -INFINITY) atomicMax(&S.rmax[cidx], f2ord(v));
             }
             __syncthreads();
-            // ---- phase bookkeeping (every thread, same numbers)
-            {
-                const int tok = S.tok;                 // slice index of the end token, or -1
-                const int nb = tok >= 0 ? tok + 1 : T; // full_b / mma_done phases
-                const int nw = tok >= 0 ? tok : T;     // wd_full phases
-                const int ne = tok >= 0 ? tok - 1 : T; // acc_empty / wd_empty arrivals (tok >= 1)
-                for (int s = 0; s < 2; ++s) {
-                    const uint32_t cb = (uint32_t)((nb + 1 - s) >> 1);
-                    const uint32_t ce = (uint32_t)((ne + 1 - s) >> 1);
-                    ph.full[s] += cb;
-                    ph.done[s] += cb;
-                    ph.acc[s] += ce;
-                }
-                ph.wdf += (uint32_t)nw;
-                ph.wde += (uint32_t)ne;
-            }
+            G += (uint32_t)(S.tok >= 0 ? S.tok + 1 : T); // every thread, the same number
             if (threadIdx.x < UM_TC && tile * UM_TC + threadIdx.x < C &&
                 S.rmax[threadIdx.x] != f2ord(-INFINITY))
                 atomicMax(rho_max + S.cp[threadIdx.x], S.rmax[threadIdx.x]);
@@ -968,10 +1214,12 @@ k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
         // the last phase the loader issued on each before the shared memory goes
         // away (a phase it never issued is not waited for)
         if (threadIdx.x == 32) {
-            for (int s = 0; s < 2; ++s)
+            for (int s = 0; s < UM_STAGES; ++s) {
                 if (S.last_full[s] >= 0)
-                    mbar_wait_bounded(&S.full_b[s], par((uint32_t)S.last_full[s]), kDrainCycles);
-            if (S.last_wd >= 0) mbar_wait_bounded(&S.wd_full, par((uint32_t)S.last_wd), kDrainCycles);
+                    mbar_wait_bounded(&S.full_b[s], (uint32_t)S.last_full[s], kDrainCycles);
+                if (S.last_wd[s] >= 0)
+                    mbar_wait_bounded(&S.wd_full[s], (uint32_t)S.last_wd[s], kDrainCycles);
+            }
         }
     }
     tc_fence_before();
@@ -1004,7 +1252,7 @@ int64_t paddi_tile_blocks(int64_t N) { return (N + UM_TW - 1) / UM_TW; }
 
 int64_t paddi_tile_block_elems_max() { return 2 * (int64_t)slice_cnt(UM_KMAX64); }
 
-int64_t paddi_tile_wd_entries() { return (int64_t)8 * WD_ROW; }
+int64_t paddi_tile_wd_entries() { return WD_ENTRIES; }
 
 PaddiBound paddi_bound_tc(int m, bool bf16)
 {
@@ -1057,7 +1305,7 @@ cudaError_t paddi_launch_refine_umma(bool bf16, const float *x, const float4 *ws
                                      int32_t N, int32_t m, int32_t col_lo, int32_t col_hi,
                                      float thr_prune, int32_t num_sms, cudaStream_t st,
                                      long long wait_cycles, int32_t withhold, bool rows64,
-                                     const PaddiWitness *W, const PaddiBlockMax *B)
+                                     const PaddiWitness *W, const PaddiBlockMax *B, float guard)
 {
     const int kp = kpad_of(m);
     if (kp > UM_KMAX64 || m < 3) return cudaErrorInvalidValue;
@@ -1069,7 +1317,7 @@ cudaError_t paddi_launch_refine_umma(bool bf16, const float *x, const float4 *ws
     void (*kern)(const float *, const float4 *, const float *, const int32_t *, int32_t *,
                  int32_t *, const uint16_t *, const float4 *, PaddiAttemptDev *, uint32_t *,
                  uint8_t *, int32_t, int32_t, int32_t, int32_t, float, int32_t, long long, int32_t,
-                 PaddiWitness, PaddiBlockMax);
+                 PaddiWitness, PaddiBlockMax, int32_t, float);
     if (MM == 128) kern = bf16 ? k_refine_umma<true, 128> : k_refine_umma<false, 128>;
     else kern = bf16 ? k_refine_umma<true, 64> : k_refine_umma<false, 64>;
     cudaError_t e = paddi_raise_smem_limit((const void *)kern, smem);
@@ -1078,5 +1326,6 @@ cudaError_t paddi_launch_refine_umma(bool bf16, const float *x, const float4 *ws
     return paddi_launch(true, kern, grid, UM_THREADS, smem, st, x, wst, mu, cand, list0, list1, bq, wdq, att, rho_max,
                                          pruned, N, m, col_lo, col_hi, thr_prune, grid,
                                          wait_cycles > 0 ? wait_cycles : 4000000000ll, withhold,
-                                         W ? *W : PaddiWitness{}, B ? *B : PaddiBlockMax{});
+                                         W ? *W : PaddiWitness{}, B ? *B : PaddiBlockMax{},
+                        !bf16 && kp >= UM_SCREEN_K ? 1 : 0, guard);
 }

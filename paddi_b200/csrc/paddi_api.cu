@@ -419,7 +419,7 @@ paddi_status refine_rounds(paddi_ctx *ctx, const float *x, int32_t N, int m, int
                                     ctx->d_cand, ctx->d_list[0], ctx->d_list[1], ctx->d_bq,
                                     ctx->d_wdq, ctx->d_att, ctx->d_rho, ctx->d_pruned, N, m,
                                     col_lo, col_hi, thr, ctx->num_sms, st, ctx->wait_cycles,
-                                    ctx->withhold, ctx->opts.tile_rows == 64, W, &B));
+                                    ctx->withhold, ctx->opts.tile_rows == 64, W, &B, guard));
     else
         CK(paddi_launch_refine_fp32(x, ctx->d_wst, ctx->d_mu, ctx->d_cand, ctx->d_list[0],
                                     ctx->d_list[1], ctx->d_att, ctx->d_rho, ctx->d_pruned, N, m,

@@ -443,7 +443,7 @@ cudaError_t paddi_launch_refine_umma(bool bf16, const float *x, const float4 *ws
                                      float thr_prune, int32_t num_sms, cudaStream_t st,
                                      long long wait_cycles = 0, int32_t withhold = 0,
                                      bool rows64 = false, const PaddiWitness *W = nullptr,
-                                     const PaddiBlockMax *B = nullptr);
+                                     const PaddiBlockMax *B = nullptr, float guard = 1e-3f);
 
 // Per-length tile data of the tensor-core refine: for every block of
 // paddi_tile_width() windows, the split 16-bit series slice (bq, at most

@@ -13,20 +13,20 @@ from paddi_b200 import datagen
 
 pytestmark = pytest.mark.gpu
 
-M = 40
-
-
-@pytest.fixture(scope="module", params=[65536 - 1, 65536, 65536 + 2048 + 7])
+# windows, length (K' = 48: all products at once; 128, 416: tiles are screened
+# where a work item has four or more, i.e. with thousands of candidates)
+@pytest.fixture(scope="module", params=[(65536 - 1, 40), (65536, 40), (65536 + 2048 + 7, 40),
+                                        (65536 + 2048 + 7, 120), (66001, 400)])
 def case(request):
-    n = request.param + M - 1
-    x, _ = datagen.pd3_series(n=n, seed=11, n_anom=4, anom_len=100)
-    return x, np.sort(O.nn_profile_fast(x, M).astype(np.float32))
+    N, m = request.param
+    x, _ = datagen.pd3_series(n=N + m - 1, seed=11, n_anom=4, anom_len=100)
+    return x, m, np.sort(O.nn_profile_fast(x, m).astype(np.float32))
 
 
 @pytest.mark.parametrize("dist,rows", [("fp32", 0), ("fp16", 0), ("fp16", 64), ("bf16", 0)])
 def test_survivor_counts_across_rounds(case, dist, rows):
     import paddi_b200 as P
-    x, nn = case
+    x, M, nn = case
     k = {"fp32": P.DIST_FP32, "fp16": P.DIST_SPLIT_FP16, "bf16": P.DIST_SPLIT_BF16}[dist]
     with P.Context(device=0, distance_kernel=k, tile_rows=rows) as ctx:
         for keep in (0, 1, 8, 9, 16, 17, 300, 5000):
