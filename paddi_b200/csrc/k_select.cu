@@ -38,13 +38,19 @@ constexpr int RC_MAXM = 1024;
 // any r").  Phase 1 leaves flat-flat pairs out (rho 0 there), so this is
 // where such windows are dropped; the span {INT_MAX - lowest, highest + 1}
 // of the flat windows decides it per window.
+// With settle_flats (thr >= 0 too), the flat windows that stay have only
+// non-flat neighbours, of correlation 0 by the same policy: the value is written
+// here and the refine and fragile passes leave them out (PADDI_SETTLED).  They
+// cannot be pruned by any pair, so each met every window: at n = 2^18 with
+// a flat run of some 490 values, the refine spent 1.34 ms on 124 of them at
+// m = 363, now 8 us; PALMAD 64..512 there 240 ms, now 127.
 constexpr int CP_WIN = 16;                 // windows per thread
 constexpr int CP_CTHREADS = 256;
 __global__ void __launch_bounds__(CP_CTHREADS)
 k_compact(uint8_t *__restrict__ alive, int32_t reset, int32_t N, int32_t *cand, uint32_t *rho_max,
           uint8_t *pruned, int32_t *rc_slot, PaddiAttemptDev *att,
           const uint8_t *__restrict__ flat, const int32_t *__restrict__ flat_span, int32_t m,
-          int32_t prune_flats)
+          int32_t prune_flats, int32_t settle_flats)
 {
     __shared__ int wcnt[CP_CTHREADS / 32];
     __shared__ int base;
@@ -68,7 +74,7 @@ k_compact(uint8_t *__restrict__ alive, int32_t reset, int32_t N, int32_t *cand, 
             if (reset && i0 + b < N) alive[i0 + b] = 1;
         }
     }
-    uint32_t mask = 0;
+    uint32_t mask = 0, settled = 0;
     int lo = 0, hi = -1;
     if (prune_flats) {
         lo = INT_MAX - flat_span[0];
@@ -78,7 +84,12 @@ k_compact(uint8_t *__restrict__ alive, int32_t reset, int32_t N, int32_t *cand, 
     for (int b = 0; b < CP_WIN; ++b) {
         bool a = f[b] != 0;
         const int i = i0 + b;
-        if (a && prune_flats && flat[i] && (i - lo >= m - 1 || hi - i >= m - 1)) a = false;
+        if (a && prune_flats && flat[i]) {
+            if (i - lo >= m - 1 || hi - i >= m - 1)
+                a = false;
+            else if (settle_flats && (i >= m - 1 || i + m - 1 < N)) // has a neighbour at all
+                settled |= 1u << b;
+        }
         mask |= (uint32_t)a << b;
     }
     const int cnt = __popc(mask);
@@ -107,8 +118,9 @@ k_compact(uint8_t *__restrict__ alive, int32_t reset, int32_t N, int32_t *cand, 
         const int b = __ffs(mask) - 1;
         mask &= mask - 1;
         cand[pos] = i0 + b;
-        rho_max[pos] = f2ord(-INFINITY);
-        pruned[pos] = 0;
+        const bool z = (settled >> b) & 1u;
+        rho_max[pos] = f2ord(z ? 0.f : -INFINITY);
+        pruned[pos] = z ? PADDI_SETTLED : 0;
         rc_slot[pos] = -1;
         ++pos;
     }
@@ -225,7 +237,7 @@ k_finalize(const int32_t *__restrict__ cand, PaddiAttemptDev *att,
     // classified here; the borderline ones after the recheck.
     long long certain_c = 0, certain_d = 0;
     for (int c = threadIdx.x; c < C; c += FZ_THREADS) {
-        if (pruned[c]) continue;
+        if (pruned[c] == 1) continue;
         const float r = ord2f(rho_max[c]);
         if (flat[cand[c]]) {
             const float v = fminf(2.f * (float)m * (1.f - r), FLT_MAX);
@@ -244,7 +256,7 @@ k_finalize(const int32_t *__restrict__ cand, PaddiAttemptDev *att,
     for (int p = 0; p < top_k; ++p) {
         VI best{-INFINITY, 0x7fffffff};
         for (int c = threadIdx.x; c < C; c += FZ_THREADS) {
-            if (pruned[c]) continue;
+            if (pruned[c] == 1) continue;
             const float r = ord2f(rho_max[c]);
             if (!(r <= thr + guard)) continue;
             const int w = cand[c];
@@ -264,7 +276,7 @@ k_finalize(const int32_t *__restrict__ cand, PaddiAttemptDev *att,
     // the cut.  A flat window's value is exact already (rho is 0 or 1 by the
     // flat-window policy), so it is never queued.
     for (int c = threadIdx.x; c < C; c += FZ_THREADS) {
-        if (pruned[c] || flat[cand[c]]) continue;
+        if (pruned[c] == 1 || flat[cand[c]]) continue;
         const float r = ord2f(rho_max[c]);
         const bool border = r >= thr - guard;
         const bool neartop = np > 0 && r <= cut + widen * guard;
@@ -475,7 +487,7 @@ k_select(const int32_t *__restrict__ cand, PaddiAttemptDev *att,
     for (int p = 0; p < top_k; ++p) {
         VI best{-INFINITY, 0x7fffffff};
         for (int c = threadIdx.x; c < C; c += FZ_THREADS) {
-            if (pruned[c]) continue;
+            if (pruned[c] == 1) continue;
             const float r = ord2f(rho_max[c]);
             if (!(r <= thr + guard)) continue;
             // exact value if rechecked, else the FP32 estimate
@@ -554,7 +566,7 @@ __global__ void k_scatter(const int32_t *__restrict__ cand, const PaddiAttemptDe
 {
     const int C = att->n_cand_p1;
     for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < C; c += gridDim.x * blockDim.x) {
-        if (pruned[c]) continue;
+        if (pruned[c] == 1) continue;
         const int w = cand[c];
         const int slot = rc_slot[c];
         float v;
@@ -585,12 +597,13 @@ cudaError_t paddi_launch_compact(uint8_t *alive, bool reset, int32_t N, int32_t 
                                  uint32_t *rho_max, uint8_t *pruned, int32_t *rc_slot,
                                  PaddiAttemptDev *att, const uint8_t *flat,
                                  const int32_t *flat_span, int32_t m, bool prune_flats,
-                                 cudaStream_t st)
+                                 bool settle_flats, cudaStream_t st)
 {
     const int per_cta = CP_CTHREADS * CP_WIN;
     const unsigned grid = (unsigned)((N + per_cta - 1) / per_cta);
     return paddi_launch(true, k_compact, grid, CP_CTHREADS, 0, st, alive, reset ? 1 : 0, N, cand, rho_max, pruned, rc_slot, att, flat,
-                                           flat_span, m, prune_flats ? 1 : 0);
+                                           flat_span, m, prune_flats ? 1 : 0,
+                        prune_flats && settle_flats ? 1 : 0);
 }
 
 cudaError_t paddi_launch_finalize(const int32_t *cand, PaddiAttemptDev *att,

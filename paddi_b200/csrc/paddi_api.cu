@@ -549,7 +549,7 @@ paddi_status run_attempt(paddi_ctx *ctx, const float *x, size_t n, int m, float 
     ++launches;
     CK(paddi_launch_compact(ctx->d_alive, !wit, N, ctx->d_cand, ctx->d_rho, ctx->d_pruned,
                             ctx->d_rcslot, ctx->d_att, ctx->d_flat, ctx->d_flatcount + 1, m,
-                            r2 > 0.f, st));
+                            r2 > 0.f, thr >= 0.f, st));
     ++launches;
     out->kernel = kernel;
     out->p1_rows = R;
@@ -1319,7 +1319,7 @@ PADDI_API paddi_status paddi_shard_refine(paddi_ctx *ctx, const float *d_series,
     CK(cudaMemsetAsync(ctx->d_att, 0, sizeof(PaddiAttemptDev), st));
     CK(paddi_launch_compact(const_cast<uint8_t *>(d_alive), false, (int32_t)N, ctx->d_cand, ctx->d_rho, ctx->d_pruned,
                             ctx->d_rcslot, ctx->d_att, ctx->d_flat, ctx->d_flatcount + 1, (int)m,
-                            r2 > 0.f, st));
+                            r2 > 0.f, false, st));
     int launches = 0;
     paddi_status s = refine_rounds(ctx, d_series, (int32_t)N, (int)m, kernel, thr,
                                    guard_of(ctx, kernel), (int32_t)col_lo, (int32_t)col_hi,

@@ -390,11 +390,14 @@ cudaError_t paddi_launch_phase1_dev(const float *x, const float4 *wst, const flo
 // reset: alive[] is all ones again when the kernel is done.
 // prune_flats (r^2 > 0): flat windows with another flat window at least m-1
 // away are dropped (distance 0); flat_span as filled by paddi_launch_stats.
+// settle_flats (thr >= 0): the others get their value (correlation 0) and
+// pruned = PADDI_SETTLED, which the passes over pairs skip and the selection keeps.
+constexpr uint8_t PADDI_SETTLED = 2;
 cudaError_t paddi_launch_compact(uint8_t *alive, bool reset, int32_t N, int32_t *cand,
                                  uint32_t *rho_max, uint8_t *pruned, int32_t *rc_slot,
                                  PaddiAttemptDev *att, const uint8_t *flat,
                                  const int32_t *flat_span, int32_t m, bool prune_flats,
-                                 cudaStream_t st);
+                                 bool settle_flats, cudaStream_t st);
 
 // FP32 refine of all att->n_cand_p1 candidates over the windows [col_lo, col_hi)
 // (col_lo a multiple of 256), all rounds in one launch; list0 / list1 and
