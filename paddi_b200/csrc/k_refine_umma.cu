@@ -5,10 +5,10 @@
 // 32x32-tiled FP32 SGEMM of a host-gathered candidate matrix against the
 // Hankel windows of the series.  Same contraction here, mapped onto UMMA:
 //
-//   D[(c,b), a] = sum_k' A[(c,b), k'] * B[a, k']       M = 128, N = 256, K' = m+7 rounded to 16
-//   A[(c,b), k'] = zhat_c[k' - b]    (16 candidates x 8 shifted copies, zero padded)
+//   D[(b,c), a] = sum_k' A[(b,c), k'] * B[a, k']       M = 128, N = 256, K' = m+7 rounded to 16
+//   A[(b,c), k'] = zhat_c[k' - b]    (8 shifted copies x 16 candidates, zero padded)
 //   B[a, k']     = y[8a + k']        (y = scaled series slice minus a shift)
-// so D[(c,b), a] = <zhat_c, y[j .. j+m)> for window j = j0 + 8a + b: one tile
+// so D[(b,c), a] = <zhat_c, y[j .. j+m)> for window j = j0 + 8a + b: one tile
 // covers 16 candidates x 2048 windows.
 //
 // The Hankel operand is never expanded: with SWIZZLE_NONE a K-major core
@@ -33,11 +33,11 @@
 // inv_j) in global memory (L2-resident).  The refine is then a pipeline of
 // roles inside one persistent CTA per SM, coupled only by mbarriers:
 //   * loader (one thread): bulk async copies (cp.async.bulk, no multicast)
-//     of the next tile's slice into one of two shared-memory stages, and of
-//     the current tile's window data;
+//     of the next tiles' slices and window data into a ring of shared-memory
+//     stages;
 //   * MMA issuer (one thread): 3 x K'/16 tcgen05.mma of 128x256x16 per tile
 //     into one of two TMEM accumulators (all 512 columns), then commit;
-//   * epilogue (8 warps, two per TMEM lane quarter, 128 columns each):
+//   * epilogue (8 warps, four per accumulator, one per TMEM lane quarter):
 //     double-buffered tcgen05.ld, rho with packed f32x2 FMAs, running maxima,
 //     prune flags.
 // Screening.  The three products of a tile are needed to 2e-4, but most tiles
@@ -48,10 +48,8 @@
 // CTAs' through rho_max, the candidate's witness), the other two products and the
 // full epilogue are skipped.  A candidate whose lower bound is above thr is pruned
 // at once.  Nothing kept is computed with less than all three products.  The MMA
-// thread issues tile u+1's hi * hi before it takes the verdict on tile u; 8 to 30 %
-// of the tiles need everything.  What bounds a screened tile is the epilogue (2000
-// cycles with all window data, 1000 with the screen's weights) and the hops
-// between the roles, about 3700 cycles together; headline run 154 -> 144 ms.
+// thread issues tile u+1's hi * hi before it takes the verdict on tile u; 5 to 25 %
+// of the tiles need everything.  (Figures at UM_SCREEN_K and EPI_WARP0.)
 //
 // The candidate operand is built by all 384 threads at the start of a work
 // item.  When every candidate of the item is pruned the loader stops and
@@ -82,38 +80,47 @@ constexpr int UM_FEW = 4;        // tiles that take all remaining windows after 
 // A tile is screened by its hi * hi product first (split-FP16, where the work item
 // has several tiles and K' is long enough; the comment at the kernel has the
 // figures): refine launches at n = 300007 with tens of thousands of candidates, all
-// products at once / screened, us: m = 64 (K' 80) 2067 / 2152, m = 100 (112) 2270 /
-// 2238, m = 200 (208) 3935 / 3035, m = 500 (512) 18700 / 10000, m = 700 (720) 27450 /
-// 14140; PALMAD 64..512 at 2^18 151 ms / 139.  With one to three tiles an item's first
-// tile, which nothing is known about yet, is most of it: MERLIN at n = 2^18 1.27 ms,
-// 1.49 screened.  BF16 leaves out 2^-8 of the slice: its screen rejects little.
+// products at once / screened, us: m = 64 (K' 80) 1770 / 1883, m = 100 (112) 2125 /
+// 2057, m = 200 (208) 3715 / 2945, m = 500 (512) 18800 / 9990, m = 700 (720) 27500 /
+// 13600; PALMAD 64..512 at 2^18 149 ms / 137.  With one to three tiles an item's first
+// tile, which nothing is known about yet, is most of it.  BF16 leaves out 2^-8 of the
+// slice: its screen rejects little.
 constexpr int UM_SCREEN_T = 4;
 constexpr int UM_SCREEN_K = 112;
 constexpr int UM_WAVES = 1;      // work items per CTA and round when candidate tiles are few
 constexpr int UM_KMAX128 = 368;  // largest K' with M = 128 (shared-memory bound)
 constexpr int UM_KMAX64 = 736;   // largest K' with M = 64
 constexpr int UM_STAGES = 4;      // at most
+// barriers for the window data of nw stages: an even number of uses around, so that
+// each barrier serves one accumulator's epilogue, which sees all of its phases
+constexpr int UM_WBARS = 6;
+__host__ __device__ constexpr int wd_bars(int nw) { return nw & 1 ? 2 * nw : nw; }
 constexpr int ZSCALE = 8;        // zhat scaled by 2^8 before splitting
 constexpr int WD_ROW = 129;      // float4 entries per shift row of the window data (128 + pad)
-constexpr int WQ_ROW = 132;      // words per shift row of the screen's weights (128 + pad)
-constexpr int WQ_OFF = 8 * WD_ROW;   // they follow the window data (float4 entries)
-constexpr int WD_ENTRIES = WQ_OFF + 8 * WQ_ROW / 4;
+constexpr int WD_ENTRIES = 8 * WD_ROW;
 constexpr int WD_BYTES = WD_ENTRIES * 16;
-constexpr uint32_t UM_SMEM_MAX = 227 * 1024 - 896; // dynamic; the rest is UmShared
+constexpr uint32_t UM_SMEM_MAX = 227 * 1024 - 1920; // dynamic; the rest is UmShared
 // limit of the abort path's drain waits (~2 s at 1.9 GHz): copies and MMAs the
 // kernel issued complete on their own, so these waits end long before it
 constexpr long long kDrainCycles = 4000000000ll;
-constexpr int EPI_WARP0 = 4;     // warps 4..11: epilogue (two per TMEM lane quarter)
-constexpr int EPI_WARPS = 8;
+// Warps 4..11: epilogue, one group of four per accumulator, so that one group's math
+// runs under the other's waits (its product, the screen's verdict): with all eight on
+// every tile and candidates major in A (below), refine launches at n = 300007 took 2080
+// us at m = 64, now 1770; m = 130 2425, now 2245; ECG of 2^23 points 5.0 ms, now 4.5.
+// What bounds it: handing each lane its windows' weights (4 or 8 bytes a correlation, 128
+// bytes a cycle from shared memory, beside the operands of the products) and, about as
+// much, the wait for the next product: the tensor memory holds two accumulators.
+constexpr int EPI_WARP0 = 4;
+constexpr int EPI_GROUP = 4;     // warps per accumulator
 constexpr int MMA_WARP = 0, LOAD_WARP = 1;
 
 __host__ __device__ constexpr int kpad_of(int m) { return ((m + 7) + 15) & ~15; }
 __host__ __device__ constexpr int slice_cnt(int kp) { return UM_TW + kp + 16; }
 // scratch row stride (32-bit words) of the candidate operand build: 4 words of
-// front padding + kp/2 words, rounded up to 8 modulo 32
+// front padding + kp/2 words, rounded up to 2 modulo 32
 __host__ __device__ constexpr int zrow_words(int kp)
 {
-    return (4 + kp / 2) + ((8 - (4 + kp / 2) % 32) + 32) % 32;
+    return (4 + kp / 2) + ((2 - (4 + kp / 2) % 32) + 32) % 32;
 }
 
 // ------------------------------------------------------------------ PTX helpers
@@ -393,7 +400,6 @@ k_prep(const float *__restrict__ x, int64_t nser, int32_t cnt, int32_t m, int32_
     }
     // built in shared memory (the prefixes are done with), written out in one sweep
     float *wf = reinterpret_cast<float *>(st_mem);
-    __nv_bfloat16 *wq = reinterpret_cast<__nv_bfloat16 *>(wf + 4 * WQ_OFF);
     const float F = Fu * mx, fm = (float)m;
     float gmax = 0.f, amax = 1.f;
 #pragma unroll
@@ -410,7 +416,6 @@ k_prep(const float *__restrict__ x, int64_t nser, int32_t cnt, int32_t m, int32_
         const int s = q & 7, i = q >> 3, k = i >> 1, slot = i & 1;
         const float a = frag ? __int_as_float(0x7fffffff) : iv[kq] * dsc;
         wf[(s * WD_ROW + k) * 4 + slot] = a;
-        wq[(s * WQ_ROW + k) * 2 + slot] = __float2bfloat16_rn(a);
         wf[(s * WD_ROW + k) * 4 + 2 + slot] = (mv[kq] - sh) * iv[kq];
         // fragile windows in index order within each warp (runs stay contiguous)
         const unsigned bal = __ballot_sync(0xffffffffu, frag);
@@ -488,17 +493,18 @@ __host__ __device__ inline UmLayout um_layout(int MM, int kp)
 struct UmShared {
     // rings over the stages (full, empty) and over the two accumulators
     uint64_t full_b[UM_STAGES];   // loader -> MMA: the stage holds the tile's slice (or an end token)
-    uint64_t wd_full[UM_STAGES];  // loader -> epilogue: and its window data (or an end token)
+    uint64_t wd_full[UM_WBARS];   // loader -> epilogue: and its window data (or an end token)
     uint64_t sl_empty[UM_STAGES]; // epilogue -> loader: done with the slice
     uint64_t wd_empty[UM_STAGES]; // epilogue -> loader: done with the window data
     uint64_t mma_done[2];  // tcgen05.commit: the tile's MMAs are complete
     uint64_t acc_empty[2]; // epilogue -> MMA: accumulator drained
     uint64_t dec[2];       // epilogue -> MMA: hi * hi product screened, need[] decided
     uint64_t rest_done[2]; // tcgen05.commit: the products with lo halves are complete
+    uint64_t put[2];       // epilogue: a fully multiplied tile's block maxima are in bmax
     uint64_t drain;        // final MMA drain on abort
     // phase of the last arrival the loader issued on full_b[s] / wd_full[s] (-1: none
     // yet); the abort path waits only for those
-    int last_full[UM_STAGES], last_wd[UM_STAGES];
+    signed char last_full[UM_STAGES], last_wd[UM_WBARS];
     uint32_t tmem_base;
     int item, abort, tok;
     int built_tile; // candidate tile whose operand sits in A (-1: none)
@@ -506,19 +512,21 @@ struct UmShared {
                     // candidates of the next round (-1: give up)
     int wsum[UM_THREADS / 32];
     volatile int item_dead;
-    volatile int vb[UM_STAGES], vw[UM_STAGES];
+    volatile uint8_t vb[UM_STAGES], vw[UM_WBARS];
     int cw[UM_TCMAX], cp[UM_TCMAX];
     float cflat[UM_TCMAX], zsum[UM_TCMAX];
     // screening: sum of the hi halves, norm of what they leave out, a correlation
     // the candidate is known to reach; need[s]: tag of the last tile in accumulator
     // s that needs its other products
-    float zsumh[UM_TCMAX], zrest[UM_TCMAX], known[UM_TCMAX];
+    float zsumh[UM_TCMAX], zrest[UM_TCMAX];
+    volatile uint32_t known[UM_TCMAX]; // (ordered image)
     volatile uint32_t need[2];
+    float bmax[2][4][2][UM_TCMAX]; // half-block maxima per accumulator and warp
     uint32_t rmax[UM_TCMAX];
     volatile uint8_t dead[UM_TCMAX];
 };
 
-static_assert(sizeof(UmShared) <= 896, "beside the largest operand and window data");
+static_assert(sizeof(UmShared) <= 1920, "beside the largest operand and window data");
 
 // The n-th use of a ring of `stages` barriers: its barrier and phase parity.  Every
 // tile (and every end token) of a CTA takes one use of every ring, so one count
@@ -567,16 +575,20 @@ k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
     if (threadIdx.x == 0) {
         for (int s = 0; s < UM_STAGES; ++s) {
             mbar_init(&S.full_b[s], 1);
+            mbar_init(&S.sl_empty[s], EPI_GROUP);
+            mbar_init(&S.wd_empty[s], EPI_GROUP);
+            S.last_full[s] = -1;
+        }
+        for (int s = 0; s < UM_WBARS; ++s) {
             mbar_init(&S.wd_full[s], 1);
-            mbar_init(&S.sl_empty[s], EPI_WARPS);
-            mbar_init(&S.wd_empty[s], EPI_WARPS);
-            S.last_full[s] = S.last_wd[s] = -1;
+            S.last_wd[s] = -1;
         }
         for (int s = 0; s < 2; ++s) {
             mbar_init(&S.mma_done[s], 1);
-            mbar_init(&S.acc_empty[s], EPI_WARPS);
-            mbar_init(&S.dec[s], EPI_WARPS);
+            mbar_init(&S.acc_empty[s], EPI_GROUP);
+            mbar_init(&S.dec[s], EPI_GROUP);
             mbar_init(&S.rest_done[s], 1);
+            mbar_init(&S.put[s], EPI_GROUP);
             S.need[s] = 0;
         }
         mbar_init(&S.drain, 1);
@@ -597,16 +609,16 @@ k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
     const uint32_t tmem = S.tmem_base;
     uint32_t G = 0; // tiles and end tokens of this CTA before the current work item
     bool mma_issued = false; // MMA thread: any MMA issued
-    uint32_t n_rest0 = 0u, n_rest1 = 0u; // epilogue: completed phases of rest_done
+    uint32_t n_rest = 0u, n_put = 0u; // epilogue: completed phases of its rest_done and put
 
     const uint32_t idesc = idesc_f16(X::fmt, UM_M, UM_N);
     const uint32_t a_hi_s = smem_u32(um_smem + L.a_hi), a_lo_s = smem_u32(um_smem + L.a_lo);
     const int kblocks = kp / 16;
     // epilogue geometry: lane group g (TMEM lanes 32g..32g+31)
-    const int g = warp & 3, hcol = (warp - EPI_WARP0) >> 2; // lane quarter, column half
+    const int g = warp & 3, grp = (warp - EPI_WARP0) >> 2; // lane quarter, accumulator
     const bool rowok = MM == 128 || lane < 16;
     const int row = MM == 128 ? 32 * g + lane : 16 * g + (lane & 15);
-    const int cidx = row >> 3, bsh = row & 7;
+    const int cidx = row % UM_TC, bsh = row / UM_TC; // candidate, shift
 
     // ---- rounds: the windows [jb, je) of growing ranges (1/16, 1/4, 1/2, all of
     // them), the survivors compacted in between so that every tile is dense.  A
@@ -656,8 +668,8 @@ k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
                 S.rmax[threadIdx.x] = f2ord(-INFINITY);
                 // a correlation this candidate reaches, from its witness (the kept value
                 // of that window is within the guard band of it)
-                S.known[threadIdx.x] =
-                    (v && W.wit) ? fmaxf(W.wrho[w] - guard - 1e-5f, -INFINITY) : -INFINITY;
+                S.known[threadIdx.x] = f2ord(
+                    (v && W.wit) ? fmaxf(W.wrho[w] - guard - 1e-5f, -INFINITY) : -INFINITY);
             }
             if (threadIdx.x == 0) {
                 S.item_dead = 0;
@@ -674,7 +686,7 @@ k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
             // the slice of tile u (its stage is free) or an end token
             auto put_slice = [&](int u, bool token) {
                 const Ring r(G + (uint32_t)u, L.nb);
-                S.last_full[r.s] = (int)r.par;
+                S.last_full[r.s] = (signed char)r.par;
                 S.vb[r.s] = !token;
                 if (token) {
                     mbar_arrive(&S.full_b[r.s]);
@@ -700,8 +712,8 @@ k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
             //      work: its results no longer matter)
             if (S.built_tile != tile) {
                 // scratch rows of 32-bit words: 4 zero words (8 elements) of front
-                // padding, then zhat[0..kp); stride ksw words with ksw % 32 == 8, so
-                // the four candidates a warp reads sit in disjoint bank ranges
+                // padding, then zhat[0..kp); stride ksw words with ksw % 32 == 2, so
+                // the 16 candidates and two shifts a warp reads sit in different banks
                 const int ksw = zrow_words(kp);
                 uint32_t *zhw = reinterpret_cast<uint32_t *>(um_smem + (L.nw >= 2 || stage0 == 0 ? L.wd[0] : L.b[0][0]));
                 uint32_t *zlw = zhw + UM_TC * ksw;
@@ -748,14 +760,17 @@ k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
                     S.zrest[c] = sqrtf(zr) * (1.01f / 256.f);
                 }
                 __syncthreads();
-                // A[(c,b), k'] = z_c[k' - b] in K-major core matrices:
+                // A[(b,c), k'] = z_c[k' - b] in K-major core matrices, the shift b major: an
+                // epilogue warp then works on two shifts, and its reads of the window data go
+                // to two addresses (with candidates major, eight: a 16-byte read took 4 cycles
+                // of shared memory, now 2):
                 // byte offset ((k'/8)*RG + r/8)*128 + (r%8)*16 + (k'%8)*2.
                 // Elements k'-b .. k'-b+7 start at padded element p0 = 8 + 8 kc - b:
                 // five 32-bit words from word p0/2, funnel-shifted by 16 bits when p0 is odd.
                 const int chunks = kp / 8;
                 for (int e = threadIdx.x; e < UM_M * chunks; e += UM_THREADS) {
                     const int r = e & (UM_M - 1), kc = e / UM_M;
-                    const int cc = r >> 3, b = r & 7;
+                    const int cc = r % UM_TC, b = r / UM_TC;
                     const int p0 = 8 + 8 * kc - b;
                     const uint32_t shf = (uint32_t)(p0 & 1) * 16u;
                     const uint32_t *rh = zhw + cc * ksw + (p0 >> 1);
@@ -792,25 +807,28 @@ k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
                     return mbar_wait_bounded(empty + r.s, r.par, wl);
                 };
                 auto put_wd = [&](int u, bool token) {
-                    const Ring r(G + (uint32_t)u, L.nw);
-                    S.last_wd[r.s] = (int)r.par;
+                    const uint32_t n = G + (uint32_t)u;
+                    const Ring r(n, wd_bars(L.nw));
+                    S.last_wd[r.s] = (signed char)r.par;
                     S.vw[r.s] = !token;
                     if (token) {
                         mbar_arrive(&S.wd_full[r.s]);
                         return;
                     }
                     mbar_arrive_expect_tx(&S.wd_full[r.s], (uint32_t)WD_BYTES);
-                    bulk_g2s(um_smem + L.wd[r.s], wdq + (size_t)(blk0 + u) * WD_ENTRIES,
+                    bulk_g2s(um_smem + L.wd[Ring(n, L.nw).s], wdq + (size_t)(blk0 + u) * WD_ENTRIES,
                              (uint32_t)WD_BYTES, &S.wd_full[r.s]);
                 };
-                // once the item is dead, an end token takes the place of a tile
+                // once the item is dead, end tokens take the place of the next two tiles (one
+                // per accumulator)
                 bool ok = freed(S.wd_empty, 0, L.nw);
                 if (ok) put_wd(0, false); // slice 0 was issued before the operand build
-                for (int u = 1; ok && u < T && S.tok < 0; ++u) {
+                int tok = -1;
+                for (int u = 1; ok && u < T && (tok < 0 || u == tok + 1); ++u) {
                     ok = freed(S.sl_empty, u, L.nb);
                     if (!ok) break;
-                    const bool token = S.item_dead;
-                    if (token) S.tok = u;
+                    const bool token = tok >= 0 || S.item_dead;
+                    if (token && tok < 0) S.tok = tok = u;
                     put_slice(u, token);
                     ok = freed(S.wd_empty, u, L.nw);
                     if (ok) put_wd(u, token);
@@ -853,9 +871,8 @@ k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
                     }
                     return true;
                 };
-                bool ok = true;
-                int u = 0;
-                for (; ok && u < T; ++u) {
+                bool ok = true, ended = false;
+                for (int u = 0; ok && u < T; ++u) {
                     const uint32_t n = G + (uint32_t)u;
                     const Ring r(n, L.nb), a(n, 2);
                     if (!mbar_wait_bounded(&S.full_b[r.s], r.par, wl)) {
@@ -870,43 +887,53 @@ k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
                         break;
                     }
                     if (!S.vb[r.s]) { // end token: pass it on (the commit also covers earlier MMAs)
-                        if (screen && u > 0) ok = settle(u - 1);
+                        if (screen && u > 0 && !ended) ok = settle(u - 1);
                         umma_commit(&S.mma_done[a.s]);
-                        break;
+                        if (ended) break;
+                        ended = true;
+                        continue;
                     }
                     issue(u, true, !screen);
                     umma_commit(&S.mma_done[a.s]);
                     // the tile before was screened while this one's product started
                     if (screen && u > 0) ok = settle(u - 1);
                 }
-                if (ok && screen && u == T) ok = settle(T - 1);
+                if (ok && screen && !ended) ok = settle(T - 1);
                 if (!ok) S.abort = 1;
             } else if (warp >= EPI_WARP0) {
                 float rmax = -INFINITY;
                 const int wc = S.cw[cidx];
                 const float zsc = S.zsum[cidx], fc = S.cflat[cidx];
                 const float zsh = S.zsumh[cidx], zrest = S.zrest[cidx];
-                float known = S.known[cidx];
                 const float rsm = rsqrtf((float)m) * 1.001f;
                 // tiles of the item and their live candidates (instrumentation)
                 int n_tiles = 0, n_alive = 0;
                 int alive = __popc(__ballot_sync(0xffffffffu, lane < UM_TC && !S.dead[lane & (UM_TC - 1)]));
-                const uint8_t *gone_p = pruned + S.cp[(UM_TC / 4) * g + (lane & (UM_TC / 4 - 1))];
+                // (the group's first warp asks, for all its candidates)
+                const uint8_t *gone_p = pruned + S.cp[cidx];
                 const uint32_t *known_p = rho_max + S.cp[cidx];
+                const bool asks = g == 0 && lane < UM_TC;
                 int gone_next = 0;
                 uint32_t kg_next = 0u;
                 // Every lane waits (acquire) and the warp then agrees through a vote, so
                 // the warp is converged and takes the same branch at every tcgen05.ld.  (One
                 // lane polling for the warp was slower: 40 instead of 37 ms per headline run.)
-                for (int u = 0; u < T; ++u) {
+                for (int u = grp ^ (int)(G & 1u); u < T; u += 2) {
                     const uint32_t n = G + (uint32_t)u;
-                    const Ring a(n, 2), rw(n, L.nw);
+                    const Ring a(n, 2), rw(n, wd_bars(L.nw));
+                    const int ws = Ring(n, L.nw).s;
                     const int s = a.s;
                     // what other CTAs have found meanwhile, asked for a tile ahead
                     const int gone = gone_next;
-                    uint32_t kg = kg_next;
-                    if (lane < UM_TC / 4) gone_next = __ldcg(gone_p);
-                    if (screen && bsh == 0) kg_next = __ldcg(known_p);
+                    const uint32_t kg = kg_next;
+                    if (asks) {
+                        gone_next = __ldcg(gone_p);
+                        if (screen) {
+                            kg_next = __ldcg(known_p);
+                            if (kg > S.known[cidx])
+                                atomicMax(const_cast<uint32_t *>(&S.known[cidx]), kg);
+                        }
+                    }
                     if (!__all_sync(0xffffffffu, mbar_wait_bounded(&S.wd_full[rw.s], rw.par, wl) &&
                                                      mbar_wait_bounded(&S.mma_done[s], a.par, wl))) {
                         S.abort = 1;
@@ -918,29 +945,50 @@ k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
                         if (lane == 0) {
                             mbar_arrive(&S.dec[s]);
                             mbar_arrive(&S.acc_empty[s]);
-                            mbar_arrive(&S.wd_empty[rw.s]);
+                            mbar_arrive(&S.wd_empty[ws]);
                             mbar_arrive(&S.sl_empty[Ring(n, L.nb).s]);
                         }
                         break;
                     }
-                    const float4 *wd4 = reinterpret_cast<const float4 *>(um_smem + L.wd[rw.s]);
+                    const float4 *wd4 = reinterpret_cast<const float4 *>(um_smem + L.wd[ws]);
                     tc_fence_after();
                     const int j0 = j_lo + u * UM_TW;
                     const uint32_t tag = n + 1u; // the tile's tag in need[s]
                     const bool live = !__shfl_sync(0xffffffffu, S.item_dead, 0);
                     bool full = true;
+                    auto keep_block = [&]() {
+                        const int c = lane % UM_TC, h = lane / UM_TC;
+                        if (g != 0 || h > 1 || S.cw[c] < 0) return;
+                        const float v = fmaxf(fmaxf(S.bmax[grp][0][h][c], S.bmax[grp][1][h][c]),
+                                              fmaxf(S.bmax[grp][2][h][c], S.bmax[grp][3][h][c]));
+                        B.v[(int64_t)S.cp[c] * B.halves + j0 / PADDI_HALF + h] = f2ord(v);
+                    };
                     if (live || screen) {
                         const uint32_t tb = tmem + ((uint32_t)(32 * g) << 16) +
-                                            (uint32_t)(s * UM_N + 128 * hcol);
+                                            (uint32_t)(s * UM_N);
                         const bool masked = (j0 + UM_TW > j_hi) ||
                                             (wc > j0 - m + 1 && wc < j0 + UM_TW + m - 1) || fc != 0.f;
-                        const float4 *wrow = wd4 + bsh * WD_ROW + 64 * hcol;
+                        const float4 *wrow = wd4 + bsh * WD_ROW;
                         // the tile's rounding bound and largest amplification (k_prep)
                         const float Gt = wd4[128].x, At = wd4[128].y;
                         uint32_t ra[32], rb[32];
-                        // maximum over the row's 128 columns of D a - z b - sub.  4 chunks of 32
-                        // columns; the load of chunk cb+1 overlaps the math of cb
-                        auto row_max = [&](float z, float sub) -> float {
+                        // f(registers, chunk) over the row's 8 chunks of 32 columns, the load of
+                        // a chunk overlapping the math on the one before; half() ends a half block
+                        auto columns = [&](auto f, auto half) {
+                            tmem_ld32_async(tb, ra);
+#pragma unroll 1
+                            for (int c2 = 0; c2 < 4; ++c2) {
+                                tmem_wait_ld(ra);
+                                tmem_ld32_async(tb + 64 * c2 + 32, rb);
+                                f(ra, 2 * c2);
+                                tmem_wait_ld(rb);
+                                if (c2 < 3) tmem_ld32_async(tb + 64 * c2 + 64, ra);
+                                f(rb, 2 * c2 + 1);
+                                if (c2 & 1) half(c2 >> 1);
+                            }
+                        };
+                        // maxima over the row's two half blocks of D a - z b - sub
+                        auto row_max = [&](float z, float sub) -> float2 {
                             const float2 nz2 = make_float2(-z, -z), ns2 = make_float2(-sub, -sub);
                             float tm[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
                             auto chunk = [&](const uint32_t (&r)[32], int cb) {
@@ -958,7 +1006,7 @@ k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
                                 } else {
 #pragma unroll
                                     for (int i = 0; i < 32; ++i) {
-                                        const int col = 128 * hcol + 32 * cb + i;
+                                        const int col = 32 * cb + i;
                                         const int j = j0 + 8 * col + bsh;
                                         const float4 wv = wrow[(32 * cb + i) >> 1];
                                         const float wa = (i & 1) ? wv.y : wv.x;
@@ -970,56 +1018,40 @@ k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
                                     }
                                 }
                             };
-                            tmem_ld32_async(tb, ra);
-                            tmem_wait_ld(ra);
-                            tmem_ld32_async(tb + 32, rb);
-                            chunk(ra, 0);
-                            tmem_wait_ld(rb);
-                            tmem_ld32_async(tb + 64, ra);
-                            chunk(rb, 1);
-                            tmem_wait_ld(ra);
-                            tmem_ld32_async(tb + 96, rb);
-                            chunk(ra, 2);
-                            tmem_wait_ld(rb);
-                            chunk(rb, 3);
-                            return rowok ? fmaxf(fmaxf(tm[0], tm[1]), fmaxf(tm[2], tm[3])) : -INFINITY;
+                            float2 out = make_float2(-INFINITY, -INFINITY);
+                            columns(chunk, [&](int h) {
+                                const float v =
+                                    rowok ? fmaxf(fmaxf(tm[0], tm[1]), fmaxf(tm[2], tm[3])) : -INFINITY;
+                                if (h == 0) out.x = v;
+                                else out.y = v;
+                                tm[0] = tm[1] = tm[2] = tm[3] = -INFINITY;
+                            });
+                            return out;
                         };
-                        // maximum of D a alone, the weights in BF16: 8 columns per load
-                        auto screen_max = [&]() -> float {
-                            const uint4 *q4 = reinterpret_cast<const uint4 *>(wd4 + WQ_OFF) +
-                                              (bsh * WQ_ROW + 64 * hcol) / 4;
+                        // the same of D a alone
+                        auto screen_max = [&]() -> float2 {
                             float tm[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
                             auto chunk = [&](const uint32_t (&r)[32], int cb) {
 #pragma unroll
-                                for (int i8 = 0; i8 < 4; ++i8) {
-                                    const uint4 w4 = q4[4 * cb + i8];
-                                    const uint32_t ww[4] = {w4.x, w4.y, w4.z, w4.w};
-#pragma unroll
-                                    for (int e = 0; e < 4; ++e) {
-                                        const float2 dd =
-                                            make_float2(__uint_as_float(r[8 * i8 + 2 * e]),
-                                                        __uint_as_float(r[8 * i8 + 2 * e + 1]));
-                                        const float2 aa =
-                                            make_float2(__uint_as_float(ww[e] << 16),
-                                                        __uint_as_float(ww[e] & 0xffff0000u));
-                                        const float2 v = __fmul2_rn(dd, aa);
-                                        tm[e] = fmax3(tm[e], v.x, v.y);
-                                    }
+                                for (int i2 = 0; i2 < 16; ++i2) {
+                                    const float2 wa =
+                                        *reinterpret_cast<const float2 *>(&wrow[16 * cb + i2]);
+                                    const float2 v = __fmul2_rn(
+                                        make_float2(__uint_as_float(r[2 * i2]),
+                                                    __uint_as_float(r[2 * i2 + 1])),
+                                        wa);
+                                    tm[i2 & 3] = fmax3(tm[i2 & 3], v.x, v.y);
                                 }
                             };
-                            tmem_ld32_async(tb, ra);
-                            tmem_wait_ld(ra);
-                            tmem_ld32_async(tb + 32, rb);
-                            chunk(ra, 0);
-                            tmem_wait_ld(rb);
-                            tmem_ld32_async(tb + 64, ra);
-                            chunk(rb, 1);
-                            tmem_wait_ld(ra);
-                            tmem_ld32_async(tb + 96, rb);
-                            chunk(ra, 2);
-                            tmem_wait_ld(rb);
-                            chunk(rb, 3);
-                            return rowok ? fmaxf(fmaxf(tm[0], tm[1]), fmaxf(tm[2], tm[3])) : -INFINITY;
+                            float2 out = make_float2(-INFINITY, -INFINITY);
+                            columns(chunk, [&](int h) {
+                                const float v =
+                                    rowok ? fmaxf(fmaxf(tm[0], tm[1]), fmaxf(tm[2], tm[3])) : -INFINITY;
+                                if (h == 0) out.x = v;
+                                else out.y = v;
+                                tm[0] = tm[1] = tm[2] = tm[3] = -INFINITY;
+                            });
+                            return out;
                         };
                         // prunes the candidates whose lower bound `low` exceeds thr, and those
                         // pruned elsewhere.  A candidate pruned here leaves the window that did
@@ -1028,10 +1060,12 @@ k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
                         auto prune = [&](float low, float z, float sub) {
                             const unsigned bal = __ballot_sync(0xffffffffu, low > thr);
                             bool hint = false;
-                            if (lane < UM_TC / 4) {
-                                const int ci = (UM_TC / 4) * g + lane;
+                            // (low is -inf in the lanes that hold no row)
+                            const unsigned hit = bal | (bal >> UM_TC);
+                            if (lane < UM_TC) {
+                                const int ci = lane;
                                 if (!S.dead[ci]) {
-                                    if ((bal >> (8 * lane)) & 0xFFu) {
+                                    if ((hit >> lane) & 1u) {
                                         S.dead[ci] = 1;
                                         pruned[S.cp[ci]] = 1;
                                         hint = W.wit != nullptr;
@@ -1043,13 +1077,13 @@ k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
                             const unsigned hints = __ballot_sync(0xffffffffu, hint);
                             if (hints) {
                                 int jh = -1;
-                                const bool mine = rowok && ((hints >> (lane >> 3)) & 1u) && low > thr;
-                                for (int cb = 0; cb < 4; ++cb) {
+                                const bool mine = rowok && ((hints >> cidx) & 1u) && low > thr;
+                                for (int cb = 0; cb < 8; ++cb) {
                                     tmem_ld32_async(tb + 32 * cb, ra);
                                     tmem_wait_ld(ra);
 #pragma unroll
                                     for (int i = 0; i < 32; ++i) {
-                                        const int j = j0 + 8 * (128 * hcol + 32 * cb + i) + bsh;
+                                        const int j = j0 + 8 * (32 * cb + i) + bsh;
                                         const float4 wv = wrow[(32 * cb + i) >> 1];
                                         const float rho =
                                             fmaf(__uint_as_float(ra[i]), (i & 1) ? wv.y : wv.x,
@@ -1062,39 +1096,44 @@ k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
                             }
                             __syncwarp();
                         };
-                        // the half block's maximum (or a bound of it) over the 8 shifts
-                        auto keep_block = [&](float bm) {
-                            if (!bkeep) return;
-#pragma unroll
-                            for (int o = 4; o > 0; o >>= 1)
-                                bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, o));
-                            if (rowok && bsh == 0 && wc >= 0)
-                                B.v[(int64_t)S.cp[cidx] * B.halves + j0 / PADDI_HALF + hcol] =
-                                    f2ord(bm);
+                        // the half blocks' maxima (or bounds of them): over the warp's two shifts,
+                        // then over the group's warps once all have put theirs
+                        auto put_block = [&](float2 bm) {
+                            bm.x = fmaxf(bm.x, __shfl_xor_sync(0xffffffffu, bm.x, UM_TC));
+                            bm.y = fmaxf(bm.y, __shfl_xor_sync(0xffffffffu, bm.y, UM_TC));
+                            if (lane < UM_TC) {
+                                S.bmax[grp][g][0][lane] = bm.x;
+                                S.bmax[grp][g][1][lane] = bm.y;
+                            }
                         };
-                        float hup = -INFINITY;
+                        float2 hup = make_float2(-INFINITY, -INFINITY);
                         if (screen && live) {
-                            kg = __shfl_sync(0xffffffffu, kg, lane & 24);
-                            known = fmaxf(known, ord2f(kg));
                             // hi * hi alone is within gc of the exact correlation: the hi halves
                             // leave out zrest of the candidate's unit norm and 2^-11 (BF16: 2^-8)
                             // of the slice, amplified by at most At; Gt covers the arithmetic
                             // and the screen drops the candidate's residual sum (|b| <= At /
-                            // sqrt(m)) and rounds the weights to 2^-8
-                            float gc = zrest + (X::uh * 1.01f + fabsf(zsh) * rsm) * At + Gt + 1e-6f;
-                            float hh;
+                            // sqrt(m))
+                            // (a flat row is exact)
+                            const bool ex = fc != 0.f;
+                            const float g0 =
+                                zrest + (X::uh * 1.01f + fabsf(zsh) * rsm) * At + Gt + 1e-6f;
+                            float2 h2;
                             // (one choice per warp: both read tensor memory, all lanes together)
                             if (!__any_sync(0xffffffffu, masked)) {
-                                hh = screen_max();
-                                gc = fmaf(0.004f, fabsf(hh), gc);
+                                h2 = screen_max();
                             } else {
-                                hh = row_max(zsh, 0.f);
+                                h2 = row_max(zsh, 0.f);
                             }
-                            if (hh == -INFINITY || fc != 0.f) gc = 0.f; // a flat row is exact
+                            const float hh = fmaxf(h2.x, h2.y);
+                            const float gc =
+                                ex || hh == -INFINITY ? 0.f : g0;
                             prune(hh - gc, zsh, gc);
-                            // a value kept after all products is at most hup
-                            hup = fc != 0.f ? hh : hh + gc + Gt;
-                            const bool want = rowok && hup > known && !S.dead[cidx];
+                            // a value kept after all products is at most this
+                            const float up = ex ? 0.f : g0 + Gt;
+                            hup = make_float2(h2.x + up, h2.y + up);
+                            const bool want = rowok && !S.dead[cidx] &&
+                                              f2ord(fmaxf(hup.x, hup.y)) > S.known[cidx];
+                            if (bkeep) put_block(hup);
                             if (__any_sync(0xffffffffu, want) && lane == 0) S.need[s] = tag;
                         }
                         if (screen) { // every warp, also one that saw the item dead already
@@ -1108,63 +1147,71 @@ k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
                             full = __shfl_sync(0xffffffffu, S.need[s], 0) == tag;
                             if (full) {
                                 if (!__all_sync(0xffffffffu,
-                                                mbar_wait_bounded(&S.rest_done[s],
-                                                                  (s ? n_rest1 : n_rest0) & 1u, wl))) {
+                                                mbar_wait_bounded(&S.rest_done[s], n_rest & 1u, wl))) {
                                     S.abort = 1;
                                     break;
                                 }
-                                n_rest0 += s ^ 1;
-                                n_rest1 += s;
+                                ++n_rest;
                                 tc_fence_after();
-                            } else if (live) {
-                                keep_block(hup);
+                            } else if (live && bkeep) {
+                                keep_block();
                             }
                         }
                         if (full && live) {
                             // correlations lowered by the tile's bound for the prune test, raised
                             // back for the kept maximum (the interval's middle; -inf stays)
-                            const float tmax = row_max(zsc, Gt);
+                            const float2 t2 = row_max(zsc, Gt);
+                            const float tmax = fmaxf(t2.x, t2.y);
                             rmax = fmaxf(rmax, tmax + Gt);
-                            keep_block(tmax + Gt);
+                            if (bkeep) put_block(make_float2(t2.x + Gt, t2.y + Gt));
                             prune(tmax, zsc, Gt);
                             if (screen) { // for the other CTAs' screens, and this item's next tiles
-                                float v = rmax;
-#pragma unroll
-                                for (int o = 4; o > 0; o >>= 1)
-                                    v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-                                known = fmaxf(known, v);
-                                if (rowok && bsh == 0 && v > -INFINITY && wc >= 0)
-                                    atomicMax(rho_max + S.cp[cidx], f2ord(v));
+                                const float v =
+                                    fmaxf(rmax, __shfl_xor_sync(0xffffffffu, rmax, UM_TC));
+                                if (lane < UM_TC && wc >= 0 && f2ord(v) > S.known[lane] &&
+                                    atomicMax(const_cast<uint32_t *>(&S.known[lane]), f2ord(v)) <
+                                        f2ord(v))
+                                    atomicMax(rho_max + S.cp[lane], f2ord(v));
                             }
                         }
-                        if (live && warp == EPI_WARP0) {
+                        if (live && g == 0) {
                             ++n_tiles;
                             n_alive += alive;
                             alive = __popc(__ballot_sync(0xffffffffu, lane < UM_TC && !S.dead[lane & (UM_TC - 1)]));
                             if (!alive) S.item_dead = 1;
                         }
                     }
+                    if (full && bkeep) { // the first warp stores what all four have put
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&S.put[s]);
+                        if (g == 0) {
+                            if (!__all_sync(0xffffffffu, mbar_wait_bounded(&S.put[s], n_put & 1u, wl))) {
+                                S.abort = 1;
+                                break;
+                            }
+                            if (live) keep_block();
+                        }
+                        ++n_put;
+                    }
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) {
                         if (!screen) mbar_arrive(&S.dec[s]); // no screen: only its use of the ring
                         mbar_arrive(&S.acc_empty[s]);
-                        mbar_arrive(&S.wd_empty[rw.s]);
+                        mbar_arrive(&S.wd_empty[ws]);
                         mbar_arrive(&S.sl_empty[Ring(n, L.nb).s]);
                     }
                 }
-                if (warp == EPI_WARP0 && lane == 0) {
+                if (g == 0 && lane == 0) {
                     atomicAdd(&att->n_pairs, (unsigned long long)n_tiles * (UM_TC * UM_TW));
                     atomicAdd(&att->n_live, (unsigned long long)n_alive * UM_TW);
                 }
-                // fold the running maxima (8 shifts per candidate)
-                float v = rmax;
-#pragma unroll
-                for (int o = 4; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-                if (rowok && (lane & 7) == 0 && v > -INFINITY) atomicMax(&S.rmax[cidx], f2ord(v));
+                // fold the running maxima
+                const float v = fmaxf(rmax, __shfl_xor_sync(0xffffffffu, rmax, UM_TC));
+                if (lane < UM_TC && v > -INFINITY) atomicMax(&S.rmax[lane], f2ord(v));
             }
             __syncthreads();
-            G += (uint32_t)(S.tok >= 0 ? S.tok + 1 : T); // every thread, the same number
+            G += (uint32_t)(S.tok >= 0 ? min(S.tok + 2, T) : T); // every thread, the same number
             if (threadIdx.x < UM_TC && tile * UM_TC + threadIdx.x < C &&
                 S.rmax[threadIdx.x] != f2ord(-INFINITY))
                 atomicMax(rho_max + S.cp[threadIdx.x], S.rmax[threadIdx.x]);
@@ -1217,6 +1264,8 @@ k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
             for (int s = 0; s < UM_STAGES; ++s) {
                 if (S.last_full[s] >= 0)
                     mbar_wait_bounded(&S.full_b[s], (uint32_t)S.last_full[s], kDrainCycles);
+            }
+            for (int s = 0; s < UM_WBARS; ++s) {
                 if (S.last_wd[s] >= 0)
                     mbar_wait_bounded(&S.wd_full[s], (uint32_t)S.last_wd[s], kDrainCycles);
             }
