@@ -17,17 +17,18 @@
 // candidate (the margin covers the FP32 rounding of thr); every value enters
 // the candidate's kept maximum.
 //
-// Work items: (a group of 8 entries of the candidate list, 64 consecutive
+// Work items: (a group of 8 entries of the candidate list, 64, 32 or 16 consecutive
 // entries of the fragile list).  The group's centred candidate values sit in
 // shared memory (read as broadcasts, two terms per load); a fragile window is
-// shared by four threads, two halves of the group times two halves of the
+// shared by 4, 8 or 16 threads, two halves of the group times 2, 4 or 8 parts of the
 // length, each with 4 FP64 accumulators and reading the window's values straight
-// from the series (consecutive addresses per thread, so 7 of 8 loads hit L1).
+// from the series (consecutive addresses per part, so most loads hit L1).
 // What bounds it is the serial chain of one thread, not FP64 issue: a headline
-// attempt has about 3000 fragile windows and a dozen candidates, 100 items for
-// 592 resident CTAs; with one thread per window and both halves in turn it took
-// 25 us, now 5.  Halves whose candidates are all pruned, and items
-// with no live candidate, are skipped.
+// attempt has about 3000 fragile windows and a handful of candidates, 50 to 100 items
+// of 64 windows for 592 resident CTAs, so the windows per item shrink (and the parts
+// grow) while the items still fit the CTAs.  All fragile passes of a headline run: with
+// one split of 4 threads a window 10.9 ms, now 6.0 (run 137.7 -> 132.5).  Halves whose
+// candidates are all pruned, and items with no live candidate, are skipped.
 #include <float.h>
 
 #include "paddi_internal.cuh"
@@ -38,10 +39,12 @@ using paddi::ord2f;
 namespace {
 
 constexpr int FG_THREADS = 256;
-constexpr int FG_WIN = 64;      // fragile windows per item
+constexpr int FG_WIN = 64;      // fragile windows per item, at most
+constexpr int FG_SPLIT = 2;     // halvings of it, at most
 constexpr int FG_CAND = 8;      // candidate-list entries per item
 constexpr int FG_HALF = 4;      // accumulators per thread
 constexpr int FG_MAXM = 1024;
+static_assert(FG_THREADS / 32 == FG_CAND, "a warp stages a candidate");
 
 __global__ void __launch_bounds__(FG_THREADS)
 k_fragile(const float *__restrict__ x, const double2 *__restrict__ ms64,
@@ -55,7 +58,7 @@ k_fragile(const float *__restrict__ x, const double2 *__restrict__ ms64,
     // [FG_CAND][mp] centred candidate values, mp = m rounded up to even
     extern __shared__ __align__(16) double fg_a[];
     __shared__ int cw[FG_CAND], cp[FG_CAND], live[FG_CAND];
-    __shared__ double civ[FG_CAND];
+    __shared__ double civ[FG_CAND], cmu[FG_CAND];
     __shared__ double best_s[FG_CAND][4];
     __shared__ int s_any;
     paddi::chain_begin();
@@ -68,7 +71,12 @@ k_fragile(const float *__restrict__ x, const double2 *__restrict__ ms64,
     const bool bkeep = B.kept(att->n_cand_p1);
     const int mp = (m + 1) & ~1;
     const int groups = (C + FG_CAND - 1) / FG_CAND;
-    const int chunks = (F + FG_WIN - 1) / FG_WIN;
+    int sh = 0; // FG_WIN >> sh windows per item
+    while (sh < FG_SPLIT &&
+           (long long)groups * ((F + (FG_WIN >> sh) / 2 - 1) / ((FG_WIN >> sh) / 2)) <= gridDim.x)
+        ++sh;
+    const int win = FG_WIN >> sh;
+    const int chunks = (F + win - 1) / win;
     const long long total = (long long)groups * chunks;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     for (long long item = blockIdx.x; item < total; item += gridDim.x) {
@@ -83,19 +91,26 @@ k_fragile(const float *__restrict__ x, const double2 *__restrict__ ms64,
             cp[t] = pos;
             cw[t] = w;
             live[t] = pos >= 0 && !__ldcg(pruned + pos);
-            civ[t] = ms64[w].y;
+            const double2 s2 = ms64[w];
+            cmu[t] = s2.x;
+            civ[t] = s2.y;
             if (live[t]) atomicOr(&s_any, 1);
         }
         __syncthreads();
         if (!s_any) continue;
-        for (int e = t; e < FG_CAND * mp; e += FG_THREADS) {
-            const int c = e / mp, k = e - c * mp;
-            fg_a[e] = (live[c] && k < m) ? (double)x[cw[c] + k] - ms64[cw[c]].x : 0.0;
+        { // a warp per candidate
+            const bool lv = live[warp] != 0;
+            const float *xc = x + cw[warp];
+            const double mc = cmu[warp];
+#pragma unroll 4
+            for (int k = lane; k < mp; k += 32)
+                fg_a[warp * mp + k] = (lv && k < m) ? (double)__ldg(xc + k) - mc : 0.0;
         }
         __syncthreads();
-        // warp: half of the group (h), 16 windows; lane: window, half of the length (s)
-        const int h = warp & 1, wsub = warp >> 1, s = lane >> 4;
-        const int fi = chunk * FG_WIN + 16 * wsub + (lane & 15);
+        // warp: half of the group (h), 16 >> sh windows; lane: window, part of the length (s)
+        const int lw = 4 - sh; // log2 of the warp's windows
+        const int h = warp & 1, wsub = warp >> 1, s = lane >> lw;
+        const int fi = chunk * win + (wsub << lw) + (lane & ((1 << lw) - 1));
         const int f = fi < F ? frag[fi] : -1;
         const bool fok = f >= col_lo && f < col_hi;
         const int c0 = h * FG_HALF;
@@ -111,7 +126,7 @@ k_fragile(const float *__restrict__ x, const double2 *__restrict__ ms64,
             for (int c = 0; c < FG_HALF; ++c) acc[c] = 0.0;
             const double2 sf = fok ? ms64[f] : make_double2(0.0, 0.0);
             const double2 *a2 = reinterpret_cast<const double2 *>(fg_a + c0 * mp);
-            const int mh = mp >> 1, q0 = s ? (mh + 1) >> 1 : 0, q1 = s ? mh : (mh + 1) >> 1;
+            const int mh = mp >> 1, q0 = (mh * s) >> (sh + 1), q1 = (mh * (s + 1)) >> (sh + 1);
             if (fok) {
                 const float *y = x + f;
 #pragma unroll 4
@@ -128,7 +143,8 @@ k_fragile(const float *__restrict__ x, const double2 *__restrict__ ms64,
             }
 #pragma unroll
             for (int c = 0; c < FG_HALF; ++c) {
-                acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], 16);
+                for (int o = 16; o >> lw; o >>= 1)
+                    acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
                 const int ci = c0 + c;
                 const int d = cw[ci] > f ? cw[ci] - f : f - cw[ci];
                 if (fok && live[ci] && d >= m - 1) {
