@@ -302,10 +302,13 @@ template <> struct E16<true> {
 // are used where they are, in shared memory and registers.  As two kernels (the
 // second one re-reading 20 B a window) they took 34 us a length at n = 1500007,
 // m = 300, as one 25; headline run 168 -> 153 ms.
+// Four CTAs per SM (64 registers, 22 bytes of shared memory per staged value: m <= 470):
+// a length of 2^21 windows is 1025 blocks, two waves instead of three; 37 us at m = 256
+// with three, now 31.
 static_assert(ST_TILE == UM_TW, "a statistics tile is a block of the refine's grid");
 
 template <bool BF>
-__global__ void __launch_bounds__(ST_THREADS)
+__global__ void __launch_bounds__(ST_THREADS, 4)
 k_prep(const float *__restrict__ x, int64_t nser, int32_t cnt, int32_t m, int32_t N, StOut O,
        uint16_t *__restrict__ bq, float4 *__restrict__ wdq, float E, float Fu, float gcap,
        int32_t *frag_list, int32_t *frag_count, unsigned long long *t_end)

@@ -18,17 +18,18 @@ constexpr int ST_WPT = ST_TILE / ST_THREADS; // windows per thread
 constexpr int ST_MAXM = 1024; // longest supported window
 
 // dynamic shared memory of one CTA for length m: P1, P2 (FP64 prefixes), E
-// (int prefix of equal neighbours) and the staged values, ST_TILE + m + 2 each
+// (prefix of equal neighbours, at most ST_TILE + m) and the staged values, ST_TILE + m + 2
+// each
 __host__ __device__ inline size_t st_smem(int m)
 {
     const size_t L = (size_t)ST_TILE + (size_t)m + 2;
-    return L * (2 * sizeof(double) + sizeof(int) + sizeof(float));
+    return L * (2 * sizeof(double) + sizeof(float) + sizeof(uint16_t));
 }
 
 struct StTile {
     double *P1, *P2;
-    int *E;
     float *xs;
+    uint16_t *E;
     float c;
 };
 
@@ -49,8 +50,8 @@ __device__ __forceinline__ StTile st_prefix(unsigned char *mem, StShared &S, con
     StTile T;
     T.P1 = reinterpret_cast<double *>(mem);
     T.P2 = T.P1 + LS;
-    T.E = reinterpret_cast<int *>(T.P2 + LS);
-    T.xs = reinterpret_cast<float *>(T.E + LS);
+    T.xs = reinterpret_cast<float *>(T.P2 + LS);
+    T.E = reinterpret_cast<uint16_t *>(T.xs + LS);
     const int len = ST_TILE + m + 1; // values staged
     T.c = x[t0 < n ? t0 : n - 1];
     for (int k = threadIdx.x; k < len; k += ST_THREADS) {
@@ -112,7 +113,7 @@ __device__ __forceinline__ StTile st_prefix(unsigned char *mem, StShared &S, con
     for (int k = k0; k < k1; ++k) {
         T.P1[k] = b1;
         T.P2[k] = b2;
-        T.E[k] = be;
+        T.E[k] = (uint16_t)be;
         const double d = (double)T.xs[k] - c;
         b1 += d;
         b2 = fma(d, d, b2);
@@ -121,7 +122,7 @@ __device__ __forceinline__ StTile st_prefix(unsigned char *mem, StShared &S, con
     if (k0 < len && k1 == len) {
         T.P1[len] = b1;
         T.P2[len] = b2;
-        T.E[len] = be;
+        T.E[len] = (uint16_t)be;
     }
     __syncthreads();
     return T;

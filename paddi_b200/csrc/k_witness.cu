@@ -514,7 +514,11 @@ cudaError_t paddi_launch_witness_step(const float *x, const double2 *ms64,
 {
     if (m < 3 || m > WT_MAXM || N < 1 || from < m - 1 || from > m + 1) return cudaErrorInvalidValue;
     const int per = WT_THREADS * WT_SWIN;
-    cudaError_t e = paddi_launch(true, k_witness_step, (unsigned)(N / per + 1), WT_THREADS, 0, st, x,
+    // the partner gathers live off L1, and the kernel before (k_prep) leaves the SM with
+    // nearly all of it as shared memory: without a preference of its own the step ran
+    // under that split (headline run, statistics and step of a length: 104 us behind
+    // four k_prep CTAs per SM, 79 behind three, 66 with the preference and four)
+    cudaError_t e = paddi_launch_carveout(0, true, k_witness_step, (unsigned)(N / per + 1), WT_THREADS, 0, st, x,
                                  ms64, N, m, from, W.wit, W.wc, W.wrho, hint, W.scal,
                                  wt_dscale(m0));
     if (e != cudaSuccess) return e;

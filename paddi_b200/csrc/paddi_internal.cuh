@@ -111,21 +111,34 @@ PaddiBound paddi_bound_fp32(int m);
 
 // Launches `kern`; chained: as the successor of the stream's previous kernel (see
 // paddi::chain_begin, which the kernel must call first).
+// carveout >= 0: the percentage of an SM's L1 that the kernel prefers as shared memory.
 template <typename... P, typename... A>
-cudaError_t paddi_launch(bool chained, void (*kern)(P...), unsigned grid, unsigned block,
-                         size_t smem, cudaStream_t st, A... args)
+cudaError_t paddi_launch_carveout(int carveout, bool chained, void (*kern)(P...), unsigned grid,
+                                  unsigned block, size_t smem, cudaStream_t st, A... args)
 {
-    cudaLaunchAttribute at = {};
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute at[2] = {};
     cudaLaunchConfig_t c = {};
     c.gridDim = dim3(grid);
     c.blockDim = dim3(block);
     c.dynamicSmemBytes = smem;
     c.stream = st;
-    c.attrs = &at;
-    c.numAttrs = chained ? 1 : 0;
+    c.attrs = at;
+    if (chained) {
+        at[c.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[c.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (carveout >= 0) {
+        at[c.numAttrs].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+        at[c.numAttrs++].val.sharedMemCarveout = (unsigned)carveout;
+    }
     return cudaLaunchKernelEx(&c, kern, P(args)...);
+}
+
+template <typename... P, typename... A>
+cudaError_t paddi_launch(bool chained, void (*kern)(P...), unsigned grid, unsigned block,
+                         size_t smem, cudaStream_t st, A... args)
+{
+    return paddi_launch_carveout(-1, chained, kern, grid, block, smem, st, args...);
 }
 
 // Time stamps (ns, globaltimer) of a length's preparation and of an attempt.
