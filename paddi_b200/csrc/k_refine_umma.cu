@@ -45,7 +45,7 @@
 // known to reach.  hi * hi alone, a third of the MMAs, is within gc (about 5e-3 on
 // the headline series) of the exact value; when its maximum plus that bound stays
 // below the best value known of every live candidate (this item's tiles, other
-// CTAs' through rho_max, the candidate's witness), the other two products and the
+// CTAs' through rho_max, the candidate's witness), the three products and the
 // full epilogue are skipped.  A candidate whose lower bound is above thr is pruned
 // at once.  Nothing kept is computed with less than all three products.  The MMA
 // thread issues tile u+1's hi * hi before it takes the verdict on tile u; 5 to 25 %
@@ -80,9 +80,9 @@ constexpr int UM_FEW = 4;        // tiles that take all remaining windows after 
 // A tile is screened by its hi * hi product first (split-FP16, where the work item
 // has several tiles and K' is long enough; the comment at the kernel has the
 // figures): refine launches at n = 300007 with tens of thousands of candidates, all
-// products at once / screened, us: m = 64 (K' 80) 1770 / 1883, m = 100 (112) 2125 /
-// 2057, m = 200 (208) 3715 / 2945, m = 500 (512) 18800 / 9990, m = 700 (720) 27500 /
-// 13600; PALMAD 64..512 at 2^18 149 ms / 137.  With one to three tiles an item's first
+// products at once / screened, us: m = 64 (K' 80) 1770 / 1890, m = 100 (112) 2125 /
+// 2120, m = 200 (208) 3715 / 3110, m = 500 (512) 18800 / 10810, m = 700 (720) 27500 /
+// 14400; PALMAD 64..512 at 2^21 137 ms / 125.  With one to three tiles an item's first
 // tile, which nothing is known about yet, is most of it.  BF16 leaves out 2^-8 of the
 // slice: its screen rejects little.
 constexpr int UM_SCREEN_T = 4;
@@ -502,7 +502,7 @@ struct UmShared {
     uint64_t mma_done[2];  // tcgen05.commit: the tile's MMAs are complete
     uint64_t acc_empty[2]; // epilogue -> MMA: accumulator drained
     uint64_t dec[2];       // epilogue -> MMA: hi * hi product screened, need[] decided
-    uint64_t rest_done[2]; // tcgen05.commit: the products with lo halves are complete
+    uint64_t rest_done[2]; // tcgen05.commit: a screened tile's three products are complete
     uint64_t put[2];       // epilogue: a fully multiplied tile's block maxima are in bmax
     uint64_t drain;        // final MMA drain on abort
     // phase of the last arrival the loader issued on full_b[s] / wd_full[s] (-1: none
@@ -520,7 +520,7 @@ struct UmShared {
     float cflat[UM_TCMAX], zsum[UM_TCMAX];
     // screening: sum of the hi halves, norm of what they leave out, a correlation
     // the candidate is known to reach; need[s]: tag of the last tile in accumulator
-    // s that needs its other products
+    // s that needs all its products
     float zsumh[UM_TCMAX], zrest[UM_TCMAX];
     volatile uint32_t known[UM_TCMAX]; // (ordered image)
     volatile uint32_t need[2];
@@ -838,8 +838,8 @@ k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
                 }
                 if (!ok) S.abort = 1;
             } else if (warp == MMA_WARP && lane == 0) {
-                // products of tile u: hi * hi, and (rest) hi * lo + lo * hi
-                auto issue = [&](int u, bool hihi, bool rest) {
+                // products of tile u: hi * hi, or all three
+                auto issue = [&](int u, bool all) {
                     const uint32_t n = G + (uint32_t)u;
                     const int st = Ring(n, L.nb).s;
                     tc_fence_after();
@@ -851,13 +851,13 @@ k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
                     uint64_t ah = sdesc(a_hi_s, RG * 128, 128), al = sdesc(a_lo_s, RG * 128, 128);
                     uint64_t bhd = sdesc(bh, 16, 128), bld = sdesc(bl, 16, 128);
                     constexpr uint64_t da = 2 * RG * 128 / 16, db = 32 / 16;
-                    if (!rest) {
+                    if (!all) {
 #pragma unroll 4
                         for (int kb = 0; kb < kblocks; ++kb, ah += da, bhd += db)
                             umma_f16(d, ah, bhd, idesc, kb > 0 ? 1u : 0u);
                     } else {
                         for (int kb = 0; kb < kblocks; ++kb, ah += da, al += da, bhd += db, bld += db) {
-                            if (hihi) umma_f16(d, ah, bhd, idesc, kb > 0 ? 1u : 0u);
+                            umma_f16(d, ah, bhd, idesc, kb > 0 ? 1u : 0u);
                             umma_f16(d, ah, bld, idesc, 1u);
                             umma_f16(d, al, bhd, idesc, 1u);
                         }
@@ -869,7 +869,12 @@ k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
                     const Ring a(G + (uint32_t)u, 2);
                     if (!mbar_wait_bounded(&S.dec[a.s], a.par, wl)) return false;
                     if (S.need[a.s] == G + (uint32_t)u + 1u) {
-                        issue(u, false, true);
+                        // all three from zero, block by block of K as without the screen: the
+                        // two small ones on top of a finished hi * hi would be rounded at the
+                        // full sum's size every time (kept correlations at m = 200: 7.9e-7
+                        // rms from FP64 instead of 6.2e-7).  The product that is done
+                        // twice is 7 % of a refine of many candidates, 1 % of PALMAD
+                        issue(u, true);
                         umma_commit(&S.rest_done[a.s]);
                     }
                     return true;
@@ -896,7 +901,7 @@ k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
                         ended = true;
                         continue;
                     }
-                    issue(u, true, !screen);
+                    issue(u, !screen);
                     umma_commit(&S.mma_done[a.s]);
                     // the tile before was screened while this one's product started
                     if (screen && u > 0) ok = settle(u - 1);
