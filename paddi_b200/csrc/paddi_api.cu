@@ -1498,20 +1498,22 @@ PADDI_API paddi_status paddi_model_grad(paddi_ctx *ctx, const float *X, const fl
     CK(dmalloc(ctx, &dX.p, sizeof(float) * MLP_NFEAT * n));
     CK(dmalloc(ctx, &dY.p, sizeof(float) * n));
     CK(dmalloc(ctx, &dP.p, sizeof(float) * MLP_NPARAM));
-    CK(dmalloc(ctx, &dG.p, sizeof(float) * MLP_NPARAM));
+    CK(dmalloc(ctx, &dG.p, sizeof(double) * MLP_NPARAM));
     CK(dmalloc(ctx, &dL.p, sizeof(double)));
     cudaStream_t st = ctx->st;
     CK(cudaMemcpyAsync(dX.p, X, sizeof(float) * MLP_NFEAT * n, cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(dY.p, Y, sizeof(float) * n, cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(dP.p, params, sizeof(float) * MLP_NPARAM, cudaMemcpyHostToDevice, st));
-    CK(cudaMemsetAsync(dG.p, 0, sizeof(float) * MLP_NPARAM, st));
+    CK(cudaMemsetAsync(dG.p, 0, sizeof(double) * MLP_NPARAM, st));
     CK(cudaMemsetAsync(dL.p, 0, sizeof(double), st));
     CK(paddi_launch_mlp_grad((float *)dX.p, (float *)dY.p, nullptr, (int)n, tau, (float *)dP.p,
-                             (float *)dG.p, (double *)dL.p, ctx->num_sms, st));
-    CK(cudaMemcpyAsync(grad, dG.p, sizeof(float) * MLP_NPARAM, cudaMemcpyDeviceToHost, st));
+                             (double *)dG.p, (double *)dL.p, ctx->num_sms, st));
+    std::vector<double> g(MLP_NPARAM);
+    CK(cudaMemcpyAsync(g.data(), dG.p, sizeof(double) * MLP_NPARAM, cudaMemcpyDeviceToHost, st));
     double lsum = 0.0;
     CK(cudaMemcpyAsync(&lsum, dL.p, sizeof(double), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
+    for (int i = 0; i < MLP_NPARAM; ++i) grad[i] = (float)g[i];
     *loss = (float)lsum;
     return PADDI_OK;
 }
@@ -1551,8 +1553,8 @@ PADDI_API paddi_status paddi_model_train(paddi_ctx *ctx, const float *X, const f
         return fail(ctx, PADDI_ERR_INVALID_ARG, "model_train: bad argument");
     CK(cudaSetDevice(ctx->device));
     cudaStream_t st = ctx->st;
-    // one allocation: the samples, an epoch's order, parameters, gradient, Adam
-    // moments, losses
+    // one allocation: the samples, an epoch's order, parameters (FP32), gradient, Adam's
+    // state and losses (64 bits)
     DevBuf buf;
     size_t bytes = 0;
     auto place = [&](size_t b) {
@@ -1562,10 +1564,11 @@ PADDI_API paddi_status paddi_model_train(paddi_ctx *ctx, const float *X, const f
     };
     const size_t np = sizeof(float) * MLP_NPARAM, nl = sizeof(double) * (epochs ? epochs : 1);
     const size_t oX = place(sizeof(float) * MLP_NFEAT * n), oY = place(sizeof(float) * n);
-    const size_t oI = place(sizeof(uint32_t) * n), oP = place(np), oG = place(np), oM = place(np);
-    const size_t oV = place(np), oL = place(nl);
+    const size_t oI = place(sizeof(uint32_t) * n), oP = place(np), oG = place(2 * np);
+    const size_t oA = place(6 * np), oL = place(nl);
     CK(dmalloc(ctx, &buf.p, bytes));
     auto at = [&](size_t o) { return reinterpret_cast<float *>(static_cast<char *>(buf.p) + o); };
+    auto at64 = [&](size_t o) { return reinterpret_cast<double *>(at(o)); };
     uint32_t *dI = reinterpret_cast<uint32_t *>(at(oI));
     CK(cudaMemsetAsync(at(oG), 0, bytes - oG, st));
     CK(cudaMemcpyAsync(at(oP), params, np, cudaMemcpyHostToDevice, st));
@@ -1586,9 +1589,9 @@ PADDI_API paddi_status paddi_model_train(paddi_ctx *ctx, const float *X, const f
         CK(cudaMemcpyAsync(dI, perm.data(), sizeof(uint32_t) * n, cudaMemcpyHostToDevice, st));
         for (uint32_t b0 = 0; b0 < n; b0 += batch) {
             const uint32_t bn = std::min(batch, n - b0);
-            CK(paddi_launch_mlp_grad(at(oX), at(oY), dI + b0, (int)bn, tau, at(oP), at(oG),
-                                     reinterpret_cast<double *>(at(oL)) + e, ctx->num_sms, st));
-            CK(paddi_launch_mlp_adam(at(oP), at(oG), at(oM), at(oV), lr, ++step, st));
+            CK(paddi_launch_mlp_grad(at(oX), at(oY), dI + b0, (int)bn, tau, at(oP), at64(oG),
+                                     at64(oL) + e, ctx->num_sms, st));
+            CK(paddi_launch_mlp_adam(at(oP), at64(oG), at64(oA), lr, ++step, st));
         }
     }
     CK(cudaMemcpyAsync(params, at(oP), np, cudaMemcpyDeviceToHost, st));

@@ -540,9 +540,10 @@ cudaError_t paddi_launch_mlp_forward(const float *X, int n, const void *P, bool 
                                      cudaStream_t st);
 // perm (optional): rows of X and Y to take, in order.
 cudaError_t paddi_launch_mlp_grad(const float *X, const float *Y, const uint32_t *perm, int n,
-                                  float tau, const float *P, float *G, double *loss, int num_sms,
+                                  float tau, const float *P, double *G, double *loss, int num_sms,
                                   cudaStream_t st);
-cudaError_t paddi_launch_mlp_adam(float *P, float *G, float *M, float *V, float lr, int step,
+// A: 3 * MLP_NPARAM values, zero before step 1.
+cudaError_t paddi_launch_mlp_adam(float *P, double *G, double *A, float lr, int step,
                                   cudaStream_t st);
 cudaError_t paddi_launch_mlp_to_bf16(const float *P, void *Q, cudaStream_t st);
 
