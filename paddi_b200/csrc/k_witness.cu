@@ -39,6 +39,14 @@
 // t + t^2 with t = 34 delta (inv_i + inv_w); 2 t is subtracted, and 1e-7 for the
 // FP32 rounding of thr.  A pair with t of the order of 1 proves nothing and
 // prunes nothing.
+// A step back (a missed attempt whose next length was already queued) takes one
+// term away again: the norms shrink, and what the two steps over that term
+// rounded may be large beside the shorter windows (a window of small values just
+// before a spike).  With a, b the term's centred values at the shorter length, a
+// step over it rounds by at most delta (|a| + |b| + delta) and 5 u |a b| (beside
+// u |cov|, which the 1e-7 covers 1e8 times over), so 2.1 delta (|a| + |b| + 2
+// delta) + 16 u (|a| + delta)(|b| + delta) per return, times inv_i inv_w, are
+// subtracted as well.  At the longer length a and b are below the norms again.
 #include <float.h>
 
 #include "paddi_internal.cuh"
@@ -93,11 +101,14 @@ __device__ __forceinline__ WtGroups wt_decode(double code)
 // mostly have neighbouring witnesses.  WT_SWIN windows per thread keep that
 // many chains wit -> partner in flight.  Hinted windows are listed for
 // k_witness_hints.
+// BACK: a step from m + 1, its rounding bounded as above (its own kernel: in one with
+// the forward step the run of 449 lengths took 1.5 % longer).
+template <bool BACK>
 __global__ void __launch_bounds__(WT_THREADS)
 k_witness_step(const float *__restrict__ x, const double2 *__restrict__ ms64, int32_t N,
                int32_t m, int32_t from, int32_t *__restrict__ wit, double *__restrict__ wc,
                float *__restrict__ wrho, int32_t *__restrict__ hint, uint32_t *scal,
-               double dscale)
+               double dscale, double delta1, int32_t returns)
 {
     paddi::chain_begin();
     const int i0 = blockIdx.x * (WT_THREADS * WT_SWIN) + threadIdx.x;
@@ -108,6 +119,7 @@ k_witness_step(const float *__restrict__ x, const double2 *__restrict__ ms64, in
     const double f = from == m - 1   ? (double)m / (double)(m - 1)
                      : from == m + 1 ? -(double)m / (double)(m + 1)
                                      : 0.0;
+    const double delta = delta1 * (double)__uint_as_float(scal[WT_AMAX]);
     int w[WT_SWIN];
 #pragma unroll
     for (int q = 0; q < WT_SWIN; ++q) {
@@ -136,11 +148,16 @@ k_witness_step(const float *__restrict__ x, const double2 *__restrict__ ms64, in
         const int i = i0 + q * WT_THREADS;
         float out = -INFINITY;
         if (ok[q]) {
+            double ret = 0.0; // rounding of the returns over the term taken away
             if (f != 0.0) {
-                c[q] = fma(f * ((double)xi[q] - si[q].x), (double)xw[q] - sw[q].x, c[q]);
+                const double a = (double)xi[q] - si[q].x, b = (double)xw[q] - sw[q].x;
+                c[q] = fma(f * a, b, c[q]);
                 wc[i] = c[q];
+                if (BACK)
+                    ret = (double)returns * (2.1 * delta * (fabs(a) + fabs(b) + 2.0 * delta) +
+                                             16.0 * kU64 * (fabs(a) + delta) * (fabs(b) + delta));
             }
-            out = wt_bound(c[q], si[q].y, sw[q].y, t1);
+            out = wt_bound(BACK ? c[q] - ret : c[q], si[q].y, sw[q].y, t1);
         } else if (w[q] >= 0) {
             wit[i] = -1;
         }
@@ -491,7 +508,9 @@ k_witness_rescue(const float *__restrict__ x, const double2 *__restrict__ ms64, 
     }
 }
 
-double wt_dscale(int32_t m0) { return 34.0 * 5e5 / (double)m0 * kU64; }
+// delta over the largest |x|, and the same times the steps' sum
+double wt_delta(int32_t m0) { return 5e5 / (double)m0 * kU64; }
+double wt_dscale(int32_t m0) { return 34.0 * wt_delta(m0); }
 
 } // namespace
 
@@ -509,8 +528,8 @@ cudaError_t paddi_launch_witness_start(const float *x, int64_t n, int32_t N, con
 
 cudaError_t paddi_launch_witness_step(const float *x, const double2 *ms64,
                                       int32_t N, int32_t m, int32_t from, int32_t m0,
-                                      const PaddiWitness &W, int32_t *hint, int32_t num_sms,
-                                      cudaStream_t st, unsigned long long *t_end)
+                                      int32_t returns, const PaddiWitness &W, int32_t *hint,
+                                      int32_t num_sms, cudaStream_t st, unsigned long long *t_end)
 {
     if (m < 3 || m > WT_MAXM || N < 1 || from < m - 1 || from > m + 1) return cudaErrorInvalidValue;
     const int per = WT_THREADS * WT_SWIN;
@@ -518,9 +537,10 @@ cudaError_t paddi_launch_witness_step(const float *x, const double2 *ms64,
     // nearly all of it as shared memory: without a preference of its own the step ran
     // under that split (headline run, statistics and step of a length: 104 us behind
     // four k_prep CTAs per SM, 79 behind three, 66 with the preference and four)
-    cudaError_t e = paddi_launch_carveout(0, true, k_witness_step, (unsigned)(N / per + 1), WT_THREADS, 0, st, x,
+    auto kern = from == m + 1 ? k_witness_step<true> : k_witness_step<false>;
+    cudaError_t e = paddi_launch_carveout(0, true, kern, (unsigned)(N / per + 1), WT_THREADS, 0, st, x,
                                  ms64, N, m, from, W.wit, W.wc, W.wrho, hint, W.scal,
-                                 wt_dscale(m0));
+                                 wt_dscale(m0), wt_delta(m0), returns);
     if (e != cudaSuccess) return e;
     return paddi_launch(true, k_witness_hints, num_sms * 4, WT_THREADS, 0, st, x, ms64, N, m, W.wit,
                         W.wc, W.wrho, hint, W.scal, wt_dscale(m0), t_end);

@@ -87,6 +87,7 @@ struct paddi_ctx {
     PaddiWitness W = {};
     size_t W_cap = 0; // windows
     int wit_m = 0, wit_m0 = 0;
+    int wit_edge = 0, wit_returns = 0; // steps back from wit_edge + 1 to wit_edge so far
     // learned r predictor
     bool model_ok = false;
     float model_margin = 1.f;
@@ -341,6 +342,7 @@ paddi_status start_witness(paddi_ctx *ctx, const float *x, size_t n, int m0)
     CK(paddi_launch_witness_start(x, (int64_t)n, (int32_t)(n - m0 + 1), ctx->W, ctx->num_sms,
                                   ctx->st));
     ctx->wit_m = ctx->wit_m0 = m0;
+    ctx->wit_edge = ctx->wit_returns = 0;
     return PADDI_OK;
 }
 
@@ -348,9 +350,17 @@ paddi_status start_witness(paddi_ctx *ctx, const float *x, size_t n, int m0)
 paddi_status witness_to(paddi_ctx *ctx, const float *x, size_t n, int m)
 {
     if (ctx->wit_m == 0 || ctx->wit_m == m) return PADDI_OK;
+    const int edge = std::min(ctx->wit_m, m);
+    if (edge != ctx->wit_edge) {
+        ctx->wit_edge = edge;
+        ctx->wit_returns = 0;
+    }
+    const bool back = ctx->wit_m > m;
+    if (back) ++ctx->wit_returns;
     CK(paddi_launch_witness_step(x, ctx->d_ms64, (int32_t)(n - m + 1), m,
-                                 ctx->wit_m, ctx->wit_m0, ctx->W, ctx->d_list[1],
-                                 ctx->num_sms, ctx->st, ctx->d_tprep + PADDI_T_STATS_E));
+                                 ctx->wit_m, ctx->wit_m0, back ? ctx->wit_returns : 0, ctx->W,
+                                 ctx->d_list[1], ctx->num_sms, ctx->st,
+                                 ctx->d_tprep + PADDI_T_STATS_E));
     ctx->prep_launches += 2;
     ctx->wit_m = m;
     return PADDI_OK;

@@ -373,11 +373,14 @@ cudaError_t paddi_launch_stats(const float *x, int64_t n, int32_t m, float4 *wst
 cudaError_t paddi_launch_witness_start(const float *x, int64_t n, int32_t N, const PaddiWitness &W,
                                        int32_t num_sms, cudaStream_t st);
 // Advances the witnesses from length `from` (m - 1, m or m + 1) to m, with the
-// statistics of m; m0 is the shortest length of the run; hint: scratch, N entries.
+// statistics of m; m0 is the shortest length of the run; returns: how often the run has
+// stepped from m + 1 back to m, this step included (0: a step forward); hint: scratch,
+// N entries.
 cudaError_t paddi_launch_witness_step(const float *x, const double2 *ms64,
                                       int32_t N, int32_t m, int32_t from, int32_t m0,
-                                      const PaddiWitness &W, int32_t *hint, int32_t num_sms,
-                                      cudaStream_t st, unsigned long long *t_end = nullptr);
+                                      int32_t returns, const PaddiWitness &W, int32_t *hint,
+                                      int32_t num_sms, cudaStream_t st,
+                                      unsigned long long *t_end = nullptr);
 // Writes alive[0..N) from the witnesses at threshold thr and looks for new
 // witnesses of the others (listed in fail) while they are at most `limit`.
 cudaError_t paddi_launch_witness_check(const double2 *ms64, const float *x,
