@@ -34,11 +34,14 @@
 // thr.  The FP64 means carry an error of at most delta = 5e5 u A / m0 (prefix
 // sums over a tile of at most 3074 values, <= 36 additions deep; u = 2^-53, A the
 // largest |x|, m0 the shortest length of the run).  A step's term is off by
-// |a| delta + |b| delta, at most 1100 steps sum to sqrt(1100) delta (n_i + n_w)
-// by Cauchy-Schwarz (norms grow with the length), so the correlation is within
-// t + t^2 with t = 34 delta (inv_i + inv_w); 2 t is subtracted, and 1e-7 for the
-// FP32 rounding of thr.  A pair with t of the order of 1 proves nothing and
-// prunes nothing.
+// |a| delta + |b| delta; a pair that has taken c_l steps over the value l (one, and
+// two more per step back) is off by sum c_l (|a_l| + |b_l|) delta, at most
+// s delta (n_i + n_w) with s^2 = sum c_l^2, by Cauchy-Schwarz (norms grow with the
+// length), so the correlation is within t + t^2 with t = (s + 1) delta (inv_i +
+// inv_w), the 1 for the pair's first dot product.  The host counts s^2 of the run
+// (at least 1089: the at most 1021 lengths of a run without steps back all take
+// s + 1 = 34).  2 t is subtracted, and 1e-7 for the FP32 rounding of thr.  A pair
+// with t of the order of 1 proves nothing and prunes nothing.
 // A step back (a missed attempt whose next length was already queued) takes one
 // term away again: the norms shrink, and what the two steps over that term
 // rounded may be large beside the shorter windows (a window of small values just
@@ -48,6 +51,9 @@
 // delta) + 16 u (|a| + delta)(|b| + delta) per return, times inv_i inv_w, are
 // subtracted as well.  At the longer length a and b are below the norms again.
 #include <float.h>
+
+#include <algorithm>
+#include <cmath>
 
 #include "paddi_internal.cuh"
 
@@ -508,9 +514,12 @@ k_witness_rescue(const float *__restrict__ x, const double2 *__restrict__ ms64, 
     }
 }
 
-// delta over the largest |x|, and the same times the steps' sum
+// delta over the largest |x|, and t over that and the inverse norms
 double wt_delta(int32_t m0) { return 5e5 / (double)m0 * kU64; }
-double wt_dscale(int32_t m0) { return 34.0 * wt_delta(m0); }
+double wt_dscale(const PaddiWitnessRun &R)
+{
+    return (std::sqrt(std::max(1089.0, R.steps2)) + 1.0) * wt_delta(R.m0);
+}
 
 } // namespace
 
@@ -527,9 +536,10 @@ cudaError_t paddi_launch_witness_start(const float *x, int64_t n, int32_t N, con
 }
 
 cudaError_t paddi_launch_witness_step(const float *x, const double2 *ms64,
-                                      int32_t N, int32_t m, int32_t from, int32_t m0,
-                                      int32_t returns, const PaddiWitness &W, int32_t *hint,
-                                      int32_t num_sms, cudaStream_t st, unsigned long long *t_end)
+                                      int32_t N, int32_t m, int32_t from,
+                                      const PaddiWitnessRun &R, const PaddiWitness &W,
+                                      int32_t *hint, int32_t num_sms, cudaStream_t st,
+                                      unsigned long long *t_end)
 {
     if (m < 3 || m > WT_MAXM || N < 1 || from < m - 1 || from > m + 1) return cudaErrorInvalidValue;
     const int per = WT_THREADS * WT_SWIN;
@@ -540,15 +550,15 @@ cudaError_t paddi_launch_witness_step(const float *x, const double2 *ms64,
     auto kern = from == m + 1 ? k_witness_step<true> : k_witness_step<false>;
     cudaError_t e = paddi_launch_carveout(0, true, kern, (unsigned)(N / per + 1), WT_THREADS, 0, st, x,
                                  ms64, N, m, from, W.wit, W.wc, W.wrho, hint, W.scal,
-                                 wt_dscale(m0), wt_delta(m0), returns);
+                                 wt_dscale(R), wt_delta(R.m0), R.returns);
     if (e != cudaSuccess) return e;
     return paddi_launch(true, k_witness_hints, num_sms * 4, WT_THREADS, 0, st, x, ms64, N, m, W.wit,
-                        W.wc, W.wrho, hint, W.scal, wt_dscale(m0), t_end);
+                        W.wc, W.wrho, hint, W.scal, wt_dscale(R), t_end);
 }
 
 cudaError_t paddi_launch_witness_check(const double2 *ms64, const float *x,
-                                       int32_t N, int32_t m, float thr, int32_t m0,
-                                       const PaddiWitness &W, uint8_t *alive, int32_t *fail,
+                                       int32_t N, int32_t m, float thr,
+                                       const PaddiWitnessRun &R, const PaddiWitness &W, uint8_t *alive, int32_t *fail,
                                        PaddiAttemptDev *att, int32_t limit, int32_t num_sms,
                                        cudaStream_t st)
 {
@@ -559,5 +569,5 @@ cudaError_t paddi_launch_witness_check(const double2 *ms64, const float *x,
     const size_t smem = sizeof(float) * (size_t)WT_RWARPS * (size_t)m;
     return paddi_launch(true, k_witness_rescue, num_sms * 8, 32 * WT_RWARPS, smem, st, x, ms64, N, m,
                         thr, fail, &att->n_fail, limit, W.wit, W.wc, W.wrho, alive,
-                        &att->n_rescued, W.scal, wt_dscale(m0));
+                        &att->n_rescued, W.scal, wt_dscale(R));
 }

@@ -83,11 +83,12 @@ struct paddi_ctx {
     double *d_G = nullptr;                  // shifted dot products, two buffers (on first use)
     size_t G_cap = 0;                       // windows per buffer
     // witnesses of the current PALMAD run (allocated on first use): the length
-    // they stand at (0: none in use) and the run's shortest length
+    // they stand at (0: none in use) and the steps taken so far
     PaddiWitness W = {};
     size_t W_cap = 0; // windows
-    int wit_m = 0, wit_m0 = 0;
-    int wit_edge = 0, wit_returns = 0; // steps back from wit_edge + 1 to wit_edge so far
+    int wit_m = 0;
+    PaddiWitnessRun wit = {};
+    int wit_edge = 0, wit_steps = 0; // steps between wit_edge and wit_edge + 1 so far
     // learned r predictor
     bool model_ok = false;
     float model_margin = 1.f;
@@ -341,8 +342,9 @@ paddi_status start_witness(paddi_ctx *ctx, const float *x, size_t n, int m0)
     }
     CK(paddi_launch_witness_start(x, (int64_t)n, (int32_t)(n - m0 + 1), ctx->W, ctx->num_sms,
                                   ctx->st));
-    ctx->wit_m = ctx->wit_m0 = m0;
-    ctx->wit_edge = ctx->wit_returns = 0;
+    ctx->wit_m = m0;
+    ctx->wit = {m0, 0, 0.0};
+    ctx->wit_edge = ctx->wit_steps = 0;
     return PADDI_OK;
 }
 
@@ -353,13 +355,13 @@ paddi_status witness_to(paddi_ctx *ctx, const float *x, size_t n, int m)
     const int edge = std::min(ctx->wit_m, m);
     if (edge != ctx->wit_edge) {
         ctx->wit_edge = edge;
-        ctx->wit_returns = 0;
+        ctx->wit_steps = 0;
     }
-    const bool back = ctx->wit_m > m;
-    if (back) ++ctx->wit_returns;
-    CK(paddi_launch_witness_step(x, ctx->d_ms64, (int32_t)(n - m + 1), m,
-                                 ctx->wit_m, ctx->wit_m0, back ? ctx->wit_returns : 0, ctx->W,
-                                 ctx->d_list[1], ctx->num_sms, ctx->st,
+    ctx->wit.steps2 += 2.0 * ctx->wit_steps + 1.0; // (c + 1)^2 - c^2
+    ++ctx->wit_steps;
+    ctx->wit.returns = ctx->wit_steps / 2; // forward, back, forward, ...
+    CK(paddi_launch_witness_step(x, ctx->d_ms64, (int32_t)(n - m + 1), m, ctx->wit_m, ctx->wit,
+                                 ctx->W, ctx->d_list[1], ctx->num_sms, ctx->st,
                                  ctx->d_tprep + PADDI_T_STATS_E));
     ctx->prep_launches += 2;
     ctx->wit_m = m;
@@ -548,7 +550,7 @@ paddi_status run_attempt(paddi_ctx *ctx, const float *x, size_t n, int m, float 
     int launches = 0;
     const bool wit = ctx->wit_m == m;
     if (wit) {
-        CK(paddi_launch_witness_check(ctx->d_ms64, x, N, m, thr, ctx->wit_m0, ctx->W,
+        CK(paddi_launch_witness_check(ctx->d_ms64, x, N, m, thr, ctx->wit, ctx->W,
                                       ctx->d_alive, ctx->d_list[0], ctx->d_att, wit_limit(N),
                                       ctx->num_sms, st));
         launches += 2;
@@ -1455,6 +1457,7 @@ PADDI_API paddi_status paddi_debug_get(paddi_ctx *ctx, int32_t key, int64_t *val
     case PADDI_DEBUG_WITHHOLD_STAGE: *value = ctx->withhold; return PADDI_OK;
     case PADDI_DEBUG_LAST_PASSES: *value = ctx->last_passes; return PADDI_OK;
     case PADDI_DEBUG_RECHECK_CAP: *value = ctx->rc_cap; return PADDI_OK;
+    case PADDI_DEBUG_WITNESS_STEPS: *value = (int64_t)ctx->wit.steps2; return PADDI_OK;
     default: break;
     }
     return fail(ctx, PADDI_ERR_INVALID_ARG, "paddi_debug_get: unknown key");

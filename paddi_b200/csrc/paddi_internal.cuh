@@ -372,20 +372,27 @@ cudaError_t paddi_launch_stats(const float *x, int64_t n, int32_t m, float4 *wst
 // Empties the witnesses of a run whose shortest length has N windows.
 cudaError_t paddi_launch_witness_start(const float *x, int64_t n, int32_t N, const PaddiWitness &W,
                                        int32_t num_sms, cudaStream_t st);
+// What the host counts of a run: its shortest length; how often it has stepped back over
+// the value that `returns` of the next step is for (this step included); the sum over the
+// values of the squared number of steps taken over each.
+struct PaddiWitnessRun {
+    int32_t m0, returns;
+    double steps2;
+};
+
 // Advances the witnesses from length `from` (m - 1, m or m + 1) to m, with the
-// statistics of m; m0 is the shortest length of the run; returns: how often the run has
-// stepped from m + 1 back to m, this step included (0: a step forward); hint: scratch,
-// N entries.
+// statistics of m; hint: scratch, N entries.
 cudaError_t paddi_launch_witness_step(const float *x, const double2 *ms64,
-                                      int32_t N, int32_t m, int32_t from, int32_t m0,
-                                      int32_t returns, const PaddiWitness &W, int32_t *hint,
-                                      int32_t num_sms, cudaStream_t st,
+                                      int32_t N, int32_t m, int32_t from,
+                                      const PaddiWitnessRun &R, const PaddiWitness &W,
+                                      int32_t *hint, int32_t num_sms, cudaStream_t st,
                                       unsigned long long *t_end = nullptr);
 // Writes alive[0..N) from the witnesses at threshold thr and looks for new
 // witnesses of the others (listed in fail) while they are at most `limit`.
 cudaError_t paddi_launch_witness_check(const double2 *ms64, const float *x,
-                                       int32_t N, int32_t m, float thr, int32_t m0,
-                                       const PaddiWitness &W, uint8_t *alive, int32_t *fail,
+                                       int32_t N, int32_t m, float thr,
+                                       const PaddiWitnessRun &R, const PaddiWitness &W,
+                                       uint8_t *alive, int32_t *fail,
                                        PaddiAttemptDev *att, int32_t limit, int32_t num_sms,
                                        cudaStream_t st);
 

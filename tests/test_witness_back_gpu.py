@@ -14,6 +14,7 @@ import numpy as np
 import pytest
 
 import paddi_b200 as P
+from paddi_b200 import datagen
 
 pytestmark = pytest.mark.gpu
 
@@ -47,3 +48,23 @@ def test_a_value_taken_back_leaves_no_false_proof(seed, spike):
         for a in log:  # (the schedule's r may be negative; its square is the threshold)
             _, rows = one.pd3(x, a["m"], r=abs(a["r"]))
             assert [(b["n_cand"], b["n_disc"]) for b in rows] == [(a["n_cand"], a["n_disc"])], a
+
+
+@pytest.mark.parametrize("guided", [True, False])
+def test_the_bound_counts_every_step(guided):
+    """The rounding bound of a carried pair scales with the steps taken over each
+    value: one per length, and two more per attempt that missed with the next length
+    queued (the guided policies queue it, for all lengths but the last).  (The
+    reference's schedule runs on noise anomalies: it can stand still on others.)"""
+    if guided:
+        x, lo = _series(0, 10.0), 60
+    else:
+        x, _ = datagen.palmad_series(n=30000, seed=2, n_anom=4, min_len=64, max_len=96,
+                                     kinds_cycle=("noise",))
+        lo = 64
+    with P.Context(device=0, r_policy=P.R_BOUND if guided else P.R_MERLIN) as ctx:
+        _, log = ctx.palmad(x, lo, lo + 8)
+        steps2 = ctx.debug_get(P.DEBUG_WITNESS_STEPS)
+    tries = [sum(a["m"] == m for a in log) for m in range(lo, lo + 8)]
+    assert tries[0] > 1
+    assert steps2 == sum((2 * t - 1 if guided else 1) ** 2 for t in tries)
