@@ -284,6 +284,13 @@ int refine_kernel_for(const paddi_ctx *ctx, int m)
     return k == PADDI_DIST_SPLIT_BF16 ? PADDI_DIST_SPLIT_BF16 : PADDI_DIST_SPLIT_FP16;
 }
 
+// The message of a refine that gave up on a wait.
+std::string refine_timeout(int kernel, int m)
+{
+    return std::string(kernel == PADDI_DIST_FP32 ? "FP32 refine" : "tensor-core refine") +
+           ": a barrier wait timed out (m=" + std::to_string(m) + ")";
+}
+
 // Guard band, in correlation units: the largest per-window rounding bound a
 // bounded refine kernel accepts, and the half-width of the FP64 recheck band.
 float guard_of(const paddi_ctx *ctx, int kernel)
@@ -1339,7 +1346,11 @@ PADDI_API paddi_status paddi_shard_refine(paddi_ctx *ctx, const float *d_series,
     if (s != PADDI_OK) return s;
     CK(cudaMemcpyAsync(&ctx->h_res->n_p1, &ctx->d_att->n_cand_p1, sizeof(int32_t),
                        cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(&ctx->h_res->status, &ctx->d_att->status, sizeof(int32_t),
+                       cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
+    if (ctx->h_res->status == 3) // the arrays miss pairs
+        return fail(ctx, PADDI_ERR_CUDA, refine_timeout(kernel, (int)m));
     const int32_t C = ctx->h_res->n_p1;
     *n_cand = (uint32_t)C;
     if ((uint32_t)C > cap)
