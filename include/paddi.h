@@ -350,6 +350,13 @@ typedef enum paddi_debug_key {
 paddi_status paddi_debug_set(paddi_ctx *ctx, int32_t key, int64_t value);
 paddi_status paddi_debug_get(paddi_ctx *ctx, int32_t key, int64_t *value);
 
+/* Windows of the largest work item (and *items, optional: the items per tile of
+ * candidates) of a refine round over `windows` windows, for a kernel
+ * (paddi_distance_kernel), a length, a number of candidates and of resident
+ * blocks; -1 for arguments outside the library's ranges.  Needs no device. */
+int64_t paddi_debug_refine_item(int32_t kernel, uint32_t m, uint32_t candidates,
+                                uint32_t windows, uint32_t ctas, int64_t *items);
+
 /* Largest window count (n - m + 1) that paddi_compute_statistics_noalloc accepts. */
 #define PADDI_NOALLOC_MAX_WINDOWS 131072
 

@@ -177,6 +177,8 @@ _SIGS = {
     "paddi_merlin_first_r": ([C.POINTER(_Discord), C.c_uint32, C.c_uint32,
                               C.POINTER(C.c_float)], C.c_float),
     "paddi_merlin_lower": ([C.c_float, C.c_uint32, C.c_float], C.c_float),
+    "paddi_debug_refine_item": ([C.c_int32, C.c_uint32, C.c_uint32, C.c_uint32, C.c_uint32,
+                                 C.c_void_p], C.c_int64),
     "paddi_debug_set": ([C.c_void_p, C.c_int32, C.c_int64], C.c_int),
     "paddi_debug_get": ([C.c_void_p, C.c_int32, C.POINTER(C.c_int64)], C.c_int),
 }

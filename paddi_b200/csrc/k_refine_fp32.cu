@@ -69,6 +69,17 @@ struct RfSmem {
     float *cgm;   // [RF_CW]: the bound subtracted from each window's correlations
 };
 
+// About two items per CTA; with thousands of candidates one split would do that, and an
+// item would be 8 candidates times the whole round.  RF_ITEM bounds its windows times m:
+// 8 * 2^30 FMA are some 2.2e8 cycles of a CTA (at 38 a cycle), a twentieth of the
+// waits' limit (without it a round of 3.4e7 windows at m = 1000 came to 7e9 cycles).
+constexpr int RF_ITEM = 1 << 30;
+__host__ __device__ __forceinline__ paddi::RefineItems rf_items(int m, int tiles, int range,
+                                                                int ctas)
+{
+    return paddi::refine_items(range, tiles, (2 * ctas + tiles - 1) / tiles, RF_CW, RF_ITEM / m);
+}
+
 constexpr int RF_SUMBLK = 64; // two-level sums: terms per partial sum
 
 __global__ void __launch_bounds__(RF_THREADS)
@@ -113,9 +124,8 @@ k_refine_fp32(const float *__restrict__ x, const float4 *__restrict__ wst,
         const int range = je - jb;
         const int tiles = (C + RF_TC - 1) / RF_TC;
         // about two items per CTA, of at least one chunk
-        int splits = (2 * (int)gridDim.x + tiles - 1) / tiles;
-        splits = max(1, min(splits, range / RF_CW));
-        const int span = (((range + splits - 1) / splits) + RF_CW - 1) / RF_CW * RF_CW;
+        const paddi::RefineItems I = rf_items(m, tiles, range, (int)gridDim.x);
+        const int splits = I.splits, span = I.span;
         const int total = tiles * splits;
         bool counted = true; // this CTA's latest item is in done_rd
         for (;;) {
@@ -354,8 +364,13 @@ cudaError_t paddi_launch_refine_fp32(const float *x, const float4 *wst, const fl
     if (per_sm < 1) return cudaErrorInvalidConfiguration;
     const int grid = num_sms * per_sm;
     return paddi_launch(true, k_refine_fp32, grid, RF_THREADS, smem, st, x, wst, mu, cand, list0, list1, att, rho_max, pruned, N, m, col_lo, col_hi, thr,
-        paddi_bound_fp32(m).E, gcap, wait_cycles > 0 ? wait_cycles : 4000000000ll,
+        paddi_bound_fp32(m).E, gcap, wait_cycles > 0 ? wait_cycles : paddi::REFINE_WAIT,
         W ? *W : PaddiWitness{});
+}
+
+paddi::RefineItems paddi_refine_items_fp32(int32_t m, int32_t C, int32_t range, int32_t ctas)
+{
+    return rf_items(m, (C + RF_TC - 1) / RF_TC, range, ctas);
 }
 
 PaddiBound paddi_bound_fp32(int m)

@@ -88,6 +88,13 @@ constexpr int UM_FEW = 4;        // tiles that take all remaining windows after 
 constexpr int UM_SCREEN_T = 4;
 constexpr int UM_SCREEN_K = 112;
 constexpr int UM_WAVES = 1;      // work items per CTA and round when candidate tiles are few
+// An item is at most 2048 tiles of at most some 4e4 cycles each (3 K'/16 products of 128
+// cycles, twice that for the rest): 8e7 cycles, a fiftieth of the waits' limit.
+constexpr int UM_ITEM = 1 << 22; // windows
+__host__ __device__ __forceinline__ paddi::RefineItems um_items(int tiles, int range, int ctas)
+{
+    return paddi::refine_items(range, tiles, UM_WAVES * ctas / tiles, UM_TW, UM_ITEM);
+}
 constexpr int UM_KMAX128 = 368;  // largest K' with M = 128 (shared-memory bound)
 constexpr int UM_KMAX64 = 736;   // largest K' with M = 64
 constexpr int UM_STAGES = 4;      // at most
@@ -638,8 +645,8 @@ k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
         const int tiles = (C + UM_TC - 1) / UM_TC;
         // at most UM_WAVES items per CTA when the candidate tiles are few, items of
         // at least one 2048-window block
-        const int splits = max(1, min(range / UM_TW, (UM_WAVES * grid_ctas) / tiles));
-        const int span = (((range + splits - 1) / splits) + UM_TW - 1) / UM_TW * UM_TW;
+        const paddi::RefineItems I = um_items(tiles, range, grid_ctas);
+        const int splits = I.splits, span = I.span;
         const int total = tiles * splits;
         if (threadIdx.x == 0) S.built_tile = -1;
         bool counted = true; // this CTA's latest item is in done_rd
@@ -1305,6 +1312,13 @@ int paddi_umma_max_m() { return UM_KMAX64 - 7; } // kpad_of(m) <= UM_KMAX64
 
 int32_t paddi_tile_width() { return UM_TW; }
 
+paddi::RefineItems paddi_refine_items_umma(int32_t m, bool rows64, int32_t C, int32_t range,
+                                           int32_t ctas)
+{
+    const int tc = kpad_of(m) <= UM_KMAX128 && !rows64 ? UM_TCMAX : UM_TCMAX / 2;
+    return um_items((C + tc - 1) / tc, range, ctas);
+}
+
 int64_t paddi_tile_blocks(int64_t N) { return (N + UM_TW - 1) / UM_TW; }
 
 int64_t paddi_tile_block_elems_max() { return 2 * (int64_t)slice_cnt(UM_KMAX64); }
@@ -1382,7 +1396,7 @@ cudaError_t paddi_launch_refine_umma(bool bf16, const float *x, const float4 *ws
     const int grid = num_sms;
     return paddi_launch(true, kern, grid, UM_THREADS, smem, st, x, wst, mu, cand, list0, list1, bq, wdq, att, rho_max,
                                          pruned, N, m, col_lo, col_hi, thr_prune, grid,
-                                         wait_cycles > 0 ? wait_cycles : 4000000000ll, withhold,
+                                         wait_cycles > 0 ? wait_cycles : paddi::REFINE_WAIT, withhold,
                                          W ? *W : PaddiWitness{}, B ? *B : PaddiBlockMax{},
                         !bf16 && kp >= UM_SCREEN_K ? 1 : 0, guard);
 }

@@ -495,8 +495,7 @@ paddi_status select_passes(paddi_ctx *ctx, const float *x, size_t n, int m, floa
         ctx->att_dirty = false;
         ctx->last_passes = pass + 1;
         if (ctx->h_res->status == 3) // a refine wait ran out: no redo can help
-            return fail(ctx, PADDI_ERR_CUDA, "tensor-core refine: a barrier wait timed out (m=" +
-                                                 std::to_string(m) + ")");
+            return fail(ctx, PADDI_ERR_CUDA, refine_timeout(refine_kernel_for(ctx, m), m));
         if (ctx->h_res->status == 1) {
             // more windows need the exact value than the queue holds: grow it and redo
             int32_t cap = ctx->rc_cap;
@@ -1472,6 +1471,22 @@ PADDI_API paddi_status paddi_debug_get(paddi_ctx *ctx, int32_t key, int64_t *val
     default: break;
     }
     return fail(ctx, PADDI_ERR_INVALID_ARG, "paddi_debug_get: unknown key");
+}
+
+PADDI_API int64_t paddi_debug_refine_item(int32_t kernel, uint32_t m, uint32_t candidates,
+                                          uint32_t windows, uint32_t ctas, int64_t *items)
+{
+    if (m < 3 || m > 1024 || candidates < 1 || windows < 1 || ctas < 1 || ctas > 1 << 16 ||
+        candidates > INT32_MAX - 64 || windows > INT32_MAX - 64)
+        return -1;
+    const bool fp32 = kernel == PADDI_DIST_FP32 || (int)m > paddi_umma_max_m();
+    const paddi::RefineItems I =
+        fp32 ? paddi_refine_items_fp32((int32_t)m, (int32_t)candidates, (int32_t)windows,
+                                       (int32_t)ctas)
+             : paddi_refine_items_umma((int32_t)m, false, (int32_t)candidates, (int32_t)windows,
+                                       (int32_t)ctas);
+    if (items) *items = I.splits;
+    return I.span;
 }
 
 // ============================================================ learned r model

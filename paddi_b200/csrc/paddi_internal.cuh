@@ -181,6 +181,28 @@ __host__ __device__ __forceinline__ int refine_round_end(int rd, int rounds, int
     return rd == rounds - 1 ? hi : lo + ((hi - lo) >> (rd ? 3 - rd : 4)) / tw * tw;
 }
 
+// Work items of a round: `tiles` candidate tiles times `splits` spans of the round's
+// windows (spans on a grid of `grid` windows, the last ones may be empty).  `want`
+// splits fill the GPU; beyond that an item is at most about `cap` windows, because
+// the CTAs that find no item left wait for the others' with a limit: an item has to
+// be a small part of that whatever the series' length.  (tiles * splits fits 31 bits.)
+struct RefineItems {
+    int splits, span;
+};
+__host__ __device__ __forceinline__ RefineItems refine_items(int range, int tiles, int want,
+                                                             int grid, int cap)
+{
+    RefineItems I;
+    const int fill = want < range / grid ? want : range / grid;
+    const int need = (int)(((long long)range + cap - 1) / cap), room = (1 << 30) / tiles;
+    I.splits = need > fill ? (need < room ? need : room) : fill;
+    if (I.splits < 1) I.splits = 1;
+    I.span = (int)((((long long)range + I.splits - 1) / I.splits + grid - 1) / grid * grid);
+    return I;
+}
+// Default limit of the refine's waits in clock cycles, about 2 s.
+constexpr long long REFINE_WAIT = 4000000000ll;
+
 __device__ __forceinline__ int32_t ld_acquire(const int32_t *p)
 {
     int32_t v;
@@ -476,6 +498,10 @@ cudaError_t paddi_launch_refine_umma(bool bf16, const float *x, const float4 *ws
 // paddi_tile_block_elems_max() elements per block) and the epilogue's window
 // data (wdq, paddi_tile_wd_entries() float4 per block).
 int32_t paddi_tile_width();
+// The work items of a round of `range` windows and C candidates on `ctas` CTAs.
+paddi::RefineItems paddi_refine_items_umma(int32_t m, bool rows64, int32_t C, int32_t range,
+                                           int32_t ctas);
+paddi::RefineItems paddi_refine_items_fp32(int32_t m, int32_t C, int32_t range, int32_t ctas);
 int64_t paddi_tile_blocks(int64_t N);
 int64_t paddi_tile_block_elems_max();
 int64_t paddi_tile_wd_entries();

@@ -41,3 +41,23 @@ def test_sharded_refine_reports_a_timeout(dist):
         ind, rho, pr = be.refine(m, r2, alive, 0, N)
         again, _ = be.select(m, r2, ind, rho, pr, 1)
         assert again == want
+
+
+def test_the_message_names_the_refine_that_gave_up():
+    """n above 65536 windows: four rounds.  The FP32 refine's blocks without work in a
+    round wait for the others', here at most one cycle."""
+    x, _ = datagen.palmad_series(n=1 << 17, seed=4, n_anom=8, min_len=32, max_len=96)
+    m = 80
+    with P.Context(device=0, distance_kernel=P.DIST_FP32) as ctx:
+        (top,), _ = ctx.pd3(x, m)
+        r = 0.7 * float(np.sqrt(top.dist))
+        want, (row,) = ctx.pd3(x, m, r=r)
+        assert row["n_cand"] > 8  # more than one tile: the rounds go on
+        ctx.debug_set(P.DEBUG_WAIT_CYCLES, 1)
+        with pytest.raises(P.PaddiError) as e:
+            ctx.pd3(x, m, r=r)
+        assert e.value.status == P.PADDI_ERR_CUDA
+        assert "FP32 refine" in str(e.value) and "timed out" in str(e.value)
+        ctx.debug_set(P.DEBUG_WAIT_CYCLES, 0)
+        again, _ = ctx.pd3(x, m, r=r)
+        assert again == want
