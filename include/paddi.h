@@ -334,7 +334,9 @@ float paddi_merlin_lower(float r, uint32_t j, float S);
  * tensor memory and returns. */
 typedef enum paddi_debug_key {
     PADDI_DEBUG_FAIL_ALLOC = 1,     /* value k > 0: the k-th next device allocation of the
-                                       context fails (PADDI_ERR_OUT_OF_MEMORY); 0: off */
+                                       context is refused once (PADDI_ERR_OUT_OF_MEMORY,
+                                       unless the context holds memory that it can do
+                                       without: it gives that up and tries again); 0: off */
     PADDI_DEBUG_WAIT_CYCLES = 2,    /* limit of the refine's barrier waits in clock cycles
                                        (0: the default, about 2 s) */
     PADDI_DEBUG_WITHHOLD_STAGE = 3, /* 1: the next tensor-core refine launches never fill one

@@ -85,7 +85,8 @@ struct paddi_ctx {
     // witnesses of the current PALMAD run (allocated on first use): the length
     // they stand at (0: none in use) and the steps taken so far
     PaddiWitness W = {};
-    size_t W_cap = 0; // windows
+    void *W_mem = nullptr; // one allocation
+    size_t W_cap = 0;      // windows
     int wit_m = 0;
     PaddiWitnessRun wit = {};
     int wit_edge = 0, wit_steps = 0; // steps between wit_edge and wit_edge + 1 so far
@@ -102,6 +103,7 @@ struct paddi_ctx {
     // clears the other (dirty: an attempt broke off before that)
     PaddiAttemptDev *d_att = nullptr, *d_att2[2] = {nullptr, nullptr};
     bool att_dirty = false;
+    bool alive_used = false; // d_alive is not all ones: written from witnesses, not reset
     unsigned long long *d_tprep = nullptr; // time stamps of the current length's preparation
     PaddiAttemptResult *d_res = nullptr;
     // {flat windows, flat span (2), fragile windows} of the current length: one of
@@ -159,22 +161,6 @@ void drop_workers(paddi_ctx *ctx, size_t keep = 0)
     }
 }
 
-// Every device allocation of a context goes through here, so a test can make
-// one fail (PADDI_DEBUG_FAIL_ALLOC) and check that PADDI_ERR_OUT_OF_MEMORY
-// reaches the caller.
-template <typename T>
-cudaError_t dmalloc(paddi_ctx *ctx, T **p, size_t bytes)
-{
-    if (ctx->fail_alloc > 0 && --ctx->fail_alloc == 0) return cudaErrorMemoryAllocation;
-    cudaError_t e = cudaMalloc((void **)p, bytes);
-    if (e == cudaErrorMemoryAllocation && !ctx->workers.empty()) {
-        cudaGetLastError();
-        drop_workers(ctx);
-        e = cudaMalloc((void **)p, bytes);
-    }
-    return e;
-}
-
 template <typename T>
 void dfree(T *&p)
 {
@@ -184,12 +170,33 @@ void dfree(T *&p)
 
 void free_witness(paddi_ctx *ctx)
 {
-    dfree(ctx->W.wit);
-    dfree(ctx->W.wc);
-    dfree(ctx->W.wrho);
-    dfree(ctx->W.scal);
+    dfree(ctx->W_mem);
+    ctx->W = {};
     ctx->W_cap = 0;
     ctx->wit_m = 0;
+}
+
+// Every device allocation of a context goes through here, so a test can have
+// one refused (PADDI_DEBUG_FAIL_ALLOC) and check that PADDI_ERR_OUT_OF_MEMORY
+// reaches the caller.  What the context holds only to be faster is given up
+// before that: idle workers, and the witnesses (a run goes on without them).
+template <typename T>
+cudaError_t dmalloc(paddi_ctx *ctx, T **p, size_t bytes)
+{
+    const bool refuse = ctx->fail_alloc > 0 && --ctx->fail_alloc == 0;
+    cudaError_t e = refuse ? cudaErrorMemoryAllocation : cudaMalloc((void **)p, bytes);
+    if (e == cudaErrorMemoryAllocation && !ctx->workers.empty()) {
+        cudaGetLastError();
+        drop_workers(ctx);
+        e = cudaMalloc((void **)p, bytes);
+    }
+    if (e == cudaErrorMemoryAllocation && ctx->W_mem) {
+        cudaGetLastError();
+        free_witness(ctx); // (cudaFree waits for the kernels that use them)
+        e = cudaMalloc((void **)p, bytes);
+    }
+    if (e != cudaSuccess) cudaGetLastError(); // reported by this call alone
+    return e;
 }
 
 void free_buffers(paddi_ctx *ctx)
@@ -311,6 +318,7 @@ paddi_status run_stats(paddi_ctx *ctx, const float *x, size_t n, int m, bool cha
 {
     const int cur = ctx->d_flatcount == ctx->d_flat2[0] ? 1 : 0;
     ctx->d_flatcount = ctx->d_flat2[cur];
+    ctx->alive_used = false;
     PaddiStatsExtra ex;
     ex.alive = ctx->d_alive;
     ex.next = ctx->d_flat2[cur ^ 1];
@@ -335,22 +343,25 @@ paddi_status run_stats(paddi_ctx *ctx, const float *x, size_t n, int m, bool cha
     return PADDI_OK;
 }
 
-// Starts a run's witnesses: no window has one.
+// Starts a run's witnesses: no window has one.  Without memory for them (16 bytes a
+// window) the run goes on without (wit_m stays 0): every attempt then runs phase 1.
 paddi_status start_witness(paddi_ctx *ctx, const float *x, size_t n, int m0)
 {
     const size_t W = ctx->cap_n + PADDI_PAD_WIN + 64;
+    ctx->wit = {m0, 0, 0.0};
     if (ctx->W_cap < W) {
         free_witness(ctx);
-        CK(dmalloc(ctx, &ctx->W.wit, sizeof(int32_t) * W));
-        CK(dmalloc(ctx, &ctx->W.wc, sizeof(double) * W));
-        CK(dmalloc(ctx, &ctx->W.wrho, sizeof(float) * W));
-        CK(dmalloc(ctx, &ctx->W.scal, sizeof(uint32_t) * 4));
+        const size_t Wa = (W + 63) & ~(size_t)63; // 256-byte steps
+        if (dmalloc(ctx, &ctx->W_mem, 16 * Wa + 256) != cudaSuccess) return PADDI_OK;
+        ctx->W.wc = (double *)ctx->W_mem;
+        ctx->W.wit = (int32_t *)(ctx->W.wc + Wa);
+        ctx->W.wrho = (float *)(ctx->W.wit + Wa);
+        ctx->W.scal = (uint32_t *)(ctx->W.wrho + Wa);
         ctx->W_cap = W;
     }
     CK(paddi_launch_witness_start(x, (int64_t)n, (int32_t)(n - m0 + 1), ctx->W, ctx->num_sms,
                                   ctx->st));
     ctx->wit_m = m0;
-    ctx->wit = {m0, 0, 0.0};
     ctx->wit_edge = ctx->wit_steps = 0;
     return PADDI_OK;
 }
@@ -555,6 +566,9 @@ paddi_status run_attempt(paddi_ctx *ctx, const float *x, size_t n, int m, float 
     ctx->att_dirty = true;
     int launches = 0;
     const bool wit = ctx->wit_m == m;
+    if (!wit && ctx->alive_used) // the witnesses were given up since the last attempt
+        CK(cudaMemsetAsync(ctx->d_alive, 1, (size_t)N, st));
+    ctx->alive_used = wit;
     if (wit) {
         CK(paddi_launch_witness_check(ctx->d_ms64, x, N, m, thr, ctx->wit, ctx->W,
                                       ctx->d_alive, ctx->d_list[0], ctx->d_att, wit_limit(N),

@@ -1,0 +1,73 @@
+"""Memory that a context can do without is given up before a call fails.
+
+A refused allocation is made on the host (PADDI_DEBUG_FAIL_ALLOC refuses the
+k-th next one once).  The buffers of the series are reserved before, so the
+count starts at the run's own allocations.
+"""
+import numpy as np
+import pytest
+
+import paddi_b200 as P
+from paddi_b200 import datagen
+
+pytestmark = pytest.mark.gpu
+
+
+def _noise_series(n=30000):
+    x, _ = datagen.palmad_series(n=n, seed=2, n_anom=4, min_len=64, max_len=96,
+                                 kinds_cycle=("noise",))
+    return x
+
+
+def _rows(log):
+    return [(a["m"], a["r"], a["n_cand"], a["n_disc"]) for a in log]
+
+
+@pytest.mark.parametrize("policy,k", [(P.R_MERLIN, 1), (P.R_BOUND, 2)])
+def test_a_run_goes_on_without_memory_for_the_witnesses(policy, k):
+    """(the bound's dot products are allocated before the witnesses)"""
+    x = _noise_series()
+    with P.Context(device=0, r_policy=policy) as ctx:
+        ctx.reserve(len(x), 80)
+        ctx.debug_set(P.DEBUG_FAIL_ALLOC, k)
+        got, log = ctx.palmad(x, 64, 80)
+        assert ctx.debug_get(P.DEBUG_FAIL_ALLOC) == 0
+        assert ctx.debug_get(P.DEBUG_WITNESS_STEPS) == 0  # none carried
+        want, wlog = ctx.palmad(x, 64, 80)
+        assert ctx.debug_get(P.DEBUG_WITNESS_STEPS) > 0
+    assert got == want and _rows(log) == _rows(wlog)
+
+
+@pytest.mark.parametrize("policy,k", [(P.R_MERLIN, 2), (P.R_BOUND, 3), (P.R_BOUND, 4)])
+def test_witnesses_are_given_up_for_memory_needed_later(policy, k):
+    """The profile's buffers are allocated after the first length's attempts: refused
+    once, they take the witnesses' memory, and the lengths after run without."""
+    x = _noise_series()
+    with P.Context(device=0, r_policy=policy) as ctx:
+        ctx.reserve(len(x), 80)
+        ctx.debug_set(P.DEBUG_FAIL_ALLOC, k)
+        got, log, prof = ctx.palmad_profiled(x, 64, 70)
+        assert ctx.debug_get(P.DEBUG_FAIL_ALLOC) == 0
+        assert ctx.debug_get(P.DEBUG_WITNESS_STEPS) == 0
+        want, wlog, wprof = ctx.palmad_profiled(x, 64, 70)
+    assert got == want and _rows(log) == _rows(wlog)
+    # a distance is known to the guard band (2e-4 in correlation) on each side
+    for j, (a, b) in enumerate(zip(prof, wprof)):
+        np.testing.assert_array_equal(a > 0, b > 0)
+        assert np.abs(a - b)[a > 0].max() <= 2 * 2 * (64 + j) * 2e-4
+
+
+@pytest.mark.parametrize("policy", [P.R_MERLIN, P.R_BOUND])
+def test_witnesses_are_given_up_for_the_recheck_queue(policy):
+    """A recheck queue of one window overflows (with a wide guard band) while the
+    run's witnesses are in use; its growth, refused once, takes their memory."""
+    x = _noise_series()
+    with P.Context(device=0, r_policy=policy, guard=0.01) as ctx:
+        want, wlog = ctx.palmad(x, 64, 80)  # all buffers are there from now on
+        assert max(a["n_recheck"] for a in wlog) > 1
+        ctx.debug_set(P.DEBUG_RECHECK_CAP, 1)
+        ctx.debug_set(P.DEBUG_FAIL_ALLOC, 1)
+        got, log = ctx.palmad(x, 64, 80)
+        assert ctx.debug_get(P.DEBUG_FAIL_ALLOC) == 0
+        assert ctx.debug_get(P.DEBUG_WITNESS_STEPS) < 16
+    assert got == want and _rows(log) == _rows(wlog)
