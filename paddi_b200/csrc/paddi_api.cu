@@ -228,6 +228,26 @@ void free_buffers(paddi_ctx *ctx)
     ctx->rc_cap = 0;
 }
 
+// A recheck queue of `cap` windows in place of the present one, which stays when the
+// memory is refused.  No kernel that uses it may be in flight.
+cudaError_t set_recheck_cap(paddi_ctx *ctx, int32_t cap)
+{
+    int32_t *q = nullptr;
+    unsigned long long *v = nullptr;
+    cudaError_t e = dmalloc(ctx, &q, sizeof(int32_t) * (size_t)cap);
+    if (e == cudaSuccess) e = dmalloc(ctx, &v, sizeof(unsigned long long) * (size_t)cap);
+    if (e != cudaSuccess) {
+        dfree(q);
+        return e;
+    }
+    dfree(ctx->d_recheck);
+    dfree(ctx->d_nn64);
+    ctx->d_recheck = q;
+    ctx->d_nn64 = v;
+    ctx->rc_cap = cap;
+    return cudaSuccess;
+}
+
 paddi_status ensure_capacity(paddi_ctx *ctx, size_t n)
 {
     if (n <= ctx->cap_n) return PADDI_OK;
@@ -258,9 +278,7 @@ paddi_status ensure_capacity(paddi_ctx *ctx, size_t n)
         CK(dmalloc(ctx, &ctx->d_bmax, sizeof(uint32_t) * (size_t)ctx->bmax_cap));
         CK(dmalloc(ctx, &ctx->d_wdq, sizeof(float4) * (size_t)(blocks * paddi_tile_wd_entries())));
     }
-    CK(dmalloc(ctx, &ctx->d_recheck, sizeof(int32_t) * PADDI_MAX_RECHECK));
-    CK(dmalloc(ctx, &ctx->d_nn64, sizeof(unsigned long long) * PADDI_MAX_RECHECK));
-    ctx->rc_cap = PADDI_MAX_RECHECK;
+    CK(set_recheck_cap(ctx, PADDI_MAX_RECHECK));
     CK(cudaMemsetAsync(ctx->d_wst, 0, sizeof(float4) * W, ctx->st));
     CK(cudaMemsetAsync(ctx->d_mu, 0, sizeof(float) * W, ctx->st));
     ctx->cap_n = n;
@@ -511,11 +529,7 @@ paddi_status select_passes(paddi_ctx *ctx, const float *x, size_t n, int m, floa
             // more windows need the exact value than the queue holds: grow it and redo
             int32_t cap = ctx->rc_cap;
             while (cap < ctx->h_res->n_recheck) cap *= 2;
-            dfree(ctx->d_recheck);
-            dfree(ctx->d_nn64);
-            CK(dmalloc(ctx, &ctx->d_recheck, sizeof(int32_t) * (size_t)cap));
-            CK(dmalloc(ctx, &ctx->d_nn64, sizeof(unsigned long long) * (size_t)cap));
-            ctx->rc_cap = cap;
+            CK(set_recheck_cap(ctx, cap));
         } else if (ctx->h_res->status == 2) {
             // a pick had no exact value: queue everything up to the cut and redo
             widen = 1e30f;
@@ -1459,11 +1473,7 @@ PADDI_API paddi_status paddi_debug_set(paddi_ctx *ctx, int32_t key, int64_t valu
         if (value < 1 || value > (1 << 24) || !ctx->d_recheck) break;
         CK(cudaSetDevice(ctx->device));
         CK(cudaStreamSynchronize(ctx->st));
-        dfree(ctx->d_recheck);
-        dfree(ctx->d_nn64);
-        CK(dmalloc(ctx, &ctx->d_recheck, sizeof(int32_t) * (size_t)value));
-        CK(dmalloc(ctx, &ctx->d_nn64, sizeof(unsigned long long) * (size_t)value));
-        ctx->rc_cap = (int32_t)value;
+        CK(set_recheck_cap(ctx, (int32_t)value));
         return PADDI_OK;
     }
     default:

@@ -71,3 +71,21 @@ def test_witnesses_are_given_up_for_the_recheck_queue(policy):
         assert ctx.debug_get(P.DEBUG_FAIL_ALLOC) == 0
         assert ctx.debug_get(P.DEBUG_WITNESS_STEPS) < 16
     assert got == want and _rows(log) == _rows(wlog)
+
+
+@pytest.mark.parametrize("k", [1, 2])
+def test_a_refused_growth_leaves_the_recheck_queue(k):
+    """Either buffer of the larger queue refused: the call fails, the queue stays as it
+    was and the next call, which grows it, is a good one."""
+    x = _noise_series(8192)
+    with P.Context(device=0) as ctx:
+        want, _ = ctx.pd3(x, 64, top_k=4)
+        ctx.debug_set(P.DEBUG_RECHECK_CAP, 1)
+        ctx.debug_set(P.DEBUG_FAIL_ALLOC, k)
+        with pytest.raises(P.PaddiError) as e:
+            ctx.pd3(x, 64, top_k=4)
+        assert e.value.status == P.PADDI_ERR_OUT_OF_MEMORY
+        assert ctx.debug_get(P.DEBUG_RECHECK_CAP) == 1
+        got, _ = ctx.pd3(x, 64, top_k=4)
+        assert ctx.debug_get(P.DEBUG_RECHECK_CAP) > 1
+    assert got == want
