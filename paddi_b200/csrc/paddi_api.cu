@@ -179,7 +179,8 @@ void free_witness(paddi_ctx *ctx)
 // Every device allocation of a context goes through here, so a test can have
 // one refused (PADDI_DEBUG_FAIL_ALLOC) and check that PADDI_ERR_OUT_OF_MEMORY
 // reaches the caller.  What the context holds only to be faster is given up
-// before that: idle workers, and the witnesses (a run goes on without them).
+// before that: idle workers, the witnesses (a run goes on without them) and the
+// block maxima (the recheck then scans the whole series).
 template <typename T>
 cudaError_t dmalloc(paddi_ctx *ctx, T **p, size_t bytes)
 {
@@ -193,6 +194,12 @@ cudaError_t dmalloc(paddi_ctx *ctx, T **p, size_t bytes)
     if (e == cudaErrorMemoryAllocation && ctx->W_mem) {
         cudaGetLastError();
         free_witness(ctx); // (cudaFree waits for the kernels that use them)
+        e = cudaMalloc((void **)p, bytes);
+    }
+    if (e == cudaErrorMemoryAllocation && ctx->d_bmax) {
+        cudaGetLastError();
+        dfree(ctx->d_bmax); // (as above)
+        ctx->bmax_cap = 0;
         e = cudaMalloc((void **)p, bytes);
     }
     if (e != cudaSuccess) cudaGetLastError(); // reported by this call alone
@@ -271,14 +278,19 @@ paddi_status ensure_capacity(paddi_ctx *ctx, size_t n)
     if (ctx->umma_ok) {
         const int64_t blocks = paddi_tile_blocks((int64_t)n);
         CK(dmalloc(ctx, &ctx->d_bq, sizeof(uint16_t) * (size_t)(blocks * paddi_tile_block_elems_max())));
-        // a row of block maxima for 2048 candidates of a long series, and for all
-        // that an attempt commonly leaves of a short one
-        ctx->bmax_cap = std::min<int64_t>((int64_t)n * 2 * blocks,
-                                          std::max<int64_t>(2 * (int64_t)W, 1 << 21));
-        CK(dmalloc(ctx, &ctx->d_bmax, sizeof(uint32_t) * (size_t)ctx->bmax_cap));
         CK(dmalloc(ctx, &ctx->d_wdq, sizeof(float4) * (size_t)(blocks * paddi_tile_wd_entries())));
     }
     CK(set_recheck_cap(ctx, PADDI_MAX_RECHECK));
+    if (ctx->umma_ok) {
+        // a row of block maxima for 2048 candidates of a long series, and for all
+        // that an attempt commonly leaves of a short one; without memory for them
+        // the recheck scans the whole series
+        const int64_t blocks = paddi_tile_blocks((int64_t)n);
+        ctx->bmax_cap = std::min<int64_t>((int64_t)n * 2 * blocks,
+                                          std::max<int64_t>(2 * (int64_t)W, 1 << 21));
+        if (dmalloc(ctx, &ctx->d_bmax, sizeof(uint32_t) * (size_t)ctx->bmax_cap) != cudaSuccess)
+            ctx->bmax_cap = 0;
+    }
     CK(cudaMemsetAsync(ctx->d_wst, 0, sizeof(float4) * W, ctx->st));
     CK(cudaMemsetAsync(ctx->d_mu, 0, sizeof(float) * W, ctx->st));
     ctx->cap_n = n;
@@ -443,7 +455,7 @@ float thr_of(float r2, int m) { return (float)(1.0 - (double)r2 / (2.0 * (double
 PaddiBlockMax block_max(const paddi_ctx *ctx, int kernel, int32_t N, bool whole)
 {
     PaddiBlockMax B = {};
-    if (kernel != PADDI_DIST_FP32 && whole) {
+    if (kernel != PADDI_DIST_FP32 && whole && ctx->d_bmax) {
         B.v = ctx->d_bmax;
         B.cap = ctx->bmax_cap;
         B.halves = 2 * (int32_t)paddi_tile_blocks(N);
@@ -487,19 +499,24 @@ paddi_status refine_rounds(paddi_ctx *ctx, const float *x, int32_t N, int m, int
 
 // Classification, FP64 recheck and top-k selection of the refined
 // candidates, redone (at most 6 passes) when the recheck queue overflows or a
-// pick lacks an exact value.  next_m > 0: the statistics (and, with
-// next_guided, the bound) of length next_m are queued behind the first pass,
-// before its result is synced; *spec tells whether they were.
+// pick lacks an exact value.  kept: the refine has stored block maxima.
+// next_m > 0: the statistics (and, with next_guided, the bound) of length next_m
+// are queued behind the first pass, before its result is synced; *spec tells
+// whether they were.
 paddi_status select_passes(paddi_ctx *ctx, const float *x, size_t n, int m, float r2,
-                           float guard, const PaddiBlockMax &B, int top_k, int32_t known_w, unsigned long long known_ord,
-                           int next_m, bool next_guided, bool *spec, int *launches)
+                           float guard, bool kept, int top_k, int32_t known_w,
+                           unsigned long long known_ord, int next_m, bool next_guided,
+                           bool *spec, int *launches)
 {
     const int32_t N = (int32_t)(n - m + 1);
     const float thr = thr_of(r2, m);
     cudaStream_t st = ctx->st;
     *spec = false;
     float widen = 2.f;
+    const int kernel = refine_kernel_for(ctx, m);
     for (int pass = 0; pass < 6; ++pass) {
+        // (a pass that grew the recheck queue may have given up the block maxima)
+        const PaddiBlockMax B = block_max(ctx, kernel, N, kept);
         CK(paddi_launch_finalize(ctx->d_cand, ctx->d_att, ctx->d_rho, ctx->d_pruned, m, r2, thr,
                                  guard, widen, top_k, ctx->d_flat, ctx->rc_cap, ctx->d_recheck,
                                  ctx->d_rcslot, ctx->d_nn64, ctx->d_res, known_w, known_ord, st));
@@ -524,7 +541,7 @@ paddi_status select_passes(paddi_ctx *ctx, const float *x, size_t n, int m, floa
         ctx->att_dirty = false;
         ctx->last_passes = pass + 1;
         if (ctx->h_res->status == 3) // a refine wait ran out: no redo can help
-            return fail(ctx, PADDI_ERR_CUDA, refine_timeout(refine_kernel_for(ctx, m), m));
+            return fail(ctx, PADDI_ERR_CUDA, refine_timeout(kernel, m));
         if (ctx->h_res->status == 1) {
             // more windows need the exact value than the queue holds: grow it and redo
             int32_t cap = ctx->rc_cap;
@@ -602,8 +619,8 @@ paddi_status run_attempt(paddi_ctx *ctx, const float *x, size_t n, int m, float 
     paddi_status s = refine_rounds(ctx, x, N, m, kernel, thr, guard, 0, N, &launches);
     if (s != PADDI_OK) return s;
     bool spec = false;
-    s = select_passes(ctx, x, n, m, r2, guard, block_max(ctx, kernel, N, true), top_k, known_w, known_ord, next_m, next_guided,
-                      &spec, &launches);
+    s = select_passes(ctx, x, n, m, r2, guard, true, top_k, known_w, known_ord, next_m,
+                      next_guided, &spec, &launches);
     if (s != PADDI_OK) return s;
     out->res = *ctx->h_res;
     out->launches = launches;
@@ -1424,7 +1441,7 @@ PADDI_API paddi_status paddi_shard_select(paddi_ctx *ctx, const float *d_series,
                        cudaMemcpyHostToDevice, st));
     int launches = 0;
     bool spec = false;
-    paddi_status s = select_passes(ctx, d_series, n, (int)m, r2, guard_of(ctx, kernel), {},
+    paddi_status s = select_passes(ctx, d_series, n, (int)m, r2, guard_of(ctx, kernel), false,
                                    (int)top_k, -1, 0, 0, false, &spec, &launches);
     if (s != PADDI_OK) return s;
     AttemptOut a;

@@ -19,6 +19,13 @@ def _noise_series(n=30000):
     return x
 
 
+def _give_up_block_maxima(ctx):
+    """A refused allocation takes the block maxima's memory first, and fails only then."""
+    ctx.debug_set(P.DEBUG_FAIL_ALLOC, 1)
+    ctx.debug_set(P.DEBUG_RECHECK_CAP, 1024)
+    assert ctx.debug_get(P.DEBUG_FAIL_ALLOC) == 0
+
+
 def _rows(log):
     return [(a["m"], a["r"], a["n_cand"], a["n_disc"]) for a in log]
 
@@ -29,6 +36,7 @@ def test_a_run_goes_on_without_memory_for_the_witnesses(policy, k):
     x = _noise_series()
     with P.Context(device=0, r_policy=policy) as ctx:
         ctx.reserve(len(x), 80)
+        _give_up_block_maxima(ctx)
         ctx.debug_set(P.DEBUG_FAIL_ALLOC, k)
         got, log = ctx.palmad(x, 64, 80)
         assert ctx.debug_get(P.DEBUG_FAIL_ALLOC) == 0
@@ -80,6 +88,7 @@ def test_a_refused_growth_leaves_the_recheck_queue(k):
     x = _noise_series(8192)
     with P.Context(device=0) as ctx:
         want, _ = ctx.pd3(x, 64, top_k=4)
+        _give_up_block_maxima(ctx)
         ctx.debug_set(P.DEBUG_RECHECK_CAP, 1)
         ctx.debug_set(P.DEBUG_FAIL_ALLOC, k)
         with pytest.raises(P.PaddiError) as e:
@@ -89,3 +98,24 @@ def test_a_refused_growth_leaves_the_recheck_queue(k):
         got, _ = ctx.pd3(x, 64, top_k=4)
         assert ctx.debug_get(P.DEBUG_RECHECK_CAP) > 1
     assert got == want
+
+
+@pytest.mark.parametrize("dist", [P.DIST_SPLIT_FP16, P.DIST_SPLIT_BF16])
+@pytest.mark.parametrize("when", ["at the start", "in use"])
+def test_searches_run_without_memory_for_the_block_maxima(dist, when):
+    """Refused at the start (the last of the 18 buffers of a series), or given up for a
+    growing recheck queue: the recheck then scans the whole series."""
+    x = _noise_series()
+    with P.Context(device=0, distance_kernel=dist) as ctx:
+        want, wlog = ctx.pd3(x, 64, top_k=4)
+    with P.Context(device=0, distance_kernel=dist) as ctx:
+        if when == "at the start":
+            ctx.debug_set(P.DEBUG_FAIL_ALLOC, 18)
+        else:
+            ctx.reserve(len(x), 64)
+            ctx.debug_set(P.DEBUG_RECHECK_CAP, 1)
+            ctx.debug_set(P.DEBUG_FAIL_ALLOC, 1)
+        got, log = ctx.pd3(x, 64, top_k=4)
+        assert ctx.debug_get(P.DEBUG_FAIL_ALLOC) == 0
+        again, _ = ctx.pd3(x, 64, top_k=4)
+    assert got == want and again == want and _rows(log) == _rows(wlog)
