@@ -336,7 +336,8 @@ typedef enum paddi_debug_key {
     PADDI_DEBUG_FAIL_ALLOC = 1,     /* value k > 0: the k-th next device allocation of the
                                        context is refused once (PADDI_ERR_OUT_OF_MEMORY,
                                        unless the context holds memory that it can do
-                                       without: it gives that up and tries again); 0: off */
+                                       without: it gives that up and tries again); a batched
+                                       call hands it to its first worker; 0: off */
     PADDI_DEBUG_WAIT_CYCLES = 2,    /* limit of the refine's barrier waits in clock cycles
                                        (0: the default, about 2 s) */
     PADDI_DEBUG_WITHHOLD_STAGE = 3, /* 1: the next tensor-core refine launches never fill one
@@ -344,10 +345,12 @@ typedef enum paddi_debug_key {
     PADDI_DEBUG_LAST_PASSES = 4,    /* read only: selection passes of the last attempt */
     PADDI_DEBUG_RECHECK_CAP = 5,    /* capacity of the FP64 recheck queue (it grows on demand
                                        when a selection overflows it) */
-    PADDI_DEBUG_WITNESS_STEPS = 6   /* read only: of the last PALMAD run, the sum over its
+    PADDI_DEBUG_WITNESS_STEPS = 6,  /* read only: of the last PALMAD run, the sum over its
                                        length changes of the squared number of times the
                                        witnesses were taken over each (the scale of their
                                        rounding bound) */
+    PADDI_DEBUG_WORKERS = 7         /* read only: worker contexts kept from the last batched
+                                       call */
 } paddi_debug_key;
 paddi_status paddi_debug_set(paddi_ctx *ctx, int32_t key, int64_t value);
 paddi_status paddi_debug_get(paddi_ctx *ctx, int32_t key, int64_t *value);

@@ -122,8 +122,9 @@ struct paddi_ctx {
     // the small buffers above live in one device and one pinned block
     void *d_small = nullptr, *h_small = nullptr;
     // worker contexts of paddi_palmad_batched, kept for the next call: as many as
-    // the last call used, destroyed with the context, after a failed call, or when
-    // an allocation of this context needs their memory
+    // the last call used, while they hold at most kWorkerPoints points together;
+    // destroyed with the context, after a failed call, or when an allocation of this
+    // context needs their memory
     std::vector<paddi_ctx *> workers;
 };
 
@@ -152,6 +153,13 @@ paddi_status fail(paddi_ctx *c, paddi_status s, const std::string &msg)
                                                              : PADDI_ERR_CUDA,              \
                         std::string(#call) + ": " + cudaGetErrorString(e_));                \
     } while (0)
+
+// Points that kept workers may hold, in all: about 1 GB of buffers (120 bytes a
+// point).  A call on four streams, lengths 32..55, with kept workers and without: 32
+// series of 2^14..2^17 points 55 and 75 ms, 16 of 2^18..2^20 507 and 548, 8 of
+// 2^20..2^21 1215 and 1324 to 1400.  Longer ones take longer still and would hold
+// memory that others on the device may need.
+constexpr size_t kWorkerPoints = (size_t)1 << 23;
 
 void drop_workers(paddi_ctx *ctx, size_t keep = 0)
 {
@@ -1508,6 +1516,7 @@ PADDI_API paddi_status paddi_debug_get(paddi_ctx *ctx, int32_t key, int64_t *val
     case PADDI_DEBUG_WITHHOLD_STAGE: *value = ctx->withhold; return PADDI_OK;
     case PADDI_DEBUG_LAST_PASSES: *value = ctx->last_passes; return PADDI_OK;
     case PADDI_DEBUG_RECHECK_CAP: *value = ctx->rc_cap; return PADDI_OK;
+    case PADDI_DEBUG_WORKERS: *value = (int64_t)ctx->workers.size(); return PADDI_OK;
     case PADDI_DEBUG_WITNESS_STEPS: *value = (int64_t)ctx->wit.steps2; return PADDI_OK;
     default: break;
     }
@@ -1686,6 +1695,31 @@ PADDI_API paddi_status paddi_model_train(paddi_ctx *ctx, const float *X, const f
 }
 
 // ============================================================ batched PALMAD
+namespace {
+paddi_status add_worker(paddi_ctx *ctx)
+{
+    paddi_ctx *c = nullptr;
+    const paddi_status s = paddi_ctx_create(&c, &ctx->opts);
+    if (s == PADDI_OK) ctx->workers.push_back(c);
+    return s;
+}
+
+// A worker shares the options and the model of its context.
+paddi_status set_up_worker(paddi_ctx *ctx, paddi_ctx *c)
+{
+    c->opts = ctx->opts;
+    c->model_ok = ctx->model_ok;
+    c->model_margin = ctx->model_margin;
+    if (ctx->model_ok) {
+        CK(cudaMemcpy(c->d_model, ctx->d_model, sizeof(float) * MLP_NPARAM,
+                      cudaMemcpyDeviceToDevice));
+        CK(cudaMemcpy(c->d_model_bf16, ctx->d_model_bf16, 2 * MLP_NPARAM,
+                      cudaMemcpyDeviceToDevice));
+    }
+    return PADDI_OK;
+}
+} // namespace
+
 PADDI_API paddi_status paddi_palmad_batched(paddi_ctx *ctx, const float *const *series,
                                             const size_t *lens, uint32_t count, uint32_t minL,
                                             uint32_t maxL, uint32_t streams, paddi_discord *out,
@@ -1701,27 +1735,15 @@ PADDI_API paddi_status paddi_palmad_batched(paddi_ctx *ctx, const float *const *
     const uint32_t L = maxL - minL + 1;
     int W = streams ? (int)streams : 4;
     if ((uint32_t)W > count) W = (int)count;
-    // worker contexts share the options and the model of ctx
     drop_workers(ctx, (size_t)W);
-    paddi_status first_err = PADDI_OK;
     CK(cudaSetDevice(ctx->device));
-    while (ctx->workers.size() < (size_t)W) {
-        paddi_ctx *c = nullptr;
-        const paddi_status s = paddi_ctx_create(&c, &ctx->opts);
-        if (s != PADDI_OK) return fail(ctx, s, "batched: cannot create worker contexts");
-        ctx->workers.push_back(c);
-    }
-    for (paddi_ctx *c : ctx->workers) {
-        c->opts = ctx->opts;
-        c->model_ok = ctx->model_ok;
-        c->model_margin = ctx->model_margin;
-        if (ctx->model_ok) {
-            CK(cudaMemcpy(c->d_model, ctx->d_model, sizeof(float) * MLP_NPARAM,
-                          cudaMemcpyDeviceToDevice));
-            CK(cudaMemcpy(c->d_model_bf16, ctx->d_model_bf16, 2 * MLP_NPARAM,
-                          cudaMemcpyDeviceToDevice));
-        }
-    }
+    paddi_status ws = PADDI_OK;
+    while (ws == PADDI_OK && ctx->workers.size() < (size_t)W) ws = add_worker(ctx);
+    for (size_t k = 0; ws == PADDI_OK && k < ctx->workers.size(); ++k)
+        ws = set_up_worker(ctx, ctx->workers[k]);
+    if (ws != PADDI_OK) return fail(ctx, ws, "batched: cannot create worker contexts");
+    // (a test's refused allocation is the first worker's)
+    std::swap(ctx->fail_alloc, ctx->workers[0]->fail_alloc);
     CK(cudaDeviceSynchronize()); // the copies precede the workers' (non-blocking) streams
     // longest series first: a worker's buffers are sized by its first one, and the
     // short ones even out the end
@@ -1733,24 +1755,41 @@ PADDI_API paddi_status paddi_palmad_batched(paddi_ctx *ctx, const float *const *
     std::vector<int32_t> st(count, (int32_t)PADDI_OK);
     std::vector<std::string> errs(count);
     std::vector<uint64_t> na(count, 0);
+    auto run = [&](paddi_ctx *c, std::vector<paddi_attempt_log> &lg, uint32_t k) {
+        uint32_t nl = 0;
+        st[k] = (int32_t)paddi_palmad(c, series[k], lens[k], minL, maxL, out + (size_t)k * L,
+                                      lg.data(), (uint32_t)lg.size(), &nl);
+        errs[k] = st[k] != PADDI_OK ? c->err : std::string();
+        na[k] = nl;
+    };
     std::vector<std::thread> pool;
     for (int w = 0; w < W; ++w) {
         pool.emplace_back([&, w]() {
             paddi_ctx *c = ctx->workers[w];
             cudaSetDevice(c->device);
             std::vector<paddi_attempt_log> lg(4096);
-            for (uint32_t q = next++; q < count; q = next++) {
-                const uint32_t k = order[q];
-                uint32_t nl = 0;
-                st[k] = (int32_t)paddi_palmad(c, series[k], lens[k], minL, maxL,
-                                              out + (size_t)k * L, lg.data(),
-                                              (uint32_t)lg.size(), &nl);
-                if (st[k] != PADDI_OK) errs[k] = c->err;
-                na[k] = nl;
-            }
+            for (uint32_t q = next++; q < count; q = next++) run(c, lg, order[q]);
         });
     }
     for (auto &t : pool) t.join();
+    std::swap(ctx->fail_alloc, ctx->workers[0]->fail_alloc);
+    // a worker cannot take the memory of the others, which may have kept theirs from
+    // longer series: what did not fit runs again, one by one, on a single worker
+    const auto refused = [&](uint32_t k) { return st[k] == (int32_t)PADDI_ERR_OUT_OF_MEMORY; };
+    if (std::any_of(order.begin(), order.end(), refused)) {
+        drop_workers(ctx);
+        std::vector<paddi_attempt_log> lg(4096);
+        for (uint32_t k : order) {
+            if (!refused(k)) continue;
+            if (ctx->workers.empty() &&
+                (add_worker(ctx) != PADDI_OK ||
+                 set_up_worker(ctx, ctx->workers[0]) != PADDI_OK ||
+                 cudaDeviceSynchronize() != cudaSuccess))
+                break;
+            run(ctx->workers[0], lg, k);
+        }
+    }
+    paddi_status first_err = PADDI_OK;
     std::string msg;
     for (uint32_t k = 0; k < count; ++k) {
         if (status) status[k] = st[k];
@@ -1764,6 +1803,11 @@ PADDI_API paddi_status paddi_palmad_batched(paddi_ctx *ctx, const float *const *
         drop_workers(ctx);
         return fail(ctx, first_err, msg);
     }
+    size_t points = 0, keep = 0;
+    while (keep < ctx->workers.size() &&
+           (points += ctx->workers[keep]->cap_n) <= kWorkerPoints)
+        ++keep;
+    drop_workers(ctx, keep);
     return PADDI_OK;
 }
 
