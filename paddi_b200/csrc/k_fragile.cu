@@ -47,12 +47,12 @@ constexpr int FG_MAXM = 1024;
 static_assert(FG_THREADS / 32 == FG_CAND, "a warp stages a candidate");
 
 __global__ void __launch_bounds__(FG_THREADS)
-k_fragile(const float *__restrict__ x, const double2 *__restrict__ ms64,
-          const int32_t *__restrict__ cand,
-          const int32_t *__restrict__ list0, const int32_t *__restrict__ list1,
+k_fragile(const float *__restrict__ x, const double2 *ms64,
+          const int32_t *cand,
+          const int32_t *list0, const int32_t *list1,
           PaddiAttemptDev *att, uint8_t *pruned, uint32_t *rho_max,
-          const int32_t *__restrict__ frag,
-          const int32_t *__restrict__ frag_count, int32_t m, float thr, int32_t col_lo,
+          const int32_t *frag,
+          const int32_t *frag_count, int32_t m, float thr, int32_t col_lo,
           int32_t col_hi, PaddiBlockMax B, float guard)
 {
     // [FG_CAND][mp] centred candidate values, mp = m rounded up to even

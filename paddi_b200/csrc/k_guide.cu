@@ -149,10 +149,10 @@ __device__ __forceinline__ void guide_finish(double best, double *red, PaddiGuid
 
 // Reuse and slide.  Leaves without a trace when a rebuild is due.
 __global__ void __launch_bounds__(GD_THREADS, GD_STREAM_CTAS_PER_SM)
-k_guide_stream(const float *__restrict__ x, const double2 *__restrict__ ms64, const uint8_t *__restrict__ flat, int32_t N,
-               int32_t m, const PaddiAttemptResult *__restrict__ prev, int32_t w_host,
-               PaddiGuide *g, double *__restrict__ G0, double *__restrict__ G1,
-               volatile PaddiGuide *host, const int32_t *__restrict__ flat_count,
+k_guide_stream(const float *__restrict__ x, const double2 *ms64, const uint8_t *flat, int32_t N,
+               int32_t m, const PaddiAttemptResult *prev, int32_t w_host,
+               PaddiGuide *g, double *G0, double *G1,
+               volatile PaddiGuide *host, const int32_t *flat_count,
                unsigned long long *t_prep)
 {
     paddi::chain_begin();
@@ -276,10 +276,10 @@ k_guide_stream(const float *__restrict__ x, const double2 *__restrict__ ms64, co
 // register ring over the staged series.  Leaves when the state is current
 // (k_guide_stream did this length) or there is no window.
 __global__ void __launch_bounds__(GD_THREADS)
-k_guide_build(const float *__restrict__ x, const double2 *__restrict__ ms64, const uint8_t *__restrict__ flat, int32_t N,
-              int32_t m, const PaddiAttemptResult *__restrict__ prev, int32_t w_host,
-              PaddiGuide *g, double *__restrict__ G0, double *__restrict__ G1,
-              volatile PaddiGuide *host, const int32_t *__restrict__ flat_count,
+k_guide_build(const float *__restrict__ x, const double2 *ms64, const uint8_t *flat, int32_t N,
+              int32_t m, const PaddiAttemptResult *prev, int32_t w_host,
+              PaddiGuide *g, double *G0, double *G1,
+              volatile PaddiGuide *host, const int32_t *flat_count,
               unsigned long long *t_prep)
 {
     paddi::chain_begin();

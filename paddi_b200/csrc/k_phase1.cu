@@ -207,8 +207,8 @@ __device__ __forceinline__ void p1_walk(const P1Smem &S, float2 (&cov)[P1_GPT], 
 
 template <bool WT>
 __global__ void __launch_bounds__(P1_THREADS, 16)
-k_phase1(const float *__restrict__ x, const float4 *__restrict__ wst, const float *__restrict__ mu,
-         const double2 *__restrict__ ms64, uint8_t *alive, int32_t N, int32_t m, int32_t R,
+k_phase1(const float *__restrict__ x, const float4 *wst, const float *mu,
+         const double2 *ms64, uint8_t *alive, int32_t N, int32_t m, int32_t R,
          int32_t max_chunks, float thr, int32_t row_lo, int32_t row_hi, PaddiAttemptDev *att,
          PaddiWitness W, int32_t enough)
 {

@@ -83,8 +83,8 @@ __host__ __device__ __forceinline__ paddi::RefineItems rf_items(int m, int tiles
 constexpr int RF_SUMBLK = 64; // two-level sums: terms per partial sum
 
 __global__ void __launch_bounds__(RF_THREADS)
-k_refine_fp32(const float *__restrict__ x, const float4 *__restrict__ wst,
-              const float *__restrict__ mu, const int32_t *__restrict__ cand, int32_t *list0,
+k_refine_fp32(const float *__restrict__ x, const float4 *wst,
+              const float *mu, const int32_t *cand, int32_t *list0,
               int32_t *list1, PaddiAttemptDev *att, uint32_t *rho_max, uint8_t *pruned, int32_t N,
               int32_t m, int32_t col_lo, int32_t col_hi, float thr, float E, float gcap,
               long long wl, PaddiWitness W)
@@ -389,8 +389,8 @@ PaddiBound paddi_bound_fp32(int m)
 
 // Fragile windows of length m for the FP32 refine's geometry (chunks of 256
 // windows shifted by their first value): the same test as the refine applies.
-__global__ void k_fragile_scan_fp32(const float *__restrict__ x, const float4 *__restrict__ wst,
-                                    const float *__restrict__ mu, int32_t N, int32_t m, float E,
+__global__ void k_fragile_scan_fp32(const float *__restrict__ x, const float4 *wst,
+                                    const float *mu, int32_t N, int32_t m, float E,
                                     float gcap, int32_t *frag_list, int32_t *frag_count,
                                     unsigned long long *t_end)
 {

@@ -317,7 +317,7 @@ static_assert(ST_TILE == UM_TW, "a statistics tile is a block of the refine's gr
 template <bool BF>
 __global__ void __launch_bounds__(ST_THREADS, 4)
 k_prep(const float *__restrict__ x, int64_t nser, int32_t cnt, int32_t m, int32_t N, StOut O,
-       uint16_t *__restrict__ bq, float4 *__restrict__ wdq, float E, float Fu, float gcap,
+       uint16_t *bq, float4 *wdq, float E, float Fu, float gcap,
        int32_t *frag_list, int32_t *frag_count, unsigned long long *t_end)
 {
     using X = E16<BF>;
@@ -555,9 +555,9 @@ struct Ring {
 //           (lanes 16..31 of every subpartition stay unused).
 template <bool BF, int MM>
 __global__ void __launch_bounds__(UM_THREADS, 1)
-k_refine_umma(const float *__restrict__ x, const float4 *__restrict__ wst,
-              const float *__restrict__ mu, const int32_t *__restrict__ cand, int32_t *list0,
-              int32_t *list1, const uint16_t *__restrict__ bq, const float4 *__restrict__ wdq,
+k_refine_umma(const float *__restrict__ x, const float4 *wst,
+              const float *mu, const int32_t *cand, int32_t *list0,
+              int32_t *list1, const uint16_t *bq, const float4 *wdq,
               PaddiAttemptDev *att, uint32_t *rho_max, uint8_t *pruned, int32_t N, int32_t m,
               int32_t col_lo, int32_t col_hi, float thr, int32_t grid_ctas, long long wl,
               int32_t withhold, PaddiWitness W, PaddiBlockMax B, int32_t may_screen, float guard)

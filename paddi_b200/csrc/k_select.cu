@@ -47,9 +47,9 @@ constexpr int RC_MAXM = 1024;
 constexpr int CP_WIN = 16;                 // windows per thread
 constexpr int CP_CTHREADS = 256;
 __global__ void __launch_bounds__(CP_CTHREADS)
-k_compact(uint8_t *__restrict__ alive, int32_t reset, int32_t N, int32_t *cand, uint32_t *rho_max,
+k_compact(uint8_t *alive, int32_t reset, int32_t N, int32_t *cand, uint32_t *rho_max,
           uint8_t *pruned, int32_t *rc_slot, PaddiAttemptDev *att,
-          const uint8_t *__restrict__ flat, const int32_t *__restrict__ flat_span, int32_t m,
+          const uint8_t *flat, const int32_t *flat_span, int32_t m,
           int32_t prune_flats, int32_t settle_flats)
 {
     __shared__ int wcnt[CP_CTHREADS / 32];
@@ -217,10 +217,10 @@ __device__ __forceinline__ bool overlaps(int a, int b, int m)
 //   thr - guard <= rho <= thr+g -> borderline, exact value needed
 //   and every candidate whose FP32 value could reach the top-k picks.
 __global__ void __launch_bounds__(FZ_THREADS)
-k_finalize(const int32_t *__restrict__ cand, PaddiAttemptDev *att,
-           const uint32_t *__restrict__ rho_max, const uint8_t *__restrict__ pruned, int32_t m,
+k_finalize(const int32_t *cand, PaddiAttemptDev *att,
+           const uint32_t *rho_max, const uint8_t *pruned, int32_t m,
            float r2, float thr, float guard, float widen, int32_t top_k,
-           const uint8_t *__restrict__ flat, int32_t rc_cap,
+           const uint8_t *flat, int32_t rc_cap,
            int32_t *recheck, int32_t *rc_slot, unsigned long long *nn64_ord,
            PaddiAttemptResult *res, int32_t known_w, unsigned long long known_ord)
 {
@@ -331,10 +331,10 @@ static_assert(RC_SPAN == 2 * PADDI_HALF, "two half blocks per block");
 __device__ __forceinline__ int rpad(int d) { return d + (d >> 4); } // conflict-free at stride 8
 
 __global__ void __launch_bounds__(RC_THREADS)
-k_recheck(const float *__restrict__ x, const double2 *__restrict__ ms64, const uint8_t *__restrict__ flat, int32_t N,
-          int32_t m, const int32_t *__restrict__ cand, const int32_t *__restrict__ recheck,
+k_recheck(const float *__restrict__ x, const double2 *ms64, const uint8_t *flat, int32_t N,
+          int32_t m, const int32_t *cand, const int32_t *recheck,
           PaddiAttemptDev *att, unsigned long long *nn64_ord, int32_t known_w,
-          const uint32_t *__restrict__ rho_max, PaddiBlockMax B, float guard)
+          const uint32_t *rho_max, PaddiBlockMax B, float guard)
 {
     __shared__ double a[RC_MAXM];
     __shared__ double xs[RC_SPAN + RC_MAXM + (RC_SPAN + RC_MAXM) / 16 + 16];
@@ -452,12 +452,12 @@ k_recheck(const float *__restrict__ x, const double2 *__restrict__ ms64, const u
 // Final counts and greedy top-k with exact values where they matter.
 // status 2: a pick has no exact value yet (host appends it and re-runs).
 __global__ void __launch_bounds__(FZ_THREADS)
-k_select(const int32_t *__restrict__ cand, PaddiAttemptDev *att,
-         const uint32_t *__restrict__ rho_max, const uint8_t *__restrict__ pruned,
-         const int32_t *__restrict__ recheck, const int32_t *__restrict__ rc_slot,
-         const unsigned long long *__restrict__ nn64_ord, int32_t m, float r2, float thr,
-         float guard, int32_t top_k, const uint8_t *__restrict__ flat,
-         const int32_t *__restrict__ flat_count, const unsigned long long *__restrict__ t_prep,
+k_select(const int32_t *cand, PaddiAttemptDev *att,
+         const uint32_t *rho_max, const uint8_t *pruned,
+         const int32_t *recheck, const int32_t *rc_slot,
+         const unsigned long long *nn64_ord, int32_t m, float r2, float thr,
+         float guard, int32_t top_k, const uint8_t *flat,
+         const int32_t *flat_count, const unsigned long long *t_prep,
          PaddiAttemptDev *next, PaddiAttemptResult *res, PaddiAttemptResult *host)
 {
     paddi::chain_begin();

@@ -111,9 +111,9 @@ __device__ __forceinline__ WtGroups wt_decode(double code)
 // the forward step the run of 449 lengths took 1.5 % longer).
 template <bool BACK>
 __global__ void __launch_bounds__(WT_THREADS)
-k_witness_step(const float *__restrict__ x, const double2 *__restrict__ ms64, int32_t N,
-               int32_t m, int32_t from, int32_t *__restrict__ wit, double *__restrict__ wc,
-               float *__restrict__ wrho, int32_t *__restrict__ hint, uint32_t *scal,
+k_witness_step(const float *__restrict__ x, const double2 *ms64, int32_t N,
+               int32_t m, int32_t from, int32_t *wit, double *wc,
+               float *wrho, int32_t *hint, uint32_t *scal,
                double dscale, double delta1, int32_t returns)
 {
     paddi::chain_begin();
@@ -202,9 +202,9 @@ __device__ __forceinline__ void wt_settle(WtBest &B, int i, int j, double c, con
 }
 
 __global__ void __launch_bounds__(WT_THREADS)
-k_witness_hints(const float *__restrict__ x, const double2 *__restrict__ ms64, int32_t N,
-                int32_t m, int32_t *__restrict__ wit, double *__restrict__ wc,
-                float *__restrict__ wrho, const int32_t *__restrict__ hint, uint32_t *scal,
+k_witness_hints(const float *__restrict__ x, const double2 *ms64, int32_t N,
+                int32_t m, int32_t *wit, double *wc,
+                float *wrho, const int32_t *hint, uint32_t *scal,
                 double dscale, unsigned long long *t_end)
 {
     paddi::chain_begin();
@@ -327,8 +327,8 @@ k_absmax(const float *__restrict__ x, int64_t n, uint32_t *amax)
 // alive[i] = 0 where the witness proves it; the others are listed (order
 // within a CTA kept).  5 B per window.
 __global__ void __launch_bounds__(WT_THREADS)
-k_witness_check(const float *__restrict__ wrho, int32_t N, float thr, uint8_t *__restrict__ alive,
-                int32_t *__restrict__ fail, PaddiAttemptDev *att)
+k_witness_check(const float *wrho, int32_t N, float thr, uint8_t *alive,
+                int32_t *fail, PaddiAttemptDev *att)
 {
     paddi::chain_begin();
     paddi::stamp_begin(att->t + PADDI_T_BEGIN);
@@ -394,11 +394,11 @@ __device__ __forceinline__ uint32_t wt_hash(uint32_t a)
 }
 
 __global__ void __launch_bounds__(32 * WT_RWARPS)
-k_witness_rescue(const float *__restrict__ x, const double2 *__restrict__ ms64, int32_t N, int32_t m, float thr,
-                 const int32_t *__restrict__ fail, const int32_t *__restrict__ n_fail,
-                 int32_t limit, int32_t *wit, double *__restrict__ wc, float *__restrict__ wrho,
-                 uint8_t *__restrict__ alive, int32_t *n_rescued,
-                 const uint32_t *__restrict__ scal, double dscale)
+k_witness_rescue(const float *__restrict__ x, const double2 *ms64, int32_t N, int32_t m, float thr,
+                 const int32_t *fail, const int32_t *n_fail,
+                 int32_t limit, int32_t *wit, double *wc, float *wrho,
+                 uint8_t *alive, int32_t *n_rescued,
+                 const uint32_t *scal, double dscale)
 {
     extern __shared__ float wt_a[]; // per warp: the centred window
     paddi::chain_begin();
