@@ -221,7 +221,8 @@ paddi_status paddi_palmad_batched(paddi_ctx *ctx, const float *const *series,
  * chunk depth {8, 12, 16}, checks that all combinations return the same
  * discords, installs the fastest in ctx and copies the chosen options to
  * *chosen.  ms (optional, 18 entries) receives the probe time of each
- * combination, tile rows outermost, then segment, then chunks.  No reference
+ * combination, tile rows outermost, then segment, then chunks (combinations that
+ * are the same program on a short series are timed once).  No reference
  * counterpart (the reference fixes SEGMENT_N and its 32x32 refine tiles at
  * compile time, src/parameters.hpp:8-10).
  */

@@ -1836,6 +1836,9 @@ PADDI_API paddi_status paddi_autotune(paddi_ctx *ctx, const float *series, size_
     float best = FLT_MAX;
     paddi_opts best_opts = saved;
     std::vector<paddi_discord> out(3);
+    // configurations that are the same program on these lengths (p1_rows_of caps the
+    // rows of a segment) are timed once
+    std::map<std::vector<int>, float> timed;
     int idx = 0;
     for (uint32_t tr : tiles)
         for (uint32_t sg : segs)
@@ -1844,9 +1847,14 @@ PADDI_API paddi_status paddi_autotune(paddi_ctx *ctx, const float *series, size_
             ctx->opts.tile_rows = tr;
             ctx->opts.segment_len = sg;
             ctx->opts.phase1_chunks = ch;
+            std::vector<int> program = {(int)tr, (int)ch};
+            for (const auto &p : probes)
+                for (uint32_t m = p.first; m <= p.second; ++m)
+                    program.push_back(p1_rows_of(ctx, (int64_t)(n - m + 1), (int)m));
+            const auto same = timed.find(program);
             // one untimed pass (kernel attributes, caches), then the timed one
-            float t_total = 0.f;
-            for (int pass = 0; pass < 2; ++pass) {
+            float t_total = same == timed.end() ? 0.f : same->second;
+            for (int pass = 0; pass < 2 && same == timed.end(); ++pass) {
                 t_total = 0.f;
                 for (size_t p = 0; p < probes.size(); ++p) {
                     const uint32_t a = probes[p].first, b = probes[p].second;
@@ -1874,6 +1882,7 @@ PADDI_API paddi_status paddi_autotune(paddi_ctx *ctx, const float *series, size_
                     }
                 }
             }
+            timed[program] = t_total;
             if (ms) ms[idx] = t_total;
             ++idx;
             if (t_total < best) {
