@@ -192,6 +192,17 @@ def cpu_sample_slices(x, count: int, minl: int = MIN_L):
     return out
 
 
+def reference_missing():
+    """Why the reference's CPU kernels cannot run here, or None when they can."""
+    from oracle import oracle as O
+    try:
+        ok = O.ref() is not None
+    except (OSError, subprocess.CalledProcessError) as e:
+        return f"the reference's CPU kernels (oracle/_ref) do not load or build: {e}"
+    return None if ok else ("the reference's CPU kernels (oracle/_ref) are not built and its "
+                            "sources are not on this machine")
+
+
 def cpu_reference(x, steps: int, warmup: int, threads: int, minl: int = MIN_L):
     from oracle import oracle as O
     maxl = minl + CPU_SAMPLE_LENGTHS - 1
@@ -313,6 +324,10 @@ def cpu_sample_of(x, args):
 
 def run_reference(args, world, rank):
     if rank != 0:
+        return
+    why = reference_missing()
+    if why:
+        print(json.dumps({"impl": "reference", "unavailable": why}), flush=True)
         return
     x, name = workload(args)
     threads = min(host_threads(), 64)
@@ -530,11 +545,16 @@ def run_paddi(args, world, rank, local):
                                                     if "plain_form" in line else None)}
     if rank == 0 and world == 1 and not args.no_cpu_baseline:
         _progress(rank, "CPU baseline")
-        cb = cpu_reference(cpu_sample_of(x, args), 1, 0, min(host_threads(), 64), args.minL)
-        line["cpu_baseline"] = {k: cb[k] for k in ("value", "unit", "cores", "kind", "sample")}
-        line["cpu_baseline"]["like_for_like"] = False
+        why = reference_missing()  # the measurements above stand without it
+        if why:
+            line["cpu_baseline"] = {"unavailable": why}
+        else:
+            cb = cpu_reference(cpu_sample_of(x, args), 1, 0, min(host_threads(), 64), args.minL)
+            line["cpu_baseline"] = {k: cb[k] for k in ("value", "unit", "cores", "kind", "sample")}
+            line["cpu_baseline"]["like_for_like"] = False
+            if args.workload == "palmad":
+                line["cpu_baseline"]["full_length"] = full_length_point(ctx, st, x, disc, args)
         if args.workload == "palmad":
-            line["cpu_baseline"]["full_length"] = full_length_point(ctx, st, x, disc, args)
             line["reference_gpu"] = reference_gpu_point(x, disc, args, lpl if not
                                                         args.no_plain_form else None)
     if rank == 0:
