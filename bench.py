@@ -49,10 +49,12 @@ CPU_SLICES_PER_THREAD = 2
 CPU_SAMPLE_LENGTHS = 8          # lengths 64..71
 REF_GPU_ATTEMPTS = 8            # attempts of the reference's GPU path timed (~1 s each)
 L2_FLUSH_BYTES = 512 << 20      # > 126 MB L2
-# DRAM bytes (read + write) of one k_refine_umma launch from an ncu capture:
-# the last refine round (windows N/2..N) of an m=300 attempt on this series
-REFINE_TRAFFIC_BYTES = 13450752
-REFINE_TRAFFIC_LAUNCH = "refine round over windows N/2..N at m=300, ncu dram__bytes_read+write"
+# DRAM bytes (read + write) of one k_refine_umma launch (all rounds) from an ncu
+# capture: the first attempt with candidates of a run from m=300 on this series
+REFINE_TRAFFIC_BYTES = 28207360
+REFINE_TRAFFIC_LAUNCH = ("first refine of a run from m=300 that has candidates, all rounds, "
+                         "ncu dram__bytes_read+write")
+RESULT_BYTES = 280              # an attempt's record in pinned host memory
 
 
 def matrix_pairs(n: int, minL: int, maxL: int) -> float:
@@ -418,7 +420,7 @@ def run_paddi(args, world, rank, local):
     e2e_step = reduce_max(world, float(np.mean(e2e_ms)))
     e2e_value = world * pairs / (e2e_step / 1e3)
     n_att = len(logs[-1])
-    d2h = n_att * 152  # one attempt result record per attempt
+    d2h = n_att * RESULT_BYTES
 
     # ---- roofline of the dominant kernel group (refine or phase 1)
     last = logs[-1]
@@ -444,12 +446,15 @@ def run_paddi(args, world, rank, local):
 
     if tc:
         achieved, ms_tc = rate(tc)
-        peak = bf16 / 3.0  # three 16-bit products per FP32-accurate product
+        # a split-FP16 tile needs one 16-bit product or three (screening), a split-BF16
+        # tile three: against the peak of one, the fraction is a lower bound
+        peak = bf16
         roof = {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                 "frac": achieved / peak, "traffic": REFINE_TRAFFIC_BYTES,
                 "traffic_launch": REFINE_TRAFFIC_LAUNCH, "kernel": "k_refine_umma",
-                "peak_source": f"bf16 dense {src} {bf16} TFLOP/s / 3 (split operands issue 3 MMAs)",
-                "work": "2*m FLOP per (candidate, window) pair evaluated",
+                "peak_source": f"bf16 dense {src} {bf16} TFLOP/s",
+                "work": "2*m FLOP per (candidate, window) pair evaluated, one product counted "
+                        "(a tile issues one product or three)",
                 "kernel_ms_per_step": ms_tc, "attempts": len(tc),
                 "live_pairs_achieved": live_rate(tc),
                 "live_pairs_note": "pairs whose candidate was still unpruned when its tile "

@@ -20,8 +20,9 @@
 // global gradient once; an Adam kernel applies the step.  With one warp per
 // sample and a gradient per warp in shared memory, a batch of 4096 spent its
 // time on 2368 warps loading the parameters and adding 5057 values each to the
-// same addresses; now 128 CTAs do: 70 us a batch, now 24 (staging the parameters,
-// a chain of five small products, and the atomics, in about equal parts).
+// same addresses; now 128 CTAs do: 70 us a batch, 24 with FP32 sums and 28 with the
+// FP64 sums of k_mlp_adam's gradient (staging the parameters, a chain of five small
+// products, and the atomics, in about equal parts).
 #include <cuda_bf16.h>
 
 #include <cmath>
@@ -54,7 +55,9 @@ __device__ __forceinline__ float ld<__nv_bfloat16>(const __nv_bfloat16 *p, int i
     return __bfloat162float(p[i]);
 }
 
-// Parameters of one model.
+// Parameters of one model.  (This struct and what mlp_forward returns beside y served
+// the earlier training kernel too; a forward pass without them let the compiler
+// contract the output sum the other way, which moved predictions in the last place.)
 template <typename W>
 struct MlpView {
     const W *w1, *b1, *w2, *b2, *w3, *b3;
@@ -280,8 +283,8 @@ k_mlp_grad(const float *__restrict__ X, const float *__restrict__ Yt,
 // batch.  In FP32 the parameters rounded at each step and the batch gradient's atomics
 // at each addition: distance of the trained parameters from 64 bits (two epochs of
 // 65536 and 20011 samples, 12 seeds) 1.6e-7 to 2.4e-6 and two runs 1e-4, now 4e-8 to
-// 2.4e-6, smaller on each seed; the time is the same at 4096 samples a step (61 us with
-// the gradient) and 1.5 us more at 1024.
+// 2.4e-6, smaller on each seed.  A step takes 33 us at 4096 samples (gradient 28, this
+// kernel 3.4), beside some 1.2 ms a call for the copies and the first shuffle.
 __global__ void k_mlp_adam(float *P, double *G, double *A, int np, double lr, double b1,
                            double b2, double eps, double bc1, double bc2, bool first)
 {

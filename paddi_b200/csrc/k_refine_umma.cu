@@ -48,8 +48,11 @@
 // CTAs' through rho_max, the candidate's witness), the three products and the
 // full epilogue are skipped.  A candidate whose lower bound is above thr is pruned
 // at once.  Nothing kept is computed with less than all three products.  The MMA
-// thread issues tile u+1's hi * hi before it takes the verdict on tile u; 5 to 25 %
-// of the tiles need everything.  (Figures at UM_SCREEN_K and EPI_WARP0.)
+// thread issues tile u+1's hi * hi before it takes the verdict on tile u.  From the
+// counts of products and pairs: of 166 thousand tiles of 48357 candidates at n =
+// 300007, m = 200, 19 % need everything; of the first attempt's 31 thousand at n = 2^21,
+// m = 300, 15 %; of the next ones' thousand to three thousand, 1 to 29 %.  (Times at
+// UM_SCREEN_K and EPI_WARP0.)
 //
 // The candidate operand is built by all 384 threads at the start of a work
 // item.  When every candidate of the item is pruned the loader stops and
@@ -114,9 +117,10 @@ constexpr long long kDrainCycles = 4000000000ll;
 // runs under the other's waits (its product, the screen's verdict): with all eight on
 // every tile and candidates major in A (below), refine launches at n = 300007 took 2080
 // us at m = 64, now 1770; m = 130 2425, now 2245; ECG of 2^23 points 5.0 ms, now 4.5.
-// What bounds it: handing each lane its windows' weights (4 or 8 bytes a correlation, 128
-// bytes a cycle from shared memory, beside the operands of the products) and, about as
-// much, the wait for the next product: the tensor memory holds two accumulators.
+// What bounds it: no unit alone.  At n = 300007, m = 200 (48357 candidates) the tensor
+// pipe is active 48 % of the time, L1 and shared memory 35 %, issue slots 25 %; at 31
+// thousand tiles (n = 2^21, m = 300) 36, 26 and 15 %.  The rest is waiting: a group for its
+// next product, the products for an accumulator (the tensor memory holds two).
 constexpr int EPI_WARP0 = 4;
 constexpr int EPI_GROUP = 4;     // warps per accumulator
 constexpr int MMA_WARP = 0, LOAD_WARP = 1;

@@ -23,7 +23,7 @@
 // Measured (n = 2^21, lengths 64..512, learned r, per run): without witnesses
 // phase 1 160 ms and the refine of its survivors 165 ms, the run 442 ms; with
 // them step 13, hints 4, check 2, rescue 15, phase 1 4, refine 87 ms, the run
-// 249 ms.  A step at n = 2^21 takes 28 us (bound by memory: 56 B per window, 4.2
+// 249 ms (120 to 135 ms with what was made faster since).  A step at n = 2^21 takes 28 us (bound by memory: 56 B per window, 4.2
 // TB/s); one window per thread, the mean and the norm in two arrays, took 50.
 // Phase 1 runs only when more windows are left than the refine should take
 // (the first attempts of a run, where no window has a witness yet).  Phase 1
@@ -384,6 +384,7 @@ k_witness_check(const float *wrho, int32_t N, float thr, uint8_t *alive,
 }
 
 // ------------------------------------------------------------------ rescue
+// 32-bit integer hash "lowbias32" (C. Wellons, hash-prospector)
 __device__ __forceinline__ uint32_t wt_hash(uint32_t a)
 {
     a ^= a >> 16;

@@ -12,8 +12,8 @@
 //   selection   k_finalize, k_recheck, k_select
 //                                 (get_node_discords_num + find_top1_discord,
 //                                  src/sets_processing.hpp:11-87)
-// all on one stream with one device->host copy of a small result record at
-// the end.  The r-schedules are restated from src/main.cu:136-233 in the
+// all on one stream as a chain of launches; the selection writes a small result
+// record to pinned host memory.  The r-schedules are restated from src/main.cu:136-233 in the
 // same float arithmetic as the reference, so equal distances give equal
 // thresholds.
 #include <cuda_runtime.h>
@@ -445,7 +445,9 @@ int p1_rows_of(const paddi_ctx *ctx, int64_t rows, int m)
     int R = (int)ctx->opts.segment_len;
     if (R <= 0) R = 256;
     R = (R + 7) & ~7;
-    const int64_t tasks = 15ll * ctx->num_sms; // resident one-warp tasks
+    // one-warp tasks that are resident at once: 15 a SM at 256 rows and m = 300 (the
+    // launcher asks for the occupancy of the rows chosen here)
+    const int64_t tasks = 15ll * ctx->num_sms;
     const int fit = rows <= 64 * tasks && m <= 256 ? 64 : rows <= 512 * tasks ? 128 : 512;
     return std::min(R, fit);
 }
