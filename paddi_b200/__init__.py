@@ -99,6 +99,8 @@ class _LogRows:
     writes to it (the default of 100000 rows is 17 MB)."""
 
     def __init__(self, cap: int):
+        if not 0 <= cap < 1 << 32:  # the library's uint32_t
+            raise ValueError(f"log_cap {cap} outside 0..2^32-1")
         self.buf = np.empty(max(cap, 1), _LOG_DTYPE)
         self.cap = cap
         self.n = C.c_uint32(0)
